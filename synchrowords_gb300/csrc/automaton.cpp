@@ -159,26 +159,6 @@ HostTables build_tables(const Automaton& A) {
   return T;
 }
 
-void to_device_rows(const uint64_t* ref, uint64_t count, uint32_t n, int W, unsigned long long* out) {
-  const uint32_t rw = (n + 63) / 64;
-  for (uint64_t i = 0; i < count; ++i) {
-    unsigned long long* o = out + i * W;
-    for (int w = 0; w < W; ++w) o[w] = 0;
-    for (uint32_t q = 0; q < n; ++q)
-      if ((ref[i * rw + q / 64] >> (q % 64)) & 1ULL) o[q >> 6] |= state_bit((int)q);
-  }
-}
-
-void from_device_rows(const unsigned long long* rows, uint64_t count, uint32_t n, int W, uint64_t* out) {
-  const uint32_t rw = (n + 63) / 64;
-  for (uint64_t i = 0; i < count; ++i) {
-    uint64_t* o = out + i * rw;
-    for (uint32_t w = 0; w < rw; ++w) o[w] = 0;
-    for (uint32_t q = 0; q < n; ++q)
-      if (rows[i * W + (q >> 6)] & state_bit((int)q)) o[q / 64] |= 1ULL << (q % 64);
-  }
-}
-
 std::vector<uint32_t> apply_word(const Automaton& A, const std::vector<uint32_t>& word) {
   std::vector<char> cur(A.n, 1), nxt(A.n);
   for (uint32_t a : word) {

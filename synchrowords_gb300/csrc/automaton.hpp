@@ -49,10 +49,6 @@ struct HostTables {
 };
 HostTables build_tables(const Automaton& A);
 
-// Reference-layout (LSB-first, ceil(n/64) words) <-> device MSB-first rows of W words.
-void to_device_rows(const uint64_t* ref, uint64_t count, uint32_t n, int W, unsigned long long* out);
-void from_device_rows(const unsigned long long* rows, uint64_t count, uint32_t n, int W, uint64_t* out);
-
 // Image of the full state set under a word (the word check).
 std::vector<uint32_t> apply_word(const Automaton& A, const std::vector<uint32_t>& word);
 

@@ -1149,15 +1149,15 @@ void Solver::apply_transition(const Automaton& A, uint32_t letter, bool inverse,
   one.t.resize(A.n);
   for (uint32_t q = 0; q < A.n; ++q) one.t[q] = A.at(q, letter);
   E.upload_tables(one);
-  std::vector<u64> rows((size_t)W * count);
-  to_device_rows(from, count, A.n, W, rows.data());
-  E.uq_rows.reserve(sizeof(u64) * rows.size());
-  E.ch_rows.reserve(sizeof(u64) * rows.size());
-  SW_CUDA(cudaMemcpyAsync(E.uq_rows.p, rows.data(), sizeof(u64) * rows.size(), cudaMemcpyHostToDevice, E.stream));
+  const size_t bytes = sizeof(u64) * (size_t)W * count;
+  E.uq_rows.reserve(bytes);
+  E.ch_rows.reserve(bytes);
+  SW_CUDA(cudaMemcpyAsync(E.uq_rows.p, from, bytes, cudaMemcpyHostToDevice, E.stream));
+  launch_convert_rows(W, E.uq_rows.as<u64>(), count, n, true, E.stream);
   launch_expand(W, !inverse, E.uq_rows.as<u64>(), (u32)count, E.tables, E.ch_rows.as<u64>(), E.stream);
-  SW_CUDA(cudaMemcpyAsync(rows.data(), E.ch_rows.p, sizeof(u64) * rows.size(), cudaMemcpyDeviceToHost, E.stream));
+  launch_convert_rows(W, E.ch_rows.as<u64>(), count, n, false, E.stream);
+  SW_CUDA(cudaMemcpyAsync(to, E.ch_rows.p, bytes, cudaMemcpyDeviceToHost, E.stream));
   SW_CUDA(cudaStreamSynchronize(E.stream));
-  from_device_rows(rows.data(), count, A.n, W, to);
 }
 
 void Solver::subsets_check(uint32_t n, const uint64_t* sets, uint64_t set_count, const uint64_t* checks,
@@ -1169,18 +1169,18 @@ void Solver::subsets_check(uint32_t n, const uint64_t* sets, uint64_t set_count,
   SW_CUDA(cudaSetDevice(device_));
   Engine& E = *eng_;
   const int W = words_for((int)n);
-  std::vector<u64> srows((size_t)W * set_count), qrows((size_t)W * check_count);
-  to_device_rows(sets, set_count, n, W, srows.data());
-  to_device_rows(checks, check_count, n, W, qrows.data());
   const u32 m = (u32)set_count, q = (u32)check_count;
-  E.uq_rows.reserve(sizeof(u64) * srows.size());
+  const size_t sbytes = sizeof(u64) * (size_t)W * m, qbytes = sizeof(u64) * (size_t)W * q;
+  E.uq_rows.reserve(sbytes);
   E.uq_vals.reserve(sizeof(u32) * m);
-  E.ch_rows.reserve(sizeof(u64) * qrows.size());
+  E.ch_rows.reserve(qbytes);
   E.flags_a.reserve(sizeof(u32) * m);
   E.flags_b.reserve(sizeof(u32) * q);
-  E.keys.reserve(sizeof(u64) * srows.size());
-  SW_CUDA(cudaMemcpyAsync(E.uq_rows.p, srows.data(), sizeof(u64) * srows.size(), cudaMemcpyHostToDevice, E.stream));
-  SW_CUDA(cudaMemcpyAsync(E.ch_rows.p, qrows.data(), sizeof(u64) * qrows.size(), cudaMemcpyHostToDevice, E.stream));
+  E.keys.reserve(sbytes);
+  SW_CUDA(cudaMemcpyAsync(E.uq_rows.p, sets, sbytes, cudaMemcpyHostToDevice, E.stream));
+  SW_CUDA(cudaMemcpyAsync(E.ch_rows.p, checks, qbytes, cudaMemcpyHostToDevice, E.stream));
+  launch_convert_rows(W, E.uq_rows.as<u64>(), m, (int)n, true, E.stream);
+  launch_convert_rows(W, E.ch_rows.as<u64>(), q, (int)n, true, E.stream);
   // sort + unique the set list (check_contains_subset sorts both, :30-33)
   launch_iota(E.uq_vals.as<u32>(), m, E.stream);
   E.sort_rows(W, E.uq_rows.as<u64>(), E.uq_vals.as<u32>(), m);
@@ -1205,21 +1205,21 @@ uint64_t Solver::sort_unique(uint32_t n, uint64_t* sets, uint64_t count) {
   SW_CUDA(cudaSetDevice(device_));
   Engine& E = *eng_;
   const int W = words_for((int)n);
-  std::vector<u64> rows((size_t)W * count);
-  to_device_rows(sets, count, n, W, rows.data());
   const u32 m = (u32)count;
-  E.uq_rows.reserve(sizeof(u64) * rows.size());
+  const size_t bytes = sizeof(u64) * (size_t)W * m;
+  E.uq_rows.reserve(bytes);
   E.uq_vals.reserve(sizeof(u32) * m);
-  E.keys.reserve(sizeof(u64) * rows.size());
+  E.keys.reserve(bytes);
   E.flags_a.reserve(sizeof(u32) * m);
-  SW_CUDA(cudaMemcpyAsync(E.uq_rows.p, rows.data(), sizeof(u64) * rows.size(), cudaMemcpyHostToDevice, E.stream));
+  SW_CUDA(cudaMemcpyAsync(E.uq_rows.p, sets, bytes, cudaMemcpyHostToDevice, E.stream));
+  launch_convert_rows(W, E.uq_rows.as<u64>(), m, (int)n, true, E.stream);
   launch_iota(E.uq_vals.as<u32>(), m, E.stream);
   E.sort_rows(W, E.uq_rows.as<u64>(), E.uq_vals.as<u32>(), m);
   launch_unique_flags(W, E.uq_rows.as<u64>(), m, E.flags_a.as<u32>(), E.stream);
   u32 u = E.compact(W, E.uq_rows.as<u64>(), E.uq_vals.as<u32>(), E.flags_a.as<u32>(), m, E.keys.as<u64>(), nullptr);
-  SW_CUDA(cudaMemcpyAsync(rows.data(), E.keys.p, sizeof(u64) * W * u, cudaMemcpyDeviceToHost, E.stream));
+  launch_convert_rows(W, E.keys.as<u64>(), u, (int)n, false, E.stream);
+  SW_CUDA(cudaMemcpyAsync(sets, E.keys.p, sizeof(u64) * W * u, cudaMemcpyDeviceToHost, E.stream));
   SW_CUDA(cudaStreamSynchronize(E.stream));
-  from_device_rows(rows.data(), u, n, W, sets);
   return u;
 }
 
@@ -1506,21 +1506,7 @@ void Solver::reduce(const Automaton& A, const sw_reduce_config& cfg, Bounds& b, 
 // Learned distance model: training pairs, scoring, training, learned beam.
 // ---------------------------------------------------------------------------
 namespace {
-// 8-word reference layout (state q = bit q % 64 of word q / 64) <-> device rows
-// of W words.
-std::vector<u64> ref8_to_rows(const uint64_t* ref, uint64_t count, uint32_t n, int W) {
-  std::vector<u64> out((size_t)count * W, 0);
-  for (uint64_t i = 0; i < count; ++i)
-    for (int w = 0; w < 8; ++w) {
-      uint64_t v = ref[i * 8 + w];
-      while (v) {
-        const int q = w * 64 + __builtin_ctzll(v);
-        v &= v - 1;
-        if ((uint32_t)q < n) out[(size_t)i * W + (q >> 6)] |= state_bit(q);
-      }
-    }
-  return out;
-}
+// device rows of W words -> the 8-word reference layout of the model's sets
 void rows_to_ref8(const u64* rows, uint64_t count, uint32_t n, int W, uint64_t* out) {
   for (uint64_t i = 0; i < count; ++i) {
     for (int w = 0; w < 8; ++w) out[i * 8 + w] = 0;
@@ -1649,11 +1635,11 @@ void Solver::mlp_forward(const Automaton& A, const uint64_t* sets, uint64_t coun
   SW_CUDA(cudaSetDevice(device_));
   Engine& E = *eng_;
   if (!count) return;
-  const std::vector<u64> rows = ref8_to_rows(sets, count, A.n, 8);
   DevBuf d_rows, d_y;
-  d_rows.reserve(sizeof(u64) * rows.size());
+  d_rows.reserve(sizeof(u64) * 8 * count);
   d_y.reserve(sizeof(float) * count);
-  SW_CUDA(cudaMemcpyAsync(d_rows.p, rows.data(), sizeof(u64) * rows.size(), cudaMemcpyHostToDevice, E.stream));
+  SW_CUDA(cudaMemcpyAsync(d_rows.p, sets, sizeof(u64) * 8 * count, cudaMemcpyHostToDevice, E.stream));
+  launch_convert_rows(8, d_rows.as<u64>(), count, (int)A.n, true, E.stream);
   E.mlp->prepare(A);
   E.mlp->forward(d_rows.as<u64>(), 8, (u32)count, d_y.as<float>());
   SW_CUDA(cudaMemcpyAsync(out, d_y.p, sizeof(float) * count, cudaMemcpyDeviceToHost, E.stream));
@@ -1665,12 +1651,12 @@ float Solver::mlp_gradient(const Automaton& A, const uint64_t* sets, const float
   SW_CUDA(cudaSetDevice(device_));
   Engine& E = *eng_;
   if (!count) throw std::invalid_argument("empty batch");
-  const std::vector<u64> rows = ref8_to_rows(sets, count, A.n, 8);
   DevBuf d_rows, d_y, d_t;
-  d_rows.reserve(sizeof(u64) * rows.size());
+  d_rows.reserve(sizeof(u64) * 8 * count);
   d_y.reserve(sizeof(float) * count);
   d_t.reserve(sizeof(float) * count);
-  SW_CUDA(cudaMemcpyAsync(d_rows.p, rows.data(), sizeof(u64) * rows.size(), cudaMemcpyHostToDevice, E.stream));
+  SW_CUDA(cudaMemcpyAsync(d_rows.p, sets, sizeof(u64) * 8 * count, cudaMemcpyHostToDevice, E.stream));
+  launch_convert_rows(8, d_rows.as<u64>(), count, (int)A.n, true, E.stream);
   SW_CUDA(cudaMemcpyAsync(d_t.p, labels, sizeof(float) * count, cudaMemcpyHostToDevice, E.stream));
   E.mlp->prepare(A);
   E.mlp->zero_grad();
@@ -1696,12 +1682,10 @@ float Solver::mlp_train(const std::vector<Automaton>& autos, const uint64_t* off
   d_rows.reserve(sizeof(u64) * 8 * total);
   d_lab.reserve(sizeof(float) * total);
   d_y.reserve(sizeof(float) * batch);
-  for (size_t a = 0; a < A_n; ++a) {
-    const uint64_t o = offsets[a], c = offsets[a + 1] - o;
-    if (!c) continue;
-    const std::vector<u64> rows = ref8_to_rows(sets + o * 8, c, autos[a].n, 8);
-    SW_CUDA(cudaMemcpy(d_rows.as<u64>() + o * 8, rows.data(), sizeof(u64) * rows.size(), cudaMemcpyHostToDevice));
-  }
+  SW_CUDA(cudaMemcpyAsync(d_rows.p, sets, sizeof(u64) * 8 * total, cudaMemcpyHostToDevice, E.stream));
+  for (size_t a = 0; a < A_n; ++a)
+    launch_convert_rows(8, d_rows.as<u64>() + offsets[a] * 8, offsets[a + 1] - offsets[a], (int)autos[a].n, true,
+                        E.stream);
   SW_CUDA(cudaMemcpy(d_lab.p, labels, sizeof(float) * total, cudaMemcpyHostToDevice));
   DevBuf d_grp;
   if (groups && rank_w > 0.0f) {

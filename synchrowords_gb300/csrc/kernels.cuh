@@ -112,6 +112,11 @@ void launch_merge(int W, const u64* A, u32 na, const u64* B, u32 nb, u64* out, c
 // rows[i] = complement of rows[i] within n states.
 void launch_complement(int W, u64* rows, u32 m, int n, cudaStream_t s);
 
+// In-place conversion of `count` rows between the reference bit layout (state
+// q = bit q % 64 of word q / 64) and the device layout (bit 63 - q % 64); bits
+// of states >= n come out zero.
+void launch_convert_rows(int W, u64* rows, u64 count, int n, bool to_device, cudaStream_t s);
+
 // out[i] = popcount of row i.
 void launch_popcount(int W, const u64* rows, u32 m, u32* out, cudaStream_t s);
 
