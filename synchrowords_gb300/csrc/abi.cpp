@@ -42,11 +42,16 @@ struct SmallBatchState {
   }
 };
 
+// Default n * log2(k) bound of the cluster launch, and the meet pairs of one
+// level it takes on at that bound.
+constexpr double kDefaultClusterLimit = 160.0;
+constexpr uint64_t kClusterMaxPairs = 1ull << 28;
+
 struct sw_context {
   std::unique_ptr<sw::Solver> solver;
   std::vector<std::unique_ptr<sw::Solver>> workers;  // extra streams for sw_solve_batch
   SmallBatchState small;
-  sw_batch_tuning tuning{0, 104.0, 0, 160.0};  // sw_autotune_batch / sw_set_batch_tuning
+  sw_batch_tuning tuning{0, 104.0, 0, kDefaultClusterLimit};  // sw_autotune_batch / sw_set_batch_tuning
 };
 
 namespace {
@@ -291,6 +296,11 @@ void start_round(sw_context* ctx, DeviceRound& D, const std::vector<uint32_t> sm
   // cluster launch geometry and scratch
   const int cs = ctx->tuning.cluster_size > 0 ? std::min<int>(ctx->tuning.cluster_size, 16) : 8;
   const sw::ClusterCaps caps = sw::cluster_default_caps();
+  // A cluster gives an automaton back (to the worker streams, which search it
+  // with the whole GPU) after a level of more than kClusterMaxPairs meet pairs,
+  // unless the caller raised cluster_limit to have larger automata searched here.
+  sw::ClusterLimits limits;
+  if (ctx->tuning.cluster_limit <= kDefaultClusterLimit) limits.max_pairs = kClusterMaxPairs;
   uint32_t clusters[4] = {0, 0, 0, 0};
   uint32_t max_clusters = 0;
   for (int c = 0; c < 4; ++c)
@@ -308,14 +318,14 @@ void start_round(sw_context* ctx, DeviceRound& D, const std::vector<uint32_t> sm
       S.c_scratch.reserve(need);
       S.c_zeroed = 0;
     }
-    if (S.c_zeroed < S.c_scratch.cap || S.c_tags_used + tags >= 0xF0000000ull) {
+    if (S.c_zeroed < S.c_scratch.cap || S.c_tags_used + tags >= sw::kClusterTagLimit) {
       // new memory, or the tag counter could wrap: every slot back to "empty"
       SW_CUDA(cudaMemsetAsync(S.c_scratch.p, 0, S.c_scratch.cap, S.stream));
       S.c_zeroed = S.c_scratch.cap;
       S.c_tags_used = 0;
     }
     S.c_tags_used += tags;
-    S.c_stats.reserve(sizeof(uint64_t) * 9);
+    S.c_stats.reserve(sizeof(uint64_t) * 7);
   }
   SW_CUDA(cudaMemcpyAsync(S.inst.p, inst.data(), sizeof(sw::SmallInstance) * inst.size(), cudaMemcpyHostToDevice,
                           S.stream));
@@ -326,7 +336,7 @@ void start_round(sw_context* ctx, DeviceRound& D, const std::vector<uint32_t> sm
   // the round's device work: the cluster statistics reset and one persistent
   // launch per non-empty class
   auto issue = [&] {
-    if (max_clusters) SW_CUDA(cudaMemsetAsync(S.c_stats.p, 0, sizeof(uint64_t) * 9, S.stream));
+    if (max_clusters) SW_CUDA(cudaMemsetAsync(S.c_stats.p, 0, sizeof(uint64_t) * 7, S.stream));
     for (int c = 0; c < 8; ++c) {
       const size_t a = class_start[c], b = class_start[c + 1];
       if (a == b) continue;
@@ -339,7 +349,7 @@ void start_round(sw_context* ctx, DeviceRound& D, const std::vector<uint32_t> sm
       else
         sw::launch_cluster_batch(W, cs, clusters[c - 4], S.inst.as<sw::SmallInstance>() + a, (uint32_t)(b - a),
                                  S.delta.as<uint8_t>(), S.seeds.as<uint8_t>(), S.results.as<sw::SmallResult>() + a,
-                                 S.words.as<uint8_t>() + a * D.word_stride, D.word_stride, S.c_scratch.p, caps,
+                                 S.words.as<uint8_t>() + a * D.word_stride, D.word_stride, S.c_scratch.p, caps, limits,
                                  S.counter.as<uint32_t>(), S.c_stats.as<sw::u64>(), S.stream);
     }
   };
@@ -352,6 +362,7 @@ void start_round(sw_context* ctx, DeviceRound& D, const std::vector<uint32_t> sm
                             (uint64_t)(uintptr_t)S.c_stats.p};
   for (int c = 0; c < 9; ++c) key.push_back(class_start[c]);
   for (int c = 0; c < 4; ++c) key.push_back(clusters[c]);
+  key.push_back(limits.max_pairs);
   cudaGraphExec_t exec = nullptr;
   for (auto& g : S.graphs)
     if (g.first == key) exec = g.second;
@@ -398,7 +409,7 @@ std::vector<uint32_t> finish_round(sw_context* ctx, DeviceRound& D, const uint32
   const size_t m = D.order.size();
   std::vector<sw::SmallResult> R(m);
   std::vector<uint8_t> words((size_t)D.word_stride * m);
-  uint64_t cst[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  uint64_t cst[7] = {0, 0, 0, 0, 0, 0, 0};
   SW_CUDA(cudaMemcpyAsync(R.data(), S.results.p, sizeof(sw::SmallResult) * m, cudaMemcpyDeviceToHost, S.stream));
   SW_CUDA(cudaMemcpyAsync(words.data(), S.words.p, words.size(), cudaMemcpyDeviceToHost, S.stream));
   const bool any_cluster = std::find(D.engine.begin(), D.engine.end(), 1) != D.engine.end();
@@ -474,9 +485,8 @@ std::vector<uint32_t> finish_round(sw_context* ctx, DeviceRound& D, const uint32
                  "capacity / %zu unfinished; cluster launch %zu / %zu / %zu\n",
                  m, D.launches, (double)ms, st[0][0], st[0][1], st[0][2], st[1][0], st[1][1], st[1][2]);
     if (any_cluster)
-      std::fprintf(stderr, "[sw] cluster launch cycles (rank 0, summed over automata): expand %.3g, dedup %.3g, "
-                   "visited insert %.3g, meet %.3g, result %.3g\n", (double)cst[4], (double)cst[5],
-                   (double)cst[6], (double)cst[7], (double)cst[8]);
+      std::fprintf(stderr, "[sw] cluster launch cycles (rank 0, summed over automata): expand and dedup %.3g, meet %.3g, "
+                   "result %.3g\n", (double)cst[4], (double)cst[5], (double)cst[6]);
   }
   return again;
 }

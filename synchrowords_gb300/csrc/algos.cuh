@@ -53,9 +53,6 @@ void launch_brute_parent(const uint16_t* delta, int n, int k, const u32* level, 
 struct SmallInstance {
   u32 n, k, delta_off, seed_off, seed_count, max_len;
 };
-// status 0: found, length and word_len letters at words + i * word_stride;
-// 1: lists outgrew the shared-memory capacities (solve it another way);
-// 2: no meeting pair within max_len.
 // status: 0 solved, 1 over a capacity, 2 no meeting within max_len.
 // why (status 1): bits 0-7 the capacity (1 children, 2 layer, 3 visited,
 // 4 depth, 5 word buffer), bits 8+ the layers searched when it stopped.
@@ -78,26 +75,65 @@ void launch_small_batch(int W, const SmallInstance* inst, u32 count, const uint8
 // Device-resident search on thread-block clusters (batch_cluster.cu): one
 // cluster of `cs` CTAs per automaton (n <= 256, n * k <= 4096), lists in a
 // per-cluster global region.  Same instances and results as the small batch;
-// status 1 may also report why 6 (a hash-table probe ran out).
+// status 1 may also report why 6 (a hash-table probe ran out), status 2 why 8
+// (a side died out) or 9 (max_len reached), and status 3 says that the search
+// stopped at a work limit; where no word was found, `length` counts the
+// lengths excluded so far.
 struct ClusterCaps {
-  u32 vis = 0;        // visited rows per side (every layer of the side, in order)
+  u32 vis = 0;        // row slots per side (one per child ever expanded on that side)
   u32 ch = 0;         // children of one step
-  u32 vtab_bits = 0;  // log2 slots of a side's visited table (>= 2 * vis)
-  u32 ltab_bits = 0;  // log2 slots of the step's child table (>= 2 * ch)
+  u32 vtab_bits = 0;  // log2 slots of a side's hash table (at least 4/3 of vis)
 };
+// Work limits of a launch: a search stops before a level of more than
+// max_children children, after a level of more than max_pairs meet pairs, and
+// once its lists and the next level pass a quarter of `budget` bytes by the
+// streamed search's count (which then changes its reductions).
+struct ClusterLimits {
+  u64 max_pairs = ~0ull;
+  u64 budget = ~0ull;
+  u32 max_children = ~0u;
+  u32 counter_ready = 0;    // the caller zeroed the counter on the launch's stream
+  size_t header_bytes = 0;  // bytes before the first region; 0: room for every cluster index
+};
+// How a single search ended (written at kClusterExitOffset of its scratch):
+// meet pairs, children and meet queries (backward rows, summed over levels),
+// then per side (forward, backward) depth, kept rows and current layer size.
+struct ClusterExit {
+  u64 pairs, children, queries;
+  u32 depth[2], kept[2], cnt[2];
+};
+constexpr size_t kClusterExitOffset = 256 + 32;
+// Scratch of a single search: tag counter, control block, its SmallResult, its
+// word (up to kClusterSingleWord letters); then the region.
+constexpr size_t kClusterSingleResult = 512, kClusterSingleWords = 576, kClusterSingleHeader = 2048;
+constexpr u32 kClusterSingleWord = 1024;
 ClusterCaps cluster_default_caps();
+ClusterCaps cluster_single_caps();
 // Bytes of scratch for `clusters` clusters.  It must be zero-filled before its
 // first launch, and again before the tags the launches take from its counter
-// (cluster_tags_per_launch) could wrap around 2^32.
+// (cluster_tags_per_launch) could pass kClusterTagLimit.
 size_t cluster_scratch_bytes(u32 clusters, const ClusterCaps& c);
+size_t cluster_single_scratch_bytes(const ClusterCaps& c);
 u32 cluster_max_clusters_supported();
 // Clusters of `cs` CTAs that fit on the current device at once.
 u32 cluster_batch_max_clusters(int W, int cs);
-// Tags a launch of `count` automata can take: one per search, one per step.
-constexpr u64 cluster_tags_per_launch(u32 count) { return (u64)count * (2 + 2 * 1024); }
+// Tags a launch of `count` automata can take: one per search and one per
+// cluster that finds the batch done.
+constexpr u64 cluster_tags_per_launch(u32 count) { return (u64)count + 512; }
+constexpr u64 kClusterTagLimit = 1ull << 26;
 void launch_cluster_batch(int W, int cs, u32 clusters, const SmallInstance* inst, u32 count,
                           const uint8_t* delta_pool, const uint8_t* seed_pool, SmallResult* results, uint8_t* words,
-                          u32 word_stride, void* scratch, const ClusterCaps& caps, u32* counter, u64* stats,
-                          cudaStream_t s);
+                          u32 word_stride, void* scratch, const ClusterCaps& caps, const ClusterLimits& limits,
+                          u32* counter, u64* stats, cudaStream_t s);
+// Kept rows of one side (0 forward, 1 backward complements) of a search that
+// stopped, layer after layer, and each row's origin (letter * parents +
+// parent position; a seed's entry is its seed index).
+// The layer table a search left (host copy of it: kClusterMetaWords words from
+// cluster_meta_offset): per side the first row slot, the first list entry and
+// the row count of every layer, each kClusterMetaStride words.
+constexpr size_t kClusterMetaStride = 1025, kClusterMetaWords = 6 * kClusterMetaStride;
+size_t cluster_meta_offset(int W, size_t header_bytes, const ClusterCaps& c);
+void launch_cluster_export(int W, const void* scratch, size_t header_bytes, const ClusterCaps& caps, int side, u32 kept,
+                           u32 depth, u64* rows, u32* origin, cudaStream_t s);
 
 }  // namespace sw

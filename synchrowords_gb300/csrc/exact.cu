@@ -36,6 +36,8 @@ namespace {
 
 struct Layer {
   DevBuf origin;        // per kept set: child position a*parent_count + parent
+  const u32* view = nullptr;  // the same, in a buffer this layer shares with others (then `origin` is unused)
+  const u32* org() const { return view ? view : origin.as<u32>(); }
   u32 count = 0;
   u32 parent_count = 0;
 };
@@ -67,6 +69,7 @@ struct Side {
     spare[best] = std::move(spare.back());
     spare.pop_back();
     L->count = L->parent_count = 0;
+    L->view = nullptr;
     return L;
   }
   void reset() {
@@ -79,6 +82,13 @@ struct Side {
     seed_states.clear();
   }
 };
+
+// Where a search leaves the single cluster it starts on (Engine::run_single).
+// CTAs of that cluster, and the children and meet pairs of a level above which
+// the level goes to the whole GPU.
+constexpr int kSingleClusterCtas = 8;
+constexpr u32 kSingleMaxChildren = 1u << 14;
+constexpr u64 kSingleMaxPairs = 1ull << 26;
 
 // One level of the bounded inverse phase (a chunk of parents' children).
 struct DLevel {
@@ -596,16 +606,138 @@ class Engine {
   }
 
   // Trace letters of set `idx` at the top layer of side X down to depth 0.
+  DevBuf trace_dev;
+  HostPinned trace_host;
   std::vector<uint32_t> trace(const Side& X, u32 idx, u32* seed_index) {
-    std::vector<uint32_t> letters;  // from the top layer down
-    for (size_t d = X.layers.size(); d-- > 0;) {
-      const Layer& L = *X.layers[d];
-      u32 o = read_u32(L.origin.as<u32>() + idx);
-      letters.push_back(o / L.parent_count);
-      idx = o % L.parent_count;
+    const size_t L = X.layers.size();  // letters come from the top layer down
+    const size_t steps_bytes = sizeof(TraceStep) * L, out_bytes = sizeof(u32) * (L + 1);
+    trace_dev.reserve(steps_bytes + out_bytes);
+    trace_host.reserve(steps_bytes + out_bytes);
+    TraceStep* h = trace_host.as<TraceStep>();
+    for (size_t i = 0; i < L; ++i) h[i] = TraceStep{X.layers[L - 1 - i]->org(), X.layers[L - 1 - i]->parent_count};
+    SW_CUDA(cudaMemcpyAsync(trace_dev.p, h, steps_bytes, cudaMemcpyHostToDevice, stream));
+    u32* d_out = reinterpret_cast<u32*>(trace_dev.as<uint8_t>() + steps_bytes);
+    launch_trace(trace_dev.as<TraceStep>(), (u32)L, idx, d_out, stream);
+    u32* out = reinterpret_cast<u32*>(trace_host.as<uint8_t>() + steps_bytes);
+    SW_CUDA(cudaMemcpyAsync(out, d_out, out_bytes, cudaMemcpyDeviceToHost, stream));
+    SW_CUDA(cudaStreamSynchronize(stream));
+    if (seed_index) *seed_index = out[L];
+    return std::vector<uint32_t>(out, out + L);
+  }
+
+  // ---- the first levels in one launch (batch_cluster.cu) ----
+  // A search starts on one thread-block cluster, which runs it level by level
+  // on the device: to its end where the lists stay small, else until a level
+  // is worth the whole GPU; import_single() then turns the cluster's lists into
+  // the two sides' layers.
+  DevBuf single_scratch, single_in, single_org[2];
+  HostPinned single_host;
+  u64 single_tags = 0;
+  size_t single_zeroed = 0;
+  struct Single {
+    SmallResult res;
+    ClusterExit exit;
+    const uint8_t* word;
+  };
+  Single run_single(const Automaton& A, const std::vector<uint32_t>& seeds, u32 max_len, u64 budget) {
+    const int W = words_for((int)A.n);
+    const ClusterCaps caps = cluster_single_caps();
+    single_scratch.reserve(cluster_single_scratch_bytes(caps));
+    if (single_zeroed < single_scratch.cap || single_tags + cluster_tags_per_launch(1) >= kClusterTagLimit) {
+      SW_CUDA(cudaMemsetAsync(single_scratch.p, 0, single_scratch.cap, stream));
+      single_zeroed = single_scratch.cap;
+      single_tags = 0;
     }
-    if (seed_index) *seed_index = idx;
-    return letters;
+    single_tags += cluster_tags_per_launch(1);
+    // input: the launch's counter (zero), the instance, its table and seeds
+    const size_t inst_off = 32, pool_off = 64, seeds_off = pool_off + A.t.size();
+    const size_t in_bytes = seeds_off + seeds.size();
+    const size_t out_bytes = kClusterSingleWords + kClusterSingleWord - 256;
+    single_in.reserve(in_bytes);
+    single_host.reserve(16384 + sizeof(u32) * kClusterMetaWords);
+    uint8_t* h = single_host.as<uint8_t>();
+    std::memset(h, 0, pool_off);
+    const SmallInstance I{A.n, A.k, (u32)pool_off, (u32)seeds_off, (u32)seeds.size(), max_len};
+    std::memcpy(h + inst_off, &I, sizeof(I));
+    for (size_t i = 0; i < A.t.size(); ++i) h[pool_off + i] = (uint8_t)A.t[i];
+    for (size_t i = 0; i < seeds.size(); ++i) h[seeds_off + i] = (uint8_t)seeds[i];
+    SW_CUDA(cudaMemcpyAsync(single_in.p, h, in_bytes, cudaMemcpyHostToDevice, stream));
+    ClusterLimits lim;
+    lim.max_children = kSingleMaxChildren;
+    lim.max_pairs = kSingleMaxPairs;
+    lim.budget = budget;
+    lim.counter_ready = 1;
+    lim.header_bytes = kClusterSingleHeader;
+    uint8_t* sc = single_scratch.as<uint8_t>();
+    const uint8_t* in = single_in.as<uint8_t>();
+    timed(3, 0.0, [&] {
+      launch_cluster_batch(W, kSingleClusterCtas, 1, reinterpret_cast<const SmallInstance*>(in + inst_off), 1, in, in,
+                           reinterpret_cast<SmallResult*>(sc + kClusterSingleResult), sc + kClusterSingleWords,
+                           kClusterSingleWord, sc, caps, lim, single_in.as<u32>(), nullptr, stream);
+    });
+    count_launch();
+    uint8_t* out = h + 8192;
+    SW_CUDA(cudaMemcpyAsync(out, sc + 256, out_bytes, cudaMemcpyDeviceToHost, stream));
+    SW_CUDA(cudaStreamSynchronize(stream));
+    Single r;
+    std::memcpy(&r.res, out + kClusterSingleResult - 256, sizeof(r.res));
+    std::memcpy(&r.exit, out + kClusterExitOffset - 256, sizeof(r.exit));
+    r.word = out + kClusterSingleWords - 256;
+    if (st) {
+      st->bfs_steps += r.exit.depth[0];
+      st->ibfs_steps += r.exit.depth[1];
+      st->subsets_expanded += r.exit.children;
+      st->subsets_kept += r.exit.kept[0] + r.exit.kept[1] - 1 - seeds.size();
+      st->trie_queries += r.exit.queries;
+      st->logical_pairs += r.exit.pairs;
+      st->meet_pairs += r.exit.pairs;
+    }
+    return r;
+  }
+  void import_single(int W, const ClusterExit& ex) {
+    const ClusterCaps caps = cluster_single_caps();
+    u32* meta = reinterpret_cast<u32*>(single_host.as<uint8_t>() + 16384);
+    SW_CUDA(cudaMemcpyAsync(meta, single_scratch.as<uint8_t>() + cluster_meta_offset(W, kClusterSingleHeader, caps),
+                            sizeof(u32) * kClusterMetaWords, cudaMemcpyDeviceToHost, stream));
+    for (int side = 0; side < 2; ++side) {
+      Side& X = side ? B : F;
+      const u32 kept = ex.kept[side], cnt = ex.cnt[side], depth = ex.depth[side];
+      X.vis.reserve(sizeof(u64) * W * kept);
+      single_org[side].reserve(sizeof(u32) * kept);
+      launch_cluster_export(W, single_scratch.p, kClusterSingleHeader, caps, side, kept, depth, X.vis.as<u64>(),
+                            single_org[side].as<u32>(), stream);
+      // the current layer in key order, its origins with it
+      X.rows.reserve(sizeof(u64) * W * cnt);
+      X.count = cnt;
+      X.vis_count = kept;
+      const u64* cur = X.vis.as<u64>() + (size_t)(kept - cnt) * W;
+      keys.reserve(sizeof(u64) * 2 * cnt);
+      ch_vals.reserve(sizeof(u32) * cnt);
+      launch_layer_keys(W, cur, cnt, keys.as<u64>(), stream, X.keymap);
+      launch_iota(ch_vals.as<u32>(), cnt, stream);
+      sort_rows(2, keys.as<u64>(), ch_vals.as<u32>(), cnt);
+      launch_gather_rows(W, cur, ch_vals.as<u32>(), cnt, X.rows.as<u64>(), stream);
+      count_launch(4);
+      std::unique_ptr<Layer> top;
+      if (depth) {
+        top = X.new_layer(sizeof(u32) * cnt);
+        top->origin.reserve(sizeof(u32) * cnt);
+        launch_gather_u32(single_org[side].as<u32>() + (kept - cnt), ch_vals.as<u32>(), cnt, top->origin.as<u32>(),
+                          stream);
+        count_launch();
+      }
+      sort_by_layer_key(W, X.vis.as<u64>(), kept, X.keymap);
+      if (side == 0) SW_CUDA(cudaStreamSynchronize(stream));  // the layer table has arrived
+      const u32* loff = meta + (2 + side) * kClusterMetaStride;
+      const u32* lcnt = meta + (4 + side) * kClusterMetaStride;
+      for (u32 d = 1; d <= depth; ++d) {
+        std::unique_ptr<Layer> L = d == depth ? std::move(top) : X.new_layer(0);
+        if (d < depth) L->view = single_org[side].as<u32>() + loff[d];
+        L->count = lcnt[d];
+        L->parent_count = lcnt[d - 1];
+        X.layers.push_back(std::move(L));
+      }
+    }
   }
 };
 
@@ -755,23 +887,66 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
     b.word.clear();
     return;
   }
-  if (!is_synchronizing(A)) {
-    // The reference's Exact has no such check and runs until its bound; a
-    // non-synchronizing automaton is reported as such instead.
-    b.non_synchro = true;
-    return;
-  }
   SW_CUDA(cudaSetDevice(device_));
   Engine& E = *eng_;
   AllocScope alloc_scope(E.stream);  // buffer growth ordered on this solve's stream only
   E.st = &st;
   auto t0 = std::chrono::steady_clock::now();
   const int n = (int)A.n, k = (int)A.k, W = words_for(n);
-  E.upload_tables(A);
+  const size_t budget = (size_t)cfg.max_memory_mb * 1024 * 1024;
+  const size_t row_bytes = sizeof(u64) * W;
+  // exact.cpp:65 searches lengths below the upper bound; when no word backs
+  // that bound (it came from the plan's upper_bound), length == bound is
+  // searched too so that a word can be returned.
+  const u64 max_rt = b.has_word ? b.upper - 1 : b.upper;
+  u64 rt = 0;
+  const std::vector<uint32_t> seeds = backward_seeds(A);
   E.F.reset();
   E.B.reset();
-  // seeds
-  {
+  auto finish = [&] {
+    st.device_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    E.st = nullptr;
+  };
+  // A search with duplicate removal only starts on one thread-block cluster
+  // (the other reductions and reduced forward seeds are the streamed path's).
+  bool imported = false;
+  ClusterExit single_exit{};
+  if (!red && !b.has_word && cfg.reductions != SW_REDUCE_ALWAYS && n <= 256 && n * k <= 4096 && !seeds.empty() &&
+      max_rt > 0) {
+    const Engine::Single S = E.run_single(A, seeds, (u32)std::min<u64>(max_rt, kClusterSingleWord), budget);
+    if (E.verbose)
+      std::fprintf(stderr, "[sw] first levels on a cluster: status %u why %u, len %u, |F|=%u |B|=%u, %llu children\n",
+                   S.res.status, S.res.why & 255u, S.res.length, S.exit.cnt[0], S.exit.cnt[1], S.exit.children);
+    if (S.res.status == 0) {
+      std::vector<uint32_t> word(S.word, S.word + S.res.word_len);
+      if (word.size() != S.res.length || apply_word(A, word).size() != 1)
+        throw std::runtime_error("internal error: the cluster search's word does not synchronize");
+      b.lower = std::max<u64>(b.lower, S.res.length);
+      b.upper = S.res.length;
+      b.has_word = true;
+      b.word = std::move(word);
+      finish();
+      return;
+    }
+    const u32 why = S.res.why & 255u;
+    imported = S.res.status == 3 || (S.res.status == 1 && (why == 1 || why == 3 || why == 4)) ||
+               (S.res.status == 2 && why == 9);
+    if (imported) {
+      single_exit = S.exit;
+      rt = S.res.length;
+    }
+  }
+  if (!is_synchronizing(A)) {
+    // The reference's Exact has no such check and runs until its bound; a
+    // non-synchronizing automaton is reported as such instead.
+    b.non_synchro = true;
+    finish();
+    return;
+  }
+  E.upload_tables(A);
+  if (imported) {
+    E.import_single(W, single_exit);
+  } else {  // seeds
     std::vector<u64> full(W, 0);
     for (int q = 0; q < n; ++q) full[q >> 6] |= state_bit(q);
     std::vector<u64> fseeds;
@@ -787,7 +962,6 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
     E.F.rows.reserve(sizeof(u64) * W * std::max<u32>(nf, 1));
     SW_CUDA(cudaMemcpyAsync(E.F.rows.p, fseeds.data(), sizeof(u64) * W * nf, cudaMemcpyHostToDevice, E.stream));
     E.F.count = nf;
-    std::vector<uint32_t> seeds = backward_seeds(A);
     std::vector<u64> rows((size_t)W * std::max<size_t>(seeds.size(), 1), 0);
     for (size_t i = 0; i < seeds.size(); ++i) {
       for (int q = 0; q < n; ++q)
@@ -813,13 +987,6 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
       E.B.vis_count = (u32)seeds.size();
     }
   }
-  const size_t budget = (size_t)cfg.max_memory_mb * 1024 * 1024;
-  const size_t row_bytes = sizeof(u64) * W;
-  // exact.cpp:65 searches lengths below the upper bound; when no word backs
-  // that bound (it came from the plan's upper_bound), length == bound is
-  // searched too so that a word can be returned.
-  const u64 max_rt = b.has_word ? b.upper - 1 : b.upper;
-  u64 rt = 0;
   bool found = false, oom = false;
   u32 wit_q = 0, wit_s = 0;
   // Bounded inverse phase (the device counterpart of the reference's DFS
@@ -980,8 +1147,7 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
       b.lower = std::max<u64>(b.lower, rt + 1);
     }
   }
-  st.device_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-  E.st = nullptr;
+  finish();
 }
 
 // ---------------------------------------------------------------------------
@@ -1042,7 +1208,7 @@ static BeamRun beam_cutoff(Engine& E, const Automaton& A, u32 beam_size, u64 max
       u32 idx = first_val % m;
       for (size_t d = X.layers.size(); d-- > 0;) {
         const Layer& L = *X.layers[d];
-        u32 o = E.read_u32(L.origin.as<u32>() + idx);
+        u32 o = E.read_u32(L.org() + idx);
         letters.push_back(o / L.parent_count);
         idx = o % L.parent_count;
       }

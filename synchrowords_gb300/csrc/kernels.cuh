@@ -172,6 +172,14 @@ void launch_gather_u32(const u32* src, const u32* idx, u32 m, u32* dst, cudaStre
 // (score null), or counts[i] << 16 | leading 16 bits of score[i] (both).
 void launch_score_keys(const float* score, const u32* counts, u32 m, u64* keys, cudaStream_t s);
 
+// Walks a word back: step i reads o = steps[i].origin[idx], emits the letter
+// out[i] = o / parents and goes on at idx = o % parents; out[count] = the last idx.
+struct TraceStep {
+  const u32* origin;
+  u32 parents;
+};
+void launch_trace(const TraceStep* steps, u32 count, u32 idx, u32* out, cudaStream_t s);
+
 // Fill u32 array with a value.
 void launch_fill_u32(u32* p, u32 value, u32 m, cudaStream_t s);
 
