@@ -47,6 +47,7 @@
 #include <utility>
 
 #include "algos.cuh"
+#include "rowset.cuh"
 
 namespace sw {
 
@@ -80,45 +81,6 @@ __device__ __forceinline__ u32 cluster_index() {
 // before the barrier by any CTA of the cluster are visible after it.
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ u32 ld_volatile(const u32* p) { return *(const volatile u32*)p; }
-__device__ __forceinline__ u64 ld_volatile64(const u64* p) { return *(const volatile u64*)p; }
-
-template <int W>
-__device__ __forceinline__ u64 row_hash(const u64* x) {
-  u64 h = 0x243F6A8885A308D3ULL;
-#pragma unroll
-  for (int w = 0; w < W; ++w) {
-    h ^= x[w];
-    h *= 0x9E3779B97F4A7C15ULL;
-    h ^= h >> 29;
-  }
-  h *= 0xD6E8FEB86659FD93ULL;
-  return h ^ (h >> 32);
-}
-
-// Row at p (written by another CTA of the cluster in this phase) equals x.
-template <int W>
-__device__ __forceinline__ bool row_eq_volatile(const u64* p, const u64* x) {
-  bool e = true;
-#pragma unroll
-  for (int w = 0; w < W; ++w) e = e && ld_volatile64(p + w) == x[w];
-  return e;
-}
-
-// 32 x 32 bit transpose across a warp: bit l of lane i's result is bit i of
-// lane l's value (five exchange stages, each swapping the off-diagonal halves).
-__device__ __forceinline__ u32 transpose32(u32 v) {
-  const u32 lane = threadIdx.x & 31u;
-  const u32 low[5] = {0x0000ffffu, 0x00ff00ffu, 0x0f0f0f0fu, 0x33333333u, 0x55555555u};
-#pragma unroll
-  for (int i = 0; i < 5; ++i) {
-    const u32 s = 16u >> i;
-    const u32 o = __shfl_xor_sync(0xffffffffu, v, s);
-    v = (lane & s) ? (v & ~low[i]) | ((o >> s) & low[i]) : (v & low[i]) | ((o & low[i]) << s);
-  }
-  return v;
 }
 
 // A table slot: the search's tag (26 bits), a fingerprint of the row (16), its
@@ -417,7 +379,7 @@ __global__ void __launch_bounds__(kCtThreads, 1)
         // a warp takes 32 parents under one letter as columns (a word per
         // state, a bit per parent): a child's column is a gather of the
         // parents', and two bit transposes lead in and out; about 12
-        // instructions a child instead of 100 by ballots
+        // instructions a child instead of 100 by ballots (rowset.cuh)
         u32* const col = s_col + warp * 64 * W;
         const u32 groups = (m + 31) / 32;
         for (u32 u = gwarp; u < groups * k; u += NW) {
@@ -427,31 +389,12 @@ __global__ void __launch_bounds__(kCtThreads, 1)
           u64 x[W];
 #pragma unroll
           for (int w = 0; w < W; ++w) x[w] = valid ? row[w] : 0ULL;
-#pragma unroll
-          for (int w = 0; w < W; ++w) {  // lane i gets the column of bit i: state 31 - i of the half
-            col[64 * w + 31 - lane] = transpose32((u32)(x[w] >> 32));
-            col[64 * w + 63 - lane] = transpose32((u32)x[w]);
-          }
+          rows_to_columns<W>(x, col);
           __syncwarp();
-#pragma unroll
-          for (int w = 0; w < W; ++w) {
-            u32 half[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const u32 s = 64 * w + 32 * h + lane;
-              u32 v = 0;
-              if (s < n) {
-                if (X == 1) {
-                  v = col[s_delta[s * k + a]];
-                } else {
-                  const u32 b0 = s_ibeg[a * (n + 1) + s], b1 = s_ibeg[a * (n + 1) + s + 1];
-                  for (u32 j = b0; j < b1; ++j) v |= col[s_isrc[j]];
-                }
-              }
-              half[h] = __brev(transpose32(v));
-            }
-            x[w] = ((u64)half[0] << 32) | half[1];
-          }
+          if (X == 1)
+            expand_columns<W, false>(col, n, s_delta + a, k, s_ibeg, s_isrc, x);
+          else
+            expand_columns<W, true>(col, n, s_delta, 0u, s_ibeg + a * (n + 1), s_isrc, x);
           __syncwarp();
           insert(x, valid, a * m + p);
         }

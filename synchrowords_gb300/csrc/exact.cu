@@ -47,6 +47,15 @@ struct Side {
   u32 count = 0;
   DevBuf vis, vis_alt;
   u32 vis_count = 0;
+  // While only duplicates are removed (Engine::step_hashed) the visited list is
+  // appended to layer by layer and a hash table names its rows; the current
+  // layer is then its tail (in_vis), else it is `rows`.  The reductions need the
+  // visited list in key order: the first of them ends this (Engine::unhash).
+  bool hashed = false, reduced = false, in_vis = false;
+  u32 cur_off = 0;  // first row of the current layer in vis
+  DevBuf table;
+  u64 table_slots = 0;  // 0: to be built from vis
+  const u64* cur_rows(int W) const { return in_vis ? vis.as<u64>() + (size_t)cur_off * W : rows.as<u64>(); }
   std::vector<std::unique_ptr<Layer>> layers;
   std::vector<u64> seed_states;  // backward side: the state of each seed row
   double unique_growth = 0;      // distinct children per parent at the last step
@@ -74,6 +83,8 @@ struct Side {
   }
   void reset() {
     count = vis_count = 0;
+    hashed = reduced = in_vis = false;
+    table_slots = 0;
     unique_growth = 0;
     keymap = KeyMap{};
     keymap_chosen = false;
@@ -195,9 +206,10 @@ class Engine {
   static constexpr int kScanErrWord = 4;  // read back with the witness, never cleared by it
   // Throws if a launch reported a bounded wait that ran out: 1 = a subset
   // check's tile copy never arrived, 2 = a compaction tile's look-back never
-  // saw its predecessor; `w` is the pinned copy of d_misc[kScanErrWord].
+  // saw its predecessor, 3 = a hash table's probe found no slot; `w` is the pinned copy of d_misc[kScanErrWord].
   static void check_scan_error(u32 w) {
     if (w == 2) throw CudaError("layer compaction: a look-back wait ran out");
+    if (w == 3) throw CudaError("duplicate removal: a hash table ran out of slots");
     if (w) throw CudaError("subset check: a tile copy did not complete within its wait limit");
   }
   // Single-pass duplicate removal (launch_dedup_compact): its tile status
@@ -369,11 +381,112 @@ class Engine {
   bool self_check = true;
   bool visited_subsets = true;
 
+  // ---- duplicate removal by hash table ----
+  DevBuf bk_counts, bk_first, bk_place, level_table;
+  BucketScratch buckets(u64 children) {
+    const size_t bytes = sizeof(u32) << kBucketBitsLarge;
+    if (bk_counts.cap < bytes) {
+      bk_counts.reserve(bytes);
+      SW_CUDA(cudaMemsetAsync(bk_counts.p, 0, bk_counts.cap, stream));
+    }
+    bk_first.reserve(bytes);
+    bk_place.reserve(sizeof(uint2) * children);
+    return BucketScratch{bucket_bits(children), bk_counts.as<u32>(), bk_first.as<u32>(), bk_place.as<uint2>()};
+  }
+  // Power-of-two slots, two to four per row.
+  static u64 slots_for(u64 rows) {
+    u64 s = 1024;
+    while (s < 2 * rows) s *= 2;
+    return s;
+  }
+  // Room for `rows` more rows at the end of X's visited list; returns the row
+  // index they start at (even where rows are an odd number of words, so that
+  // the layer stays 16-byte aligned for the subset check's tile copies; the row
+  // before it then repeats row 0, which is visited anyway).
+  u32 append_base(Side& X, int W, u64 rows) {
+    const u32 base = X.vis_count + ((W & 1) ? (X.vis_count & 1u) : 0u);
+    const size_t need = sizeof(u64) * W * (base + rows);
+    if (X.vis.cap < need) {
+      X.vis_alt.reserve(std::max(need, 2 * X.vis.cap));
+      SW_CUDA(cudaMemcpyAsync(X.vis_alt.p, X.vis.p, sizeof(u64) * W * (size_t)X.vis_count, cudaMemcpyDeviceToDevice,
+                              stream));
+      std::swap(X.vis.p, X.vis_alt.p);
+      std::swap(X.vis.cap, X.vis_alt.cap);
+    }
+    if (base != X.vis_count)
+      SW_CUDA(cudaMemcpyAsync(X.vis.as<u64>() + (size_t)X.vis_count * W, X.vis.p, sizeof(u64) * W,
+                              cudaMemcpyDeviceToDevice, stream));
+    return base;
+  }
+  void step_hashed(Side& X, bool forward, int W, int k) {
+    const u32 m = X.count, Nc = m * (u32)k;
+    const double t_step0 = vclock();
+    X.hashed = true;
+    const u32 base = append_base(X, W, Nc);
+    if (2 * X.table_slots < 3 * ((u64)base + Nc)) {  // fewer than 1.5 slots a row: rebuild
+      X.table_slots = slots_for((u64)base + Nc);
+      X.table.reserve(sizeof(u64) * X.table_slots);
+      SW_CUDA(cudaMemsetAsync(X.table.p, 0, sizeof(u64) * X.table_slots, stream));
+      timed(3, (double)base * (8.0 * W + 8), [&] {
+        launch_hash_build(W, X.vis.as<u64>(), base, X.table.as<u64>(), (u32)(X.table_slots - 1), d_misc + kScanErrWord,
+                          stream);
+      });
+      count_launch();
+    }
+    ch_rows.reserve(sizeof(u64) * W * (size_t)Nc);
+    const BucketScratch bk = buckets(Nc);
+    // reads each parent row, writes k child rows, a table slot and a place each
+    timed(1, (double)m * 8.0 * W * (1 + k) + (double)Nc * 16.0, [&] {
+      launch_expand_hash(W, forward, X.cur_rows(W), m, tables, ch_rows.as<u64>(), X.vis.as<u64>(), base,
+                         X.table.as<u64>(), (u32)(X.table_slots - 1), bk, d_misc + kScanErrWord, stream);
+    });
+    std::unique_ptr<Layer> L = X.new_layer(sizeof(u32) * (size_t)std::max<u32>(Nc, 1));
+    L->origin.reserve(sizeof(u32) * (size_t)std::max<u32>(Nc, 1));
+    timed(3, (double)Nc * (2 * 8.0 * W + 8 + 4), [&] {
+      launch_bucket_scatter(W, ch_rows.as<u64>(), Nc, bk, base, X.vis.as<u64>() + (size_t)base * W,
+                            L->origin.as<u32>(), X.table.as<u64>(), d_misc + 8, stream);
+    });
+    count_launch(3);
+    const u32 f = read_total_checked();
+    if (m) X.unique_growth = (double)f / m;
+    if (st) {
+      st->subsets_expanded += Nc;
+      st->subsets_kept += f;
+    }
+    L->count = f;
+    L->parent_count = m;
+    X.layers.push_back(std::move(L));
+    X.in_vis = true;
+    X.cur_off = base;
+    X.count = f;
+    X.vis_count = base + f;
+    if (verbose)
+      std::fprintf(stderr, "[sw] %s parents=%u children=%u kept=%u (duplicates only) | %.3f ms\n",
+                   forward ? "BFS " : "IBFS", m, Nc, f, vclock() - t_step0);
+  }
+  // Back to a current layer of its own and a visited list in key order.
+  void unhash(Side& X, int W) {
+    if (!X.hashed) return;
+    if (X.in_vis) {
+      X.rows.reserve(sizeof(u64) * W * (size_t)std::max<u32>(X.count, 1));
+      SW_CUDA(cudaMemcpyAsync(X.rows.p, X.cur_rows(W), sizeof(u64) * W * (size_t)X.count, cudaMemcpyDeviceToDevice,
+                              stream));
+    }
+    X.hashed = X.in_vis = false;
+    X.table_slots = 0;
+    sort_by_layer_key(W, X.vis.as<u64>(), X.vis_count, X.keymap);
+  }
+
   void step(Side& X, bool forward, int W, int n, int k, bool dominance = true) {
     const u32 m = X.count;
     const u64 N = (u64)m * k;
     if (N > 0xffffffffULL) throw std::runtime_error("layer exceeds 2^32 children");
     const u32 Nc = (u32)N;
+    if (dominance && !self_check && !visited_subsets && !X.reduced && !sort_key_option() &&
+        2 * ((u64)X.vis_count + N + 1) <= 1ull << 32)
+      return step_hashed(X, forward, W, k);
+    unhash(X, W);
+    X.reduced = true;
     ch_rows.reserve(sizeof(u64) * W * N);
     ch_vals.reserve(sizeof(u32) * N);
     uq_rows.reserve(sizeof(u64) * W * N);
@@ -525,14 +638,18 @@ class Engine {
   // sort key with 64 chosen states of its current layer (for the backward
   // side, states of the complements) and re-sort its visited list.
   DevBuf d_counts;
+  static const char* sort_key_option() {
+    static const char* opt = std::getenv("SW_SORT_KEY");
+    return opt && (std::string(opt) == "frequent" || std::string(opt) == "balanced") ? opt : nullptr;
+  }
   void choose_keymap(Side& X, int W, int n) {
     X.keymap_chosen = true;
     if (n <= 64) return;  // the identity map already covers every state
     // Measured on random binary DFAs (n = 200 and 320), re-keying made the
     // subset checks slower than the identity key, so it is opt-in:
     // SW_SORT_KEY=frequent or SW_SORT_KEY=balanced.
-    static const char* opt = std::getenv("SW_SORT_KEY");
-    if (!opt || (std::string(opt) != "frequent" && std::string(opt) != "balanced")) return;
+    const char* opt = sort_key_option();
+    if (!opt) return;
     d_counts.reserve(sizeof(u32) * 64 * W);
     SW_CUDA(cudaMemsetAsync(d_counts.p, 0, sizeof(u32) * 64 * W, stream));
     launch_state_counts(W, X.rows.as<u64>(), X.count, d_counts.as<u32>(), stream);
@@ -566,24 +683,26 @@ class Engine {
     const u64 N = (u64)m * k;
     if (N > 0xffffffffULL) throw std::runtime_error("level exceeds 2^32 children");
     const u32 Nc = (u32)N;
+    const u64 slots = slots_for(N);
+    if (slots > 1ull << 32) throw std::runtime_error("level exceeds 2^31 children");
     ch_rows.reserve(sizeof(u64) * W * N);
-    ch_vals.reserve(sizeof(u32) * N);
-    flags_a.reserve(sizeof(u32) * N);
-    keys.reserve(sizeof(u64) * 2 * N);
-    sorted_rows.reserve(sizeof(u64) * W * N);
+    level_table.reserve(sizeof(u64) * slots);
     out_rows.reserve(sizeof(u64) * W * std::max<u64>(N, 1));
     out_origin.reserve(sizeof(u32) * std::max<u64>(N, 1));
+    const BucketScratch bk = buckets(N);
     const double t0 = vclock();
-    timed(1, (double)m * 8.0 * W * (1 + k), [&] { launch_expand(W, false, parents, m, tables, ch_rows.as<u64>(), stream); });
-    launch_iota(ch_vals.as<u32>(), Nc, stream);
-    launch_layer_keys(W, ch_rows.as<u64>(), Nc, keys.as<u64>(), stream);
-    sort_rows(2, keys.as<u64>(), ch_vals.as<u32>(), Nc);
-    launch_gather_rows(W, ch_rows.as<u64>(), ch_vals.as<u32>(), Nc, sorted_rows.as<u64>(), stream);
-    launch_unique_flags(W, sorted_rows.as<u64>(), Nc, flags_a.as<u32>(), stream);
-    count_launch(5);
+    SW_CUDA(cudaMemsetAsync(level_table.p, 0, sizeof(u64) * slots, stream));
+    timed(1, (double)m * 8.0 * W * (1 + k) + (double)N * 16.0, [&] {
+      launch_expand_hash(W, false, parents, m, tables, ch_rows.as<u64>(), nullptr, 0, level_table.as<u64>(),
+                         (u32)(slots - 1), bk, d_misc + kScanErrWord, stream);
+    });
+    timed(3, (double)N * (2 * 8.0 * W + 8 + 4), [&] {
+      launch_bucket_scatter(W, ch_rows.as<u64>(), Nc, bk, 0, out_rows.as<u64>(), out_origin.as<u32>(), nullptr,
+                            d_misc + 8, stream);
+    });
+    count_launch(3);
     if (st) st->subsets_expanded += N;
-    out_count = compact(W, sorted_rows.as<u64>(), ch_vals.as<u32>(), flags_a.as<u32>(), Nc, out_rows.as<u64>(),
-                        out_origin.as<u32>());
+    out_count = read_total_checked();
     if (verbose)
       std::fprintf(stderr, "[sw] IBFS (bounded) parents=%u children=%u unique=%u | %.3f ms\n", m, Nc, out_count,
                    vclock() - t0);
@@ -593,7 +712,7 @@ class Engine {
   // query index and the F index.
   bool meet(int W, int n, const u64* Q, u32 q, u32* qi, u32* si) {
     SW_CUDA(cudaMemsetAsync(d_misc, 0, 4 * sizeof(u32), stream));
-    query(W, kQueryDisjoint, F.rows.as<u64>(), F.count, Q, q, n, nullptr, true);
+    query(W, kQueryDisjoint, F.cur_rows(W), F.count, Q, q, n, nullptr, true);
     if (st) st->meet_pairs += (u64)F.count * q;
     SW_CUDA(cudaMemcpyAsync(pinned.p, d_misc, 5 * sizeof(u32), cudaMemcpyDeviceToHost, stream));  // witness + error
     SW_CUDA(cudaStreamSynchronize(stream));
@@ -702,31 +821,35 @@ class Engine {
     for (int side = 0; side < 2; ++side) {
       Side& X = side ? B : F;
       const u32 kept = ex.kept[side], cnt = ex.cnt[side], depth = ex.depth[side];
-      X.vis.reserve(sizeof(u64) * W * kept);
+      ch_rows.reserve(sizeof(u64) * W * kept);
       single_org[side].reserve(sizeof(u32) * kept);
-      launch_cluster_export(W, single_scratch.p, kClusterSingleHeader, caps, side, kept, depth, X.vis.as<u64>(),
+      launch_cluster_export(W, single_scratch.p, kClusterSingleHeader, caps, side, kept, depth, ch_rows.as<u64>(),
                             single_org[side].as<u32>(), stream);
-      // the current layer in key order, its origins with it
-      X.rows.reserve(sizeof(u64) * W * cnt);
-      X.count = cnt;
-      X.vis_count = kept;
-      const u64* cur = X.vis.as<u64>() + (size_t)(kept - cnt) * W;
-      keys.reserve(sizeof(u64) * 2 * cnt);
+      // the visited list: the earlier layers as they are, then the current one in bucket order
+      X.vis_count = kept - cnt;
+      X.vis.reserve(sizeof(u64) * W * ((size_t)kept + 1));
+      SW_CUDA(cudaMemcpyAsync(X.vis.p, ch_rows.p, sizeof(u64) * W * std::max<u32>(X.vis_count, 1),
+                              cudaMemcpyDeviceToDevice, stream));
+      const u32 base = append_base(X, W, cnt);
+      const u64* cur = ch_rows.as<u64>() + (size_t)(kept - cnt) * W;
+      const BucketScratch bk = buckets(cnt);
       ch_vals.reserve(sizeof(u32) * cnt);
-      launch_layer_keys(W, cur, cnt, keys.as<u64>(), stream, X.keymap);
-      launch_iota(ch_vals.as<u32>(), cnt, stream);
-      sort_rows(2, keys.as<u64>(), ch_vals.as<u32>(), cnt);
-      launch_gather_rows(W, cur, ch_vals.as<u32>(), cnt, X.rows.as<u64>(), stream);
+      launch_bucket_rank(W, cur, cnt, bk, stream);
+      launch_bucket_scatter(W, cur, cnt, bk, base, X.vis.as<u64>() + (size_t)base * W, ch_vals.as<u32>(), nullptr,
+                            d_misc + 8, stream);
       count_launch(4);
+      X.hashed = X.in_vis = true;
+      X.cur_off = base;
+      X.count = cnt;
+      X.vis_count = base + cnt;
       std::unique_ptr<Layer> top;
-      if (depth) {
+      if (depth) {  // the current layer's origins in the order of its rows
         top = X.new_layer(sizeof(u32) * cnt);
         top->origin.reserve(sizeof(u32) * cnt);
         launch_gather_u32(single_org[side].as<u32>() + (kept - cnt), ch_vals.as<u32>(), cnt, top->origin.as<u32>(),
                           stream);
         count_launch();
       }
-      sort_by_layer_key(W, X.vis.as<u64>(), kept, X.keymap);
       if (side == 0) SW_CUDA(cudaStreamSynchronize(stream));  // the layer table has arrived
       const u32* loff = meta + (2 + side) * kClusterMetaStride;
       const u32* lcnt = meta + (4 + side) * kClusterMetaStride;
@@ -773,7 +896,7 @@ struct BoundedSearch {
   }
 
   const u64* level_rows(size_t li) const {
-    return li == 0 ? E.B.rows.as<u64>() : levels[li]->rows.as<u64>();
+    return li == 0 ? E.B.cur_rows(W) : levels[li]->rows.as<u64>();
   }
 
   // Letters from level `li` index x back to the B frontier, plus the MITM B trace.
@@ -911,7 +1034,7 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
   // (the other reductions and reduced forward seeds are the streamed path's).
   bool imported = false;
   ClusterExit single_exit{};
-  if (!red && !b.has_word && cfg.reductions != SW_REDUCE_ALWAYS && n <= 256 && n * k <= 4096 && !seeds.empty() &&
+  if (!red && !b.has_word && cfg.reductions != SW_REDUCE_ALWAYS && !Engine::sort_key_option() && n <= 256 && n * k <= 4096 && !seeds.empty() &&
       max_rt > 0) {
     const Engine::Single S = E.run_single(A, seeds, (u32)std::min<u64>(max_rt, kClusterSingleWord), budget);
     if (E.verbose)
@@ -1045,8 +1168,7 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
     if (time_meet) SW_CUDA(cudaStreamSynchronize(E.stream));
     const auto t_meet_host0 = std::chrono::steady_clock::now();
     SW_CUDA(cudaMemsetAsync(E.d_misc, 0, 4 * sizeof(u32), E.stream));
-    E.query(W, kQueryDisjoint, E.F.rows.as<u64>(), E.F.count, E.B.rows.as<u64>(), E.B.count,
-            n, nullptr, true);
+    E.query(W, kQueryDisjoint, E.F.cur_rows(W), E.F.count, E.B.cur_rows(W), E.B.count, n, nullptr, true);
     st.meet_pairs += (u64)E.F.count * E.B.count;
     SW_CUDA(cudaMemcpyAsync(E.pinned.p, E.d_misc, 5 * sizeof(u32), cudaMemcpyDeviceToHost, E.stream));  // witness + error
     SW_CUDA(cudaStreamSynchronize(E.stream));

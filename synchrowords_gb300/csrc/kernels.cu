@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "kernels.cuh"
+#include "rowset.cuh"
 
 namespace sw {
 
@@ -132,114 +133,6 @@ __device__ __forceinline__ void layer_key(const u64* r, const KeyMap& map, u64& 
   }
   k0 = a;
   k1 = row_mix<W>(r, 0);
-}
-
-// ===========================================================================
-// Layer expansion.  One warp per input set.  The set row is staged in shared
-// memory; lane l decides output states l, l+32, ... by a gather:
-//   preimage  out[p] = S[delta_a(p)]                  (delta in smem)
-//   image     out[t] = OR_{q : delta_a(q) = t} S[q]   (preimage CSR in smem)
-// and each 32-state round becomes half an output word through __ballot_sync
-// (bit-reversed into the MSB-first layout).  Both directions are
-// gathers, so no atomics are needed.
-// ===========================================================================
-template <int W, bool kImage>
-__global__ void __launch_bounds__(256) k_expand(const u64* __restrict__ in, u32 m, TransTables t,
-                                                u64* __restrict__ out, u64* __restrict__ keys,
-                                                u32* __restrict__ vals, KeyMap map) {
-  extern __shared__ uint16_t s_tab[];
-  __shared__ u64 s_row[8][W];
-  __shared__ u64 s_out[8][W];
-  const int n = t.n, k = t.k;
-  uint16_t* s_a = s_tab;                  // delta (preimage) or inv_beg (image)
-  uint16_t* s_b = s_tab + k * (n + 1);    // inv_src (image)
-  if (kImage) {
-    for (int i = threadIdx.x; i < k * (n + 1); i += blockDim.x) s_a[i] = t.inv_beg[i];
-    for (int i = threadIdx.x; i < k * n; i += blockDim.x) s_b[i] = t.inv_src[i];
-  } else {
-    for (int i = threadIdx.x; i < k * n; i += blockDim.x) s_a[i] = t.delta[i];
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const u32 stride = gridDim.x * 8u;
-  const int rounds = (n + 31) >> 5;
-  for (u32 i = blockIdx.x * 8u + warp; i < m; i += stride) {
-    if (lane < W) s_row[warp][lane] = in[(size_t)i * W + lane];
-    __syncwarp();
-    for (int a = 0; a < k; ++a) {
-      u64 word = 0;
-      for (int r = 0; r < rounds; ++r) {
-        const int q = r * 32 + lane;
-        bool bit = false;
-        if (q < n) {
-          if (kImage) {
-            const int b = s_a[a * (n + 1) + q], e = s_a[a * (n + 1) + q + 1];
-            for (int j = b; j < e; ++j) {
-              const int p = s_b[a * n + j];
-              if ((s_row[warp][p >> 6] >> (63 - (p & 63))) & 1ULL) {
-                bit = true;
-                break;
-              }
-            }
-          } else {
-            const int p = s_a[a * n + q];
-            bit = (s_row[warp][p >> 6] >> (63 - (p & 63))) & 1ULL;
-          }
-        }
-        const u32 bal = __ballot_sync(kFull, bit);
-        if (lane == (r >> 1)) {
-          const u64 v = (u64)__brev(bal);
-          word |= (r & 1) ? v : (v << 32);
-        }
-      }
-      const size_t o = (size_t)a * m + i;
-      if (lane < W) out[o * W + lane] = word;
-      if (keys) {  // the child's layer key and its index as the sort payload
-        if (lane < W) s_out[warp][lane] = word;
-        __syncwarp();
-        if (lane == 0) {
-          u64 k0, k1;
-          layer_key<W>(s_out[warp], map, k0, k1);
-          keys[2 * o] = k0;
-          keys[2 * o + 1] = k1;
-          vals[o] = (u32)o;
-        }
-        __syncwarp();
-      }
-    }
-    __syncwarp();
-  }
-}
-
-void launch_expand(int W, bool image, const u64* in, u32 m, const TransTables& t, u64* out, cudaStream_t s,
-                   u64* keys, u32* vals, const KeyMap& map) {
-  if (m == 0) return;
-  size_t smem = image ? sizeof(uint16_t) * (size_t)t.k * (2 * t.n + 1) : sizeof(uint16_t) * (size_t)t.k * t.n;
-  u32 blocks = std::min<u32>((m + 7) / 8, (u32)sm_count() * 8);
-#define SW_EXP(WW)                                                                                  \
-  case WW:                                                                                          \
-    if (image) {                                                                                    \
-      if (smem > 48 * 1024) ensure_smem_limit((const void*)k_expand<WW, true>, (int)smem);         \
-      k_expand<WW, true><<<blocks, 256, smem, s>>>(in, m, t, out, keys, vals, map);                 \
-    } else {                                                                                        \
-      if (smem > 48 * 1024) ensure_smem_limit((const void*)k_expand<WW, false>, (int)smem);        \
-      k_expand<WW, false><<<blocks, 256, smem, s>>>(in, m, t, out, keys, vals, map);                \
-    }                                                                                               \
-    break;
-  switch (W) {
-    SW_EXP(1)
-    SW_EXP(2)
-    SW_EXP(3)
-    SW_EXP(4)
-    SW_EXP(5)
-    SW_EXP(6)
-    SW_EXP(7)
-    SW_EXP(8)
-    default:
-      throw std::runtime_error("expand: unsupported width");
-  }
-#undef SW_EXP
-  SW_LAUNCH_CHECK();
 }
 
 // ===========================================================================
@@ -378,6 +271,308 @@ void launch_scan(const u32* in, u32* out, u32 n, u32* total_dev, void* temp, cud
   k_scan_reduce<<<nb, kScanThreads, 0, s>>>(in, n, partial);
   k_scan_partials<<<1, kScanThreads, 0, s>>>(partial, nb, total_dev);
   k_scan_final<<<nb, kScanThreads, 0, s>>>(in, out, n, partial);
+  SW_LAUNCH_CHECK();
+}
+
+// ===========================================================================
+// Layer expansion.  A warp takes 32 parent rows under one letter, turns them
+// into columns (a word per state, a bit per parent: shared memory), gathers the
+// children's columns
+//   preimage  child[p] = parent[delta_a(p)]
+//   image     child[t] = OR_{q : delta_a(q) = t} parent[q]   (preimage CSR)
+// and turns those back into rows, one child per lane: two 32 x 32 bit
+// transposes and one gather per 32 states, about 12 instructions a child (a
+// warp per parent with a ballot per 32 states took 165).  Bound by the rows
+// written at large layers and by the latency of one warp's chain (a few
+// hundred instructions) at small ones.
+// ===========================================================================
+namespace {
+constexpr int kExpThreads = 128;
+constexpr int kExpWarps = kExpThreads / 32;
+
+// Per-letter tables staged in shared memory: delta (preimage), or list starts
+// and sources (image), as u16.
+template <bool kImage>
+__device__ __forceinline__ void stage_tables(const TransTables& t, uint16_t* s_tab) {
+  const int n = t.n, k = t.k;
+  if (kImage) {
+    for (int i = threadIdx.x; i < k * (n + 1); i += blockDim.x) s_tab[i] = t.inv_beg[i];
+    for (int i = threadIdx.x; i < k * n; i += blockDim.x) s_tab[k * (n + 1) + i] = t.inv_src[i];
+  } else {
+    for (int i = threadIdx.x; i < k * n; i += blockDim.x) s_tab[i] = t.delta[i];
+  }
+  __syncthreads();
+}
+
+// Lane's child of parent 32 g + lane under letter a, into x (garbage-free zero
+// rows for lanes past m).
+template <int W, bool kImage>
+__device__ __forceinline__ void expand_group(const u64* __restrict__ in, u32 m, const TransTables& t, u32 g, u32 a,
+                                             const uint16_t* s_tab, u32* col, u64* x) {
+  const u32 n = (u32)t.n, p = 32 * g + (threadIdx.x & 31u);
+#pragma unroll
+  for (int w = 0; w < W; ++w) x[w] = p < m ? in[(size_t)p * W + w] : 0ULL;
+  rows_to_columns<W>(x, col);
+  __syncwarp();
+  const uint16_t* const beg = s_tab + a * (n + 1);
+  const uint16_t* const src = s_tab + (u32)t.k * (n + 1) + a * n;
+  expand_columns<W, kImage>(col, n, s_tab + a * n, 1u, beg, src, x);
+  __syncwarp();
+}
+
+size_t expand_smem(bool image, const TransTables& t) {
+  return sizeof(uint16_t) * (size_t)t.k * (image ? 2 * t.n + 1 : t.n);
+}
+// Units are (32 parents, letter); four warps a block, so that small layers
+// spread over the SMs.
+u32 expand_blocks(u32 m, int k) {
+  const u64 units = (u64)((m + 31) / 32) * (u32)k;
+  return (u32)std::min<u64>((units + kExpWarps - 1) / kExpWarps, (u64)sm_count() * 12);
+}
+}  // namespace
+
+template <int W, bool kImage>
+__global__ void __launch_bounds__(kExpThreads) k_expand(const u64* __restrict__ in, u32 m, TransTables t,
+                                                        u64* __restrict__ out, u64* __restrict__ keys,
+                                                        u32* __restrict__ vals, KeyMap map) {
+  extern __shared__ uint16_t s_tab[];
+  __shared__ u32 s_cols[kExpWarps][64 * W];
+  stage_tables<kImage>(t, s_tab);
+  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const u32 groups = (m + 31) / 32, units = groups * (u32)t.k;
+  for (u32 u = blockIdx.x * kExpWarps + warp; u < units; u += gridDim.x * kExpWarps) {
+    const u32 a = u / groups, g = u - a * groups, p = 32 * g + lane;
+    u64 x[W];
+    expand_group<W, kImage>(in, m, t, g, a, s_tab, s_cols[warp], x);
+    if (p < m) {
+      const size_t o = (size_t)a * m + p;
+#pragma unroll
+      for (int w = 0; w < W; ++w) out[o * W + w] = x[w];
+      if (keys) {  // the child's layer key and its index as the sort payload
+        u64 k0, k1;
+        layer_key<W>(x, map, k0, k1);
+        keys[2 * o] = k0;
+        keys[2 * o + 1] = k1;
+        vals[o] = (u32)o;
+      }
+    }
+  }
+}
+
+#define SW_EXP_DISPATCH(LAUNCH)                                    \
+  switch (W) {                                                     \
+    case 1: { constexpr int WW = 1; LAUNCH; } break;               \
+    case 2: { constexpr int WW = 2; LAUNCH; } break;               \
+    case 3: { constexpr int WW = 3; LAUNCH; } break;               \
+    case 4: { constexpr int WW = 4; LAUNCH; } break;               \
+    case 5: { constexpr int WW = 5; LAUNCH; } break;               \
+    case 6: { constexpr int WW = 6; LAUNCH; } break;               \
+    case 7: { constexpr int WW = 7; LAUNCH; } break;               \
+    case 8: { constexpr int WW = 8; LAUNCH; } break;               \
+    default: throw std::runtime_error("expand: unsupported width"); \
+  }
+
+void launch_expand(int W, bool image, const u64* in, u32 m, const TransTables& t, u64* out, cudaStream_t s,
+                   u64* keys, u32* vals, const KeyMap& map) {
+  if (m == 0) return;
+  const size_t smem = expand_smem(image, t);
+  const u32 blocks = expand_blocks(m, t.k);
+#define SW_EXP(IMG)                                                                                  \
+  {                                                                                                  \
+    if (smem > 32 * 1024) ensure_smem_limit((const void*)k_expand<WW, IMG>, (int)smem);              \
+    k_expand<WW, IMG><<<blocks, kExpThreads, smem, s>>>(in, m, t, out, keys, vals, map);             \
+  }
+  SW_EXP_DISPATCH(if (image) SW_EXP(true) else SW_EXP(false))
+#undef SW_EXP
+  SW_LAUNCH_CHECK();
+}
+
+// ===========================================================================
+// Expansion with duplicate removal by an open-addressing hash table, and the
+// bucket order of what is kept.  Three launches a layer instead of a sort (a
+// chunk sort and a merge pass per doubling), a duplicate scan with a binary
+// search per child and a merge of the visited list:
+//   k_expand_hash   expands a layer (as k_expand), stores each child, inserts it
+//                   in the table (a slot names an earlier row or a child of this
+//                   launch with the same fingerprint, whose row decides) and
+//                   counts what it keeps per bucket: the leading bits of word 0;
+//   k_bucket_scan   first row of every bucket, and the number kept;
+//   k_bucket_scatter  moves the kept rows to their buckets, with their origins,
+//                   and points their slots there.
+// Rows of one bucket share their leading states, which is all the subset
+// check's tile masks and query groups need: counted on layers of 40 000 to
+// 100 000 sets (n = 100, 200, 300), 12 leading bits cost its tiles 1 to 15%
+// more work than the full key order, 16 bits 0 to 3%.  Bound by the table's random
+// accesses (two 8-byte sectors and a row per child) and, below some 10 000
+// children, by the latency of the three launches.
+// ===========================================================================
+namespace {
+// Slot: bit 63 set, 31 bits of the hash, row index (a row of V below `base`,
+// else child index - base of this launch).
+template <int W>
+__device__ __forceinline__ bool hash_insert(u64* tab, u32 tmask, const u64* V, u32 base, const u64* C, const u64* x,
+                                            u32 idx, u32* at, u32* err) {
+  const u64 h = row_hash<W>(x);
+  const u64 mine = (h & 0xffffffff00000000ULL) | (1ULL << 63) | idx;
+  u32 s = (u32)h & tmask;
+  for (u32 it = 0; it < tmask; ++it) {
+    u64 v = ld_volatile64(&tab[s]);
+    if (v == 0) {
+      v = atomicCAS(&tab[s], 0ULL, mine);
+      if (v == 0) {
+        *at = s;
+        return true;
+      }
+    }
+    if ((v ^ mine) >> 32 == 0) {
+      __threadfence();  // the row was written before its slot
+      const u32 r = (u32)v;
+      if (row_eq_volatile<W>(r >= base ? C + (size_t)(r - base) * W : V + (size_t)r * W, x)) return false;
+    }
+    s = (s + 1) & tmask;
+  }
+  atomicExch(err, 3u);
+  return false;
+}
+constexpr u32 kDropped = 0xffffffffu;
+
+// The lane's rank in its bucket, one atomic per bucket a warp meets: most
+// backward rows share a few buckets.  Every lane of the warp calls it.
+__device__ __forceinline__ u32 bucket_rank(u32* counts, u32 bucket, bool keep) {
+  const u32 kept = __ballot_sync(kFull, keep);
+  u32 r = kDropped;
+  if (keep) {
+    const u32 peers = __match_any_sync(kept, bucket);
+    const int leader = __ffs(peers) - 1;
+    u32 first = 0;
+    if ((threadIdx.x & 31) == (u32)leader) first = atomicAdd(&counts[bucket], (u32)__popc(peers));
+    r = __shfl_sync(peers, first, leader) + __popc(peers & lanemask_lt());
+  }
+  return r;
+}
+}  // namespace
+
+template <int W, bool kImage>
+__global__ void __launch_bounds__(kExpThreads) k_expand_hash(const u64* __restrict__ in, u32 m, TransTables t, u64* C,
+                                                             const u64* V, u32 base, u64* tab, u32 tmask,
+                                                             u32* __restrict__ counts, int shift,
+                                                             uint2* __restrict__ place, u32* err) {
+  extern __shared__ uint16_t s_tab[];
+  __shared__ u32 s_cols[kExpWarps][64 * W];
+  stage_tables<kImage>(t, s_tab);
+  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const u32 groups = (m + 31) / 32, units = groups * (u32)t.k;
+  for (u32 u = blockIdx.x * kExpWarps + warp; u < units; u += gridDim.x * kExpWarps) {
+    const u32 a = u / groups, g = u - a * groups, p = 32 * g + lane;
+    u64 x[W];
+    expand_group<W, kImage>(in, m, t, g, a, s_tab, s_cols[warp], x);
+    const u32 e = a * m + p;
+    if (p < m) {
+#pragma unroll
+      for (int w = 0; w < W; ++w) C[(size_t)e * W + w] = x[w];
+    }
+    __threadfence();  // the row before its slot
+    u32 at = 0;
+    const bool keep = p < m && hash_insert<W>(tab, tmask, V, base, C, x, base + e, &at, err);
+    const u32 rank = bucket_rank(counts, (u32)(x[0] >> shift), keep);
+    if (p < m) place[e] = make_uint2(rank, at);  // rank in its bucket (or dropped), table slot
+  }
+}
+
+// counts -> exclusive sums (first row of each bucket), counts cleared for the
+// next layer, *total = rows kept; one block, `bins` a multiple of 4096.
+__global__ void __launch_bounds__(kScanThreads) k_bucket_scan(u32* __restrict__ counts, u32* __restrict__ first,
+                                                              u32 bins, u32* total) {
+  u32 carry = 0;
+  for (u32 b0 = 0; b0 < bins; b0 += 4 * kScanThreads) {
+    const u32 i = b0 + 4 * threadIdx.x;
+    const uint4 c = *reinterpret_cast<const uint4*>(counts + i);
+    u32 tot;
+    const u32 ex = carry + block_exclusive_scan(c.x + c.y + c.z + c.w, tot);
+    *reinterpret_cast<uint4*>(first + i) = make_uint4(ex, ex + c.x, ex + c.x + c.y, ex + c.x + c.y + c.z);
+    *reinterpret_cast<uint4*>(counts + i) = make_uint4(0, 0, 0, 0);
+    carry += tot;
+  }
+  if (threadIdx.x == 0) *total = carry;
+}
+
+template <int W>
+__global__ void __launch_bounds__(256) k_bucket_scatter(const u64* __restrict__ C, u32 m, const uint2* __restrict__ place,
+                                                        const u32* __restrict__ first, int shift, u32 base,
+                                                        u64* __restrict__ out_rows, u32* __restrict__ out_vals,
+                                                        u32* __restrict__ tab_words) {
+  const u32 e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= m) return;
+  const uint2 pl = place[e];
+  if (pl.x == kDropped) return;
+  u64 x[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) x[w] = C[(size_t)e * W + w];
+  const u32 d = first[(u32)(x[0] >> shift)] + pl.x;
+#pragma unroll
+  for (int w = 0; w < W; ++w) out_rows[(size_t)d * W + w] = x[w];
+  out_vals[d] = e;
+  if (tab_words) tab_words[2 * (size_t)pl.y] = base + d;  // the slot's low half: the row index
+}
+
+// Bucket places of rows that are all kept.
+template <int W>
+__global__ void __launch_bounds__(256) k_bucket_rank(const u64* __restrict__ C, u32 m, u32* __restrict__ counts,
+                                                     int shift, uint2* __restrict__ place) {
+  const u32 e = blockIdx.x * blockDim.x + threadIdx.x;
+  const u32 bucket = e < m ? (u32)(C[(size_t)e * W] >> shift) : 0u;
+  const u32 rank = bucket_rank(counts, bucket, e < m);
+  if (e < m) place[e] = make_uint2(rank, 0u);
+}
+
+// Enters rows 0 .. m - 1 of V (equal rows once).
+template <int W>
+__global__ void __launch_bounds__(256) k_hash_build(const u64* __restrict__ V, u32 m, u64* tab, u32 tmask, u32* err) {
+  const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m) return;
+  u64 x[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) x[w] = V[(size_t)i * W + w];
+  u32 at;
+  hash_insert<W>(tab, tmask, V, ~0u, nullptr, x, i, &at, err);
+}
+
+void launch_expand_hash(int W, bool image, const u64* in, u32 m, const TransTables& t, u64* C, const u64* V, u32 base,
+                        u64* tab, u32 tmask, const BucketScratch& b, u32* err, cudaStream_t s) {
+  if (m == 0) return;
+  const size_t smem = expand_smem(image, t);
+  const u32 blocks = expand_blocks(m, t.k);
+#define SW_EXP(IMG)                                                                                          \
+  {                                                                                                          \
+    if (smem > 32 * 1024) ensure_smem_limit((const void*)k_expand_hash<WW, IMG>, (int)smem);                 \
+    k_expand_hash<WW, IMG><<<blocks, kExpThreads, smem, s>>>(in, m, t, C, V, base, tab, tmask, b.counts,     \
+                                                             64 - b.bits, b.place, err);                     \
+  }
+  SW_EXP_DISPATCH(if (image) SW_EXP(true) else SW_EXP(false))
+#undef SW_EXP
+  SW_LAUNCH_CHECK();
+}
+
+void launch_bucket_rank(int W, const u64* C, u32 m, const BucketScratch& b, cudaStream_t s) {
+  if (!m) return;
+  SW_EXP_DISPATCH((k_bucket_rank<WW><<<(m + 255) / 256, 256, 0, s>>>(C, m, b.counts, 64 - b.bits, b.place)))
+  SW_LAUNCH_CHECK();
+}
+
+void launch_bucket_scatter(int W, const u64* C, u32 m, const BucketScratch& b, u32 base, u64* out_rows, u32* out_vals,
+                           u64* tab, u32* total, cudaStream_t s) {
+  k_bucket_scan<<<1, kScanThreads, 0, s>>>(b.counts, b.first, 1u << b.bits, total);
+  SW_LAUNCH_CHECK();
+  if (!m) return;
+  SW_EXP_DISPATCH((k_bucket_scatter<WW><<<(m + 255) / 256, 256, 0, s>>>(C, m, b.place, b.first, 64 - b.bits, base,
+                                                                      out_rows, out_vals,
+                                                                      reinterpret_cast<u32*>(tab))))
+  SW_LAUNCH_CHECK();
+}
+
+void launch_hash_build(int W, const u64* V, u32 m, u64* tab, u32 tmask, u32* err, cudaStream_t s) {
+  if (!m) return;
+  SW_EXP_DISPATCH((k_hash_build<WW><<<(m + 255) / 256, 256, 0, s>>>(V, m, tab, tmask, err)))
   SW_LAUNCH_CHECK();
 }
 

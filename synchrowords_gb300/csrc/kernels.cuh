@@ -40,6 +40,34 @@ struct KeyMap {
 void launch_expand(int W, bool image, const u64* in, u32 m, const TransTables& t, u64* out, cudaStream_t s,
                    u64* keys = nullptr, u32* vals = nullptr, const KeyMap& map = KeyMap{});
 
+// Duplicate removal by hash table and bucket order (kernels.cu).  A layer is
+// expanded into C (child a*m + i) and what is new — no row of V[0, base) that
+// the table holds, no other child of this layer — is ranked within its bucket,
+// the leading `bits` bits of word 0; launch_bucket_scatter then moves the kept
+// rows to out_rows (bucket order), their child indices to out_vals, and points
+// their slots at rows base .. of V (tab given; V + base * W is then out_rows).
+// Table: tmask + 1 slots of u64, zero = empty, more slots than rows; *err is
+// set to 3 if a probe runs out.  counts: 2^bits words, zero before the first
+// launch (the scatter clears them); first: 2^bits words; place: one entry per
+// child.
+struct BucketScratch {
+  int bits = 12;
+  u32* counts = nullptr;
+  u32* first = nullptr;
+  uint2* place = nullptr;
+};
+// 12 leading bits below 2^16 children (one round of the bucket scan), 16 above.
+constexpr int kBucketBitsSmall = 12, kBucketBitsLarge = 16;
+inline int bucket_bits(u64 children) { return children < (1u << 16) ? kBucketBitsSmall : kBucketBitsLarge; }
+void launch_expand_hash(int W, bool image, const u64* in, u32 m, const TransTables& t, u64* C, const u64* V, u32 base,
+                        u64* tab, u32 tmask, const BucketScratch& b, u32* err, cudaStream_t s);
+// Ranks m rows that are all kept.
+void launch_bucket_rank(int W, const u64* C, u32 m, const BucketScratch& b, cudaStream_t s);
+void launch_bucket_scatter(int W, const u64* C, u32 m, const BucketScratch& b, u32 base, u64* out_rows, u32* out_vals,
+                           u64* tab, u32* total, cudaStream_t s);
+// Enters rows [0, m) of V in a zeroed table.
+void launch_hash_build(int W, const u64* V, u32 m, u64* tab, u32 tmask, u32* err, cudaStream_t s);
+
 // Scratch sizing for the sort / scan helpers.
 size_t scan_temp_bytes(u32 n);
 size_t sort_temp_bytes(int R, u32 m);

@@ -33,7 +33,9 @@ def test_same_lengths_without_the_cluster(ctx, n, k):
         d = random_dfa(n, k, 7000 + 31 * n + seed)
         r, s = ctx.solve(d, n, k, plan()), ctx.solve(d, n, k, plan(reductions="always"))
         assert (r.non_synchro, r.lower, r.upper) == (s.non_synchro, s.lower, s.upper)
-        if not r.non_synchro:
+        if n == 1:
+            assert r.upper == 0  # the plan's bound n^3 / 6 is zero: nothing is searched
+        elif not r.non_synchro and r.lower == r.upper:  # else both stopped at the plan's memory budget
             assert len(r.word) == r.upper and len(oracle.apply_word(d, n, k, r.word)) == 1
 
 
