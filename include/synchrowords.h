@@ -298,7 +298,7 @@ int sw_autotune_cluster(sw_context* ctx, uint32_t count, const uint32_t* deltas,
  * shape per row width (words = ceil(n / 64), 1..8) and list size class; the
  * shape changes speed only, never results. */
 typedef struct {
-  int32_t tile_rows;        /* rows of S per tile staged in shared memory: 32, 64 or 128 (default 64) */
+  int32_t tile_rows;        /* rows of S per tile mask: 32, 64 or 128 (default 64) */
   int32_t warps;            /* warps of 32 queries per block: 4, 8 or 16 (default 8) */
   int32_t tiles_per_super;  /* tiles per super-tile AND mask: 4, 8, 16 or 32 (default 16) */
   int32_t grid_factor;      /* target blocks per SM of the grid, 1..64 (default 16) */
@@ -447,13 +447,13 @@ int sw_mlp_train_ranked(sw_context* ctx, float* params, uint32_t automata, const
  * sw_subsets_check, but on device buffers the caller owns and with no
  * cudaMalloc / cudaFree / allocating library call: the scratch it needs (the
  * AND masks of the set list's row tiles) is a static device array of the
- * library, sized for SW_NOALLOC_MAX_SETS sets (about 1 MB; every GPU that
+ * library, sized for SW_NOALLOC_MAX_SETS sets (about 3.3 MB; every GPU that
  * loads the library keeps it until the process exits).  Larger set lists are
  * rejected with SW_ERR_CAPACITY.
  *
  * Rows use the device layout: W = ceil(n / 64) uint64 words (1 to 8); state
  * q is bit (63 - q % 64) of word q / 64; unused bits are 0.  d_sets must be
- * 16-byte aligned (its row tiles move as 16-byte loads), d_checks 8-byte and
+ * 16-byte aligned, d_checks 8-byte and
  * d_results 4-byte aligned; other pointers are rejected with
  * SW_ERR_INVALID_ARGUMENT before any work is queued.
  * d_results[i] (uint32) becomes 1 if some d_sets row ⊆ d_checks row i

@@ -202,15 +202,15 @@ class Engine {
     }
     prof_on = false;
   }
-  u32* d_misc = nullptr;  // [0..3] witness, [8] scan total, [kScanErrWord] bounded-wait timeouts
+  u32* d_misc = nullptr;  // [0..2] witness, [3] the subset check's size floor, [8] scan total, [9] the check's unit count, [kScanErrWord] bounded-wait timeouts
   static constexpr int kScanErrWord = 4;  // read back with the witness, never cleared by it
-  // Throws if a launch reported a bounded wait that ran out: 1 = a subset
-  // check's tile copy never arrived, 2 = a compaction tile's look-back never
-  // saw its predecessor, 3 = a hash table's probe found no slot; `w` is the pinned copy of d_misc[kScanErrWord].
+  // Throws if a launch reported a bounded wait that ran out: 2 = a compaction
+  // tile's look-back never saw its predecessor, 3 = a hash table's probe found
+  // no slot; `w` is the pinned copy of d_misc[kScanErrWord].
   static void check_scan_error(u32 w) {
     if (w == 2) throw CudaError("layer compaction: a look-back wait ran out");
     if (w == 3) throw CudaError("duplicate removal: a hash table ran out of slots");
-    if (w) throw CudaError("subset check: a tile copy did not complete within its wait limit");
+    if (w) throw CudaError("a launch reported error " + std::to_string(w));
   }
   // Single-pass duplicate removal (launch_dedup_compact): its tile status
   // words (zero-filled when allocated), tile counter and launch epoch.
@@ -321,7 +321,7 @@ class Engine {
 
   // Subset queries run on the tiled check (subset_check.cu), in the launch
   // shape the context holds for the row width and the list's size class.
-  DevBuf tile_and;
+  DevBuf tile_and, scan_items;
   ScanShapes scan_shapes;
   // while profiling: events around each check's mask build + scan, keyed by
   // (W - 1) * kScanSizeClasses + size class
@@ -333,16 +333,19 @@ class Engine {
     if (!m || !q) return;
     const ScanShape& sh = scan_shapes.pick(W, m);
     tile_and.reserve(subset_check_temp_bytes(W, m, sh));
+    scan_items.reserve(sizeof(uint2) * kSubsetItems);
     cudaEvent_t e0 = nullptr;
     if (prof_on) {
       e0 = next_event();
       SW_CUDA(cudaEventRecord(e0, stream));
     }
-    timed(3, (double)m * 8.0 * W, [&] { launch_tile_and(W, S, m, tile_and.as<u64>(), sh, stream); });
-    // algorithmic bytes: the query rows plus every S tile staged on chip
+    u32* const size_floor = d_misc + 3;  // zeroed with the witness in meet mode
+    if (!stop) SW_CUDA(cudaMemsetAsync(size_floor, 0, sizeof(u32), stream));
+    timed(3, (double)m * 8.0 * W, [&] { launch_tile_and(W, S, m, tile_and.as<u64>(), size_floor, sh, stream); });
+    // algorithmic bytes: the query rows plus every row of S a query is tested against
     timed(0, (double)q * 8.0 * W, [&] {
-      launch_subset_check(W, mode, S, m, tile_and.as<u64>(), Q, q, n, flags, d_misc, stop, sh, stream,
-                          prof_on ? d_query_bytes : nullptr, d_misc + kScanErrWord);
+      launch_subset_check(W, mode, S, m, tile_and.as<u64>(), size_floor, Q, q, n, flags, d_misc, stop, sh, stream,
+                          prof_on ? d_query_bytes : nullptr, scan_items.as<uint2>(), d_misc + 9);
     });
     if (prof_on) {
       cudaEvent_t e1 = next_event();
@@ -350,6 +353,35 @@ class Engine {
       scan_ev.push_back({(W - 1) * kScanSizeClasses + (m >= kScanLargeRows ? 1 : 0), {e0, e1}});
     }
     count_launch(2);
+    if (st) {
+      st->trie_queries += q;
+      st->logical_pairs += (u64)m * q;
+    }
+  }
+
+  // flags[i] = 1 where a row of S (a proper one) is inside child row i of Q, on
+  // the forward side or on complement rows; children `decided` already may be
+  // left out.
+  void dominated(bool forward, int W, const u64* S, u32 m, const u64* Q, u32 q, int n, bool proper, const u32* decided,
+                 u32* flags) {
+    if (!m || !q) return;
+    cudaEvent_t e0 = nullptr;
+    if (prof_on) {
+      e0 = next_event();
+      SW_CUDA(cudaEventRecord(e0, stream));
+    }
+    timed(0, (double)(m + q) * 8.0 * W, [&] {
+      if (forward)  // sets s ⊆ c: the children hold them
+        launch_dominance(W, false, true, Q, q, S, m, n, proper, decided, flags, stream);
+      else  // complements: the set of c lies in the set of s
+        launch_dominance(W, true, false, S, m, Q, q, n, proper, decided, flags, stream);
+    });
+    if (prof_on) {
+      cudaEvent_t e1 = next_event();
+      SW_CUDA(cudaEventRecord(e1, stream));
+      scan_ev.push_back({(W - 1) * kScanSizeClasses + (m >= kScanLargeRows ? 1 : 0), {e0, e1}});
+    }
+    count_launch();
     if (st) {
       st->trie_queries += q;
       st->logical_pairs += (u64)m * q;
@@ -566,7 +598,8 @@ class Engine {
     const double t_sort = vclock();
     if (X.vis_count) {
       if (visited_subsets) {
-        query(W, kQuerySubset, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, n, flags_a.as<u32>(), false);
+        dominated(forward, W, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, n, false, nullptr,
+                  flags_a.as<u32>());
       } else {
         timed(3, (double)u * 8.0 * W, [&] {
           launch_member_key(W, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, flags_a.as<u32>(), stream,
@@ -577,8 +610,8 @@ class Engine {
     }
     const double t_vis = vclock();
     if (self_check)
-      query(W, kQueryProperSubset, uq_rows.as<u64>(), u, uq_rows.as<u64>(), u, n,
-            flags_b.as<u32>(), false);
+      dominated(forward, W, uq_rows.as<u64>(), u, uq_rows.as<u64>(), u, n, true, flags_a.as<u32>(),
+                flags_b.as<u32>());
     const double t_self = vclock();
     if (verbose) {
       std::vector<u32> fa(u), fb(u);
@@ -1478,11 +1511,8 @@ void Solver::subsets_check(uint32_t n, const uint64_t* sets, uint64_t set_count,
   E.query(W, proper ? kQueryProperSubset : kQuerySubset, E.keys.as<u64>(), u,
           E.ch_rows.as<u64>(), q, (int)n, E.flags_b.as<u32>(), false);
   std::vector<u32> flags(q);
-  u32 scan_err = 0;
   SW_CUDA(cudaMemcpyAsync(flags.data(), E.flags_b.p, sizeof(u32) * q, cudaMemcpyDeviceToHost, E.stream));
-  SW_CUDA(cudaMemcpyAsync(&scan_err, E.d_misc + Engine::kScanErrWord, sizeof(u32), cudaMemcpyDeviceToHost, E.stream));
   SW_CUDA(cudaStreamSynchronize(E.stream));
-  Engine::check_scan_error(scan_err);
   for (u32 i = 0; i < q; ++i) results[i] = flags[i] ? 1 : 0;
 }
 

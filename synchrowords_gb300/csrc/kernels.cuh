@@ -100,14 +100,15 @@ enum QueryMode : int {
 // Tiled subset check (subset_check.cu): for each query row c, flags[c] |=
 // hit(c) (or, with `stop`, record one witness pair and let all warps exit
 // early: witness[0] = found flag, witness[1] = query index, witness[2] = set
-// index).  S is cut into tiles of sh.tile_rows rows; tile_and[t] (W words) =
-// AND of the tile's rows, then one mask per super-tile of
-// sh.tiles_per_super tiles, from launch_tile_and with the same shape.  `flags` must start zeroed (non-stop
-// mode).  `bytes_ctr` (optional) accumulates the bytes of S tiles staged on
-// chip.  S must start 16-byte aligned (its tiles move by bulk copies).  *err
-// is set to 1 when a wait for a tile copy runs out (its bounded poll limit);
-// the results of that launch are then incomplete.
-// Launch shape of the subset check: rows of S per staged tile (32, 64, 128),
+// index).  S is cut into tiles of sh.tile_rows rows and super-tiles of
+// sh.tiles_per_super tiles; `masks` (subset_check_temp_bytes) and *size_floor
+// (zero beforehand) come from launch_tile_and with the same shape.  `flags`
+// must start zeroed (non-stop mode).  `items` (kSubsetItems entries) and
+// item_count list the parts of S that a large check's queries need; without them
+// (nullptr) it goes over all of S.  `bytes_ctr` (optional) accumulates the
+// bytes of S rows tested.
+constexpr u64 kSubsetItems = 1u << 22;
+// Launch shape of the subset check: rows of S per tile mask (32, 64, 128),
 // warps of 32 queries per block (4, 8, 16), tiles per super-tile mask (4, 8,
 // 16, 32) and the grid's target blocks per SM (1..64), which sets how finely
 // S is chunked over blockIdx.y.  Results do not depend on it.
@@ -129,10 +130,20 @@ struct ScanShapes {
 bool scan_shape_valid(int W, const ScanShape& sh);
 size_t scan_smem_bytes(int W, const ScanShape& sh);
 size_t subset_check_temp_bytes(int W, u32 m, const ScanShape& sh);
-void launch_tile_and(int W, const u64* S, u32 m, u64* tile_and, const ScanShape& sh, cudaStream_t s);
-void launch_subset_check(int W, int mode, const u64* S, u32 m, const u64* tile_and, const u64* Q, u32 q, int n,
-                         u32* flags, u32* witness, bool stop, const ScanShape& sh, cudaStream_t s, u64* bytes_ctr,
-                         u32* err);
+void launch_tile_and(int W, const u64* S, u32 m, u64* masks, u32* size_floor, const ScanShape& sh, cudaStream_t s);
+void launch_subset_check(int W, int mode, const u64* S, u32 m, const u64* masks, const u32* size_floor, const u64* Q,
+                         u32 q, int n, u32* flags, u32* witness, bool stop, const ScanShape& sh, cudaStream_t s,
+                         u64* bytes_ctr, uint2* items, u32* item_count);
+
+// Dominance (dominance.cu): with hit_t, flags[t] = 1 for every row t of T that
+// holds some row x of X (x ⊆ t; proper: x ⊊ t), else flags[x] = 1 for every x that
+// some t holds.  comp: rows are complements of the sets meant.  Rows whose
+// `decided` entry is set (rows of T, or of X without hit_t) may be left out.
+// T up to kDomSmallRows rows is cut into 1024-row chunks, above into 4096 (2048
+// at seven words a row and more).
+constexpr u32 kDomSmallRows = 1u << 15;
+void launch_dominance(int W, bool comp, bool hit_t, const u64* T, u32 tm, const u64* X, u32 xm, int n, bool proper,
+                      const u32* decided, u32* flags, cudaStream_t s);
 
 // out = sorted merge of two sorted, mutually disjoint row arrays.
 void launch_merge(int W, const u64* A, u32 na, const u64* B, u32 nb, u64* out, cudaStream_t s);

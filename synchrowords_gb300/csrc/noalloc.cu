@@ -29,13 +29,15 @@
 namespace sw {
 namespace {
 
-// masks for SW_NOALLOC_MAX_SETS rows of 8 words: one per 64-row tile plus one
-// per 1024-row super-tile (the default ScanShape, which this entry point
-// always uses, whatever shapes a context was tuned to), plus 4 words: three
-// for the unused meet-mode witness, one for the kernel's copy-timeout word
+// masks for SW_NOALLOC_MAX_SETS rows of 8 words: one per 64-row tile, one per
+// 1024-row super-tile, one word per four rows, a size per tile and super-tile
+// (the default ScanShape, which this entry point always uses, whatever shapes a
+// context was tuned to), plus 2 words: the unused meet-mode witness and the
+// check's size floor
 constexpr size_t kMaxTiles = (SW_NOALLOC_MAX_SETS + 63) / 64;
 constexpr size_t kMaxSupers = (SW_NOALLOC_MAX_SETS + 1023) / 1024;
-constexpr size_t kScratchWords = (kMaxTiles + kMaxSupers) * 8 + 4;  // + witness, error word
+constexpr size_t kScratchWords =
+    (kMaxTiles + kMaxSupers) * 8 + SW_NOALLOC_MAX_SETS / 4 + (kMaxTiles + kMaxSupers) / 2 + 2 + 2;
 
 __device__ __align__(256) unsigned long long g_noalloc_scratch[kScratchWords];
 
@@ -102,9 +104,8 @@ extern "C" int sw_subsets_check_device_noalloc(uint32_t n, const uint64_t* d_set
     g_err = "NULL device buffer";
     return SW_ERR_INVALID_ARGUMENT;
   }
-  // the set tiles are copied with 16-byte loads, check rows with 8-byte
-  // loads, results written as 4-byte words: a misaligned pointer would fault
-  // on the GPU, so it is refused here
+  // the entry point's alignment rule (16-byte set rows, 8-byte checks, 4-byte
+  // results): a misaligned pointer could fault on the GPU, so it is refused here
   if (((uintptr_t)d_sets & 15u) || ((uintptr_t)d_checks & 7u) || ((uintptr_t)d_results & 3u)) {
     g_err = "misaligned device buffer: d_sets needs 16-byte, d_checks 8-byte and d_results 4-byte alignment";
     return SW_ERR_INVALID_ARGUMENT;
@@ -127,14 +128,17 @@ extern "C" int sw_subsets_check_device_noalloc(uint32_t n, const uint64_t* d_set
   if (set_count == 0) return SW_OK;
   const int W = words_for((int)n);
   auto* masks = static_cast<u64*>(scratch);
-  u32* witness = reinterpret_cast<u32*>(masks + kScratchWords - 4);
+  u32* witness = reinterpret_cast<u32*>(masks + kScratchWords - 2);  // three words, then the size floor
   try {
     const ScanShape sh{};
     static_assert(ScanShape{}.tile_rows == 64 && ScanShape{}.tiles_per_super == 16, "scratch sized for 64 x 16");
-    launch_tile_and(W, reinterpret_cast<const u64*>(d_sets), (u32)set_count, masks, sh, s);
+    if (subset_check_temp_bytes(W, (u32)set_count, sh) > sizeof(u64) * (kScratchWords - 2))
+      throw std::runtime_error("allocation-free check: masks outgrow the static scratch");
+    SW_CUDA(cudaMemsetAsync(witness + 3, 0, sizeof(u32), s));
+    launch_tile_and(W, reinterpret_cast<const u64*>(d_sets), (u32)set_count, masks, witness + 3, sh, s);
     launch_subset_check(W, proper ? kQueryProperSubset : kQuerySubset, reinterpret_cast<const u64*>(d_sets),
-                        (u32)set_count, masks, reinterpret_cast<const u64*>(d_checks), (u32)check_count, (int)n,
-                        d_results, witness, false, sh, s, nullptr, witness + 3);
+                        (u32)set_count, masks, witness + 3, reinterpret_cast<const u64*>(d_checks), (u32)check_count,
+                        (int)n, d_results, witness, false, sh, s, nullptr, nullptr, nullptr);
   } catch (const std::exception& ex) {
     g_err = ex.what();
     return SW_ERR_CUDA;
