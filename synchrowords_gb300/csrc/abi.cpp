@@ -22,15 +22,34 @@
 #include "exact.hpp"
 #include "plan.hpp"
 
-// Device state of the batched launches (batch_small.cu, batch_cluster.cu).
+// Scratch of cluster launches (batch_cluster.cu): tag counter, control blocks
+// and per-cluster regions; the regions' hash tables must start zero-filled (tag
+// 0 = empty slot).
+struct ClusterScratch {
+  sw::DevBuf buf;
+  size_t zeroed = 0;       // bytes zero-filled since the allocation
+  uint64_t tags_used = 0;  // upper bound on the tags taken since the last zero fill
+  void prepare(uint32_t clusters, const sw::ClusterCaps& caps, uint64_t tags, cudaStream_t s) {
+    const size_t need = sw::cluster_scratch_bytes(clusters, caps);
+    if (buf.cap < need) {
+      buf.reserve(need);
+      zeroed = 0;
+    }
+    if (zeroed < buf.cap || tags_used + tags >= sw::kClusterTagLimit) {
+      // new memory, or the tag counter could wrap: every slot back to "empty"
+      SW_CUDA(cudaMemsetAsync(buf.p, 0, buf.cap, s));
+      zeroed = buf.cap;
+      tags_used = 0;
+    }
+    tags_used += tags;
+  }
+};
+
+// Device state of the batched launches.
 struct SmallBatchState {
   cudaStream_t stream = nullptr;
-  sw::DevBuf inst, delta, seeds, results, words, origins, visited, counter;
-  // cluster launch: tag counter, control blocks and per-cluster regions; the
-  // regions' hash tables must start zero-filled (tag 0 = empty slot)
-  sw::DevBuf c_scratch, c_stats;
-  size_t c_zeroed = 0;       // bytes of c_scratch zero-filled since its allocation
-  uint64_t c_tags_used = 0;  // upper bound on the tags taken since the last zero fill
+  sw::DevBuf inst, delta, seeds, results, words, counter, c_stats;
+  ClusterScratch scratch[2];  // the batched launch's small regions, the cluster launch's large ones
   sw_batch_profile last{};
   // CUDA graphs of recent device rounds, keyed by everything their launches
   // bake in (buffers, per-width counts, cluster geometry): a batch of a shape
@@ -46,6 +65,10 @@ struct SmallBatchState {
 // level it takes on at that bound.
 constexpr double kDefaultClusterLimit = 160.0;
 constexpr uint64_t kClusterMaxPairs = 1ull << 28;
+// CTAs per automaton of the batched launch (64 automata of n = 48, three
+// batches: 1.8 / 4.9 / 1.03 ms with 4, 2.0 / 12.8 / 1.08 with 1, 1.9 / 3.8 /
+// 1.29 with 8; 1024 of them 17.4, 21.6, 20.9).
+constexpr int kSmallClusterCtas = 4;
 
 struct sw_context {
   std::unique_ptr<sw::Solver> solver;
@@ -239,12 +262,13 @@ int sw_solve(sw_context* ctx, const uint32_t* delta, uint32_t n, uint32_t k, con
 
 namespace {
 
-// One device round of sw_solve_batch: the automata of `small` (shared-memory
-// launch) and `cluster` (cluster launch), each by set width, uploaded once and
-// launched per width on the batch stream; finish_round() waits for it.
+// One device round of sw_solve_batch: the automata of `small` (batched launch:
+// clusters of kSmallClusterCtas CTAs, small regions) and `cluster` (cluster
+// launch), each by set width, uploaded once and launched per width on the batch
+// stream; finish_round() waits for it.
 struct DeviceRound {
   std::vector<uint32_t> order;  // slot -> instance
-  std::vector<uint8_t> engine;  // per slot: 0 shared-memory launch, 1 cluster launch
+  std::vector<uint8_t> engine;  // per slot: 0 batched launch, 1 cluster launch
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   int launches = 0;
   uint32_t word_stride = 1024;
@@ -284,49 +308,32 @@ void start_round(sw_context* ctx, DeviceRound& D, const std::vector<uint32_t> sm
   S.results.reserve(sizeof(sw::SmallResult) * inst.size());
   S.words.reserve((size_t)D.word_stride * inst.size());
   S.counter.reserve(sizeof(uint32_t) * 2);
-  const uint32_t blocks = (uint32_t)sw::small_batch_blocks();
-  size_t ow = 0, vw = 0;
-  for (int c = 0; c < 4; ++c)
-    if (!small[c].empty()) {
-      ow = std::max(ow, sw::small_batch_origin_words(c + 1, blocks));
-      vw = std::max(vw, sw::small_batch_visited_words(c + 1, blocks));
-    }
-  if (ow) S.origins.reserve(sizeof(uint32_t) * ow);
-  if (vw) S.visited.reserve(sizeof(uint64_t) * vw);
-  // cluster launch geometry and scratch
-  const int cs = ctx->tuning.cluster_size > 0 ? std::min<int>(ctx->tuning.cluster_size, 16) : 8;
-  const sw::ClusterCaps caps = sw::cluster_default_caps();
+  // geometry and scratch of the two launches (class c: c / 4 = launch)
+  const int cs[2] = {kSmallClusterCtas,
+                     ctx->tuning.cluster_size > 0 ? std::min<int>(ctx->tuning.cluster_size, 16) : 8};
+  const sw::ClusterCaps caps[2] = {sw::cluster_single_caps(), sw::cluster_default_caps()};
   // A cluster gives an automaton back (to the worker streams, which search it
   // with the whole GPU) after a level of more than kClusterMaxPairs meet pairs,
   // unless the caller raised cluster_limit to have larger automata searched here.
   sw::ClusterLimits limits;
   if (ctx->tuning.cluster_limit <= kDefaultClusterLimit) limits.max_pairs = kClusterMaxPairs;
-  uint32_t clusters[4] = {0, 0, 0, 0};
-  uint32_t max_clusters = 0;
-  for (int c = 0; c < 4; ++c)
-    if (!cluster[c].empty()) {
-      clusters[c] = std::min<uint32_t>({(uint32_t)cluster[c].size(), sw::cluster_batch_max_clusters(c + 1, cs),
+  uint32_t clusters[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (int l = 0; l < 2; ++l) {
+    uint32_t most = 0;
+    uint64_t tags = 0;
+    for (int c = 4 * l; c < 4 * l + 4; ++c) {
+      const uint32_t cnt = (uint32_t)(class_start[c + 1] - class_start[c]);
+      if (!cnt) continue;
+      clusters[c] = std::min<uint32_t>({cnt, sw::cluster_batch_max_clusters(c % 4 + 1, cs[l]),
                                         sw::cluster_max_clusters_supported()});
       if (!clusters[c]) throw std::runtime_error("cluster launch: no cluster of this size fits on the device");
-      max_clusters = std::max(max_clusters, clusters[c]);
+      most = std::max(most, clusters[c]);
+      tags += sw::cluster_tags_per_launch(cnt);
     }
-  if (max_clusters) {
-    const size_t need = sw::cluster_scratch_bytes(max_clusters, caps);
-    uint64_t tags = 0;
-    for (int c = 0; c < 4; ++c) tags += sw::cluster_tags_per_launch((uint32_t)cluster[c].size());
-    if (S.c_scratch.cap < need) {
-      S.c_scratch.reserve(need);
-      S.c_zeroed = 0;
-    }
-    if (S.c_zeroed < S.c_scratch.cap || S.c_tags_used + tags >= sw::kClusterTagLimit) {
-      // new memory, or the tag counter could wrap: every slot back to "empty"
-      SW_CUDA(cudaMemsetAsync(S.c_scratch.p, 0, S.c_scratch.cap, S.stream));
-      S.c_zeroed = S.c_scratch.cap;
-      S.c_tags_used = 0;
-    }
-    S.c_tags_used += tags;
-    S.c_stats.reserve(sizeof(uint64_t) * 7);
+    if (most) S.scratch[l].prepare(most, caps[l], tags, S.stream);
   }
+  const bool any_cluster = class_start[8] != class_start[4];
+  if (any_cluster) S.c_stats.reserve(sizeof(uint64_t) * 7);
   SW_CUDA(cudaMemcpyAsync(S.inst.p, inst.data(), sizeof(sw::SmallInstance) * inst.size(), cudaMemcpyHostToDevice,
                           S.stream));
   SW_CUDA(cudaMemcpyAsync(S.delta.p, dpool.data(), dpool.size(), cudaMemcpyHostToDevice, S.stream));
@@ -336,39 +343,31 @@ void start_round(sw_context* ctx, DeviceRound& D, const std::vector<uint32_t> sm
   // the round's device work: the cluster statistics reset and one persistent
   // launch per non-empty class
   auto issue = [&] {
-    if (max_clusters) SW_CUDA(cudaMemsetAsync(S.c_stats.p, 0, sizeof(uint64_t) * 7, S.stream));
+    if (any_cluster) SW_CUDA(cudaMemsetAsync(S.c_stats.p, 0, sizeof(uint64_t) * 7, S.stream));
     for (int c = 0; c < 8; ++c) {
       const size_t a = class_start[c], b = class_start[c + 1];
       if (a == b) continue;
-      const int W = c % 4 + 1;
-      if (c < 4)
-        sw::launch_small_batch(W, S.inst.as<sw::SmallInstance>() + a, (uint32_t)(b - a), S.delta.as<uint8_t>(),
-                               S.seeds.as<uint8_t>(), S.results.as<sw::SmallResult>() + a,
-                               S.words.as<uint8_t>() + a * D.word_stride, D.word_stride, S.origins.as<uint32_t>(),
-                               S.visited.as<sw::u64>(), blocks, S.counter.as<uint32_t>(), S.stream);
-      else
-        sw::launch_cluster_batch(W, cs, clusters[c - 4], S.inst.as<sw::SmallInstance>() + a, (uint32_t)(b - a),
-                                 S.delta.as<uint8_t>(), S.seeds.as<uint8_t>(), S.results.as<sw::SmallResult>() + a,
-                                 S.words.as<uint8_t>() + a * D.word_stride, D.word_stride, S.c_scratch.p, caps, limits,
-                                 S.counter.as<uint32_t>(), S.c_stats.as<sw::u64>(), S.stream);
+      const int l = c / 4;
+      sw::launch_cluster_batch(c % 4 + 1, cs[l], clusters[c], S.inst.as<sw::SmallInstance>() + a, (uint32_t)(b - a),
+                               S.delta.as<uint8_t>(), S.seeds.as<uint8_t>(), S.results.as<sw::SmallResult>() + a,
+                               S.words.as<uint8_t>() + a * D.word_stride, D.word_stride, S.scratch[l].buf.p, caps[l],
+                               limits, S.counter.as<uint32_t>(), l ? S.c_stats.as<sw::u64>() : nullptr, S.stream);
     }
   };
   for (int c = 0; c < 8; ++c) D.launches += class_start[c] != class_start[c + 1];
-  std::vector<uint64_t> key{(uint64_t)cs, blocks, D.word_stride, (uint64_t)(uintptr_t)S.inst.p,
+  std::vector<uint64_t> key{(uint64_t)cs[1], D.word_stride, (uint64_t)(uintptr_t)S.inst.p,
                             (uint64_t)(uintptr_t)S.delta.p, (uint64_t)(uintptr_t)S.seeds.p,
                             (uint64_t)(uintptr_t)S.results.p, (uint64_t)(uintptr_t)S.words.p,
-                            (uint64_t)(uintptr_t)S.origins.p, (uint64_t)(uintptr_t)S.visited.p,
-                            (uint64_t)(uintptr_t)S.counter.p, (uint64_t)(uintptr_t)S.c_scratch.p,
-                            (uint64_t)(uintptr_t)S.c_stats.p};
+                            (uint64_t)(uintptr_t)S.counter.p, (uint64_t)(uintptr_t)S.scratch[0].buf.p,
+                            (uint64_t)(uintptr_t)S.scratch[1].buf.p, (uint64_t)(uintptr_t)S.c_stats.p,
+                            limits.max_pairs};
   for (int c = 0; c < 9; ++c) key.push_back(class_start[c]);
-  for (int c = 0; c < 4; ++c) key.push_back(clusters[c]);
-  key.push_back(limits.max_pairs);
+  for (int c = 0; c < 8; ++c) key.push_back(clusters[c]);
   cudaGraphExec_t exec = nullptr;
   for (auto& g : S.graphs)
     if (g.first == key) exec = g.second;
   if (!exec) {
-    // the kernels' attributes are set before the capture (not a stream operation)
-    sw::small_batch_prepare();
+    // the kernels' attributes were set with the cluster counts, before the capture
     cudaGraph_t graph = nullptr;
     SW_CUDA(cudaStreamBeginCapture(S.stream, cudaStreamCaptureModeThreadLocal));
     try {
@@ -436,7 +435,7 @@ std::vector<uint32_t> finish_round(sw_context* ctx, DeviceRound& D, const uint32
     st[D.engine[t]][std::min<uint32_t>(R[t].status, 2)]++;
     if (R[t].status != 0) {
       if (R[t].status == 1) over[{D.engine[t], R[t].why & 255u}]++;
-      if (D.engine[t] == 0 && unfinished_small)
+      if (D.engine[t] == 0 && R[t].status == 1 && unfinished_small)  // larger regions may hold it
         unfinished_small->push_back(i);
       else
         again.push_back(i);
@@ -518,8 +517,8 @@ int sw_solve_batch(sw_context* ctx, uint32_t count, const uint32_t* deltas, cons
       model_copied = true;
     };
     // Automata whose plan is a plain Exact run are searched on the device
-    // without host round trips: the smallest by the shared-memory launch
-    // (batch_small.cu), the others by the cluster launch (batch_cluster.cu).
+    // without host round trips (batch_cluster.cu): the smallest by the batched
+    // launch (many small clusters), the others by the cluster launch.
     // What neither finishes, and every other automaton, runs on the worker
     // streams.
     const bool cluster_on = ctx->tuning.cluster_size >= 0;
@@ -614,7 +613,7 @@ int sw_solve_batch(sw_context* ctx, uint32_t count, const uint32_t* deltas, cons
     run_pool(streamed);
     const double ms_streamed = since(h1);
     const auto h2 = clk::now();
-    // what the shared-memory launch leaves gets a cluster round before the streams
+    // what outgrows the batched launch's regions gets a cluster round before the streams
     std::vector<uint32_t> small_left;
     std::vector<uint32_t> again = finish_round(ctx, round1, deltas, off, ns, ks, plans, results,
                                                cluster_on ? &small_left : nullptr, verbose);

@@ -45,9 +45,9 @@ void launch_brute_level(const uint16_t* delta, int n, int k, const u32* frontier
 void launch_brute_parent(const uint16_t* delta, int n, int k, const u32* level, u32 count, u32 target, u64* best,
                          cudaStream_t s);
 
-// ---- Batched exact search for small automata (batch_small.cu) -----------
+// ---- Device-resident exact search (batch_cluster.cu) ----------------------
 
-// One automaton of a batch: n <= 64 W states, k <= 4 letters; delta[q*k + a]
+// One automaton of a batch: n <= 64 W states; delta[q*k + a]
 // (u8) at delta_off of the delta pool, its backward seeds (ascending) at
 // seed_off of the seed pool; lengths 1..max_len are searched.
 struct SmallInstance {
@@ -60,22 +60,9 @@ struct SmallResult {
   u32 status, length, word_len, why;
 };
 
-int small_batch_blocks();
-// Raises the shared-memory limits of the batched kernels on the current
-// device (done before a launch is captured into a CUDA graph).
-void small_batch_prepare();
-size_t small_batch_origin_words(int W, u32 blocks);
-size_t small_batch_visited_words(int W, u32 blocks);
-// One persistent launch of `blocks` blocks over `count` automata of set width
-// W (1 to 4 words, n <= 64 W); origins, visited and counter are scratch.
-void launch_small_batch(int W, const SmallInstance* inst, u32 count, const uint8_t* delta_pool,
-                        const uint8_t* seed_pool, SmallResult* results, uint8_t* words, u32 word_stride, u32* origins,
-                        u64* visited, u32 blocks, u32* counter, cudaStream_t s);
-
 // Device-resident search on thread-block clusters (batch_cluster.cu): one
 // cluster of `cs` CTAs per automaton (n <= 256, n * k <= 4096), lists in a
-// per-cluster global region.  Same instances and results as the small batch;
-// status 1 may also report why 6 (a hash-table probe ran out), status 2 why 8
+// per-cluster global region.  Status 1 may also report why 6 (a hash-table probe ran out), status 2 why 8
 // (a side died out) or 9 (max_len reached), and status 3 says that the search
 // stopped at a work limit; where no word was found, `length` counts the
 // lengths excluded so far.

@@ -27,8 +27,7 @@
 //     per lane-word, stopping as soon as every word is zero; a word still
 //     nonzero when f's states run out names a B_j ⊇ f;
 //   * the word is traced back through the layers' slot lists.
-// The search is the one k_small_batch (batch_small.cu) runs, with the same
-// exactness argument: one side grows by one layer per step, every total
+// Exactness: one side grows by one layer per step, every total
 // length is checked once, and a set equal to one of an earlier layer of its
 // side is dropped (a shorter prefix reaches it).  An automaton whose lists
 // outgrow the capacities, or whose search reaches the depth or length limit,
@@ -79,6 +78,8 @@ __device__ __forceinline__ u32 cluster_index() {
 // Every thread of every CTA of the cluster arrives and waits; the arrive
 // releases and the wait acquires at cluster scope, so global-memory writes made
 // before the barrier by any CTA of the cluster are visible after it.
+// A row's words before its table slot, for the CTAs of the cluster.
+__device__ __forceinline__ void cluster_fence() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -104,7 +105,7 @@ __device__ __forceinline__ bool table_insert(u64* vt, u32 vmask, u64 tag, const 
       v = old;  // taken meanwhile, by a row of this search
     }
     if (((v ^ mine) >> kSlotRowBits) == 0) {  // same tag and fingerprint
-      __threadfence();                        // the row was written before its slot
+      cluster_fence();                        // the row was written before its slot
       if (row_eq_volatile<W>(V + (size_t)((u32)v & kSlotRowMask) * W, x)) return false;
     }
     slot = (slot + 1) & vmask;
@@ -113,13 +114,23 @@ __device__ __forceinline__ bool table_insert(u64* vt, u32 vmask, u64 tag, const 
   return false;
 }
 
-// Per-cluster control words (one 256-byte block per cluster index).
+__device__ __forceinline__ uint4 ld_volatile128(const void* p) {
+  uint4 v;
+  asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+
+// Per-cluster control words (one 256-byte block per cluster index; the first
+// four are read together).
 struct ClusterCtl {
-  u32 inst;       // automaton being solved
-  u32 vtag;       // tag of this search's table slots
   u32 fcount[2];  // kept children of the step (by step parity)
   u32 overflow;   // a table probe ran out (never expected: tables hold more slots than rows)
   u32 found;      // meet flag
+  u32 inst;       // automaton being solved
+  u32 vtag;       // tag of this search's table slots
   u32 fi, bj;     // meeting pair: index in the current F layer, in the current B layer
   ClusterExit exit;  // how the last search ended
   u32 pad[64 - 8 - sizeof(ClusterExit) / 4];
@@ -273,7 +284,7 @@ __global__ void __launch_bounds__(kCtThreads, 1)
           V[(size_t)r * W + w] = x[w];
         }
         (i == 0 ? L0 : L1)[r] = r;
-        __threadfence();
+        cluster_fence();
         table_insert<W>(i == 0 ? vt0 : vt1, vmask, vtag, V, x, r, &ctl->overflow);
       }
       if (rank == 0 && tid == 0) {
@@ -333,7 +344,7 @@ __global__ void __launch_bounds__(kCtThreads, 1)
 #pragma unroll
           for (int w = 0; w < W; ++w) VX[(size_t)r * W + w] = x[w];
         }
-        __threadfence();  // the row before its slot
+        cluster_fence();  // the row before its slot
         const bool keep = valid && table_insert<W>(vtX, vmask, vtag, VX, x, r, &ctl->overflow);
         const u32 kmask = __ballot_sync(0xffffffffu, keep);
         u32 pos0 = 0;
@@ -402,7 +413,8 @@ __global__ void __launch_bounds__(kCtThreads, 1)
       my_children += c;
       cluster_barrier();
       lap(0);
-      const u32 f = ld_volatile(&ctl->fcount[par]);
+      const uint4 now = ld_volatile128(ctl);  // both counts, overflow, meet flag
+      const u32 f = par ? now.y : now.x;
       if (rank == 0 && tid == 0) {
         ctl->fcount[par ^ 1u] = 0;
         m_voff(X)[depthX + 1] = usedX;
@@ -423,7 +435,7 @@ __global__ void __launch_bounds__(kCtThreads, 1)
         depth0 = depthX + 1;
       }
       ++steps;
-      if (ld_volatile(&ctl->overflow)) {
+      if (now.z) {
         status = 1;
         why = 6;
         break;

@@ -39,8 +39,8 @@ constexpr u32 col_stride() {
   return V == 1 ? 33 : 32 * V + (V == 4 ? 4 : 2);
 }
 template <int W, int V>
-constexpr size_t dom_smem() {
-  return sizeof(u32) * 64 * W * col_stride<V>() + sizeof(uint16_t) * 1024 * V;
+constexpr size_t dom_smem() {  // columns, open rows, row sizes
+  return sizeof(u32) * (64 * W * col_stride<V>() + 32 * V) + sizeof(uint16_t) * 1024 * V;
 }
 template <int V>
 constexpr int dom_threads() {
@@ -68,18 +68,24 @@ __device__ __forceinline__ void and_column(u32* acc, const u32* col) {
 // Block (chunk of T, slice of X).  kHitT: flags[t] = 1 for every row t of T
 // that holds some x; else flags[x] = 1 for every row x of X that some t holds.
 // kComp: rows are complements of the sets.  decided (may be null): rows of T
-// (kHitT) or X whose answer is not wanted.
+// (kHitT) or X whose answer is not wanted.  index (may be null): what row t of T is
+// called in flags and decided.
 template <int W, int V, bool kComp, bool kHitT>
 __global__ void __launch_bounds__(dom_threads<V>()) k_dominance(const u64* __restrict__ T, u32 tm,
+                                                               const u32* __restrict__ index,
                                                                const u64* __restrict__ X, u32 xm, int n, int proper,
-                                                               u32 per_slice, const u32* __restrict__ decided,
-                                                               u32* flags) {
+                                                               u32 per_slice, u32 per_warp,
+                                                               const u32* __restrict__ decided, u32* flags) {
   extern __shared__ __align__(16) u32 s_dom[];
+  __shared__ u32 s_max;
   constexpr u32 kStride = col_stride<V>();
   constexpr u32 kWarps = dom_threads<V>() / 32;
-  uint16_t* const s_size = reinterpret_cast<uint16_t*>(s_dom + 64 * W * kStride);
+  u32* const s_open = s_dom + 64 * W * kStride;
+  uint16_t* const s_size = reinterpret_cast<uint16_t*>(s_open + 32 * V);
   const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const u32 r0 = blockIdx.x * 1024u * V, rows = min(1024u * V, tm - r0);
+  if (threadIdx.x == 0) s_max = 0;
+  __syncthreads();
   for (u32 g = warp; g < 32 * V; g += kWarps) {
     const u32 r = 32 * g + lane;
     u32 size = 0;
@@ -91,35 +97,41 @@ __global__ void __launch_bounds__(dom_threads<V>()) k_dominance(const u64* __res
         if (kComp) b = ~b & valid_mask(n, w);
       }
       size += __popcll(b);
-      s_dom[(64 * w + 31 - lane) * kStride + g] = transpose32((u32)(b >> 32));
-      s_dom[(64 * w + 63 - lane) * kStride + g] = transpose32((u32)b);
+      // column c of a word holds bit c: its states from the last to the first
+      s_dom[(64 * w + 32 + lane) * kStride + g] = transpose32((u32)(b >> 32));
+      s_dom[(64 * w + lane) * kStride + g] = transpose32((u32)b);
     }
     s_size[r] = (uint16_t)size;
+    bool in = r < rows;
+    if (kHitT && decided && in) in = !decided[index ? index[r0 + r] : r0 + r];
+    const u32 open = __ballot_sync(kFullWarp, in);
+    const u32 most = __reduce_max_sync(kFullWarp, size);
+    if (lane == 0) {
+      s_open[g] = open;
+      atomicMax(&s_max, most);
+    }
   }
   __syncthreads();
-  // the lane's rows: 32 (V lane + i) + bit; those past the chunk or decided take no part
-  u32 open[V];
+  u32 open[V];  // the lane's rows that take part: 32 (V lane + i) + bit
 #pragma unroll
-  for (int i = 0; i < V; ++i) {
-    const u32 b = 32 * (V * lane + i);
-    open[i] = b >= rows ? 0u : (rows - b >= 32 ? 0xffffffffu : (1u << (rows - b)) - 1u);
-    if (kHitT && decided)
-      for (u32 left = open[i]; left; left &= left - 1)
-        if (decided[r0 + b + __ffs(left) - 1]) open[i] &= ~(left & -left);
-  }
+  for (int i = 0; i < V; ++i) open[i] = s_open[V * lane + i];
+  const u32 most = s_max;
   const u32 x_end = min(xm, (blockIdx.y + 1) * per_slice);
-  for (u32 x0 = blockIdx.y * per_slice + warp * 32; x0 < x_end; x0 += kWarps * 32) {
+  for (u32 x0 = blockIdx.y * per_slice + warp * per_warp; x0 < x_end; x0 += kWarps * per_warp) {
     const u32 xi = x0 + lane;
-    u64 x[W];
+    const bool valid = lane < per_warp && xi < x_end;
+    u32 x[2 * W];  // the set in 32-bit halves
     u32 size = 0;
 #pragma unroll
     for (int w = 0; w < W; ++w) {
-      u64 b = xi < x_end ? X[(size_t)xi * W + w] : 0ULL;
-      if (kComp && xi < x_end) b = ~b & valid_mask(n, w);
-      x[w] = b;
+      u64 b = valid ? X[(size_t)xi * W + w] : 0ULL;
+      if (kComp && valid) b = ~b & valid_mask(n, w);
+      x[2 * w] = (u32)(b >> 32);
+      x[2 * w + 1] = (u32)b;
       size += __popcll(b);
     }
-    bool want = xi < x_end;
+    // no row of the chunk is as large as a larger set (nor, for a proper subset, larger than one as large)
+    bool want = valid && (proper ? size < most : size <= most);
     if (!kHitT && want) want = !*(volatile u32*)(flags + xi) && !(decided && decided[xi]);
     u32 todo = __ballot_sync(kFullWarp, want);
     while (todo) {
@@ -132,15 +144,17 @@ __global__ void __launch_bounds__(dom_threads<V>()) k_dominance(const u64* __res
       // states are numbered by falling frequency in images: the last ones first,
       // whose columns are the emptiest
 #pragma unroll
-      for (int w = W - 1; w >= 0; --w) {
-        u64 v = __shfl_sync(kFullWarp, x[w], j);
-        const u32* const last = s_dom + (u32)(64 * w + 63) * kStride + V * lane;  // column of bit 0
+      for (int h = 2 * W - 1; h >= 0; --h) {
+        u32 v = __shfl_sync(kFullWarp, x[h], j);
+        const u32* const base = s_dom + (u32)(64 * (h >> 1) + ((h & 1) ? 0 : 32)) * kStride + V * lane;
         while (v && alive) {  // two states a turn
-          and_column<V>(acc, last - (u32)(__ffsll((long long)v) - 1) * kStride);
+          const u32 b0 = __ffs(v) - 1;
           v &= v - 1;
+          and_column<V>(acc, base + b0 * kStride);
           if (v) {
-            and_column<V>(acc, last - (u32)(__ffsll((long long)v) - 1) * kStride);
+            const u32 b1 = __ffs(v) - 1;
             v &= v - 1;
+            and_column<V>(acc, base + b1 * kStride);
           }
           u32 any = 0;
 #pragma unroll
@@ -158,7 +172,7 @@ __global__ void __launch_bounds__(dom_threads<V>()) k_dominance(const u64* __res
           const u32 r = 32 * (V * lane + i) + __ffs(left) - 1;
           if (proper && s_size[r] == sx) continue;
           if (kHitT) {
-            flags[r0 + r] = 1u;
+            flags[index ? index[r0 + r] : r0 + r] = 1u;
             open[i] &= ~(left & -left);
           } else {
             hit = true;
@@ -170,25 +184,58 @@ __global__ void __launch_bounds__(dom_threads<V>()) k_dominance(const u64* __res
   }
 }
 
+// ---- rows by falling size, so that a chunk's sizes are alike ----
+template <int W, bool kComp>
+__global__ void __launch_bounds__(256) k_size_rank(const u64* __restrict__ T, u32 m, int n, u32* __restrict__ counts,
+                                                   uint2* __restrict__ place) {
+  const u32 e = blockIdx.x * blockDim.x + threadIdx.x;
+  u32 size = 0;
+  if (e < m)
+#pragma unroll
+    for (int w = 0; w < W; ++w) size += __popcll(T[(size_t)e * W + w]);
+  const u32 bucket = kComp ? size : (u32)n - size;  // largest sets first
+  const u32 in = __ballot_sync(kFullWarp, e < m);
+  if (e >= m) return;
+  const u32 lane = threadIdx.x & 31;
+  const u32 peers = __match_any_sync(in, bucket);
+  const int leader = __ffs(peers) - 1;
+  u32 first = 0;
+  if (lane == (u32)leader) first = atomicAdd(&counts[bucket], (u32)__popc(peers));
+  place[e] = make_uint2(__shfl_sync(peers, first, leader) + __popc(peers & ((1u << lane) - 1u)), bucket);
+}
+
+template <int W>
+__global__ void __launch_bounds__(256) k_size_scatter(const u64* __restrict__ T, u32 m, const uint2* __restrict__ place,
+                                                      const u32* __restrict__ first, u64* __restrict__ out,
+                                                      u32* __restrict__ index) {
+  const u32 e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= m) return;
+  const uint2 pl = place[e];
+  const u32 d = first[pl.y] + pl.x;
+#pragma unroll
+  for (int w = 0; w < W; ++w) out[(size_t)d * W + w] = T[(size_t)e * W + w];
+  index[d] = e;
+}
+
 namespace {
 template <int W, int V>
-void launch_dom(bool comp, bool hit_t, const u64* T, u32 tm, const u64* X, u32 xm, int n, bool proper,
+void launch_dom(bool comp, bool hit_t, const u64* T, u32 tm, const u32* index, const u64* X, u32 xm, int n, bool proper,
                 const u32* decided, u32* flags, cudaStream_t s) {
   const u32 chunks = (tm + 1024 * V - 1) / (1024 * V);
-  constexpr u32 kThreads = dom_threads<V>();
-  // about two blocks an SM and chunk set, at least one pass of a block's warps
-  // (one round of 32 sets each; 8 at V = 1 would only add staging) per slice
+  constexpr u32 kThreads = dom_threads<V>(), kWarps = kThreads / 32;
+  // slices of X: as many blocks as fit the GPU a few times over, while a warp keeps eight sets or more
   u32 slices = std::max<u32>(1, (u32)device_sm_count() * (V == 1 ? 8 : 2) / chunks);
-  slices = std::min<u32>({slices, (xm + kThreads - 1) / kThreads, 65535u});
+  slices = std::min<u32>({slices, (xm + 8 * kWarps - 1) / (8 * kWarps), 65535u});
   u32 per = (xm + slices - 1) / slices;
-  per = (per + 31) / 32 * 32;
+  const u32 per_warp = std::min<u32>(32, (per + kWarps - 1) / kWarps);
   slices = (xm + per - 1) / per;
   const dim3 grid(chunks, slices);
   constexpr size_t smem = dom_smem<W, V>();
-#define SW_DOM(C, H)                                                                                      \
-  {                                                                                                       \
-    ensure_smem_limit((const void*)k_dominance<W, V, C, H>, (int)smem);                                   \
-    k_dominance<W, V, C, H><<<grid, kThreads, smem, s>>>(T, tm, X, xm, n, proper ? 1 : 0, per, decided, flags); \
+#define SW_DOM(C, H)                                                                                          \
+  {                                                                                                           \
+    ensure_smem_limit((const void*)k_dominance<W, V, C, H>, (int)smem);                                       \
+    k_dominance<W, V, C, H><<<grid, kThreads, smem, s>>>(T, tm, index, X, xm, n, proper ? 1 : 0, per, per_warp, \
+                                                         decided, flags);                                     \
   }
   if (comp) {
     if (hit_t) SW_DOM(true, true) else SW_DOM(true, false)
@@ -200,27 +247,36 @@ void launch_dom(bool comp, bool hit_t, const u64* T, u32 tm, const u64* X, u32 x
 }
 template <int W>
 void launch_dom_w(bool comp, bool hit_t, const u64* T, u32 tm, const u64* X, u32 xm, int n, bool proper,
-                  const u32* decided, u32* flags, cudaStream_t s) {
+                  const u32* decided, u32* flags, const DominanceScratch& sc, cudaStream_t s) {
   // small lists: 1024-row chunks, so that they spread over more blocks
-  if (tm <= kDomSmallRows)
-    launch_dom<W, 1>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, s);
+  if (tm <= kDomSmallRows) {
+    launch_dom<W, 1>(comp, hit_t, T, tm, nullptr, X, xm, n, proper, decided, flags, s);
+    return;
+  }
+  const u32 blocks = (tm + 255) / 256;
+  if (comp)
+    k_size_rank<W, true><<<blocks, 256, 0, s>>>(T, tm, n, sc.bucket.counts, sc.bucket.place);
   else
-    launch_dom<W, (W < 7 ? 4 : 2)>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, s);
+    k_size_rank<W, false><<<blocks, 256, 0, s>>>(T, tm, n, sc.bucket.counts, sc.bucket.place);
+  launch_bucket_scan(BucketScratch{kBucketBitsSmall, sc.bucket.counts, sc.bucket.first, sc.bucket.place}, sc.total, s);
+  k_size_scatter<W><<<blocks, 256, 0, s>>>(T, tm, sc.bucket.place, sc.bucket.first, sc.rows, sc.index);
+  SW_LAUNCH_CHECK();
+  launch_dom<W, (W < 7 ? 4 : 2)>(comp, hit_t, sc.rows, tm, sc.index, X, xm, n, proper, decided, flags, s);
 }
 }  // namespace
 
 void launch_dominance(int W, bool comp, bool hit_t, const u64* T, u32 tm, const u64* X, u32 xm, int n, bool proper,
-                      const u32* decided, u32* flags, cudaStream_t s) {
+                      const u32* decided, u32* flags, const DominanceScratch& sc, cudaStream_t s) {
   if (!tm || !xm) return;
   switch (W) {
-    case 1: return launch_dom_w<1>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, s);
-    case 2: return launch_dom_w<2>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, s);
-    case 3: return launch_dom_w<3>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, s);
-    case 4: return launch_dom_w<4>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, s);
-    case 5: return launch_dom_w<5>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, s);
-    case 6: return launch_dom_w<6>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, s);
-    case 7: return launch_dom_w<7>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, s);
-    case 8: return launch_dom_w<8>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, s);
+    case 1: return launch_dom_w<1>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
+    case 2: return launch_dom_w<2>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
+    case 3: return launch_dom_w<3>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
+    case 4: return launch_dom_w<4>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
+    case 5: return launch_dom_w<5>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
+    case 6: return launch_dom_w<6>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
+    case 7: return launch_dom_w<7>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
+    case 8: return launch_dom_w<8>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
     default: throw std::runtime_error("dominance: unsupported width");
   }
 }

@@ -96,10 +96,12 @@ struct Side {
 
 // Where a search leaves the single cluster it starts on (Engine::run_single).
 // CTAs of that cluster, and the children and meet pairs of a level above which
-// the level goes to the whole GPU.
+// the level goes to the whole GPU.  Four solves at n = 200 in ms, by children
+// (pairs = children^2 / 4): 2^11 15.1, 2^12 15.1, 2^13 14.8, 2^14 15.3; with 4
+// CTAs and 2^13 15.4, with 16 (a size not every GPU part can place) 14.5.
 constexpr int kSingleClusterCtas = 8;
-constexpr u32 kSingleMaxChildren = 1u << 14;
-constexpr u64 kSingleMaxPairs = 1ull << 26;
+constexpr u32 kSingleMaxChildren = 1u << 13;
+constexpr u64 kSingleMaxPairs = 1ull << 24;
 
 // One level of the bounded inverse phase (a chunk of parents' children).
 struct DLevel {
@@ -362,6 +364,7 @@ class Engine {
   // flags[i] = 1 where a row of S (a proper one) is inside child row i of Q, on
   // the forward side or on complement rows; children `decided` already may be
   // left out.
+  DevBuf dom_rows, dom_index;
   void dominated(bool forward, int W, const u64* S, u32 m, const u64* Q, u32 q, int n, bool proper, const u32* decided,
                  u32* flags) {
     if (!m || !q) return;
@@ -370,11 +373,22 @@ class Engine {
       e0 = next_event();
       SW_CUDA(cudaEventRecord(e0, stream));
     }
+    DominanceScratch sc;
+    const u32 tm = forward ? q : m;  // rows that hold: children forward, visited or siblings backward
+    if (tm > kDomSmallRows) {
+      sc.bucket = buckets(tm);
+      dom_rows.reserve(sizeof(u64) * W * (size_t)tm);
+      dom_index.reserve(sizeof(u32) * (size_t)tm);
+      sc.rows = dom_rows.as<u64>();
+      sc.index = dom_index.as<u32>();
+      sc.total = d_misc + 10;
+      count_launch(3);
+    }
     timed(0, (double)(m + q) * 8.0 * W, [&] {
       if (forward)  // sets s ⊆ c: the children hold them
-        launch_dominance(W, false, true, Q, q, S, m, n, proper, decided, flags, stream);
+        launch_dominance(W, false, true, Q, q, S, m, n, proper, decided, flags, sc, stream);
       else  // complements: the set of c lies in the set of s
-        launch_dominance(W, true, false, S, m, Q, q, n, proper, decided, flags, stream);
+        launch_dominance(W, true, false, S, m, Q, q, n, proper, decided, flags, sc, stream);
     });
     if (prof_on) {
       cudaEvent_t e1 = next_event();

@@ -559,10 +559,14 @@ void launch_bucket_rank(int W, const u64* C, u32 m, const BucketScratch& b, cuda
   SW_LAUNCH_CHECK();
 }
 
-void launch_bucket_scatter(int W, const u64* C, u32 m, const BucketScratch& b, u32 base, u64* out_rows, u32* out_vals,
-                           u64* tab, u32* total, cudaStream_t s) {
+void launch_bucket_scan(const BucketScratch& b, u32* total, cudaStream_t s) {
   k_bucket_scan<<<1, kScanThreads, 0, s>>>(b.counts, b.first, 1u << b.bits, total);
   SW_LAUNCH_CHECK();
+}
+
+void launch_bucket_scatter(int W, const u64* C, u32 m, const BucketScratch& b, u32 base, u64* out_rows, u32* out_vals,
+                           u64* tab, u32* total, cudaStream_t s) {
+  launch_bucket_scan(b, total, s);
   if (!m) return;
   SW_EXP_DISPATCH((k_bucket_scatter<WW><<<(m + 255) / 256, 256, 0, s>>>(C, m, b.place, b.first, 64 - b.bits, base,
                                                                       out_rows, out_vals,

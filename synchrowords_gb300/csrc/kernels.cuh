@@ -139,11 +139,20 @@ void launch_subset_check(int W, int mode, const u64* S, u32 m, const u64* masks,
 // holds some row x of X (x ⊆ t; proper: x ⊊ t), else flags[x] = 1 for every x that
 // some t holds.  comp: rows are complements of the sets meant.  Rows whose
 // `decided` entry is set (rows of T, or of X without hit_t) may be left out.
-// T up to kDomSmallRows rows is cut into 1024-row chunks, above into 4096 (2048
-// at seven words a row and more).
+// T up to kDomSmallRows rows is cut into 1024-row chunks as it is; above, its rows
+// are first ordered by falling size (so that most sets are too large for most
+// chunks) and cut into chunks of 4096 (2048 at seven words a row and more); the
+// scratch is used only then.
 constexpr u32 kDomSmallRows = 1u << 15;
+struct DominanceScratch {
+  BucketScratch bucket;   // as for launch_bucket_scatter, with room for T's rows
+  u64* rows = nullptr;    // T's rows again
+  u32* index = nullptr;   // one word per row of T
+  u32* total = nullptr;   // one word
+};
+void launch_bucket_scan(const BucketScratch& b, u32* total, cudaStream_t s);
 void launch_dominance(int W, bool comp, bool hit_t, const u64* T, u32 tm, const u64* X, u32 xm, int n, bool proper,
-                      const u32* decided, u32* flags, cudaStream_t s);
+                      const u32* decided, u32* flags, const DominanceScratch& sc, cudaStream_t s);
 
 // out = sorted merge of two sorted, mutually disjoint row arrays.
 void launch_merge(int W, const u64* A, u32 na, const u64* B, u32 nb, u64* out, cudaStream_t s);

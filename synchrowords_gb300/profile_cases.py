@@ -5,8 +5,8 @@ enough that an ncu capture of a few launches ends in seconds:
 
   cluster  16 random binary automata, n = 128, on the cluster launch
            (k_cluster_batch, clusters of 8 CTAs)
-  small2   64 random binary automata, n = 100, on the shared-memory batched
-           launch (k_small_batch, two-word rows)
+  small2   64 random binary automata, n = 100, on the batched launch
+           (k_cluster_batch in clusters of 4 CTAs, two-word rows)
   small3   the same at n = 150 (three-word rows)
   n200     one plain Exact solve, n = 200, on the streamed path
            (k_subset_scan, k_bitonic_small, k_expand, ...)
