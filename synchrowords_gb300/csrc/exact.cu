@@ -1983,21 +1983,20 @@ float Solver::mlp_gradient(const Automaton& A, const uint64_t* sets, const float
   SW_CUDA(cudaSetDevice(device_));
   Engine& E = *eng_;
   if (!count) throw std::invalid_argument("empty batch");
-  DevBuf d_rows, d_y, d_t;
+  DevBuf d_rows, d_t;
   d_rows.reserve(sizeof(u64) * 8 * count);
-  d_y.reserve(sizeof(float) * count);
   d_t.reserve(sizeof(float) * count);
   SW_CUDA(cudaMemcpyAsync(d_rows.p, sets, sizeof(u64) * 8 * count, cudaMemcpyHostToDevice, E.stream));
   launch_convert_rows(8, d_rows.as<u64>(), count, (int)A.n, true, E.stream);
   SW_CUDA(cudaMemcpyAsync(d_t.p, labels, sizeof(float) * count, cudaMemcpyHostToDevice, E.stream));
   E.mlp->prepare(A);
   E.mlp->zero_grad();
-  E.mlp->forward(d_rows.as<u64>(), 8, (u32)count, d_y.as<float>());
-  E.mlp->backward(d_t.as<float>(), (u32)count);
+  E.mlp->gradient(d_rows.as<u64>(), 8, (u32)count, d_t.as<float>(), nullptr, 0.0f, E.mlp->loss());
   float loss = 0;
   SW_CUDA(cudaMemcpyAsync(grad, E.mlp->grad(), sizeof(float) * mlp::kParams, cudaMemcpyDeviceToHost, E.stream));
   SW_CUDA(cudaMemcpyAsync(&loss, E.mlp->loss(), sizeof(float), cudaMemcpyDeviceToHost, E.stream));
   SW_CUDA(cudaStreamSynchronize(E.stream));
+  if (mlp::tc_error()) throw CudaError("distance model: a tensor-core wait ran out");
   return loss;
 }
 
@@ -2010,20 +2009,23 @@ float Solver::mlp_train(const std::vector<Automaton>& autos, const uint64_t* off
   const uint64_t total = offsets[A_n];
   if (!total || !batch) throw std::invalid_argument("no training pairs");
   // all pairs resident on the device as 8-word rows
-  DevBuf d_rows, d_lab, d_y;
+  DevBuf d_rows, d_lab, d_grp, d_loss;
   d_rows.reserve(sizeof(u64) * 8 * total);
   d_lab.reserve(sizeof(float) * total);
-  d_y.reserve(sizeof(float) * batch);
   SW_CUDA(cudaMemcpyAsync(d_rows.p, sets, sizeof(u64) * 8 * total, cudaMemcpyHostToDevice, E.stream));
   for (size_t a = 0; a < A_n; ++a)
     launch_convert_rows(8, d_rows.as<u64>() + offsets[a] * 8, offsets[a + 1] - offsets[a], (int)autos[a].n, true,
                         E.stream);
-  SW_CUDA(cudaMemcpy(d_lab.p, labels, sizeof(float) * total, cudaMemcpyHostToDevice));
-  DevBuf d_grp;
+  SW_CUDA(cudaMemcpyAsync(d_lab.p, labels, sizeof(float) * total, cudaMemcpyHostToDevice, E.stream));
   if (groups && rank_w > 0.0f) {
     d_grp.reserve(sizeof(uint32_t) * total);
-    SW_CUDA(cudaMemcpy(d_grp.p, groups, sizeof(uint32_t) * total, cudaMemcpyHostToDevice));
+    SW_CUDA(cudaMemcpyAsync(d_grp.p, groups, sizeof(uint32_t) * total, cudaMemcpyHostToDevice, E.stream));
   }
+  // one loss per step, read once an epoch: the steps queue without waiting for each other
+  uint64_t steps = 0;
+  for (size_t a = 0; a < A_n; ++a) steps += (offsets[a + 1] - offsets[a] + batch - 1) / batch;
+  d_loss.reserve(sizeof(float) * steps);
+  std::vector<float> step_loss(steps);
   std::vector<size_t> order(A_n);
   for (size_t a = 0; a < A_n; ++a) order[a] = a;
   uint64_t state = seed;
@@ -2036,26 +2038,26 @@ float Solver::mlp_train(const std::vector<Automaton>& autos, const uint64_t* off
   double last = 0;
   for (uint32_t ep = 0; ep < epochs; ++ep) {
     for (size_t a = A_n; a > 1; --a) std::swap(order[a - 1], order[next() % a]);
-    double sum = 0;
-    uint64_t steps = 0;
+    SW_CUDA(cudaMemsetAsync(d_loss.p, 0, sizeof(float) * steps, E.stream));
+    E.mlp->zero_grad();
+    uint64_t step = 0;
     for (size_t oi = 0; oi < A_n; ++oi) {
       const size_t a = order[oi];
-      for (uint64_t o = offsets[a]; o < offsets[a + 1]; o += batch) {
+      for (uint64_t o = offsets[a]; o < offsets[a + 1]; o += batch, ++step) {
         const u32 c = (u32)std::min<uint64_t>(batch, offsets[a + 1] - o);
         E.mlp->prepare(autos[a]);
-        E.mlp->zero_grad();
-        E.mlp->forward(d_rows.as<u64>() + o * 8, 8, c, d_y.as<float>());
-        E.mlp->backward(d_lab.as<float>() + o, c, d_grp.p ? d_grp.as<uint32_t>() + o : nullptr, rank_w);
+        E.mlp->gradient(d_rows.as<u64>() + o * 8, 8, c, d_lab.as<float>() + o,
+                        d_grp.p ? d_grp.as<uint32_t>() + o : nullptr, rank_w, d_loss.as<float>() + step);
         E.mlp->adam_step(lr);
-        float l = 0;
-        SW_CUDA(cudaMemcpyAsync(&l, E.mlp->loss(), sizeof(float), cudaMemcpyDeviceToHost, E.stream));
-        SW_CUDA(cudaStreamSynchronize(E.stream));
-        sum += l;
-        ++steps;
       }
     }
+    SW_CUDA(cudaMemcpyAsync(step_loss.data(), d_loss.p, sizeof(float) * steps, cudaMemcpyDeviceToHost, E.stream));
+    SW_CUDA(cudaStreamSynchronize(E.stream));
+    double sum = 0;
+    for (float l : step_loss) sum += l;
     last = steps ? sum / steps : 0.0;
   }
+  if (mlp::tc_error()) throw CudaError("distance model: a tensor-core wait ran out");
   return (float)last;
 }
 

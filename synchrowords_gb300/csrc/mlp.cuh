@@ -1,12 +1,14 @@
 // Learned distance model: a set S of states is scored by
 //   E   = relu(feat · Phi + c)                  per-state embeddings, n x 64 (bf16)
-//   x   = sum over q in S of E[q]                (= bits(S) · E, a tensor-core GEMM)
+//   x   = sum over q in S of E[q]                (= bits(S) · E, a tensor-core product)
 //   h1  = relu(x · W1 + b1),  h2 = relu(h1 · W2 + b2)   (64 -> 128 -> 128)
 //   y   = h2 · w3 + b3                            predicted shortest merge length
 // feat is a fixed per-state feature vector of the automaton (automaton.cpp),
-// so one trained model applies to automata of any size.  Dense products run
-// on the tensor cores (tcgen05.mma, bf16 inputs, fp32 accumulation in TMEM);
-// master weights, gradients and Adam moments are fp32.
+// so one trained model applies to automata of any size.  The products over a
+// batch run on the tensor cores (tcgen05.mma, bf16 inputs, fp32 accumulation in
+// TMEM); master weights, gradients and Adam moments are fp32.  A training step is
+// six launches (mlp.cu): embeddings, forward, loss, backward, the embeddings'
+// gradient, Adam.
 #pragma once
 #include <cuda_bf16.h>
 
@@ -30,54 +32,46 @@ constexpr int kOffW3 = kOffB2 + kHidden;              // [kHidden]
 constexpr int kOffB3 = kOffW3 + kHidden;              // [1]
 constexpr int kParams = kOffB3 + 1;
 
-// A bf16 matrix view: element (i, k) at p[i * si + k * sk].
-struct View {
-  const __nv_bfloat16* p;
-  long long si, sk;
+using bf16 = __nv_bfloat16;
+
+// The dense layers' weights in bf16, in the layout their products read from
+// shared memory (mlp.cu), as the forward pass and as the backward pass needs
+// them; element counts.
+constexpr int kStagedW1 = kEmb * kHidden, kStagedW2 = kHidden * kHidden;
+constexpr int kOffW1F = 0, kOffW1B = kOffW1F + kStagedW1, kOffW2F = kOffW1B + kStagedW1,
+              kOffW2B = kOffW2F + kStagedW2, kStagedWeights = kOffW2B + kStagedW2;
+
+// Elements of the staged embeddings of n states (whole 64-state slices).
+inline size_t staged_embeddings(int n) { return (size_t)((n + 63) / 64) * 64 * kEmb; }
+
+// Activations a backward pass needs (null pointers: scoring only).
+struct Activations {
+  bf16 *x = nullptr, *h1 = nullptr, *h2 = nullptr;  // [rows][64], [rows][128], [rows][128]
+  u32 *open1 = nullptr, *open2 = nullptr;           // [rows][4]: bit c of word c / 32 = pre-activation above zero
 };
 
-// C[i*ldc + j] (= or +=) sum_k A(i,k) B(k,j) for i < M, j < N <= 128; `atomic`
-// accumulates with atomicAdd (required when split > 1: K is cut in `split`
-// slices, one per grid z).
-void gemm(View A, View B, float* C, int ldc, int M, int N, int K, bool atomic, int split, cudaStream_t s);
+// epre = feat · Phi + c (fp32, n x 64), staged = bf16(relu(epre)).
+void embed(const float* feat, const float* params, int n, float* epre, bf16* staged, cudaStream_t s);
+// y of `count` sets (device rows of W words).
+void forward(const u64* rows, int W, int n, u32 count, const bf16* staged_e, const bf16* weights, const float* params,
+             float* y, const Activations& act, cudaStream_t s);
+// loss[0] += mean (y - t)^2 plus, with grp and w > 0, w / rows sum over pairs of one
+// group with t_a < t_b of softplus(y_a - y_b); dy = its gradient in y.
+void loss(const float* y, const float* t, const uint32_t* grp, int rows, float w, float* dy, float* loss,
+          cudaStream_t s);
+// grad += the gradients of W1, b1, W2, b2, w3, b3; de (n x 64, zero before) += the embeddings'.
+void backward(const u64* rows, int W, int n, u32 count, const float* dy, const bf16* weights, const float* params,
+              const Activations& act, float* grad, float* de, cudaStream_t s);
+// grad += the gradients of Phi and c; de is cleared.
+void embed_back(const float* feat, const float* epre, int n, float* de, float* grad, cudaStream_t s);
+// Adam step t (1-based) on the parameters, which also refreshes the staged
+// weights and clears the gradient.
+void adam(float* p, float* g, float* m, float* v, bf16* weights, float lr, int t, cudaStream_t s);
+void stage_weights(const float* p, bf16* weights, cudaStream_t s);
+
 // True once a product's bounded wait for its tensor-core work ran out (its
 // results are then incomplete); synchronises with the device.
 bool tc_error();
-
-// Set rows (device layout, W words) -> dense 0/1 bf16 rows of width ld (>= n).
-void bits_to_dense(const u64* rows, int W, int n, u32 count, __nv_bfloat16* out, int ld, cudaStream_t s);
-
-// act = bf16(relu(in + bias)); keeps `in + bias` in `pre` when pre != nullptr.
-// With relu == false only the bias is added.
-void bias_act(const float* in, const float* bias, int rows, int cols, bool relu, float* pre, __nv_bfloat16* act,
-              cudaStream_t s);
-
-// y[b] = sum_j H[b][j] * w3[j] + b3 (w3, b3 from the fp32 parameters).
-void head(const __nv_bfloat16* H, const float* params, int rows, float* y, cudaStream_t s);
-
-// Loss 1/B sum (y - t)^2 (loss[0] += ...) and dy = 2 (y - t) / B.
-void mse(const float* y, const float* t, int rows, float* dy, float* loss, cudaStream_t s);
-// Adds w/B sum over pairs of one group with t_a < t_b of softplus(y_a - y_b)
-// to the loss and its gradient to dy (a within-layer ranking term).
-void rank_add(const float* y, const float* t, const uint32_t* grp, int rows, float w, float* dy, float* loss,
-              cudaStream_t s);
-
-// From dy: grad of w3 and b3 (grad vector, accumulated), and the masked
-// hidden gradient dH = dy w3^T * [pre > 0] (fp32 and bf16).
-void head_back(const float* dy, const __nv_bfloat16* H, const float* pre, const float* params, int rows, float* grad,
-               float* dH, __nv_bfloat16* dHb, cudaStream_t s);
-
-// d = d * [pre > 0] in place, bf16 copy in db (nullptr: none).
-void relu_back(float* d, const float* pre, int count, __nv_bfloat16* db, cudaStream_t s);
-
-// out[j] += sum_i M[i*cols + j].
-void col_sum(const float* M, int rows, int cols, float* out, cudaStream_t s);
-
-// fp32 -> bf16.
-void to_bf16(const float* in, __nv_bfloat16* out, int count, cudaStream_t s);
-
-// Adam step (t = 1-based step count) on the parameter vector.
-void adam(float* p, const float* g, float* m, float* v, int count, float lr, int t, cudaStream_t s);
 
 }  // namespace mlp
 }  // namespace sw
