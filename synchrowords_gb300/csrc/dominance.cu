@@ -67,15 +67,13 @@ __device__ __forceinline__ void and_column(u32* acc, const u32* col) {
 
 // Block (chunk of T, slice of X).  kHitT: flags[t] = 1 for every row t of T
 // that holds some x; else flags[x] = 1 for every row x of X that some t holds.
-// kComp: rows are complements of the sets.  decided (may be null): rows of T
-// (kHitT) or X whose answer is not wanted.  index (may be null): what row t of T is
-// called in flags and decided.
+// kComp: rows are complements of the sets.  Rows flagged before are left out.
+// index (may be null): what row t of T is called in flags.
 template <int W, int V, bool kComp, bool kHitT>
 __global__ void __launch_bounds__(dom_threads<V>()) k_dominance(const u64* __restrict__ T, u32 tm,
                                                                const u32* __restrict__ index,
                                                                const u64* __restrict__ X, u32 xm, int n, int proper,
-                                                               u32 per_slice, u32 per_warp,
-                                                               const u32* __restrict__ decided, u32* flags) {
+                                                               u32 per_slice, u32 per_warp, u32* flags) {
   extern __shared__ __align__(16) u32 s_dom[];
   __shared__ u32 s_max;
   constexpr u32 kStride = col_stride<V>();
@@ -103,7 +101,7 @@ __global__ void __launch_bounds__(dom_threads<V>()) k_dominance(const u64* __res
     }
     s_size[r] = (uint16_t)size;
     bool in = r < rows;
-    if (kHitT && decided && in) in = !decided[index ? index[r0 + r] : r0 + r];
+    if (kHitT && in) in = !*(volatile u32*)(flags + (index ? index[r0 + r] : r0 + r));
     const u32 open = __ballot_sync(kFullWarp, in);
     const u32 most = __reduce_max_sync(kFullWarp, size);
     if (lane == 0) {
@@ -132,7 +130,7 @@ __global__ void __launch_bounds__(dom_threads<V>()) k_dominance(const u64* __res
     }
     // no row of the chunk is as large as a larger set (nor, for a proper subset, larger than one as large)
     bool want = valid && (proper ? size < most : size <= most);
-    if (!kHitT && want) want = !*(volatile u32*)(flags + xi) && !(decided && decided[xi]);
+    if (!kHitT && want) want = !*(volatile u32*)(flags + xi);
     u32 todo = __ballot_sync(kFullWarp, want);
     while (todo) {
       const int j = __ffs(todo) - 1;
@@ -220,7 +218,7 @@ __global__ void __launch_bounds__(256) k_size_scatter(const u64* __restrict__ T,
 namespace {
 template <int W, int V>
 void launch_dom(bool comp, bool hit_t, const u64* T, u32 tm, const u32* index, const u64* X, u32 xm, int n, bool proper,
-                const u32* decided, u32* flags, cudaStream_t s) {
+                u32* flags, cudaStream_t s) {
   const u32 chunks = (tm + 1024 * V - 1) / (1024 * V);
   constexpr u32 kThreads = dom_threads<V>(), kWarps = kThreads / 32;
   // slices of X: as many blocks as fit the GPU a few times over, while a warp keeps eight sets or more
@@ -235,7 +233,7 @@ void launch_dom(bool comp, bool hit_t, const u64* T, u32 tm, const u32* index, c
   {                                                                                                           \
     ensure_smem_limit((const void*)k_dominance<W, V, C, H>, (int)smem);                                       \
     k_dominance<W, V, C, H><<<grid, kThreads, smem, s>>>(T, tm, index, X, xm, n, proper ? 1 : 0, per, per_warp, \
-                                                         decided, flags);                                     \
+                                                         flags);                                     \
   }
   if (comp) {
     if (hit_t) SW_DOM(true, true) else SW_DOM(true, false)
@@ -247,36 +245,36 @@ void launch_dom(bool comp, bool hit_t, const u64* T, u32 tm, const u32* index, c
 }
 template <int W>
 void launch_dom_w(bool comp, bool hit_t, const u64* T, u32 tm, const u64* X, u32 xm, int n, bool proper,
-                  const u32* decided, u32* flags, const DominanceScratch& sc, cudaStream_t s) {
+                  u32* flags, const DominanceScratch& sc, cudaStream_t s) {
+  constexpr int V = W < 7 ? 4 : 2;
   // small lists: 1024-row chunks, so that they spread over more blocks
-  if (tm <= kDomSmallRows) {
-    launch_dom<W, 1>(comp, hit_t, T, tm, nullptr, X, xm, n, proper, decided, flags, s);
-    return;
-  }
+  if (tm <= kDomSmallRows) return launch_dom<W, 1>(comp, hit_t, T, tm, nullptr, X, xm, n, proper, flags, s);
+  if (tm <= kDomOrderRows) return launch_dom<W, V>(comp, hit_t, T, tm, nullptr, X, xm, n, proper, flags, s);
   const u32 blocks = (tm + 255) / 256;
   if (comp)
     k_size_rank<W, true><<<blocks, 256, 0, s>>>(T, tm, n, sc.bucket.counts, sc.bucket.place);
   else
     k_size_rank<W, false><<<blocks, 256, 0, s>>>(T, tm, n, sc.bucket.counts, sc.bucket.place);
-  launch_bucket_scan(BucketScratch{kBucketBitsSmall, sc.bucket.counts, sc.bucket.first, sc.bucket.place}, sc.total, s);
+  launch_bucket_scan(BucketScratch{kBucketBitsSmall, sc.bucket.counts, sc.bucket.first, sc.bucket.place, sc.bucket.met},
+                     sc.total, s);
   k_size_scatter<W><<<blocks, 256, 0, s>>>(T, tm, sc.bucket.place, sc.bucket.first, sc.rows, sc.index);
   SW_LAUNCH_CHECK();
-  launch_dom<W, (W < 7 ? 4 : 2)>(comp, hit_t, sc.rows, tm, sc.index, X, xm, n, proper, decided, flags, s);
+  launch_dom<W, V>(comp, hit_t, sc.rows, tm, sc.index, X, xm, n, proper, flags, s);
 }
 }  // namespace
 
 void launch_dominance(int W, bool comp, bool hit_t, const u64* T, u32 tm, const u64* X, u32 xm, int n, bool proper,
-                      const u32* decided, u32* flags, const DominanceScratch& sc, cudaStream_t s) {
+                      u32* flags, const DominanceScratch& sc, cudaStream_t s) {
   if (!tm || !xm) return;
   switch (W) {
-    case 1: return launch_dom_w<1>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
-    case 2: return launch_dom_w<2>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
-    case 3: return launch_dom_w<3>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
-    case 4: return launch_dom_w<4>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
-    case 5: return launch_dom_w<5>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
-    case 6: return launch_dom_w<6>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
-    case 7: return launch_dom_w<7>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
-    case 8: return launch_dom_w<8>(comp, hit_t, T, tm, X, xm, n, proper, decided, flags, sc, s);
+    case 1: return launch_dom_w<1>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
+    case 2: return launch_dom_w<2>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
+    case 3: return launch_dom_w<3>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
+    case 4: return launch_dom_w<4>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
+    case 5: return launch_dom_w<5>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
+    case 6: return launch_dom_w<6>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
+    case 7: return launch_dom_w<7>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
+    case 8: return launch_dom_w<8>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
     default: throw std::runtime_error("dominance: unsupported width");
   }
 }

@@ -47,14 +47,16 @@ struct Side {
   u32 count = 0;
   DevBuf vis, vis_alt;
   u32 vis_count = 0;
-  // While only duplicates are removed (Engine::step_hashed) the visited list is
-  // appended to layer by layer and a hash table names its rows; the current
-  // layer is then its tail (in_vis), else it is `rows`.  The reductions need the
-  // visited list in key order: the first of them ends this (Engine::unhash).
-  bool hashed = false, reduced = false, in_vis = false;
+  // Hashed sides (Engine::step_hashed) append each layer to the visited list,
+  // whose tail the current layer then is (in_vis; else it is `rows`), and keep a
+  // hash table of every distinct row met.  Its slots name rows of vis until a
+  // reduction drops one; from then on (split) they name rows of `met`, which
+  // keeps the dropped ones too.
+  bool hashed = false, sorted_only = false, in_vis = false, split = false;
   u32 cur_off = 0;  // first row of the current layer in vis
-  DevBuf table;
-  u64 table_slots = 0;  // 0: to be built from vis
+  DevBuf table, met;
+  u32 met_count = 0;    // rows of met (split)
+  u64 table_slots = 0;  // 0: to be built
   const u64* cur_rows(int W) const { return in_vis ? vis.as<u64>() + (size_t)cur_off * W : rows.as<u64>(); }
   std::vector<std::unique_ptr<Layer>> layers;
   std::vector<u64> seed_states;  // backward side: the state of each seed row
@@ -83,7 +85,7 @@ struct Side {
   }
   void reset() {
     count = vis_count = 0;
-    hashed = reduced = in_vis = false;
+    hashed = sorted_only = in_vis = split = false;
     table_slots = 0;
     unique_growth = 0;
     keymap = KeyMap{};
@@ -204,7 +206,7 @@ class Engine {
     }
     prof_on = false;
   }
-  u32* d_misc = nullptr;  // [0..2] witness, [3] the subset check's size floor, [8] scan total, [9] the check's unit count, [kScanErrWord] bounded-wait timeouts
+  u32* d_misc = nullptr;  // [0..2] witness, [3] the subset check's size floor, [6, 7] children met before, [8] scan total, [12, 13] the check's unit counts, [kScanErrWord] bounded-wait timeouts
   static constexpr int kScanErrWord = 4;  // read back with the witness, never cleared by it
   // Throws if a launch reported a bounded wait that ran out: 2 = a compaction
   // tile's look-back never saw its predecessor, 3 = a hash table's probe found
@@ -347,7 +349,7 @@ class Engine {
     // algorithmic bytes: the query rows plus every row of S a query is tested against
     timed(0, (double)q * 8.0 * W, [&] {
       launch_subset_check(W, mode, S, m, tile_and.as<u64>(), size_floor, Q, q, n, flags, d_misc, stop, sh, stream,
-                          prof_on ? d_query_bytes : nullptr, scan_items.as<uint2>(), d_misc + 9);
+                          prof_on ? d_query_bytes : nullptr, scan_items.as<uint2>(), d_misc + 12);
     });
     if (prof_on) {
       cudaEvent_t e1 = next_event();
@@ -362,11 +364,9 @@ class Engine {
   }
 
   // flags[i] = 1 where a row of S (a proper one) is inside child row i of Q, on
-  // the forward side or on complement rows; children `decided` already may be
-  // left out.
+  // the forward side or on complement rows; children flagged already are left out.
   DevBuf dom_rows, dom_index;
-  void dominated(bool forward, int W, const u64* S, u32 m, const u64* Q, u32 q, int n, bool proper, const u32* decided,
-                 u32* flags) {
+  void dominated(bool forward, int W, const u64* S, u32 m, const u64* Q, u32 q, int n, bool proper, u32* flags) {
     if (!m || !q) return;
     cudaEvent_t e0 = nullptr;
     if (prof_on) {
@@ -375,7 +375,7 @@ class Engine {
     }
     DominanceScratch sc;
     const u32 tm = forward ? q : m;  // rows that hold: children forward, visited or siblings backward
-    if (tm > kDomSmallRows) {
+    if (tm > kDomOrderRows) {
       sc.bucket = buckets(tm);
       dom_rows.reserve(sizeof(u64) * W * (size_t)tm);
       dom_index.reserve(sizeof(u32) * (size_t)tm);
@@ -386,9 +386,9 @@ class Engine {
     }
     timed(0, (double)(m + q) * 8.0 * W, [&] {
       if (forward)  // sets s ⊆ c: the children hold them
-        launch_dominance(W, false, true, Q, q, S, m, n, proper, decided, flags, sc, stream);
+        launch_dominance(W, false, true, Q, q, S, m, n, proper, flags, sc, stream);
       else  // complements: the set of c lies in the set of s
-        launch_dominance(W, true, false, S, m, Q, q, n, proper, decided, flags, sc, stream);
+        launch_dominance(W, true, false, S, m, Q, q, n, proper, flags, sc, stream);
     });
     if (prof_on) {
       cudaEvent_t e1 = next_event();
@@ -437,7 +437,8 @@ class Engine {
     }
     bk_first.reserve(bytes);
     bk_place.reserve(sizeof(uint2) * children);
-    return BucketScratch{bucket_bits(children), bk_counts.as<u32>(), bk_first.as<u32>(), bk_place.as<uint2>()};
+    return BucketScratch{bucket_bits(children), bk_counts.as<u32>(), bk_first.as<u32>(), bk_place.as<uint2>(),
+                         d_misc + 6};
   }
   // Power-of-two slots, two to four per row.
   static u64 slots_for(u64 rows) {
@@ -445,36 +446,46 @@ class Engine {
     while (s < 2 * rows) s *= 2;
     return s;
   }
-  // Room for `rows` more rows at the end of X's visited list; returns the row
-  // index they start at (even where rows are an odd number of words, so that
-  // the layer stays 16-byte aligned for the subset check's tile copies; the row
-  // before it then repeats row 0, which is visited anyway).
-  u32 append_base(Side& X, int W, u64 rows) {
-    const u32 base = X.vis_count + ((W & 1) ? (X.vis_count & 1u) : 0u);
-    const size_t need = sizeof(u64) * W * (base + rows);
-    if (X.vis.cap < need) {
-      X.vis_alt.reserve(std::max(need, 2 * X.vis.cap));
-      SW_CUDA(cudaMemcpyAsync(X.vis_alt.p, X.vis.p, sizeof(u64) * W * (size_t)X.vis_count, cudaMemcpyDeviceToDevice,
-                              stream));
-      std::swap(X.vis.p, X.vis_alt.p);
-      std::swap(X.vis.cap, X.vis_alt.cap);
-    }
-    if (base != X.vis_count)
-      SW_CUDA(cudaMemcpyAsync(X.vis.as<u64>() + (size_t)X.vis_count * W, X.vis.p, sizeof(u64) * W,
-                              cudaMemcpyDeviceToDevice, stream));
-    return base;
+  // Room for `rows` more rows behind the first `count` of `buf`, which are kept.
+  void grow_rows(DevBuf& buf, DevBuf& spare, int W, u64 count, u64 rows) {
+    const size_t need = sizeof(u64) * W * (count + rows);
+    if (buf.cap >= need) return;
+    spare.reserve(std::max(need, 2 * buf.cap));
+    SW_CUDA(cudaMemcpyAsync(spare.p, buf.p, sizeof(u64) * W * (size_t)count, cudaMemcpyDeviceToDevice, stream));
+    std::swap(buf.p, spare.p);
+    std::swap(buf.cap, spare.cap);
   }
-  void step_hashed(Side& X, bool forward, int W, int k) {
+  // Lists up to this size are hashed; larger ones, whose table and spare copies
+  // would take several times as much again, are kept sorted.
+  static constexpr u64 kHashBytes = 16ull << 30;
+  static bool hashable(const Side& X, int W, u64 children) {
+    const u64 rows = (X.split ? X.met_count : X.vis_count) + children + 1;
+    return !X.sorted_only && 2 * rows <= 1ull << 32 && rows * 8 * W <= kHashBytes;
+  }
+  // One layer on a hashed side: children equal to a row met before or to a sibling
+  // are dropped by the table, then, with the reductions on, those that a visited
+  // set or a sibling dominates.
+  void step_hashed(Side& X, bool forward, int W, int n, int k) {
     const u32 m = X.count, Nc = m * (u32)k;
     const double t_step0 = vclock();
+    const bool reduce = self_check || visited_subsets;
     X.hashed = true;
-    const u32 base = append_base(X, W, Nc);
+    if (reduce && !X.split) {
+      X.split = true;
+      X.met_count = X.vis_count;
+      X.met.reserve(sizeof(u64) * W * ((size_t)X.vis_count + Nc));
+      SW_CUDA(cudaMemcpyAsync(X.met.p, X.vis.p, sizeof(u64) * W * (size_t)X.vis_count, cudaMemcpyDeviceToDevice,
+                              stream));
+    }
+    DevBuf& list = X.split ? X.met : X.vis;
+    const u32 base = X.split ? X.met_count : X.vis_count;
+    grow_rows(list, X.vis_alt, W, base, Nc);
     if (2 * X.table_slots < 3 * ((u64)base + Nc)) {  // fewer than 1.5 slots a row: rebuild
       X.table_slots = slots_for((u64)base + Nc);
       X.table.reserve(sizeof(u64) * X.table_slots);
       SW_CUDA(cudaMemsetAsync(X.table.p, 0, sizeof(u64) * X.table_slots, stream));
       timed(3, (double)base * (8.0 * W + 8), [&] {
-        launch_hash_build(W, X.vis.as<u64>(), base, X.table.as<u64>(), (u32)(X.table_slots - 1), d_misc + kScanErrWord,
+        launch_hash_build(W, list.as<u64>(), base, X.table.as<u64>(), (u32)(X.table_slots - 1), d_misc + kScanErrWord,
                           stream);
       });
       count_launch();
@@ -483,32 +494,57 @@ class Engine {
     const BucketScratch bk = buckets(Nc);
     // reads each parent row, writes k child rows, a table slot and a place each
     timed(1, (double)m * 8.0 * W * (1 + k) + (double)Nc * 16.0, [&] {
-      launch_expand_hash(W, forward, X.cur_rows(W), m, tables, ch_rows.as<u64>(), X.vis.as<u64>(), base,
+      launch_expand_hash(W, forward, X.cur_rows(W), m, tables, ch_rows.as<u64>(), list.as<u64>(), base,
                          X.table.as<u64>(), (u32)(X.table_slots - 1), bk, d_misc + kScanErrWord, stream);
     });
     std::unique_ptr<Layer> L = X.new_layer(sizeof(u32) * (size_t)std::max<u32>(Nc, 1));
     L->origin.reserve(sizeof(u32) * (size_t)std::max<u32>(Nc, 1));
+    if (X.split) uq_vals.reserve(sizeof(u32) * (size_t)std::max<u32>(Nc, 1));
+    u64* const fresh = list.as<u64>() + (size_t)base * W;  // the new rows, in bucket order
+    u32* const fresh_origin = X.split ? uq_vals.as<u32>() : L->origin.as<u32>();
     timed(3, (double)Nc * (2 * 8.0 * W + 8 + 4), [&] {
-      launch_bucket_scatter(W, ch_rows.as<u64>(), Nc, bk, base, X.vis.as<u64>() + (size_t)base * W,
-                            L->origin.as<u32>(), X.table.as<u64>(), d_misc + 8, stream);
+      launch_bucket_scatter(W, ch_rows.as<u64>(), Nc, bk, base, fresh, fresh_origin, X.table.as<u64>(), d_misc + 8,
+                            stream);
     });
     count_launch(3);
-    const u32 f = read_total_checked();
-    if (m) X.unique_growth = (double)f / m;
-    if (st) {
-      st->subsets_expanded += Nc;
-      st->subsets_kept += f;
+    const u32 u = read_total_checked();
+    // branching of a level that drops siblings only (the bounded phase's)
+    if (m) X.unique_growth = (double)(u + pinned.as<u32>()[7 - kScanErrWord]) / m;
+    if (st) st->subsets_expanded += Nc;
+    u32 f = u;
+    if (X.split) {
+      X.met_count = base + u;
+      grow_rows(X.vis, X.vis_alt, W, X.vis_count, u);
+      u64* const out = X.vis.as<u64>() + (size_t)X.vis_count * W;
+      if (reduce && u) {
+        flags_a.reserve(sizeof(u32) * (size_t)u);
+        SW_CUDA(cudaMemsetAsync(flags_a.p, 0, sizeof(u32) * (size_t)u, stream));
+        if (X.vis_count && visited_subsets)
+          dominated(forward, W, X.vis.as<u64>(), X.vis_count, fresh, u, n, false, flags_a.as<u32>());
+        if (self_check) dominated(forward, W, fresh, u, fresh, u, n, true, flags_a.as<u32>());
+        const u32 epoch = next_dc_epoch(u);
+        timed(3, (double)u * (4 + 2 * (8.0 * W + 4)), [&] {
+          launch_keep_compact(W, fresh, fresh_origin, flags_a.as<u32>(), u, out, L->origin.as<u32>(), d_misc + 8,
+                              dc_status.as<u64>(), dc_ctr.as<u32>(), epoch, d_misc + kScanErrWord, stream);
+        });
+        count_launch();
+        f = read_total_checked();
+      } else if (u) {
+        SW_CUDA(cudaMemcpyAsync(out, fresh, sizeof(u64) * W * (size_t)u, cudaMemcpyDeviceToDevice, stream));
+        SW_CUDA(cudaMemcpyAsync(L->origin.p, fresh_origin, sizeof(u32) * (size_t)u, cudaMemcpyDeviceToDevice, stream));
+      }
     }
+    if (st) st->subsets_kept += f;
     L->count = f;
     L->parent_count = m;
     X.layers.push_back(std::move(L));
     X.in_vis = true;
-    X.cur_off = base;
+    X.cur_off = X.vis_count;
     X.count = f;
-    X.vis_count = base + f;
+    X.vis_count += f;
     if (verbose)
-      std::fprintf(stderr, "[sw] %s parents=%u children=%u kept=%u (duplicates only) | %.3f ms\n",
-                   forward ? "BFS " : "IBFS", m, Nc, f, vclock() - t_step0);
+      std::fprintf(stderr, "[sw] %s parents=%u children=%u unique=%u kept=%u (%s) | %.3f ms\n", forward ? "BFS " : "IBFS",
+                   m, Nc, u, f, reduce ? "reduced" : "duplicates only", vclock() - t_step0);
   }
   // Back to a current layer of its own and a visited list in key order.
   void unhash(Side& X, int W) {
@@ -518,21 +554,21 @@ class Engine {
       SW_CUDA(cudaMemcpyAsync(X.rows.p, X.cur_rows(W), sizeof(u64) * W * (size_t)X.count, cudaMemcpyDeviceToDevice,
                               stream));
     }
-    X.hashed = X.in_vis = false;
+    X.hashed = X.in_vis = X.split = false;
     X.table_slots = 0;
     sort_by_layer_key(W, X.vis.as<u64>(), X.vis_count, X.keymap);
   }
 
-  void step(Side& X, bool forward, int W, int n, int k, bool dominance = true) {
+  // `ordered`: the layer's rows come in key order, the same on every run
+  // (samples of a layer, and beams whose ties go by it, depend on that).
+  void step(Side& X, bool forward, int W, int n, int k, bool dominance = true, bool ordered = false) {
     const u32 m = X.count;
     const u64 N = (u64)m * k;
     if (N > 0xffffffffULL) throw std::runtime_error("layer exceeds 2^32 children");
     const u32 Nc = (u32)N;
-    if (dominance && !self_check && !visited_subsets && !X.reduced && !sort_key_option() &&
-        2 * ((u64)X.vis_count + N + 1) <= 1ull << 32)
-      return step_hashed(X, forward, W, k);
+    if (dominance && !ordered && !sort_key_option() && hashable(X, W, N)) return step_hashed(X, forward, W, n, k);
     unhash(X, W);
-    X.reduced = true;
+    X.sorted_only = true;
     ch_rows.reserve(sizeof(u64) * W * N);
     ch_vals.reserve(sizeof(u32) * N);
     uq_rows.reserve(sizeof(u64) * W * N);
@@ -612,8 +648,7 @@ class Engine {
     const double t_sort = vclock();
     if (X.vis_count) {
       if (visited_subsets) {
-        dominated(forward, W, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, n, false, nullptr,
-                  flags_a.as<u32>());
+        dominated(forward, W, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, n, false, flags_a.as<u32>());
       } else {
         timed(3, (double)u * 8.0 * W, [&] {
           launch_member_key(W, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, flags_a.as<u32>(), stream,
@@ -624,8 +659,7 @@ class Engine {
     }
     const double t_vis = vclock();
     if (self_check)
-      dominated(forward, W, uq_rows.as<u64>(), u, uq_rows.as<u64>(), u, n, true, flags_a.as<u32>(),
-                flags_b.as<u32>());
+      dominated(forward, W, uq_rows.as<u64>(), u, uq_rows.as<u64>(), u, n, true, flags_b.as<u32>());
     const double t_self = vclock();
     if (verbose) {
       std::vector<u32> fa(u), fb(u);
@@ -805,7 +839,9 @@ class Engine {
     ClusterExit exit;
     const uint8_t* word;
   };
-  Single run_single(const Automaton& A, const std::vector<uint32_t>& seeds, u32 max_len, u64 budget) {
+  // `meanwhile` runs on the host while the cluster searches.
+  template <class Fn>
+  Single run_single(const Automaton& A, const std::vector<uint32_t>& seeds, u32 max_len, u64 budget, Fn&& meanwhile) {
     const int W = words_for((int)A.n);
     const ClusterCaps caps = cluster_single_caps();
     single_scratch.reserve(cluster_single_scratch_bytes(caps));
@@ -844,6 +880,7 @@ class Engine {
     count_launch();
     uint8_t* out = h + 8192;
     SW_CUDA(cudaMemcpyAsync(out, sc + 256, out_bytes, cudaMemcpyDeviceToHost, stream));
+    meanwhile();
     SW_CUDA(cudaStreamSynchronize(stream));
     Single r;
     std::memcpy(&r.res, out + kClusterSingleResult - 256, sizeof(r.res));
@@ -873,11 +910,9 @@ class Engine {
       launch_cluster_export(W, single_scratch.p, kClusterSingleHeader, caps, side, kept, depth, ch_rows.as<u64>(),
                             single_org[side].as<u32>(), stream);
       // the visited list: the earlier layers as they are, then the current one in bucket order
-      X.vis_count = kept - cnt;
-      X.vis.reserve(sizeof(u64) * W * ((size_t)kept + 1));
-      SW_CUDA(cudaMemcpyAsync(X.vis.p, ch_rows.p, sizeof(u64) * W * std::max<u32>(X.vis_count, 1),
-                              cudaMemcpyDeviceToDevice, stream));
-      const u32 base = append_base(X, W, cnt);
+      const u32 base = kept - cnt;
+      X.vis.reserve(sizeof(u64) * W * (size_t)kept);
+      SW_CUDA(cudaMemcpyAsync(X.vis.p, ch_rows.p, sizeof(u64) * W * (size_t)base, cudaMemcpyDeviceToDevice, stream));
       const u64* cur = ch_rows.as<u64>() + (size_t)(kept - cnt) * W;
       const BucketScratch bk = buckets(cnt);
       ch_vals.reserve(sizeof(u32) * cnt);
@@ -1030,13 +1065,17 @@ void Solver::last_scan_profile(double ms[8 * kScanSizeClasses], uint64_t checks[
 static std::vector<uint32_t> image_frequency_order(const Automaton& A) {
   const uint32_t n = A.n, k = A.k;
   std::vector<double> pi(n, 1.0 / n), nx(n);
+  const double share = 0.99 / k;
   for (int it = 0; it < 200; ++it) {
     std::fill(nx.begin(), nx.end(), 0.01 / n);
     for (uint32_t q = 0; q < n; ++q) {
-      const double w = 0.99 * pi[q] / k;
+      const double w = share * pi[q];
       for (uint32_t a = 0; a < k; ++a) nx[A.at(q, a)] += w;
     }
+    double moved = 0;
+    for (uint32_t q = 0; q < n; ++q) moved += std::abs(nx[q] - pi[q]);
     pi.swap(nx);
+    if (moved < 1e-9) break;  // settled (random automata: after 30 to 60 rounds)
   }
   std::vector<uint32_t> idx(n);
   std::iota(idx.begin(), idx.end(), 0u);
@@ -1079,11 +1118,14 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
   };
   // A search with duplicate removal only starts on one thread-block cluster
   // (the other reductions and reduced forward seeds are the streamed path's).
-  bool imported = false;
+  bool imported = false, checked = false, synchronizing = false;
   ClusterExit single_exit{};
   if (!red && !b.has_word && cfg.reductions != SW_REDUCE_ALWAYS && !Engine::sort_key_option() && n <= 256 && n * k <= 4096 && !seeds.empty() &&
       max_rt > 0) {
-    const Engine::Single S = E.run_single(A, seeds, (u32)std::min<u64>(max_rt, kClusterSingleWord), budget);
+    const Engine::Single S = E.run_single(A, seeds, (u32)std::min<u64>(max_rt, kClusterSingleWord), budget, [&] {
+      synchronizing = is_synchronizing(A);
+      checked = true;
+    });
     if (E.verbose)
       std::fprintf(stderr, "[sw] first levels on a cluster: status %u why %u, len %u, |F|=%u |B|=%u, %llu children\n",
                    S.res.status, S.res.why & 255u, S.res.length, S.exit.cnt[0], S.exit.cnt[1], S.exit.children);
@@ -1106,7 +1148,7 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
       rt = S.res.length;
     }
   }
-  if (!is_synchronizing(A)) {
+  if (!(checked ? synchronizing : is_synchronizing(A))) {
     // The reference's Exact has no such check and runs until its bound; a
     // non-synchronizing automaton is reported as such instead.
     b.non_synchro = true;
@@ -1734,7 +1776,7 @@ void Solver::reduce(const Automaton& A, const sw_reduce_config& cfg, Bounds& b, 
     const u32 m = E.F.count;
     if (!m) continue;
     counts.reserve(sizeof(u32) * m);
-    launch_popcount(W, E.F.rows.as<u64>(), m, counts.as<u32>(), E.stream);
+    launch_popcount(W, E.F.cur_rows(W), m, counts.as<u32>(), E.stream);
     E.count_launch();
     std::vector<u32> pc(m);
     SW_CUDA(cudaMemcpyAsync(pc.data(), counts.p, sizeof(u32) * m, cudaMemcpyDeviceToHost, E.stream));
@@ -1765,7 +1807,7 @@ void Solver::reduce(const Automaton& A, const sw_reduce_config& cfg, Bounds& b, 
   // reduce.hpp:112-143 (try_to_reduce): states reachable from the list
   const u32 m = E.F.count;
   std::vector<u64> rows((size_t)m * W);
-  if (m) SW_CUDA(cudaMemcpyAsync(rows.data(), E.F.rows.p, sizeof(u64) * W * m, cudaMemcpyDeviceToHost, E.stream));
+  if (m) SW_CUDA(cudaMemcpyAsync(rows.data(), E.F.cur_rows(W), sizeof(u64) * W * m, cudaMemcpyDeviceToHost, E.stream));
   SW_CUDA(cudaStreamSynchronize(E.stream));
   std::vector<char> reach(n, 0);
   std::vector<uint32_t> stack;
@@ -1908,7 +1950,7 @@ uint32_t Solver::distance_pairs(const Automaton& A, uint32_t per_layer, uint64_t
   };
   keep_layer();
   for (u64 j = 1; j <= L && inv_total < max_inverse_sets; ++j) {
-    E.step(E.B, false, W, n, k, true);
+    E.step(E.B, false, W, n, k, true, true);
     if (!E.B.count) break;
     keep_layer();
   }
@@ -1957,7 +1999,7 @@ uint32_t Solver::distance_pairs(const Automaton& A, uint32_t per_layer, uint64_t
     labels.insert(labels.end(), lab.begin(), lab.end());
     depths.insert(depths.end(), s, (uint32_t)i);
     if (i == L) break;
-    E.step(E.F, true, W, n, k, true);
+    E.step(E.F, true, W, n, k, true, true);
     if (!E.F.count) break;
   }
   return (uint32_t)L;

@@ -409,9 +409,11 @@ void launch_expand(int W, bool image, const u64* in, u32 m, const TransTables& t
 namespace {
 // Slot: bit 63 set, 31 bits of the hash, row index (a row of V below `base`,
 // else child index - base of this launch).
+// 0: entered at *at; 1: equal to a child of this launch; 2: equal to a row of V.
+constexpr int kNew = 0, kSibling = 1, kMet = 2;
 template <int W>
-__device__ __forceinline__ bool hash_insert(u64* tab, u32 tmask, const u64* V, u32 base, const u64* C, const u64* x,
-                                            u32 idx, u32* at, u32* err) {
+__device__ __forceinline__ int hash_insert(u64* tab, u32 tmask, const u64* V, u32 base, const u64* C, const u64* x,
+                                           u32 idx, u32* at, u32* err) {
   const u64 h = row_hash<W>(x);
   const u64 mine = (h & 0xffffffff00000000ULL) | (1ULL << 63) | idx;
   u32 s = (u32)h & tmask;
@@ -421,18 +423,19 @@ __device__ __forceinline__ bool hash_insert(u64* tab, u32 tmask, const u64* V, u
       v = atomicCAS(&tab[s], 0ULL, mine);
       if (v == 0) {
         *at = s;
-        return true;
+        return kNew;
       }
     }
     if ((v ^ mine) >> 32 == 0) {
       __threadfence();  // the row was written before its slot
       const u32 r = (u32)v;
-      if (row_eq_volatile<W>(r >= base ? C + (size_t)(r - base) * W : V + (size_t)r * W, x)) return false;
+      if (row_eq_volatile<W>(r >= base ? C + (size_t)(r - base) * W : V + (size_t)r * W, x))
+        return r >= base ? kSibling : kMet;
     }
     s = (s + 1) & tmask;
   }
   atomicExch(err, 3u);
-  return false;
+  return kSibling;
 }
 constexpr u32 kDropped = 0xffffffffu;
 
@@ -456,7 +459,7 @@ template <int W, bool kImage>
 __global__ void __launch_bounds__(kExpThreads) k_expand_hash(const u64* __restrict__ in, u32 m, TransTables t, u64* C,
                                                              const u64* V, u32 base, u64* tab, u32 tmask,
                                                              u32* __restrict__ counts, int shift,
-                                                             uint2* __restrict__ place, u32* err) {
+                                                             uint2* __restrict__ place, u32* met, u32* err) {
   extern __shared__ uint16_t s_tab[];
   __shared__ u32 s_cols[kExpWarps][64 * W];
   stage_tables<kImage>(t, s_tab);
@@ -473,16 +476,19 @@ __global__ void __launch_bounds__(kExpThreads) k_expand_hash(const u64* __restri
     }
     __threadfence();  // the row before its slot
     u32 at = 0;
-    const bool keep = p < m && hash_insert<W>(tab, tmask, V, base, C, x, base + e, &at, err);
-    const u32 rank = bucket_rank(counts, (u32)(x[0] >> shift), keep);
+    const int found = p < m ? hash_insert<W>(tab, tmask, V, base, C, x, base + e, &at, err) : kSibling;
+    const u32 rank = bucket_rank(counts, (u32)(x[0] >> shift), found == kNew);
+    const u32 again = __ballot_sync(kFull, found == kMet);
+    if (lane == 0 && again) atomicAdd(met, (u32)__popc(again));
     if (p < m) place[e] = make_uint2(rank, at);  // rank in its bucket (or dropped), table slot
   }
 }
 
 // counts -> exclusive sums (first row of each bucket), counts cleared for the
-// next layer, *total = rows kept; one block, `bins` a multiple of 4096.
+// next layer, *total = rows kept, met[1] = met[0] and met[0] cleared; one block,
+// `bins` a multiple of 4096.
 __global__ void __launch_bounds__(kScanThreads) k_bucket_scan(u32* __restrict__ counts, u32* __restrict__ first,
-                                                              u32 bins, u32* total) {
+                                                              u32 bins, u32* total, u32* met) {
   u32 carry = 0;
   for (u32 b0 = 0; b0 < bins; b0 += 4 * kScanThreads) {
     const u32 i = b0 + 4 * threadIdx.x;
@@ -493,7 +499,11 @@ __global__ void __launch_bounds__(kScanThreads) k_bucket_scan(u32* __restrict__ 
     *reinterpret_cast<uint4*>(counts + i) = make_uint4(0, 0, 0, 0);
     carry += tot;
   }
-  if (threadIdx.x == 0) *total = carry;
+  if (threadIdx.x == 0) {
+    *total = carry;
+    met[1] = met[0];
+    met[0] = 0;
+  }
 }
 
 template <int W>
@@ -546,7 +556,7 @@ void launch_expand_hash(int W, bool image, const u64* in, u32 m, const TransTabl
   {                                                                                                          \
     if (smem > 32 * 1024) ensure_smem_limit((const void*)k_expand_hash<WW, IMG>, (int)smem);                 \
     k_expand_hash<WW, IMG><<<blocks, kExpThreads, smem, s>>>(in, m, t, C, V, base, tab, tmask, b.counts,     \
-                                                             64 - b.bits, b.place, err);                     \
+                                                             64 - b.bits, b.place, b.met, err);              \
   }
   SW_EXP_DISPATCH(if (image) SW_EXP(true) else SW_EXP(false))
 #undef SW_EXP
@@ -560,7 +570,7 @@ void launch_bucket_rank(int W, const u64* C, u32 m, const BucketScratch& b, cuda
 }
 
 void launch_bucket_scan(const BucketScratch& b, u32* total, cudaStream_t s) {
-  k_bucket_scan<<<1, kScanThreads, 0, s>>>(b.counts, b.first, 1u << b.bits, total);
+  k_bucket_scan<<<1, kScanThreads, 0, s>>>(b.counts, b.first, 1u << b.bits, total, b.met);
   SW_LAUNCH_CHECK();
 }
 
@@ -1284,20 +1294,20 @@ __device__ __forceinline__ void st_release_u64(u64* p, u64 v) {
   asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-template <int W>
-__global__ void __launch_bounds__(kDcTile) k_dedup_compact(const u64* __restrict__ C, const u32* __restrict__ vals,
-                                                          const u64* __restrict__ keys, u32 m,
-                                                          const u64* __restrict__ V, u32 nv, KeyMap map,
-                                                          u64* __restrict__ out_rows, u32* __restrict__ out_vals,
-                                                          u32* total, u64* status, u32* ctr, u32 epoch, u32* err) {
-  __shared__ u32 s_tile, s_warp[kDcTile / 32], s_excl;
-  const u32 ntiles = (m + kDcTile - 1) / kDcTile;
+// Output position of the block's tile-local kept element (valid where `keep`):
+// the block's part of the above, for the tile it drew.
+__device__ __forceinline__ u32 draw_tile(u32* ctr, u32 ntiles) {
+  __shared__ u32 s_tile;
   if (threadIdx.x == 0) s_tile = atomicAdd(ctr, 1u);
   __syncthreads();
   const u32 tile = s_tile;
   if (threadIdx.x == 0 && tile == ntiles - 1) *ctr = 0u;  // every block has drawn its index
-  const u32 i = tile * kDcTile + threadIdx.x;
-  const bool keep = i < m && dedup_keep<W>(C, vals, keys, i, V, nv, map);
+  return tile;
+}
+
+__device__ __forceinline__ u32 tile_position(bool keep, u32 tile, u32 ntiles, u32* total, u64* status, u32 epoch,
+                                             u32* err) {
+  __shared__ u32 s_warp[kDcTile / 32], s_excl;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const u32 ballot = __ballot_sync(0xffffffffu, keep);
   const u32 before_in_warp = __popc(ballot & ((1u << lane) - 1u));
@@ -1342,12 +1352,53 @@ __global__ void __launch_bounds__(kDcTile) k_dedup_compact(const u64* __restrict
     }
   }
   __syncthreads();
+  return s_excl + s_warp[warp] + before_in_warp;
+}
+
+template <int W>
+__global__ void __launch_bounds__(kDcTile) k_dedup_compact(const u64* __restrict__ C, const u32* __restrict__ vals,
+                                                          const u64* __restrict__ keys, u32 m,
+                                                          const u64* __restrict__ V, u32 nv, KeyMap map,
+                                                          u64* __restrict__ out_rows, u32* __restrict__ out_vals,
+                                                          u32* total, u64* status, u32* ctr, u32 epoch, u32* err) {
+  const u32 ntiles = (m + kDcTile - 1) / kDcTile, tile = draw_tile(ctr, ntiles);
+  const u32 i = tile * kDcTile + threadIdx.x;
+  const bool keep = i < m && dedup_keep<W>(C, vals, keys, i, V, nv, map);
+  const u32 d = tile_position(keep, tile, ntiles, total, status, epoch, err);
   if (keep) {
-    const u32 d = s_excl + s_warp[warp] + before_in_warp, src = vals[i];
+    const u32 src = vals[i];
 #pragma unroll
     for (int w = 0; w < W; ++w) out_rows[(size_t)d * W + w] = C[(size_t)src * W + w];
     out_vals[d] = src;
   }
+}
+
+template <int W>
+__global__ void __launch_bounds__(kDcTile) k_keep_compact(const u64* __restrict__ rows, const u32* __restrict__ vals,
+                                                         const u32* __restrict__ flags, u32 m,
+                                                         u64* __restrict__ out_rows, u32* __restrict__ out_vals,
+                                                         u32* total, u64* status, u32* ctr, u32 epoch, u32* err) {
+  const u32 ntiles = (m + kDcTile - 1) / kDcTile, tile = draw_tile(ctr, ntiles);
+  const u32 i = tile * kDcTile + threadIdx.x;
+  const bool keep = i < m && !flags[i];
+  const u32 d = tile_position(keep, tile, ntiles, total, status, epoch, err);
+  if (keep) {
+#pragma unroll
+    for (int w = 0; w < W; ++w) out_rows[(size_t)d * W + w] = rows[(size_t)i * W + w];
+    out_vals[d] = vals[i];
+  }
+}
+
+void launch_keep_compact(int W, const u64* rows, const u32* vals, const u32* flags, u32 m, u64* out_rows, u32* out_vals,
+                         u32* total, u64* status, u32* ctr, u32 epoch, u32* err, cudaStream_t s) {
+  if (!m) {
+    SW_CUDA(cudaMemsetAsync(total, 0, sizeof(u32), s));
+    return;
+  }
+  if (epoch == 0 || epoch >= (1u << 30)) throw std::invalid_argument("keep_compact: epoch must be 1..2^30-1");
+  SW_DISPATCH_W(W, (k_keep_compact<WW><<<(m + kDcTile - 1) / kDcTile, kDcTile, 0, s>>>(
+                       rows, vals, flags, m, out_rows, out_vals, total, status, ctr, epoch, err)));
+  SW_LAUNCH_CHECK();
 }
 
 size_t dedup_compact_status_words(u32 m) { return (m + kDcTile - 1) / kDcTile; }

@@ -55,6 +55,7 @@ struct BucketScratch {
   u32* counts = nullptr;
   u32* first = nullptr;
   uint2* place = nullptr;
+  u32* met = nullptr;  // two words, the first zero before the first launch; the second gets the children found in V
 };
 // 12 leading bits below 2^16 children (one round of the bucket scan), 16 above.
 constexpr int kBucketBitsSmall = 12, kBucketBitsLarge = 16;
@@ -104,7 +105,7 @@ enum QueryMode : int {
 // sh.tiles_per_super tiles; `masks` (subset_check_temp_bytes) and *size_floor
 // (zero beforehand) come from launch_tile_and with the same shape.  `flags`
 // must start zeroed (non-stop mode).  `items` (kSubsetItems entries) and
-// item_count list the parts of S that a large check's queries need; without them
+// item_counts (two words) list the parts of S that a large check's queries need; without them
 // (nullptr) it goes over all of S.  `bytes_ctr` (optional) accumulates the
 // bytes of S rows tested.
 constexpr u64 kSubsetItems = 1u << 22;
@@ -133,17 +134,18 @@ size_t subset_check_temp_bytes(int W, u32 m, const ScanShape& sh);
 void launch_tile_and(int W, const u64* S, u32 m, u64* masks, u32* size_floor, const ScanShape& sh, cudaStream_t s);
 void launch_subset_check(int W, int mode, const u64* S, u32 m, const u64* masks, const u32* size_floor, const u64* Q,
                          u32 q, int n, u32* flags, u32* witness, bool stop, const ScanShape& sh, cudaStream_t s,
-                         u64* bytes_ctr, uint2* items, u32* item_count);
+                         u64* bytes_ctr, uint2* items, u32* item_counts);
 
 // Dominance (dominance.cu): with hit_t, flags[t] = 1 for every row t of T that
 // holds some row x of X (x ⊆ t; proper: x ⊊ t), else flags[x] = 1 for every x that
-// some t holds.  comp: rows are complements of the sets meant.  Rows whose
-// `decided` entry is set (rows of T, or of X without hit_t) may be left out.
-// T up to kDomSmallRows rows is cut into 1024-row chunks as it is; above, its rows
-// are first ordered by falling size (so that most sets are too large for most
-// chunks) and cut into chunks of 4096 (2048 at seven words a row and more); the
-// scratch is used only then.
-constexpr u32 kDomSmallRows = 1u << 15;
+// some t holds.  comp: rows are complements of the sets meant.  Rows whose flag
+// is set already are left out.  T up to kDomSmallRows rows is cut into 1024-row
+// chunks (a level of 5 000 against 4 000 sets: 16 us), above into chunks of 4096
+// (2048 at seven words a row and more), which cost a quarter of the instructions
+// a pair; above kDomOrderRows its rows are first ordered by falling size (three
+// launches), so that most sets are too large for most chunks, and only then is the
+// scratch used.
+constexpr u32 kDomSmallRows = 1u << 13, kDomOrderRows = 1u << 15;
 struct DominanceScratch {
   BucketScratch bucket;   // as for launch_bucket_scatter, with room for T's rows
   u64* rows = nullptr;    // T's rows again
@@ -152,7 +154,7 @@ struct DominanceScratch {
 };
 void launch_bucket_scan(const BucketScratch& b, u32* total, cudaStream_t s);
 void launch_dominance(int W, bool comp, bool hit_t, const u64* T, u32 tm, const u64* X, u32 xm, int n, bool proper,
-                      const u32* decided, u32* flags, const DominanceScratch& sc, cudaStream_t s);
+                      u32* flags, const DominanceScratch& sc, cudaStream_t s);
 
 // out = sorted merge of two sorted, mutually disjoint row arrays.
 void launch_merge(int W, const u64* A, u32 na, const u64* B, u32 nb, u64* out, cudaStream_t s);
@@ -194,6 +196,10 @@ size_t dedup_compact_status_words(u32 m);
 void launch_dedup_compact(int W, const u64* C, const u32* vals, const u64* keys, u32 m, const u64* V, u32 nv,
                           const KeyMap& map, u64* out_rows, u32* out_vals, u32* total, u64* status, u32* ctr,
                           u32 epoch, u32* err, cudaStream_t s);
+// The rows whose flag is zero, in order, and their vals: one launch, compacted as
+// by launch_dedup_compact (same status, ctr and epoch).
+void launch_keep_compact(int W, const u64* rows, const u32* vals, const u32* flags, u32 m, u64* out_rows, u32* out_vals,
+                         u32* total, u64* status, u32* ctr, u32 epoch, u32* err, cudaStream_t s);
 void launch_member_key(int W, const u64* V, u32 nv, const u64* C, u32 nc, u32* flags, cudaStream_t s,
                        const KeyMap& map = KeyMap{});
 // flags[i] = 0 where flags[i] = 1 and row i of C equals a row of V (same

@@ -231,18 +231,21 @@ __global__ void __launch_bounds__(256) k_scan_candidates(const u64* __restrict__
   }
 }
 
-// Units: items[0 .. *count), or without items every (query group, `chunk`
+// Units: items[0 .. counts[0]), which warps fetch one by one (counts[1], the next
+// while they work on one), or without items every (query group, `chunk`
 // super-tiles) pair.  Instructions per launch against rows of needed tiles tested by the
 // whole warp one query at a time: 237 -> 88 M and 309 -> 155 M at two levels
 // of an n = 200 search.
+// Registers are held to 40 up to four words a row (48 warps an SM): the loads a
+// unit waits for are what the other warps hide.
 template <int W, int MODE>
-__global__ void __launch_bounds__(kMaxScanWarps * 32) k_subset_scan(const u64* __restrict__ S, u32 m,
+__global__ void __launch_bounds__(kMaxScanWarps * 32, W <= 4 ? 3 : 2) k_subset_scan(const u64* __restrict__ S, u32 m,
                                                                     const u64* __restrict__ masks, u32 tile_rows,
                                                                     u32 tps, const u64* __restrict__ Q, u32 q, int n,
                                                                     u32* flags, u32* witness,
                                                                     const u32* __restrict__ size_floor, int stop,
                                                                     const uint2* __restrict__ items,
-                                                                    const u32* __restrict__ count, u32 chunk,
+                                                                    u32* counts, u32 chunk,
                                                                     u64* __restrict__ bytes_ctr) {
   const u32 lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const u32 tiles = (m + tile_rows - 1) / tile_rows, supers = (tiles + tps - 1) / tps;
@@ -253,10 +256,15 @@ __global__ void __launch_bounds__(kMaxScanWarps * 32) k_subset_scan(const u64* _
   const u32* const super_min = reinterpret_cast<const u32*>(masks + L.super_min);
   const u32 gpt = tile_rows / kGroupRows;  // groups per tile: 8, 16 or 32
   const u32 chunks = (supers + chunk - 1) / chunk;
-  const u64 units = items ? *count : (u64)((q + 31) / 32) * chunks;
+  const u64 units = items ? *(volatile u32*)counts : (u64)((q + 31) / 32) * chunks;
+  auto fetch = [&]() -> u32 { return lane == 0 ? atomicAdd(counts + 1, 1u) : 0u; };
   const int floor_size = (int)~*size_floor;
   u32 rows_read = 0;
-  for (u64 u = blockIdx.x * warps + (threadIdx.x >> 5); u < units; u += gridDim.x * warps) {
+  u32 ahead = items ? fetch() : 0u;
+  for (u64 u = blockIdx.x * warps + (threadIdx.x >> 5);; u += gridDim.x * warps) {
+    if (items) u = __shfl_sync(kFullMask, ahead, 0);
+    if (u >= units) break;
+    if (items) ahead = fetch();
     if (stop) {  // leave once any warp met
       const u32 f = lane == 0 ? *(volatile u32*)witness : 0u;
       if (__shfl_sync(kFullMask, f, 0) != 0) break;
@@ -427,7 +435,7 @@ void launch_tile_and(int W, const u64* S, u32 m, u64* masks, u32* size_floor, co
 
 void launch_subset_check(int W, int mode, const u64* S, u32 m, const u64* masks, const u32* size_floor, const u64* Q,
                          u32 q, int n, u32* flags, u32* witness, bool stop, const ScanShape& sh, cudaStream_t s,
-                         u64* bytes_ctr, uint2* items, u32* item_count) {
+                         u64* bytes_ctr, uint2* items, u32* item_counts) {
   if (!m || !q) return;
   if (!scan_shape_valid(W, sh)) throw std::invalid_argument("subset check: invalid scan shape");
   const u32 tiles = n_tiles(m, sh), supers = n_supers(m, sh);
@@ -445,16 +453,16 @@ void launch_subset_check(int W, int mode, const u64* S, u32 m, const u64* masks,
     const u32 gs = std::min(slice, groups - g0);
     const u64 units = listed ? (u64)gs * supers : (u64)groups * ((supers + chunk - 1) / chunk);
     const u32 blocks = (u32)std::min<u64>((units + warps - 1) / warps, most_blocks);
-    if (listed) SW_CUDA(cudaMemsetAsync(item_count, 0, sizeof(u32), s));
+    if (listed) SW_CUDA(cudaMemsetAsync(item_counts, 0, 2 * sizeof(u32), s));
 #define SW_SC_ONE(WW, MM)                                                                                             \
   {                                                                                                                   \
     if (listed)                                                                                                       \
       k_scan_candidates<WW, MM><<<(gs + 7) / 8, 256, 0, s>>>(                                                         \
           masks + L.super_and, reinterpret_cast<const u32*>(masks + L.super_min), supers, Q, q, g0, gs, n, flags,     \
-          witness, size_floor, stop, items, item_count);                                                              \
+          witness, size_floor, stop, items, item_counts);                                                              \
     k_subset_scan<WW, MM><<<blocks, warps * 32, 0, s>>>(S, m, masks, (u32)sh.tile_rows, (u32)sh.tiles_per_super, Q,   \
                                                         q, n, flags, witness, size_floor, stop,                       \
-                                                        listed ? items : nullptr, item_count, chunk, bytes_ctr);      \
+                                                        listed ? items : nullptr, item_counts, chunk, bytes_ctr);      \
   }
 #define SW_SC(WW)                                                           \
   case WW:                                                                  \
