@@ -1208,9 +1208,15 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
   // duplicate removal only, each level meet-checked against F.  The switch is
   // taken when the projected cost of those levels (measured per-query meet
   // time, B growing by the last observed branching) is below that of
-  // continuing the dominance-pruned search (last step's time growing 1.6x per
+  // continuing the dominance-pruned search (last step's time growing 1.5x per
   // step), and the widest projected level fits the memory budget.
   bool bounded = false;
+  // Seconds of a step's and a meet check's launches, which do not grow with the
+  // lists; below kSwitchRows rows they are all of it, and neither the times nor
+  // the branching say anything about later levels (a switch at 145 rows, 29
+  // levels before the bound, took 190 ms where 35 was enough).
+  constexpr double kStepLaunch = 1.2e-4, kMeetLaunch = 2.5e-5;
+  constexpr u32 kSwitchRows = 4096;
   double t_iter_last = 0, t_meet_per_query = 0, b_growth = k * 0.95;
   while (rt < max_rt) {  // meet_in_the_middle.cpp:73
     const auto t_iter0 = std::chrono::steady_clock::now();
@@ -1267,17 +1273,24 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
     t_iter_last = std::chrono::duration<double>(t_end - t_iter0).count();
     if (E.B.count)
       t_meet_per_query = std::chrono::duration<double>(t_end - t_meet_host0).count() / (double)E.B.count;
-    if (!bounded && b.has_word && !w[0] && rt < max_rt && rt >= 4 && E.B.count) {
+    if (!bounded && b.has_word && !w[0] && rt < max_rt && rt >= 4 && E.B.count >= kSwitchRows) {
       const u64 R = max_rt - rt;  // levels still to exclude
-      // per child: dedup (~1 ns measured at 10^7 rows) + the meet check's cost per query
-      const double per_row = t_meet_per_query + 2e-9;
+      // per child: expansion and hash table (0.12-0.25 ns measured at 10^7
+      // rows) + the meet check's cost per query.  Continuing costs 1.5x more
+      // per length: the sides alternate, each list grows ~1.7x when its turn
+      // comes and the dominance checks with its square (0.8, 1.5, 3.4, 6, 10 ms
+      // measured for five lengths at n=300).  With the 2 ns and 1.35x that the
+      // sorted levels cost, the switch came one or two lengths later: n=256
+      // 70.8 -> 56 ms, n=300 within 5% either way.
+      const double per_row = std::max(t_meet_per_query - kMeetLaunch / (double)E.B.count, 0.0) + 2.5e-10;
+      t_iter_last = std::max(t_iter_last - kStepLaunch, 0.0);
       double lvl = E.B.count, total = 0, mitm = 0, grow = 1.0;
       bool fits = true;
       for (u64 i = 1; i <= R && fits; ++i) {
         const double children = lvl * k;
         total += children * per_row;
-        grow *= 1.35;  // both sides alternate: each side grows ~1.7x every other step
-        mitm += t_iter_last * grow;
+        grow *= 1.5;
+        mitm += kStepLaunch + t_iter_last * grow;
         // children rows + their sorted copy + the kept level, keys and payloads
         if (children * (3.0 * row_bytes + 32) + (lvl + (double)E.F.count) * row_bytes > (double)budget)
           fits = false;
