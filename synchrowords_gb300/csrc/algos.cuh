@@ -45,6 +45,21 @@ void launch_brute_level(const uint16_t* delta, int n, int k, const u32* frontier
 void launch_brute_parent(const uint16_t* delta, int n, int k, const u32* level, u32 count, u32 target, u64* best,
                          cudaStream_t s);
 
+// ---- Beam in one CTA (beam.cu) -------------------------------------------
+
+// Levels per launch, and the words of `out`: found, levels expanded, sets kept,
+// ancestor; kBeamLevels letters; kBeamLevels parent counts.
+constexpr u32 kBeamLevels = 256, kBeamHeader = 8, kBeamOutWords = kBeamHeader + 2 * kBeamLevels;
+constexpr size_t kBeamSmemBytes = 226 * 1024;
+// Whether `parents` sets (the larger of the beam and the seeds) and their
+// children fit.
+bool beam_fits(int W, u32 n, u32 k, u64 parents);
+// Up to `levels` (<= kBeamLevels) levels from the m sets in `rows` (room for
+// `parents`; after a launch that found nothing it holds the kept sets), each
+// kept set's letter * m + parent position in log[level * parents + position].
+void launch_beam(int W, const uint16_t* delta, u32 n, u32 k, u32 beam, u32 m, u32 parents, u32 levels, u64* rows,
+                 u32* log, u32* out, cudaStream_t s);
+
 // ---- Device-resident exact search (batch_cluster.cu) ----------------------
 
 // One automaton of a batch: n <= 64 W states; delta[q*k + a]

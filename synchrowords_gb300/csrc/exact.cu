@@ -267,8 +267,9 @@ class Engine {
   Side F, B;
   sw_stats* st = nullptr;
   std::vector<std::unique_ptr<DLevel>> dlevel_pool;  // the bounded phase's per-depth levels
-  // scratch of the learned beam and of Reduce, kept across calls
+  // scratch of the beams and of Reduce, kept across calls
   DevBuf lb_counts, lb_scores, lb_keys, lb_vals, lb_alt_k, lb_alt_v, lb_sel_rows, lb_sel_origin, red_counts;
+  DevBuf beam_log, beam_out;
 
   void upload_tables(const Automaton& A) {
     HostTables h = build_tables(A);
@@ -1396,10 +1397,62 @@ static BeamRun beam_cutoff(Engine& E, const Automaton& A, u32 beam_size, u64 max
   X.reset();
   std::vector<u64> rows((size_t)W * std::max<size_t>(seeds.size(), 1), 0);
   for (size_t i = 0; i < seeds.size(); ++i) rows[i * W + (seeds[i] >> 6)] |= state_bit((int)seeds[i]);
-  X.rows.reserve(sizeof(u64) * rows.size());
+  const u64 parents = std::max<u64>(beam_size, seeds.size());
+  const bool one_cta = beam_fits(W, (u32)n, (u32)k, parents);
+  X.rows.reserve(sizeof(u64) * std::max<size_t>(rows.size(), one_cta ? W * parents : 0));
   SW_CUDA(cudaMemcpyAsync(X.rows.p, rows.data(), sizeof(u64) * W * seeds.size(), cudaMemcpyHostToDevice, E.stream));
   X.count = (u32)seeds.size();
-  if (X.count == 0 || beam_size == 0) return out;
+  if (X.count == 0 || beam_size == 0 || max_mlsw == 0) return out;
+  if (one_cta) {
+    // Beams whose children fit in one CTA's shared memory run there (still the
+    // faster side at the largest that fit: n=256 beam 2048 123 us a level over
+    // the whole GPU, 64 here; n=100 beam 3000 127 and 54), up to kBeamLevels
+    // levels a launch; earlier launches' origins are kept on the host.
+    const u64 most = max_iter >= 0 ? std::min<u64>(max_mlsw - 1, (u64)max_iter) : max_mlsw - 1;
+    E.beam_log.reserve(sizeof(u32) * parents * kBeamLevels);
+    E.beam_out.reserve(sizeof(u32) * kBeamOutWords);
+    struct Part {
+      std::vector<u32> log, parents;  // per level: kept origins, parent count
+    };
+    std::vector<Part> parts;
+    u32 m = X.count;
+    for (u64 len = 0; len < most;) {
+      const u32 levels = (u32)std::min<u64>(most - len, kBeamLevels);
+      launch_beam(W, E.tables.delta, (u32)n, (u32)k, beam_size, m, (u32)parents, levels, X.rows.as<u64>(),
+                  E.beam_log.as<u32>(), E.beam_out.as<u32>(), E.stream);
+      E.count_launch();
+      SW_CUDA(cudaMemcpyAsync(E.pinned.p, E.beam_out.p, sizeof(u32) * kBeamOutWords, cudaMemcpyDeviceToHost, E.stream));
+      SW_CUDA(cudaStreamSynchronize(E.stream));
+      const u32 *o = E.pinned.as<u32>(), *counts = o + kBeamHeader + kBeamLevels;
+      for (u32 l = 0; l < o[1]; ++l) st.subsets_expanded += (u64)counts[l] * k;
+      len += o[1];
+      if (o[0]) {
+        // word: letters from this layer down to the first, applied in that order
+        out.word.assign(o + kBeamHeader, o + kBeamHeader + o[1]);
+        u32 idx = o[3];
+        for (size_t i = parts.size(); i-- > 0;)
+          for (size_t d = parts[i].parents.size(); d-- > 0;) {
+            const u32 v = parts[i].log[d * parents + idx];
+            out.word.push_back(v / parts[i].parents[d]);
+            idx = v % parts[i].parents[d];
+          }
+        out.bound = len;
+        std::vector<uint32_t> img = apply_word(A, out.word);
+        out.has_word = img.size() == 1 && out.word.size() == len;
+        return out;
+      }
+      m = o[2];
+      if (len < most) {
+        parts.emplace_back();
+        parts.back().parents.assign(counts, counts + levels);
+        parts.back().log.resize((size_t)levels * parents);
+        SW_CUDA(cudaMemcpyAsync(parts.back().log.data(), E.beam_log.p, sizeof(u32) * levels * parents,
+                                cudaMemcpyDeviceToHost, E.stream));
+        SW_CUDA(cudaStreamSynchronize(E.stream));
+      }
+    }
+    return out;
+  }
   for (u64 len = 1; len < max_mlsw; ++len) {
     if (max_iter >= 0 && (int64_t)len > max_iter) break;
     const u32 m = X.count;
