@@ -265,10 +265,11 @@ class Engine {
     count_launch(4);
   }
   Side F, B;
+  Side R;  // the list of the last Reduce, from which a search of the reduced automaton starts
   sw_stats* st = nullptr;
   std::vector<std::unique_ptr<DLevel>> dlevel_pool;  // the bounded phase's per-depth levels
   // scratch of the beams and of Reduce, kept across calls
-  DevBuf lb_counts, lb_scores, lb_keys, lb_vals, lb_alt_k, lb_alt_v, lb_sel_rows, lb_sel_origin, red_counts;
+  DevBuf lb_counts, lb_scores, lb_keys, lb_vals, lb_alt_k, lb_alt_v, lb_sel_rows, lb_sel_origin, red_states;
   DevBuf beam_log, beam_out;
 
   void upload_tables(const Automaton& A) {
@@ -1160,20 +1161,22 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
   if (imported) {
     E.import_single(W, single_exit);
   } else {  // seeds
+    const u32 nf = red ? red->seeds : 1;
+    E.F.rows.reserve(sizeof(u64) * W * std::max<u32>(nf, 1));
     std::vector<u64> full(W, 0);
-    for (int q = 0; q < n; ++q) full[q >> 6] |= state_bit(q);
-    std::vector<u64> fseeds;
+    std::vector<uint16_t> from(n);
     if (red) {
       // exact.cpp:130-146: the forward side starts from the reduced BFS list
-      fseeds.assign((size_t)W * red->seeds.size(), 0);
-      for (size_t i = 0; i < red->seeds.size(); ++i)
-        for (uint32_t q : red->seeds[i]) fseeds[i * W + (order[q] >> 6)] |= state_bit((int)order[q]);
+      for (int q = 0; q < n; ++q) from[order[q]] = (uint16_t)red->states[q];
+      E.red_states.reserve(sizeof(uint16_t) * n);
+      SW_CUDA(cudaMemcpyAsync(E.red_states.p, from.data(), sizeof(uint16_t) * n, cudaMemcpyHostToDevice, E.stream));
+      const int Wr = words_for((int)red->original.n);
+      launch_relabel_rows(E.R.cur_rows(Wr), Wr, nf, E.red_states.as<uint16_t>(), n, E.F.rows.as<u64>(), W, E.stream);
+      E.count_launch();
     } else {
-      fseeds = full;
+      for (int q = 0; q < n; ++q) full[q >> 6] |= state_bit(q);
+      SW_CUDA(cudaMemcpyAsync(E.F.rows.p, full.data(), sizeof(u64) * W, cudaMemcpyHostToDevice, E.stream));
     }
-    const u32 nf = (u32)(fseeds.size() / W);
-    E.F.rows.reserve(sizeof(u64) * W * std::max<u32>(nf, 1));
-    SW_CUDA(cudaMemcpyAsync(E.F.rows.p, fseeds.data(), sizeof(u64) * W * nf, cudaMemcpyHostToDevice, E.stream));
     E.F.count = nf;
     std::vector<u64> rows((size_t)W * std::max<size_t>(seeds.size(), 1), 0);
     for (size_t i = 0; i < seeds.size(); ++i) {
@@ -1350,7 +1353,10 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
     u32 seed_idx = 0;
     std::vector<uint32_t> bw = bounded_tail.empty() ? E.trace(E.B, wit_q, &seed_idx) : bounded_tail;
     std::vector<uint32_t> word;
-    if (red) word = red->prefix.at(fseed);
+    if (red) {
+      word = E.trace(E.R, fseed, nullptr);
+      std::reverse(word.begin(), word.end());
+    }
     word.insert(word.end(), fw.begin(), fw.end());
     word.insert(word.end(), bw.begin(), bw.end());
     std::vector<uint32_t> img = apply_word(red ? red->original : A, word);
@@ -1816,45 +1822,44 @@ void Solver::reduce(const Automaton& A, const sw_reduce_config& cfg, Bounds& b, 
   const int n = (int)A.n, k = (int)A.k, W = words_for(n);
   E.upload_tables(A);
   E.self_check = E.visited_subsets = true;  // the reference's step (reduce.hpp:186-187): its list sizes decide the reduction
-  E.F.reset();
+  E.R.reset();
   std::vector<u64> full(W, 0);
   for (int q = 0; q < n; ++q) full[q >> 6] |= state_bit(q);
-  E.F.rows.reserve(sizeof(u64) * W);
-  SW_CUDA(cudaMemcpyAsync(E.F.rows.p, full.data(), sizeof(u64) * W, cudaMemcpyHostToDevice, E.stream));
-  E.F.count = 1;
-  E.F.vis_count = 0;  // reduce.hpp:128: the visited list starts empty
+  E.R.rows.reserve(sizeof(u64) * W);
+  SW_CUDA(cudaMemcpyAsync(E.R.rows.p, full.data(), sizeof(u64) * W, cudaMemcpyHostToDevice, E.stream));
+  E.R.count = 1;
+  E.R.vis_count = 0;  // reduce.hpp:128: the visited list starts empty
   const u64 max_mlsw = b.upper - 1;
   u64 mlsw = 0;
   bool found = false;
   std::vector<uint32_t> word;
-  DevBuf& counts = E.red_counts;
   auto done = [&] {
     st.device_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     E.st = nullptr;
   };
+  u64* const sum = reinterpret_cast<u64*>(E.d_misc + 32);  // the list's union, then ~(its first single-state set)
+  const size_t sum_bytes = 8 * sizeof(u64) + sizeof(u32);
   // reduce.hpp:96-109 (process_short_bfs) with bfs_step :171-198
   while (mlsw < max_mlsw) {
-    if (E.F.count > cfg.list_size_threshold) break;
+    if (E.R.count > cfg.list_size_threshold) break;
     mlsw++;
     st.bfs_steps++;
-    if (E.F.count == 0) continue;  // an exhausted list stays empty up to the bound, as in the reference
-    E.step(E.F, true, W, n, k, true);
-    const u32 m = E.F.count;
-    if (!m) continue;
-    counts.reserve(sizeof(u32) * m);
-    launch_popcount(W, E.F.cur_rows(W), m, counts.as<u32>(), E.stream);
+    if (E.R.count == 0) continue;  // an exhausted list stays empty up to the bound, as in the reference
+    E.step(E.R, true, W, n, k, true);
+    if (!E.R.count) continue;
+    SW_CUDA(cudaMemsetAsync(sum, 0, sum_bytes, E.stream));
+    launch_list_summary(W, E.R.cur_rows(W), E.R.count, sum, reinterpret_cast<u32*>(sum + 8), E.stream);
     E.count_launch();
-    std::vector<u32> pc(m);
-    SW_CUDA(cudaMemcpyAsync(pc.data(), counts.p, sizeof(u32) * m, cudaMemcpyDeviceToHost, E.stream));
+    SW_CUDA(cudaMemcpyAsync(E.pinned.p, sum, sum_bytes, cudaMemcpyDeviceToHost, E.stream));
     SW_CUDA(cudaStreamSynchronize(E.stream));
-    for (u32 i = 0; i < m; ++i)
-      if (pc[i] == 1) {
-        word = E.trace(E.F, i, nullptr);
-        std::reverse(word.begin(), word.end());
-        found = true;
-        break;
-      }
-    if (found) break;
+    std::copy(E.pinned.as<u64>(), E.pinned.as<u64>() + W, full.begin());
+    const u32 single = E.pinned.as<u32>()[16];
+    if (single) {
+      word = E.trace(E.R, ~single, nullptr);
+      std::reverse(word.begin(), word.end());
+      found = true;
+      break;
+    }
   }
   if (!found && mlsw == max_mlsw) {  // reduce.hpp:60-63: every shorter length is excluded
     mlsw++;
@@ -1871,18 +1876,13 @@ void Solver::reduce(const Automaton& A, const sw_reduce_config& cfg, Bounds& b, 
     return done();
   }
   // reduce.hpp:112-143 (try_to_reduce): states reachable from the list
-  const u32 m = E.F.count;
-  std::vector<u64> rows((size_t)m * W);
-  if (m) SW_CUDA(cudaMemcpyAsync(rows.data(), E.F.cur_rows(W), sizeof(u64) * W * m, cudaMemcpyDeviceToHost, E.stream));
-  SW_CUDA(cudaStreamSynchronize(E.stream));
   std::vector<char> reach(n, 0);
   std::vector<uint32_t> stack;
-  for (u32 i = 0; i < m; ++i)
-    for (int q = 0; q < n; ++q)
-      if ((rows[(size_t)i * W + (q >> 6)] & state_bit(q)) && !reach[q]) {
-        reach[q] = 1;
-        stack.push_back((uint32_t)q);
-      }
+  for (int q = 0; q < n && E.R.count; ++q)
+    if (full[q >> 6] & state_bit(q)) {
+      reach[q] = 1;
+      stack.push_back((uint32_t)q);
+    }
   while (!stack.empty()) {  // reduce.hpp:145-169
     const uint32_t q = stack.back();
     stack.pop_back();
@@ -1909,31 +1909,9 @@ void Solver::reduce(const Automaton& A, const sw_reduce_config& cfg, Bounds& b, 
   for (int q = 0; q < n; ++q)
     if (reach[q])
       for (uint32_t a = 0; a < A.k; ++a) red.reduced.t[(size_t)map[q] * A.k + a] = map[A.at((uint32_t)q, a)];
-  // each list set and the word that produced it, traced on the host from the
-  // per-layer origin arrays
-  std::vector<std::vector<u32>> origin(E.F.layers.size());
-  for (size_t d = 0; d < E.F.layers.size(); ++d) {
-    const Layer& L = *E.F.layers[d];
-    origin[d].resize(L.count);
-    if (L.count)
-      SW_CUDA(cudaMemcpyAsync(origin[d].data(), L.origin.p, sizeof(u32) * L.count, cudaMemcpyDeviceToHost,
-                              E.stream));
-  }
-  SW_CUDA(cudaStreamSynchronize(E.stream));
-  red.seeds.resize(m);
-  red.prefix.resize(m);
-  for (u32 i = 0; i < m; ++i) {
-    for (int q = 0; q < n; ++q)
-      if (rows[(size_t)i * W + (q >> 6)] & state_bit(q)) red.seeds[i].push_back(map[q]);
-    std::vector<uint32_t>& w = red.prefix[i];
-    u32 idx = i;
-    for (size_t d = E.F.layers.size(); d-- > 0;) {
-      const u32 o = origin[d][idx];
-      w.push_back(o / E.F.layers[d]->parent_count);
-      idx = o % E.F.layers[d]->parent_count;
-    }
-    std::reverse(w.begin(), w.end());
-  }
+  for (int q = 0; q < n; ++q)
+    if (reach[q]) red.states.push_back((uint32_t)q);
+  red.seeds = E.R.count;
   st.reduce_bfs_steps = mlsw;
   st.reduced_states = rn;
   // reduce.hpp:77-84: the remaining search works on reduced lengths

@@ -29,8 +29,8 @@ struct ReduceState {
   uint64_t bfs_steps = 0; // BFS steps the reduction took (added back by Exact)
   Automaton original;     // the automaton before reduction (words are checked on it)
   Automaton reduced;      // restriction to the states reachable from the BFS list
-  std::vector<std::vector<uint32_t>> seeds;   // BFS list, as state lists in reduced labels
-  std::vector<std::vector<uint32_t>> prefix;  // word taking the full set to each seed
+  std::vector<uint32_t> states;  // reduced label -> original state
+  uint32_t seeds = 0;     // sets of the BFS list, which stays with the solver that reduced
 };
 
 class Solver {

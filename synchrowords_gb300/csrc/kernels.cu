@@ -1068,6 +1068,64 @@ void launch_convert_rows(int W, u64* rows, u64 count, int n, bool to_device, cud
   SW_LAUNCH_CHECK();
 }
 
+// What Reduce asks of a list, without reading the list back.
+template <int W>
+__global__ void k_list_summary(const u64* __restrict__ rows, u32 m, u64* __restrict__ sum, u32* __restrict__ single) {
+  u64 all[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) all[w] = 0;
+  u32 first = 0;
+  for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+    u32 c = 0;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      const u64 x = rows[(size_t)i * W + w];
+      all[w] |= x;
+      c += __popcll(x);
+    }
+    if (c == 1) first = max(first, ~i);
+  }
+  first = __reduce_max_sync(0xffffffffu, first);
+  if ((threadIdx.x & 31u) == 0 && first) atomicMax(single, first);
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    const u32 hi = __reduce_or_sync(0xffffffffu, (u32)(all[w] >> 32));
+    const u32 lo = __reduce_or_sync(0xffffffffu, (u32)all[w]);
+    if ((threadIdx.x & 31u) == 0) atomicOr((unsigned long long*)&sum[w], ((unsigned long long)hi << 32) | lo);
+  }
+}
+
+void launch_list_summary(int W, const u64* rows, u32 m, u64* sum, u32* single, cudaStream_t s) {
+  if (!m) return;
+  const u32 blocks = (u32)std::min<u64>(((u64)m + 255) / 256, (u64)sm_count() * 4);
+  SW_DISPATCH_W(W, (k_list_summary<WW><<<blocks, 256, 0, s>>>(rows, m, sum, single)));
+  SW_LAUNCH_CHECK();
+}
+
+// One thread per 32 states of a row.
+__global__ void k_relabel_rows(const u64* __restrict__ in, int Wi, u32 m, const uint16_t* __restrict__ src, int n,
+                               u32* __restrict__ out, int Wo) {
+  const u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= (u64)m * 2 * Wo) return;
+  const u64 i = e / (2 * Wo);
+  const int h = (int)(e % (2 * Wo));  // h-th half of the row, its first states in the high bits
+  u32 v = 0;
+  for (int j = 0; j < 32; ++j) {
+    const int t = 32 * h + j;
+    if (t >= n) break;
+    const u32 q = src[t];
+    if (in[i * Wi + (q >> 6)] & state_bit((int)q)) v |= 0x80000000u >> j;
+  }
+  out[e ^ 1] = v;  // little-endian words: the high half is the second
+}
+
+void launch_relabel_rows(const u64* in, int Wi, u32 m, const uint16_t* src, int n, u64* out, int Wo, cudaStream_t s) {
+  if (!m) return;
+  const u64 threads = (u64)m * 2 * Wo;
+  k_relabel_rows<<<(u32)((threads + 255) / 256), 256, 0, s>>>(in, Wi, m, src, n, (u32*)out, Wo);
+  SW_LAUNCH_CHECK();
+}
+
 void launch_popcount(int W, const u64* rows, u32 m, u32* out, cudaStream_t s) {
   if (!m) return;
   SW_DISPATCH_W(W, (k_popcount<WW><<<(m + 255) / 256, 256, 0, s>>>(rows, m, out)));

@@ -168,6 +168,12 @@ void launch_complement(int W, u64* rows, u32 m, int n, cudaStream_t s);
 void launch_convert_rows(int W, u64* rows, u64 count, int n, bool to_device, cudaStream_t s);
 
 // out[i] = popcount of row i.
+// sum[0..W) |= every row; ~(index of the first single-state row) is maxed into
+// *single (zero: none).  The caller zeroes both.
+void launch_list_summary(int W, const u64* rows, u32 m, u64* sum, u32* single, cudaStream_t s);
+// Row i of `out` (Wo words) holds state t where row i of `in` (Wi words) holds
+// state src[t], for t < n.
+void launch_relabel_rows(const u64* in, int Wi, u32 m, const uint16_t* src, int n, u64* out, int Wo, cudaStream_t s);
 void launch_popcount(int W, const u64* rows, u32 m, u32* out, cudaStream_t s);
 
 // flags[i] = AND/OR combine: out[i] = (a[i] == 0 && b[i] == 0).
