@@ -206,7 +206,7 @@ class Engine {
     }
     prof_on = false;
   }
-  u32* d_misc = nullptr;  // [0..2] witness, [3] the subset check's size floor, [6, 7] children met before, [8] scan total, [12, 13] the check's unit counts, [kScanErrWord] bounded-wait timeouts
+  u32* d_misc = nullptr;  // [0..2] witness, [3] the subset check's size floor, [6, 7] children met before, [8] scan total, [kScanErrWord] bounded-wait timeouts
   static constexpr int kScanErrWord = 4;  // read back with the witness, never cleared by it
   // Throws if a launch reported a bounded wait that ran out: 2 = a compaction
   // tile's look-back never saw its predecessor, 3 = a hash table's probe found
@@ -339,7 +339,7 @@ class Engine {
     if (!m || !q) return;
     const ScanShape& sh = scan_shapes.pick(W, m);
     tile_and.reserve(subset_check_temp_bytes(W, m, sh));
-    scan_items.reserve(sizeof(uint2) * kSubsetItems);
+    scan_items.reserve(sizeof(uint2) * kSubsetItems + sizeof(u32) * kSubsetCounterWords);
     cudaEvent_t e0 = nullptr;
     if (prof_on) {
       e0 = next_event();
@@ -351,7 +351,8 @@ class Engine {
     // algorithmic bytes: the query rows plus every row of S a query is tested against
     timed(0, (double)q * 8.0 * W, [&] {
       launch_subset_check(W, mode, S, m, tile_and.as<u64>(), size_floor, Q, q, n, flags, d_misc, stop, sh, stream,
-                          prof_on ? d_query_bytes : nullptr, scan_items.as<uint2>(), d_misc + 12);
+                          prof_on ? d_query_bytes : nullptr, scan_items.as<uint2>(),
+                          reinterpret_cast<u32*>(scan_items.as<uint2>() + kSubsetItems));
     });
     if (prof_on) {
       cudaEvent_t e1 = next_event();

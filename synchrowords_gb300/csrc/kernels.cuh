@@ -105,10 +105,11 @@ enum QueryMode : int {
 // sh.tiles_per_super tiles; `masks` (subset_check_temp_bytes) and *size_floor
 // (zero beforehand) come from launch_tile_and with the same shape.  `flags`
 // must start zeroed (non-stop mode).  `items` (kSubsetItems entries) and
-// item_counts (two words) list the parts of S that a large check's queries need; without them
+// item_counts (kSubsetCounterWords words) list the parts of S that a large check's queries need; without them
 // (nullptr) it goes over all of S.  `bytes_ctr` (optional) accumulates the
 // bytes of S rows tested.
 constexpr u64 kSubsetItems = 1u << 22;
+constexpr u32 kSubsetQueues = 64, kSubsetCounterWords = 32 * (kSubsetQueues + 1);  // counters a cache line apart
 // Launch shape of the subset check: rows of S per tile mask (32, 64, 128),
 // warps of 32 queries per block (4, 8, 16), tiles per super-tile mask (4, 8,
 // 16, 32) and the grid's target blocks per SM (1..64), which sets how finely

@@ -39,6 +39,12 @@ constexpr int kMaxTilesPerSuper = 32;
 // Units up to which a check takes every (32 queries, super-tile) pair as a unit;
 // above, the pairs are tested first (one more launch, about 4 us) and listed.
 constexpr u64 kDirectUnits = 1u << 14;
+// Checks of fewer units than this split them below super-tiles: the heaviest units
+// end such a check.  Milliseconds by 2^12 / 2^14 / 2^16 / 2^18: four solves at n = 200
+// 11.9 / 11.5 / 11.9 / 13.7 (12.5 unsplit), eight in a batch 14.2 / 15.2 / 18.6 / 25.7,
+// 65 536 x 32 768 sets 0.91 / 0.91 / 0.83 / 0.85, n = 100 reduced 18.1 / 17.0 / 16.7 /
+// 16.8.
+constexpr u32 kSplitUnits = 1u << 14;
 // Queries needing a tile up to which they are taken one at a time.
 constexpr int kFewTakers = 6;
 constexpr u32 kFullMask = 0xffffffffu;
@@ -213,27 +219,46 @@ __global__ void __launch_bounds__(256) k_scan_candidates(const u64* __restrict__
   const bool done = !valid || room < (int)~*size_floor || (!stop && flags[qi]);
   const int most = query_union<W>(nc, room, done, nu);
   if (most < 0) return;
-  for (u32 s0 = 0; s0 < supers; s0 += 32) {
-    const u32 s = s0 + lane;
-    bool cand = s < supers;
-    if (cand) {
-      cand = (int)super_min[s] <= most;
+  for (u32 b0 = 0; b0 < supers; b0 += 1024) {  // one reservation per 1024 super-tiles
+    u32 mine = 0;  // lane i: which of super-tiles b0 + 32 i .. + 31 are candidates
+    for (u32 i = 0; i < 32 && b0 + 32 * i < supers; ++i) {
+      const u32 s = b0 + 32 * i + lane;
+      bool cand = s < supers;
+      if (cand) {
+        cand = (int)super_min[s] <= most;
 #pragma unroll
-      for (int w = 0; w < W; ++w)
-        if (super_and[(size_t)s * W + w] & nu[w]) cand = false;
+        for (int w = 0; w < W; ++w)
+          if (super_and[(size_t)s * W + w] & nu[w]) cand = false;
+      }
+      const u32 mask = __ballot_sync(kFullMask, cand);
+      if (lane == i) mine = mask;
     }
-    const u32 mask = __ballot_sync(kFullMask, cand);
-    if (!mask) continue;
+    u32 incl = __popc(mine);
+#pragma unroll
+    for (u32 d = 1; d < 32; d *= 2) {
+      const u32 o = __shfl_up_sync(kFullMask, incl, d);
+      if (lane >= d) incl += o;
+    }
     u32 at = 0;
-    if (lane == 0) at = atomicAdd(count, (u32)__popc(mask));
-    at = __shfl_sync(kFullMask, at, 0);
-    if (cand) items[at + __popc(mask & ((1u << lane) - 1u))] = make_uint2(group0 + g, s);
+    if (lane == 31 && incl) at = atomicAdd(count, incl);
+    at = __shfl_sync(kFullMask, at, 31);
+    u32 left = __ballot_sync(kFullMask, mine != 0);
+    while (left) {
+      const int i = __ffs(left) - 1;
+      left &= left - 1;
+      const u32 mask = __shfl_sync(kFullMask, mine, i), before = __shfl_sync(kFullMask, incl, i) - __popc(mask);
+      if ((mask >> lane) & 1u)
+        items[at + before + __popc(mask & ((1u << lane) - 1u))] = make_uint2(group0 + g, b0 + 32 * i + lane);
+    }
   }
 }
 
-// Units: items[0 .. counts[0]), which warps fetch one by one (counts[1], the next
-// while they work on one), or without items every (query group, `chunk`
-// super-tiles) pair.  Instructions per launch against rows of needed tiles tested by the
+// Units: items[0 .. counts[0]), or without items every (query group, `chunk`
+// super-tiles) pair; where these are fewer than `split_units`, parts of them.
+// Warps fetch items one by one, the next while they work on one, from
+// kSubsetQueues counters: class c of the warps takes the items c, c + 64, ... (one
+// counter served ~0.6 fetches a ns, and 19 456 warps starting on it were 30 us of a
+// 77 us launch).  Instructions per launch against rows of needed tiles tested by the
 // whole warp one query at a time: 237 -> 88 M and 309 -> 155 M at two levels
 // of an n = 200 search.
 // Registers are held to 40 up to four words a row (48 warps an SM): the loads a
@@ -245,7 +270,7 @@ __global__ void __launch_bounds__(kMaxScanWarps * 32, W <= 4 ? 3 : 2) k_subset_s
                                                                     u32* flags, u32* witness,
                                                                     const u32* __restrict__ size_floor, int stop,
                                                                     const uint2* __restrict__ items,
-                                                                    u32* counts, u32 chunk,
+                                                                    u32* counts, u32 chunk, u32 split_units,
                                                                     u64* __restrict__ bytes_ctr) {
   const u32 lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const u32 tiles = (m + tile_rows - 1) / tile_rows, supers = (tiles + tps - 1) / tps;
@@ -256,28 +281,41 @@ __global__ void __launch_bounds__(kMaxScanWarps * 32, W <= 4 ? 3 : 2) k_subset_s
   const u32* const super_min = reinterpret_cast<const u32*>(masks + L.super_min);
   const u32 gpt = tile_rows / kGroupRows;  // groups per tile: 8, 16 or 32
   const u32 chunks = (supers + chunk - 1) / chunk;
-  const u64 units = items ? *(volatile u32*)counts : (u64)((q + 31) / 32) * chunks;
-  auto fetch = [&]() -> u32 { return lane == 0 ? atomicAdd(counts + 1, 1u) : 0u; };
+  const u64 whole = items ? *(volatile u32*)counts : (u64)((q + 31) / 32) * chunks;
+  u32 split = 1;
+  if (items || chunk == 1)
+    while (split < tps && whole * split < split_units) split *= 2;
+  const u64 units = whole * split;
+  const u32 me = blockIdx.x * warps + (threadIdx.x >> 5), queue = me % kSubsetQueues;
+  // the class's warps start on its first items, one each
+  const u32 started = (gridDim.x * warps - queue + kSubsetQueues - 1) / kSubsetQueues;
+  auto fetch = [&]() -> u32 { return lane == 0 ? atomicAdd(counts + 32 * (queue + 1), 1u) : 0u; };
   const int floor_size = (int)~*size_floor;
-  u32 rows_read = 0;
-  u32 ahead = items ? fetch() : 0u;
-  for (u64 u = blockIdx.x * warps + (threadIdx.x >> 5);; u += gridDim.x * warps) {
-    if (items) u = __shfl_sync(kFullMask, ahead, 0);
+  u32 rows_read = 0, ahead = 0;
+  bool first = true;
+  for (u64 u = me;; u += gridDim.x * warps) {
+    if (items && !first) u = (u64)(__shfl_sync(kFullMask, ahead, 0) + started) * kSubsetQueues + queue;
+    first = false;
     if (u >= units) break;
     if (items) ahead = fetch();
     if (stop) {  // leave once any warp met
       const u32 f = lane == 0 ? *(volatile u32*)witness : 0u;
       if (__shfl_sync(kFullMask, f, 0) != 0) break;
     }
-    u32 g, s0, s1;
+    u32 g, s0, s1, lo = 0, hi = tps;  // tiles lo .. hi - 1 of the super-tiles s0 .. s1 - 1
+    if (split > 1) {
+      lo = (u32)(u % split) * (tps / split);
+      hi = lo + tps / split;
+    }
+    const u64 v = u / split;
     if (items) {
-      const uint2 it = items[u];
+      const uint2 it = items[v];
       g = it.x;
       s0 = it.y;
       s1 = s0 + 1;
     } else {
-      g = (u32)(u / chunks);
-      s0 = (u32)(u - (u64)g * chunks) * chunk;
+      g = (u32)(v / chunks);
+      s0 = (u32)(v - (u64)g * chunks) * chunk;
       s1 = min(supers, s0 + chunk);
     }
     const u32 qi = g * 32 + lane;
@@ -300,7 +338,7 @@ __global__ void __launch_bounds__(kMaxScanWarps * 32, W <= 4 ? 3 : 2) k_subset_s
     while (s_todo) {
       const u32 t0 = (s0 + __ffs(s_todo) - 1) * tps;
       s_todo &= s_todo - 1;
-      bool tc = lane < tps && t0 + lane < tiles;
+      bool tc = lane >= lo && lane < hi && t0 + lane < tiles;
       if (tc) {
         tc = (int)tile_min[t0 + lane] <= most;
 #pragma unroll
@@ -442,7 +480,9 @@ void launch_subset_check(int W, int mode, const u64* S, u32 m, const u64* masks,
   const MaskLayout L = mask_layout(W, m, tiles, supers);
   const u32 groups = (q + 31) / 32, warps = (u32)sh.warps;
   const u64 pairs = (u64)groups * supers;
-  const u32 most_blocks = (u32)sm_count_sc() * (u32)sh.grid_factor;
+  // no more blocks than are resident (the launch bounds): the others only find the
+  // units gone (eight n = 200 solves in a batch 15.2 -> 14.5 ms)
+  const u32 most_blocks = (u32)sm_count_sc() * std::min<u32>((u32)sh.grid_factor, (W <= 4 ? 48u : 32u) / warps);
   // without a list: few enough units for one each, else up to 32 super-tiles a unit
   const bool listed = items && pairs > kDirectUnits && supers <= kSubsetItems;
   u32 chunk = 1;
@@ -451,9 +491,10 @@ void launch_subset_check(int W, int mode, const u64* S, u32 m, const u64* masks,
   const u32 slice = listed ? std::max<u32>(1, std::min<u32>(groups, (u32)(kSubsetItems / supers))) : groups;
   for (u32 g0 = 0; g0 < groups; g0 += slice) {
     const u32 gs = std::min(slice, groups - g0);
-    const u64 units = listed ? (u64)gs * supers : (u64)groups * ((supers + chunk - 1) / chunk);
+    u64 units = listed ? (u64)gs * supers : (u64)groups * ((supers + chunk - 1) / chunk);
+    if (listed || chunk == 1) units = std::max(units, std::min<u64>(units * sh.tiles_per_super, kSplitUnits));
     const u32 blocks = (u32)std::min<u64>((units + warps - 1) / warps, most_blocks);
-    if (listed) SW_CUDA(cudaMemsetAsync(item_counts, 0, 2 * sizeof(u32), s));
+    if (listed) SW_CUDA(cudaMemsetAsync(item_counts, 0, sizeof(u32) * kSubsetCounterWords, s));
 #define SW_SC_ONE(WW, MM)                                                                                             \
   {                                                                                                                   \
     if (listed)                                                                                                       \
@@ -462,7 +503,7 @@ void launch_subset_check(int W, int mode, const u64* S, u32 m, const u64* masks,
           witness, size_floor, stop, items, item_counts);                                                              \
     k_subset_scan<WW, MM><<<blocks, warps * 32, 0, s>>>(S, m, masks, (u32)sh.tile_rows, (u32)sh.tiles_per_super, Q,   \
                                                         q, n, flags, witness, size_floor, stop,                       \
-                                                        listed ? items : nullptr, item_counts, chunk, bytes_ctr);      \
+                                                        listed ? items : nullptr, item_counts, chunk, kSplitUnits, bytes_ctr);      \
   }
 #define SW_SC(WW)                                                           \
   case WW:                                                                  \
