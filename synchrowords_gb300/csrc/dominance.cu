@@ -73,7 +73,8 @@ template <int W, int V, bool kComp, bool kHitT>
 __global__ void __launch_bounds__(dom_threads<V>()) k_dominance(const u64* __restrict__ T, u32 tm,
                                                                const u32* __restrict__ index,
                                                                const u64* __restrict__ X, u32 xm, int n, int proper,
-                                                               u32 per_slice, u32 per_warp, u32* flags) {
+                                                               u32 per_slice, u32 per_warp, u32* flags,
+                                                               const u32* t_live, const u32* x_live) {
   extern __shared__ __align__(16) u32 s_dom[];
   __shared__ u32 s_max;
   constexpr u32 kStride = col_stride<V>();
@@ -81,7 +82,11 @@ __global__ void __launch_bounds__(dom_threads<V>()) k_dominance(const u64* __res
   u32* const s_open = s_dom + 64 * W * kStride;
   uint16_t* const s_size = reinterpret_cast<uint16_t*>(s_open + 32 * V);
   const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const u32 r0 = blockIdx.x * 1024u * V, rows = min(1024u * V, tm - r0);
+  tm = live_count(tm, t_live);
+  xm = live_count(xm, x_live);
+  const u32 r0 = blockIdx.x * 1024u * V;
+  if (r0 >= tm || blockIdx.y * per_slice >= xm) return;
+  const u32 rows = min(1024u * V, tm - r0);
   if (threadIdx.x == 0) s_max = 0;
   __syncthreads();
   for (u32 g = warp; g < 32 * V; g += kWarps) {
@@ -185,7 +190,8 @@ __global__ void __launch_bounds__(dom_threads<V>()) k_dominance(const u64* __res
 // ---- rows by falling size, so that a chunk's sizes are alike ----
 template <int W, bool kComp>
 __global__ void __launch_bounds__(256) k_size_rank(const u64* __restrict__ T, u32 m, int n, u32* __restrict__ counts,
-                                                   uint2* __restrict__ place) {
+                                                   uint2* __restrict__ place, const u32* live) {
+  m = live_count(m, live);
   const u32 e = blockIdx.x * blockDim.x + threadIdx.x;
   u32 size = 0;
   if (e < m)
@@ -205,9 +211,9 @@ __global__ void __launch_bounds__(256) k_size_rank(const u64* __restrict__ T, u3
 template <int W>
 __global__ void __launch_bounds__(256) k_size_scatter(const u64* __restrict__ T, u32 m, const uint2* __restrict__ place,
                                                       const u32* __restrict__ first, u64* __restrict__ out,
-                                                      u32* __restrict__ index) {
+                                                      u32* __restrict__ index, const u32* live) {
   const u32 e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= m) return;
+  if (e >= live_count(m, live)) return;
   const uint2 pl = place[e];
   const u32 d = first[pl.y] + pl.x;
 #pragma unroll
@@ -218,7 +224,7 @@ __global__ void __launch_bounds__(256) k_size_scatter(const u64* __restrict__ T,
 namespace {
 template <int W, int V>
 void launch_dom(bool comp, bool hit_t, const u64* T, u32 tm, const u32* index, const u64* X, u32 xm, int n, bool proper,
-                u32* flags, cudaStream_t s) {
+                u32* flags, cudaStream_t s, const u32* t_live, const u32* x_live) {
   const u32 chunks = (tm + 1024 * V - 1) / (1024 * V);
   constexpr u32 kThreads = dom_threads<V>(), kWarps = kThreads / 32;
   // slices of X: as many blocks as fit the GPU a few times over, while a warp keeps eight sets or more
@@ -233,7 +239,7 @@ void launch_dom(bool comp, bool hit_t, const u64* T, u32 tm, const u32* index, c
   {                                                                                                           \
     ensure_smem_limit((const void*)k_dominance<W, V, C, H>, (int)smem);                                       \
     k_dominance<W, V, C, H><<<grid, kThreads, smem, s>>>(T, tm, index, X, xm, n, proper ? 1 : 0, per, per_warp, \
-                                                         flags);                                     \
+                                                         flags, t_live, x_live);                     \
   }
   if (comp) {
     if (hit_t) SW_DOM(true, true) else SW_DOM(true, false)
@@ -245,36 +251,36 @@ void launch_dom(bool comp, bool hit_t, const u64* T, u32 tm, const u32* index, c
 }
 template <int W>
 void launch_dom_w(bool comp, bool hit_t, const u64* T, u32 tm, const u64* X, u32 xm, int n, bool proper,
-                  u32* flags, const DominanceScratch& sc, cudaStream_t s) {
+                  u32* flags, const DominanceScratch& sc, cudaStream_t s, const u32* t_live, const u32* x_live) {
   constexpr int V = W < 7 ? 4 : 2;
   // small lists: 1024-row chunks, so that they spread over more blocks
-  if (tm <= kDomSmallRows) return launch_dom<W, 1>(comp, hit_t, T, tm, nullptr, X, xm, n, proper, flags, s);
-  if (tm <= kDomOrderRows) return launch_dom<W, V>(comp, hit_t, T, tm, nullptr, X, xm, n, proper, flags, s);
+  if (tm <= kDomSmallRows) return launch_dom<W, 1>(comp, hit_t, T, tm, nullptr, X, xm, n, proper, flags, s, t_live, x_live);
+  if (tm <= kDomOrderRows) return launch_dom<W, V>(comp, hit_t, T, tm, nullptr, X, xm, n, proper, flags, s, t_live, x_live);
   const u32 blocks = (tm + 255) / 256;
   if (comp)
-    k_size_rank<W, true><<<blocks, 256, 0, s>>>(T, tm, n, sc.bucket.counts, sc.bucket.place);
+    k_size_rank<W, true><<<blocks, 256, 0, s>>>(T, tm, n, sc.bucket.counts, sc.bucket.place, t_live);
   else
-    k_size_rank<W, false><<<blocks, 256, 0, s>>>(T, tm, n, sc.bucket.counts, sc.bucket.place);
+    k_size_rank<W, false><<<blocks, 256, 0, s>>>(T, tm, n, sc.bucket.counts, sc.bucket.place, t_live);
   launch_bucket_scan(BucketScratch{kBucketBitsSmall, sc.bucket.counts, sc.bucket.first, sc.bucket.place, sc.bucket.met},
                      sc.total, s);
-  k_size_scatter<W><<<blocks, 256, 0, s>>>(T, tm, sc.bucket.place, sc.bucket.first, sc.rows, sc.index);
+  k_size_scatter<W><<<blocks, 256, 0, s>>>(T, tm, sc.bucket.place, sc.bucket.first, sc.rows, sc.index, t_live);
   SW_LAUNCH_CHECK();
-  launch_dom<W, V>(comp, hit_t, sc.rows, tm, sc.index, X, xm, n, proper, flags, s);
+  launch_dom<W, V>(comp, hit_t, sc.rows, tm, sc.index, X, xm, n, proper, flags, s, t_live, x_live);
 }
 }  // namespace
 
 void launch_dominance(int W, bool comp, bool hit_t, const u64* T, u32 tm, const u64* X, u32 xm, int n, bool proper,
-                      u32* flags, const DominanceScratch& sc, cudaStream_t s) {
+                      u32* flags, const DominanceScratch& sc, cudaStream_t s, const u32* t_live, const u32* x_live) {
   if (!tm || !xm) return;
   switch (W) {
-    case 1: return launch_dom_w<1>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
-    case 2: return launch_dom_w<2>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
-    case 3: return launch_dom_w<3>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
-    case 4: return launch_dom_w<4>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
-    case 5: return launch_dom_w<5>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
-    case 6: return launch_dom_w<6>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
-    case 7: return launch_dom_w<7>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
-    case 8: return launch_dom_w<8>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s);
+    case 1: return launch_dom_w<1>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s, t_live, x_live);
+    case 2: return launch_dom_w<2>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s, t_live, x_live);
+    case 3: return launch_dom_w<3>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s, t_live, x_live);
+    case 4: return launch_dom_w<4>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s, t_live, x_live);
+    case 5: return launch_dom_w<5>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s, t_live, x_live);
+    case 6: return launch_dom_w<6>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s, t_live, x_live);
+    case 7: return launch_dom_w<7>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s, t_live, x_live);
+    case 8: return launch_dom_w<8>(comp, hit_t, T, tm, X, xm, n, proper, flags, sc, s, t_live, x_live);
     default: throw std::runtime_error("dominance: unsupported width");
   }
 }

@@ -57,6 +57,14 @@ struct Side {
   DevBuf table, met;
   u32 met_count = 0;    // rows of met (split)
   u64 table_slots = 0;  // 0: to be built
+  // The last hashed step, and where its layer's count is while only the device
+  // knows it (count is then an upper bound).
+  struct Step {
+    u32 parents = 0, children = 0, base = 0, visited = 0;
+    bool forward = false, reduce = false, self = false, compacted = false, deferred = false;
+    double t0 = 0;
+  } step;
+  const u32* live = nullptr;
   const u64* cur_rows(int W) const { return in_vis ? vis.as<u64>() + (size_t)cur_off * W : rows.as<u64>(); }
   std::vector<std::unique_ptr<Layer>> layers;
   std::vector<u64> seed_states;  // backward side: the state of each seed row
@@ -86,6 +94,7 @@ struct Side {
   void reset() {
     count = vis_count = 0;
     hashed = sorted_only = in_vis = split = false;
+    live = nullptr;
     table_slots = 0;
     unique_growth = 0;
     keymap = KeyMap{};
@@ -126,6 +135,8 @@ class Engine {
   }
   ~Engine() {
     for (auto e : ev_pool) cudaEventDestroy(e);
+    for (auto e : meet_ev)
+      if (e) cudaEventDestroy(e);
     if (d_query_bytes) cudaFree(d_query_bytes);
     if (d_misc) cudaFree(d_misc);
     if (stream) cudaStreamDestroy(stream);
@@ -206,7 +217,7 @@ class Engine {
     }
     prof_on = false;
   }
-  u32* d_misc = nullptr;  // [0..2] witness, [3] the subset check's size floor, [6, 7] children met before, [8] scan total, [kScanErrWord] bounded-wait timeouts
+  u32* d_misc = nullptr;  // [0..2] witness, [3] the subset check's size floor, [6, 7] children met before, [8] scan total, [9] rows kept by the reductions, [kScanErrWord] bounded-wait timeouts
   static constexpr int kScanErrWord = 4;  // read back with the witness, never cleared by it
   // Throws if a launch reported a bounded wait that ran out: 2 = a compaction
   // tile's look-back never saw its predecessor, 3 = a hash table's probe found
@@ -335,7 +346,8 @@ class Engine {
   double scan_ms[8 * kScanSizeClasses] = {};
   u64 scan_launches[8 * kScanSizeClasses] = {};
 
-  void query(int W, int mode, const u64* S, u32 m, const u64* Q, u32 q, int n, u32* flags, bool stop) {
+  void query(int W, int mode, const u64* S, u32 m, const u64* Q, u32 q, int n, u32* flags, bool stop,
+             const u32* m_live = nullptr, const u32* q_live = nullptr) {
     if (!m || !q) return;
     const ScanShape& sh = scan_shapes.pick(W, m);
     tile_and.reserve(subset_check_temp_bytes(W, m, sh));
@@ -347,12 +359,12 @@ class Engine {
     }
     u32* const size_floor = d_misc + 3;  // zeroed with the witness in meet mode
     if (!stop) SW_CUDA(cudaMemsetAsync(size_floor, 0, sizeof(u32), stream));
-    timed(3, (double)m * 8.0 * W, [&] { launch_tile_and(W, S, m, tile_and.as<u64>(), size_floor, sh, stream); });
+    timed(3, (double)m * 8.0 * W, [&] { launch_tile_and(W, S, m, tile_and.as<u64>(), size_floor, sh, stream, m_live); });
     // algorithmic bytes: the query rows plus every row of S a query is tested against
     timed(0, (double)q * 8.0 * W, [&] {
       launch_subset_check(W, mode, S, m, tile_and.as<u64>(), size_floor, Q, q, n, flags, d_misc, stop, sh, stream,
                           prof_on ? d_query_bytes : nullptr, scan_items.as<uint2>(),
-                          reinterpret_cast<u32*>(scan_items.as<uint2>() + kSubsetItems));
+                          reinterpret_cast<u32*>(scan_items.as<uint2>() + kSubsetItems), m_live, q_live);
     });
     if (prof_on) {
       cudaEvent_t e1 = next_event();
@@ -360,16 +372,19 @@ class Engine {
       scan_ev.push_back({(W - 1) * kScanSizeClasses + (m >= kScanLargeRows ? 1 : 0), {e0, e1}});
     }
     count_launch(2);
-    if (st) {
-      st->trie_queries += q;
-      st->logical_pairs += (u64)m * q;
-    }
+    if (!m_live && !q_live) count_query(m, q);
+  }
+  void count_query(u32 m, u32 q) {
+    if (!st) return;
+    st->trie_queries += q;
+    st->logical_pairs += (u64)m * q;
   }
 
   // flags[i] = 1 where a row of S (a proper one) is inside child row i of Q, on
   // the forward side or on complement rows; children flagged already are left out.
   DevBuf dom_rows, dom_index;
-  void dominated(bool forward, int W, const u64* S, u32 m, const u64* Q, u32 q, int n, bool proper, u32* flags) {
+  void dominated(bool forward, int W, const u64* S, u32 m, const u64* Q, u32 q, int n, bool proper, u32* flags,
+                 const u32* m_live = nullptr, const u32* q_live = nullptr) {
     if (!m || !q) return;
     cudaEvent_t e0 = nullptr;
     if (prof_on) {
@@ -380,6 +395,7 @@ class Engine {
     const u32 tm = forward ? q : m;  // rows that hold: children forward, visited or siblings backward
     if (tm > kDomOrderRows) {
       sc.bucket = buckets(tm);
+      sc.bucket.met = d_misc + 14;  // not the step's
       dom_rows.reserve(sizeof(u64) * W * (size_t)tm);
       dom_index.reserve(sizeof(u32) * (size_t)tm);
       sc.rows = dom_rows.as<u64>();
@@ -389,9 +405,9 @@ class Engine {
     }
     timed(0, (double)(m + q) * 8.0 * W, [&] {
       if (forward)  // sets s ⊆ c: the children hold them
-        launch_dominance(W, false, true, Q, q, S, m, n, proper, flags, sc, stream);
+        launch_dominance(W, false, true, Q, q, S, m, n, proper, flags, sc, stream, q_live, m_live);
       else  // complements: the set of c lies in the set of s
-        launch_dominance(W, true, false, S, m, Q, q, n, proper, flags, sc, stream);
+        launch_dominance(W, true, false, S, m, Q, q, n, proper, flags, sc, stream, m_live, q_live);
     });
     if (prof_on) {
       cudaEvent_t e1 = next_event();
@@ -399,10 +415,21 @@ class Engine {
       scan_ev.push_back({(W - 1) * kScanSizeClasses + (m >= kScanLargeRows ? 1 : 0), {e0, e1}});
     }
     count_launch();
-    if (st) {
-      st->trie_queries += q;
-      st->logical_pairs += (u64)m * q;
-    }
+    if (!m_live && !q_live) count_query(m, q);
+  }
+
+  // Device time of the last meet check.
+  cudaEvent_t meet_ev[2] = {nullptr, nullptr};
+  void meet_begin() {
+    for (cudaEvent_t& e : meet_ev)
+      if (!e) SW_CUDA(cudaEventCreate(&e));
+    SW_CUDA(cudaEventRecord(meet_ev[0], stream));
+  }
+  void meet_end() { SW_CUDA(cudaEventRecord(meet_ev[1], stream)); }
+  double meet_seconds() {
+    float ms = 0;
+    SW_CUDA(cudaEventElapsedTime(&ms, meet_ev[0], meet_ev[1]));
+    return 1e-3 * ms;
   }
 
   // Step log on stderr when SYNCHRO_VERBOSE is set (synchronises per phase).
@@ -468,10 +495,18 @@ class Engine {
   // One layer on a hashed side: children equal to a row met before or to a sibling
   // are dropped by the table, then, with the reductions on, those that a visited
   // set or a sibling dominates.
-  void step_hashed(Side& X, bool forward, int W, int n, int k) {
+  // With `defer` the counts stay on the device (X.live) until finish_step():
+  // the launches that follow are sized for every child.
+  void step_hashed(Side& X, bool forward, int W, int n, int k, bool defer) {
     const u32 m = X.count, Nc = m * (u32)k;
-    const double t_step0 = vclock();
     const bool reduce = self_check || visited_subsets;
+    Side::Step& P = X.step;
+    P = Side::Step{};
+    P.t0 = vclock();
+    P.forward = forward;
+    P.reduce = reduce;
+    P.parents = m;
+    P.children = Nc;
     X.hashed = true;
     if (reduce && !X.split) {
       X.split = true;
@@ -510,44 +545,74 @@ class Engine {
                             stream);
     });
     count_launch(3);
-    const u32 u = read_total_checked();
-    // branching of a level that drops siblings only (the bounded phase's)
-    if (m) X.unique_growth = (double)(u + pinned.as<u32>()[7 - kScanErrWord]) / m;
-    if (st) st->subsets_expanded += Nc;
-    u32 f = u;
+    defer = defer && Nc && (reduce || !X.split);
+    u32 u = Nc;
+    const u32* const fresh_live = defer ? d_misc + 8 : nullptr;
+    if (!defer) u = read_total_checked();
     if (X.split) {
-      X.met_count = base + u;
+      P.visited = visited_subsets ? X.vis_count : 0;
+      P.self = self_check;
       grow_rows(X.vis, X.vis_alt, W, X.vis_count, u);
       u64* const out = X.vis.as<u64>() + (size_t)X.vis_count * W;
       if (reduce && u) {
         flags_a.reserve(sizeof(u32) * (size_t)u);
         SW_CUDA(cudaMemsetAsync(flags_a.p, 0, sizeof(u32) * (size_t)u, stream));
         if (X.vis_count && visited_subsets)
-          dominated(forward, W, X.vis.as<u64>(), X.vis_count, fresh, u, n, false, flags_a.as<u32>());
-        if (self_check) dominated(forward, W, fresh, u, fresh, u, n, true, flags_a.as<u32>());
+          dominated(forward, W, X.vis.as<u64>(), X.vis_count, fresh, u, n, false, flags_a.as<u32>(), nullptr, fresh_live);
+        if (self_check)
+          dominated(forward, W, fresh, u, fresh, u, n, true, flags_a.as<u32>(), fresh_live, fresh_live);
         const u32 epoch = next_dc_epoch(u);
         timed(3, (double)u * (4 + 2 * (8.0 * W + 4)), [&] {
-          launch_keep_compact(W, fresh, fresh_origin, flags_a.as<u32>(), u, out, L->origin.as<u32>(), d_misc + 8,
-                              dc_status.as<u64>(), dc_ctr.as<u32>(), epoch, d_misc + kScanErrWord, stream);
+          launch_keep_compact(W, fresh, fresh_origin, flags_a.as<u32>(), u, out, L->origin.as<u32>(), d_misc + 9,
+                              dc_status.as<u64>(), dc_ctr.as<u32>(), epoch, d_misc + kScanErrWord, stream, fresh_live);
         });
         count_launch();
-        f = read_total_checked();
       } else if (u) {
         SW_CUDA(cudaMemcpyAsync(out, fresh, sizeof(u64) * W * (size_t)u, cudaMemcpyDeviceToDevice, stream));
         SW_CUDA(cudaMemcpyAsync(L->origin.p, fresh_origin, sizeof(u32) * (size_t)u, cudaMemcpyDeviceToDevice, stream));
       }
     }
-    if (st) st->subsets_kept += f;
-    L->count = f;
     L->parent_count = m;
     X.layers.push_back(std::move(L));
     X.in_vis = true;
     X.cur_off = X.vis_count;
+    X.count = u;
+    P.base = base;
+    P.compacted = X.split && reduce && u;
+    P.deferred = defer;
+    if (defer) {
+      X.live = d_misc + (P.compacted ? 9 : 8);
+      return;
+    }
+    SW_CUDA(cudaMemcpyAsync(pinned.p, d_misc, sizeof(u32) * kStepWords, cudaMemcpyDeviceToHost, stream));
+    SW_CUDA(cudaStreamSynchronize(stream));
+    finish_step(X, pinned.as<u32>());
+  }
+  // The step's counts from a host copy of d_misc's first kStepWords words.
+  static constexpr int kStepWords = 10;
+  void finish_step(Side& X, const u32* w) {
+    Side::Step& P = X.step;
+    check_scan_error(w[kScanErrWord]);
+    const u32 u = w[8], f = P.compacted ? w[9] : u;
+    // branching of a level that drops siblings only (the bounded phase's)
+    if (P.parents) X.unique_growth = (double)(u + w[7]) / P.parents;
+    if (st) {
+      st->subsets_expanded += P.children;
+      st->subsets_kept += f;
+    }
+    if (P.deferred && P.compacted) {
+      if (P.visited) count_query(P.visited, u);
+      if (P.self) count_query(u, u);
+    }
+    if (X.split) X.met_count = P.base + u;
+    X.layers.back()->count = f;
     X.count = f;
     X.vis_count += f;
+    X.live = nullptr;
     if (verbose)
-      std::fprintf(stderr, "[sw] %s parents=%u children=%u unique=%u kept=%u (%s) | %.3f ms\n", forward ? "BFS " : "IBFS",
-                   m, Nc, u, f, reduce ? "reduced" : "duplicates only", vclock() - t_step0);
+      std::fprintf(stderr, "[sw] %s parents=%u children=%u unique=%u kept=%u (%s) | %.3f ms\n",
+                   P.forward ? "BFS " : "IBFS", P.parents, P.children, u, f, P.reduce ? "reduced" : "duplicates only",
+                   vclock() - P.t0);
   }
   // Back to a current layer of its own and a visited list in key order.
   void unhash(Side& X, int W) {
@@ -564,12 +629,16 @@ class Engine {
 
   // `ordered`: the layer's rows come in key order, the same on every run
   // (samples of a layer, and beams whose ties go by it, depend on that).
-  void step(Side& X, bool forward, int W, int n, int k, bool dominance = true, bool ordered = false) {
+  // `defer`: the counts of a hashed step may stay on the device until the caller's
+  // next read-back (X.live then names the layer's, and finish_step() is called).
+  void step(Side& X, bool forward, int W, int n, int k, bool dominance = true, bool ordered = false,
+            bool defer = false) {
     const u32 m = X.count;
     const u64 N = (u64)m * k;
     if (N > 0xffffffffULL) throw std::runtime_error("layer exceeds 2^32 children");
     const u32 Nc = (u32)N;
-    if (dominance && !ordered && !sort_key_option() && hashable(X, W, N)) return step_hashed(X, forward, W, n, k);
+    if (dominance && !ordered && !sort_key_option() && hashable(X, W, N)) 
+      return step_hashed(X, forward, W, n, k, defer && !verbose && !prof_on);
     unhash(X, W);
     X.sorted_only = true;
     ch_rows.reserve(sizeof(u64) * W * N);
@@ -1220,7 +1289,7 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
   // lists; below kSwitchRows rows they are all of it, and neither the times nor
   // the branching say anything about later levels (a switch at 145 rows, 29
   // levels before the bound, took 190 ms where 35 was enough).
-  constexpr double kStepLaunch = 1.2e-4, kMeetLaunch = 2.5e-5;
+  constexpr double kStepLaunch = 8e-5, kMeetLaunch = 1.5e-5;
   constexpr u32 kSwitchRows = 4096;
   double t_iter_last = 0, t_meet_per_query = 0, b_growth = k * 0.95;
   while (rt < max_rt) {  // meet_in_the_middle.cpp:73
@@ -1251,10 +1320,7 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
     const bool pressure = 4 * (live + next) > budget;
     E.self_check = E.visited_subsets = cfg.reductions == SW_REDUCE_ALWAYS ||
                                        (cfg.reductions == SW_REDUCE_AUTO && b.has_word) || pressure;
-    E.step(X, fwd, W, n, k, /*dominance=*/!bounded);
-    // projected branching of the bounded levels: distinct children per parent
-    // before pruning, never below 1.5, plus 10% margin
-    if (!fwd && parents_before) b_growth = std::max(1.2, E.B.unique_growth);
+    E.step(X, fwd, W, n, k, /*dominance=*/!bounded, false, /*defer=*/true);
     if (fwd) {
       st.bfs_steps++;
     } else {
@@ -1262,22 +1328,33 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
     }
     // meet check: some F disjoint from some B-complement (F ⊆ B)
     const double t_meet0 = E.vclock();
-    // the switch to the bounded phase prices the meet check per query: time it
-    // alone (a synchronisation first) only while that switch is possible
+    // the switch to the bounded phase prices the meet check per query: it is timed
+    // while that switch is possible
     const bool time_meet = !bounded && b.has_word;
-    if (time_meet) SW_CUDA(cudaStreamSynchronize(E.stream));
-    const auto t_meet_host0 = std::chrono::steady_clock::now();
+    if (time_meet) E.meet_begin();
     SW_CUDA(cudaMemsetAsync(E.d_misc, 0, 4 * sizeof(u32), E.stream));
-    E.query(W, kQueryDisjoint, E.F.cur_rows(W), E.F.count, E.B.cur_rows(W), E.B.count, n, nullptr, true);
-    st.meet_pairs += (u64)E.F.count * E.B.count;
-    SW_CUDA(cudaMemcpyAsync(E.pinned.p, E.d_misc, 5 * sizeof(u32), cudaMemcpyDeviceToHost, E.stream));  // witness + error
+    E.query(W, kQueryDisjoint, E.F.cur_rows(W), E.F.count, E.B.cur_rows(W), E.B.count, n, nullptr, true, E.F.live,
+            E.B.live);
+    if (time_meet) E.meet_end();
+    // the one read-back of a level: witness, error, the step's counts (a reduced
+    // level read back four times: n=100 plans of ~19 levels 2.7 -> 2.4 ms, plain
+    // n=200 levels twice: 3.1 -> 2.9 ms)
+    SW_CUDA(cudaMemcpyAsync(E.pinned.p, E.d_misc, Engine::kStepWords * sizeof(u32), cudaMemcpyDeviceToHost, E.stream));
     SW_CUDA(cudaStreamSynchronize(E.stream));
     const auto t_end = std::chrono::steady_clock::now();
-    const u32* w = E.pinned.as<u32>();
-    Engine::check_scan_error(w[4]);
+    u32 w[Engine::kStepWords];
+    std::copy(E.pinned.as<u32>(), E.pinned.as<u32>() + Engine::kStepWords, w);
+    Engine::check_scan_error(w[Engine::kScanErrWord]);
+    if (X.live) {
+      E.finish_step(X, w);
+      E.count_query(E.F.count, E.B.count);
+    }
+    st.meet_pairs += (u64)E.F.count * E.B.count;
+    // projected branching of the bounded levels: distinct children per parent
+    // before pruning, never below 1.2
+    if (!fwd && parents_before) b_growth = std::max(1.2, E.B.unique_growth);
     t_iter_last = std::chrono::duration<double>(t_end - t_iter0).count();
-    if (E.B.count)
-      t_meet_per_query = std::chrono::duration<double>(t_end - t_meet_host0).count() / (double)E.B.count;
+    if (E.B.count && time_meet) t_meet_per_query = E.meet_seconds() / (double)E.B.count;
     if (!bounded && b.has_word && !w[0] && rt < max_rt && rt >= 4 && E.B.count >= kSwitchRows) {
       const u64 R = max_rt - rt;  // levels still to exclude
       // per child: expansion and hash table (0.12-0.25 ns measured at 10^7
@@ -1846,15 +1923,17 @@ void Solver::reduce(const Automaton& A, const sw_reduce_config& cfg, Bounds& b, 
     mlsw++;
     st.bfs_steps++;
     if (E.R.count == 0) continue;  // an exhausted list stays empty up to the bound, as in the reference
-    E.step(E.R, true, W, n, k, true);
+    E.step(E.R, true, W, n, k, true, false, /*defer=*/true);
     if (!E.R.count) continue;
     SW_CUDA(cudaMemsetAsync(sum, 0, sum_bytes, E.stream));
-    launch_list_summary(W, E.R.cur_rows(W), E.R.count, sum, reinterpret_cast<u32*>(sum + 8), E.stream);
+    launch_list_summary(W, E.R.cur_rows(W), E.R.count, sum, reinterpret_cast<u32*>(sum + 8), E.stream, E.R.live);
     E.count_launch();
-    SW_CUDA(cudaMemcpyAsync(E.pinned.p, sum, sum_bytes, cudaMemcpyDeviceToHost, E.stream));
+    SW_CUDA(cudaMemcpyAsync(E.pinned.p, E.d_misc, 32 * sizeof(u32) + sum_bytes, cudaMemcpyDeviceToHost, E.stream));
     SW_CUDA(cudaStreamSynchronize(E.stream));
-    std::copy(E.pinned.as<u64>(), E.pinned.as<u64>() + W, full.begin());
-    const u32 single = E.pinned.as<u32>()[16];
+    if (E.R.live) E.finish_step(E.R, E.pinned.as<u32>());
+    if (!E.R.count) continue;
+    std::copy(E.pinned.as<u64>() + 16, E.pinned.as<u64>() + 16 + W, full.begin());
+    const u32 single = E.pinned.as<u32>()[48];
     if (single) {
       word = E.trace(E.R, ~single, nullptr);
       std::reverse(word.begin(), word.end());

@@ -1070,7 +1070,9 @@ void launch_convert_rows(int W, u64* rows, u64 count, int n, bool to_device, cud
 
 // What Reduce asks of a list, without reading the list back.
 template <int W>
-__global__ void k_list_summary(const u64* __restrict__ rows, u32 m, u64* __restrict__ sum, u32* __restrict__ single) {
+__global__ void k_list_summary(const u64* __restrict__ rows, u32 m, u64* __restrict__ sum, u32* __restrict__ single,
+                               const u32* live) {
+  m = live_count(m, live);
   u64 all[W];
 #pragma unroll
   for (int w = 0; w < W; ++w) all[w] = 0;
@@ -1095,10 +1097,10 @@ __global__ void k_list_summary(const u64* __restrict__ rows, u32 m, u64* __restr
   }
 }
 
-void launch_list_summary(int W, const u64* rows, u32 m, u64* sum, u32* single, cudaStream_t s) {
+void launch_list_summary(int W, const u64* rows, u32 m, u64* sum, u32* single, cudaStream_t s, const u32* live) {
   if (!m) return;
   const u32 blocks = (u32)std::min<u64>(((u64)m + 255) / 256, (u64)sm_count() * 4);
-  SW_DISPATCH_W(W, (k_list_summary<WW><<<blocks, 256, 0, s>>>(rows, m, sum, single)));
+  SW_DISPATCH_W(W, (k_list_summary<WW><<<blocks, 256, 0, s>>>(rows, m, sum, single, live)));
   SW_LAUNCH_CHECK();
 }
 
@@ -1435,10 +1437,11 @@ template <int W>
 __global__ void __launch_bounds__(kDcTile) k_keep_compact(const u64* __restrict__ rows, const u32* __restrict__ vals,
                                                          const u32* __restrict__ flags, u32 m,
                                                          u64* __restrict__ out_rows, u32* __restrict__ out_vals,
-                                                         u32* total, u64* status, u32* ctr, u32 epoch, u32* err) {
+                                                         u32* total, u64* status, u32* ctr, u32 epoch, u32* err,
+                                                         const u32* live) {
   const u32 ntiles = (m + kDcTile - 1) / kDcTile, tile = draw_tile(ctr, ntiles);
   const u32 i = tile * kDcTile + threadIdx.x;
-  const bool keep = i < m && !flags[i];
+  const bool keep = i < live_count(m, live) && !flags[i];
   const u32 d = tile_position(keep, tile, ntiles, total, status, epoch, err);
   if (keep) {
 #pragma unroll
@@ -1448,14 +1451,14 @@ __global__ void __launch_bounds__(kDcTile) k_keep_compact(const u64* __restrict_
 }
 
 void launch_keep_compact(int W, const u64* rows, const u32* vals, const u32* flags, u32 m, u64* out_rows, u32* out_vals,
-                         u32* total, u64* status, u32* ctr, u32 epoch, u32* err, cudaStream_t s) {
+                         u32* total, u64* status, u32* ctr, u32 epoch, u32* err, cudaStream_t s, const u32* live) {
   if (!m) {
     SW_CUDA(cudaMemsetAsync(total, 0, sizeof(u32), s));
     return;
   }
   if (epoch == 0 || epoch >= (1u << 30)) throw std::invalid_argument("keep_compact: epoch must be 1..2^30-1");
   SW_DISPATCH_W(W, (k_keep_compact<WW><<<(m + kDcTile - 1) / kDcTile, kDcTile, 0, s>>>(
-                       rows, vals, flags, m, out_rows, out_vals, total, status, ctr, epoch, err)));
+                       rows, vals, flags, m, out_rows, out_vals, total, status, ctr, epoch, err, live)));
   SW_LAUNCH_CHECK();
 }
 

@@ -20,6 +20,13 @@ namespace sw {
 // Per-letter transition tables as staged into shared memory by `expand`.
 // Layout (all u16): delta[a*n + q]; inv_beg[a*(n+1) + t] ..inv_beg[..+1] index
 // inv_src[a*n + e] (CSR of preimages).
+// Counts that only the device knows yet: a launcher's `live` pointers (null: the
+// host's count holds) name the word that holds how many of a list's first m rows
+// there are; grids and scratch are sized for m.
+#ifdef __CUDACC__
+__device__ __forceinline__ u32 live_count(u32 m, const u32* live) { return live ? min(m, *live) : m; }
+#endif
+
 struct TransTables {
   const uint16_t* delta = nullptr;   // k*n
   const uint16_t* inv_beg = nullptr; // k*(n+1)
@@ -132,10 +139,12 @@ struct ScanShapes {
 bool scan_shape_valid(int W, const ScanShape& sh);
 size_t scan_smem_bytes(int W, const ScanShape& sh);
 size_t subset_check_temp_bytes(int W, u32 m, const ScanShape& sh);
-void launch_tile_and(int W, const u64* S, u32 m, u64* masks, u32* size_floor, const ScanShape& sh, cudaStream_t s);
+void launch_tile_and(int W, const u64* S, u32 m, u64* masks, u32* size_floor, const ScanShape& sh, cudaStream_t s,
+                     const u32* m_live = nullptr);
 void launch_subset_check(int W, int mode, const u64* S, u32 m, const u64* masks, const u32* size_floor, const u64* Q,
                          u32 q, int n, u32* flags, u32* witness, bool stop, const ScanShape& sh, cudaStream_t s,
-                         u64* bytes_ctr, uint2* items, u32* item_counts);
+                         u64* bytes_ctr, uint2* items, u32* item_counts, const u32* m_live = nullptr,
+                         const u32* q_live = nullptr);
 
 // Dominance (dominance.cu): with hit_t, flags[t] = 1 for every row t of T that
 // holds some row x of X (x ⊆ t; proper: x ⊊ t), else flags[x] = 1 for every x that
@@ -155,7 +164,8 @@ struct DominanceScratch {
 };
 void launch_bucket_scan(const BucketScratch& b, u32* total, cudaStream_t s);
 void launch_dominance(int W, bool comp, bool hit_t, const u64* T, u32 tm, const u64* X, u32 xm, int n, bool proper,
-                      u32* flags, const DominanceScratch& sc, cudaStream_t s);
+                      u32* flags, const DominanceScratch& sc, cudaStream_t s, const u32* t_live = nullptr,
+                      const u32* x_live = nullptr);
 
 // out = sorted merge of two sorted, mutually disjoint row arrays.
 void launch_merge(int W, const u64* A, u32 na, const u64* B, u32 nb, u64* out, cudaStream_t s);
@@ -171,7 +181,8 @@ void launch_convert_rows(int W, u64* rows, u64 count, int n, bool to_device, cud
 // out[i] = popcount of row i.
 // sum[0..W) |= every row; ~(index of the first single-state row) is maxed into
 // *single (zero: none).  The caller zeroes both.
-void launch_list_summary(int W, const u64* rows, u32 m, u64* sum, u32* single, cudaStream_t s);
+void launch_list_summary(int W, const u64* rows, u32 m, u64* sum, u32* single, cudaStream_t s,
+                         const u32* live = nullptr);
 // Row i of `out` (Wo words) holds state t where row i of `in` (Wi words) holds
 // state src[t], for t < n.
 void launch_relabel_rows(const u64* in, int Wi, u32 m, const uint16_t* src, int n, u64* out, int Wo, cudaStream_t s);
@@ -206,7 +217,7 @@ void launch_dedup_compact(int W, const u64* C, const u32* vals, const u64* keys,
 // The rows whose flag is zero, in order, and their vals: one launch, compacted as
 // by launch_dedup_compact (same status, ctr and epoch).
 void launch_keep_compact(int W, const u64* rows, const u32* vals, const u32* flags, u32 m, u64* out_rows, u32* out_vals,
-                         u32* total, u64* status, u32* ctr, u32 epoch, u32* err, cudaStream_t s);
+                         u32* total, u64* status, u32* ctr, u32 epoch, u32* err, cudaStream_t s, const u32* live = nullptr);
 void launch_member_key(int W, const u64* V, u32 nv, const u64* C, u32 nc, u32* flags, cudaStream_t s,
                        const KeyMap& map = KeyMap{});
 // flags[i] = 0 where flags[i] = 1 and row i of C equals a row of V (same

@@ -102,13 +102,15 @@ __host__ __device__ inline MaskLayout mask_layout(int W, u32 m, u32 tiles, u32 s
 template <int W>
 __global__ void __launch_bounds__(kMaxTilesPerSuper * 32) k_range_and(const u64* __restrict__ S, u32 m,
                                                                       u64* __restrict__ masks, u32 tile_rows,
-                                                                      u32* size_floor) {
+                                                                      u32* size_floor, const u32* m_live) {
   __shared__ u64 s_and[kMaxTilesPerSuper][W];
   __shared__ u32 s_min[kMaxTilesPerSuper];
   const u32 tiles = (m + tile_rows - 1) / tile_rows;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tps = blockDim.x >> 5;
   const u32 t = blockIdx.x * tps + warp;
   const MaskLayout L = mask_layout(W, m, tiles, gridDim.x);
+  m = live_count(m, m_live);
+  if (blockIdx.x * tps * tile_rows >= m) return;
   u64 a[W];
 #pragma unroll
   for (int w = 0; w < W; ++w) a[w] = ~0ULL;
@@ -201,11 +203,14 @@ __device__ __forceinline__ int query_union(const u64* nc, int room, bool done, u
 // queries, 32 super-tiles tested at a time.
 template <int W, int MODE>
 __global__ void __launch_bounds__(256) k_scan_candidates(const u64* __restrict__ super_and,
-                                                         const u32* __restrict__ super_min, u32 supers,
+                                                         const u32* __restrict__ super_min, u32 m, u32 super_rows,
                                                          const u64* __restrict__ Q, u32 q, u32 group0, u32 groups, int n,
                                                          const u32* __restrict__ flags, const u32* witness,
                                                          const u32* __restrict__ size_floor, int stop,
-                                                         uint2* __restrict__ items, u32* count) {
+                                                         uint2* __restrict__ items, u32* count, const u32* m_live,
+                                                         const u32* q_live) {
+  const u32 supers = (live_count(m, m_live) + super_rows - 1) / super_rows;
+  q = live_count(q, q_live);
   const u32 lane = threadIdx.x & 31, g = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (g >= groups) return;
   if (stop) {  // met in an earlier slice of the queries
@@ -271,10 +276,15 @@ __global__ void __launch_bounds__(kMaxScanWarps * 32, W <= 4 ? 3 : 2) k_subset_s
                                                                     const u32* __restrict__ size_floor, int stop,
                                                                     const uint2* __restrict__ items,
                                                                     u32* counts, u32 chunk, u32 split_units,
-                                                                    u64* __restrict__ bytes_ctr) {
+                                                                    u64* __restrict__ bytes_ctr, const u32* m_live,
+                                                                    const u32* q_live) {
   const u32 lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  const u32 tiles = (m + tile_rows - 1) / tile_rows, supers = (tiles + tps - 1) / tps;
+  u32 tiles = (m + tile_rows - 1) / tile_rows, supers = (tiles + tps - 1) / tps;
   const MaskLayout L = mask_layout(W, m, tiles, supers);
+  m = live_count(m, m_live);
+  q = live_count(q, q_live);
+  tiles = (m + tile_rows - 1) / tile_rows;
+  supers = (tiles + tps - 1) / tps;
   const u64* const super_and = masks + L.super_and;
   const u64* const group_and = masks + L.group_and;
   const u32* const tile_min = reinterpret_cast<const u32*>(masks + L.tile_min);
@@ -449,13 +459,14 @@ size_t subset_check_temp_bytes(int W, u32 m, const ScanShape& sh) {
   return sizeof(u64) * mask_layout(W, mm, n_tiles(mm, sh), n_supers(mm, sh)).words;
 }
 
-void launch_tile_and(int W, const u64* S, u32 m, u64* masks, u32* size_floor, const ScanShape& sh, cudaStream_t s) {
+void launch_tile_and(int W, const u64* S, u32 m, u64* masks, u32* size_floor, const ScanShape& sh, cudaStream_t s,
+                     const u32* m_live) {
   if (!m) return;
   if (!scan_shape_valid(W, sh)) throw std::invalid_argument("range_and: invalid scan shape");
   const u32 blocks = n_supers(m, sh);
   const int threads = sh.tiles_per_super * 32;
 #define SW_RA(WW) \
-  case WW: k_range_and<WW><<<blocks, threads, 0, s>>>(S, m, masks, (u32)sh.tile_rows, size_floor); break;
+  case WW: k_range_and<WW><<<blocks, threads, 0, s>>>(S, m, masks, (u32)sh.tile_rows, size_floor, m_live); break;
   switch (W) {
     SW_RA(1)
     SW_RA(2)
@@ -473,11 +484,12 @@ void launch_tile_and(int W, const u64* S, u32 m, u64* masks, u32* size_floor, co
 
 void launch_subset_check(int W, int mode, const u64* S, u32 m, const u64* masks, const u32* size_floor, const u64* Q,
                          u32 q, int n, u32* flags, u32* witness, bool stop, const ScanShape& sh, cudaStream_t s,
-                         u64* bytes_ctr, uint2* items, u32* item_counts) {
+                         u64* bytes_ctr, uint2* items, u32* item_counts, const u32* m_live, const u32* q_live) {
   if (!m || !q) return;
   if (!scan_shape_valid(W, sh)) throw std::invalid_argument("subset check: invalid scan shape");
   const u32 tiles = n_tiles(m, sh), supers = n_supers(m, sh);
   const MaskLayout L = mask_layout(W, m, tiles, supers);
+  const u32 super_rows = (u32)(sh.tile_rows * sh.tiles_per_super);
   const u32 groups = (q + 31) / 32, warps = (u32)sh.warps;
   const u64 pairs = (u64)groups * supers;
   // no more blocks than are resident (the launch bounds): the others only find the
@@ -499,11 +511,12 @@ void launch_subset_check(int W, int mode, const u64* S, u32 m, const u64* masks,
   {                                                                                                                   \
     if (listed)                                                                                                       \
       k_scan_candidates<WW, MM><<<(gs + 7) / 8, 256, 0, s>>>(                                                         \
-          masks + L.super_and, reinterpret_cast<const u32*>(masks + L.super_min), supers, Q, q, g0, gs, n, flags,     \
-          witness, size_floor, stop, items, item_counts);                                                              \
+          masks + L.super_and, reinterpret_cast<const u32*>(masks + L.super_min), m, super_rows, Q, q, g0, gs, n,     \
+          flags, witness, size_floor, stop, items, item_counts, m_live, q_live);                                       \
     k_subset_scan<WW, MM><<<blocks, warps * 32, 0, s>>>(S, m, masks, (u32)sh.tile_rows, (u32)sh.tiles_per_super, Q,   \
                                                         q, n, flags, witness, size_floor, stop,                       \
-                                                        listed ? items : nullptr, item_counts, chunk, kSplitUnits, bytes_ctr);      \
+                                                        listed ? items : nullptr, item_counts, chunk, kSplitUnits, bytes_ctr,       \
+                                                        m_live, q_live);                                              \
   }
 #define SW_SC(WW)                                                           \
   case WW:                                                                  \
