@@ -614,6 +614,34 @@ class Engine {
                    P.forward ? "BFS " : "IBFS", P.parents, P.children, u, f, P.reduce ? "reduced" : "duplicates only",
                    vclock() - P.t0);
   }
+  // X's children without duplicates among themselves, in bucket order, as its next
+  // layer, whose count is left in d_misc[8].
+  void step_distinct(Side& X, int W, int k) {
+    const u32 m = X.count, Nc = m * (u32)k;
+    const u64 slots = slots_for(Nc);
+    level_table.reserve(sizeof(u64) * slots);
+    ch_rows.reserve(sizeof(u64) * W * (size_t)Nc);
+    X.rows_alt.reserve(sizeof(u64) * W * (size_t)Nc);
+    const BucketScratch bk = buckets(Nc);
+    SW_CUDA(cudaMemsetAsync(level_table.p, 0, sizeof(u64) * slots, stream));
+    timed(1, (double)m * 8.0 * W * (1 + k) + (double)Nc * 16.0, [&] {
+      launch_expand_hash(W, true, X.rows.as<u64>(), m, tables, ch_rows.as<u64>(), nullptr, 0, level_table.as<u64>(),
+                         (u32)(slots - 1), bk, d_misc + kScanErrWord, stream);
+    });
+    std::unique_ptr<Layer> L = X.new_layer(sizeof(u32) * (size_t)Nc);
+    L->origin.reserve(sizeof(u32) * (size_t)Nc);
+    timed(3, (double)Nc * (2 * 8.0 * W + 8 + 4), [&] {
+      launch_bucket_scatter(W, ch_rows.as<u64>(), Nc, bk, 0, X.rows_alt.as<u64>(), L->origin.as<u32>(), nullptr,
+                            d_misc + 8, stream);
+    });
+    count_launch(3);
+    if (st) st->subsets_expanded += Nc;
+    std::swap(X.rows.p, X.rows_alt.p);
+    std::swap(X.rows.cap, X.rows_alt.cap);
+    L->parent_count = m;
+    X.layers.push_back(std::move(L));
+    X.count = Nc;
+  }
   // Back to a current layer of its own and a visited list in key order.
   void unhash(Side& X, int W) {
     if (!X.hashed) return;
@@ -2257,23 +2285,34 @@ void Solver::learned_beam(const Automaton& A, const sw_learned_beam_config& cfg,
   // engine-owned, kept across calls: freeing device memory would synchronise the device
   DevBuf &counts = E.lb_counts, &scores = E.lb_scores, &keys = E.lb_keys, &vals = E.lb_vals;
   DevBuf &alt_k = E.lb_alt_k, &alt_v = E.lb_alt_v, &sel_rows = E.lb_sel_rows, &sel_origin = E.lb_sel_origin;
-  std::vector<u32> pc;
+  u64* const sum = reinterpret_cast<u64*>(E.d_misc + 32);  // as in reduce(): ~(the first single-state set) follows
+  const size_t sum_bytes = 8 * sizeof(u64) + sizeof(u32);
   u64 found_len = 0;
   std::vector<uint32_t> word;
   for (u64 depth = 1; depth < b.upper && (cfg.max_iter < 0 || depth <= (u64)cfg.max_iter); ++depth) {
-    E.step(E.F, true, W, n, k, /*dominance=*/false);  // children, duplicates removed, origins recorded
+    // Layers of up to kSelectMax children scored by the model: duplicates dropped by
+    // the hash table and the kept sets selected, where the others are sorted twice.
+    // Ordering by size stays sorted: most of its keys are equal.
+    const bool select = use_model && (u64)E.F.count * k <= kSelectMax;
+    if (select)
+      E.step_distinct(E.F, W, k);
+    else
+      E.step(E.F, true, W, n, k, /*dominance=*/false);  // children, duplicates removed, origins recorded
+    SW_CUDA(cudaMemsetAsync(sum, 0, sum_bytes, E.stream));
+    launch_list_summary(W, E.F.rows.as<u64>(), E.F.count, sum, reinterpret_cast<u32*>(sum + 8), E.stream,
+                        select ? E.d_misc + 8 : nullptr);
+    SW_CUDA(cudaMemcpyAsync(E.pinned.p, E.d_misc, 32 * sizeof(u32) + sum_bytes, cudaMemcpyDeviceToHost, E.stream));
+    SW_CUDA(cudaStreamSynchronize(E.stream));
+    Engine::check_scan_error(E.pinned.as<u32>()[Engine::kScanErrWord]);
+    const u32 single = E.pinned.as<u32>()[48];
+    if (select) {
+      E.F.count = E.F.layers.back()->count = E.pinned.as<u32>()[8];
+      st.subsets_kept += E.F.count;
+    }
     const u32 m = E.F.count;
     if (!m) break;
-    counts.reserve(sizeof(u32) * m);
-    launch_popcount(W, E.F.rows.as<u64>(), m, counts.as<u32>(), E.stream);
-    pc.resize(m);
-    SW_CUDA(cudaMemcpyAsync(pc.data(), counts.p, sizeof(u32) * m, cudaMemcpyDeviceToHost, E.stream));
-    SW_CUDA(cudaStreamSynchronize(E.stream));
-    u32 hit = UINT32_MAX;
-    for (u32 i = 0; i < m && hit == UINT32_MAX; ++i)
-      if (pc[i] == 1) hit = i;
-    if (hit != UINT32_MAX) {
-      word = E.trace(E.F, hit, nullptr);
+    if (single) {
+      word = E.trace(E.F, ~single, nullptr);
       std::reverse(word.begin(), word.end());
       found_len = depth;
       break;
@@ -2286,17 +2325,28 @@ void Solver::learned_beam(const Automaton& A, const sw_learned_beam_config& cfg,
       scores.reserve(sizeof(float) * m);
       E.mlp->forward(E.F.rows.as<u64>(), W, m, scores.as<float>());
     }
+    if (cfg.order != SW_ORDER_MODEL) {
+      counts.reserve(sizeof(u32) * m);
+      launch_popcount(W, E.F.rows.as<u64>(), m, counts.as<u32>(), E.stream);
+    }
     launch_score_keys(use_model ? scores.as<float>() : nullptr,
                       cfg.order != SW_ORDER_MODEL ? counts.as<u32>() : nullptr, m, keys.as<u64>(), E.stream);
-    launch_iota(vals.as<u32>(), m, E.stream);
-    E.sort_rows(1, keys.as<u64>(), vals.as<u32>(), m);
+    if (select) {
+      launch_select(W, keys.as<u64>(), m, width, E.F.rows.as<u64>(), vals.as<u32>(), E.stream);
+      E.count_launch();
+    } else {
+      launch_iota(vals.as<u32>(), m, E.stream);
+      E.sort_rows(1, keys.as<u64>(), vals.as<u32>(), m);
+    }
     sel_rows.reserve(sizeof(u64) * W * width);
     sel_origin.reserve(sizeof(u32) * width);
     launch_gather_rows(W, E.F.rows.as<u64>(), vals.as<u32>(), width, sel_rows.as<u64>(), E.stream);
     Layer& top = *E.F.layers.back();
     launch_gather_u32(top.origin.as<u32>(), vals.as<u32>(), width, sel_origin.as<u32>(), E.stream);
-    SW_CUDA(cudaMemcpyAsync(E.F.rows.p, sel_rows.p, sizeof(u64) * W * width, cudaMemcpyDeviceToDevice, E.stream));
-    SW_CUDA(cudaMemcpyAsync(top.origin.p, sel_origin.p, sizeof(u32) * width, cudaMemcpyDeviceToDevice, E.stream));
+    std::swap(E.F.rows.p, sel_rows.p);
+    std::swap(E.F.rows.cap, sel_rows.cap);
+    std::swap(top.origin.p, sel_origin.p);
+    std::swap(top.origin.cap, sel_origin.cap);
     top.count = width;
     E.F.count = width;
     E.count_launch(5);

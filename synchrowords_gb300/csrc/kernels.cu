@@ -1604,6 +1604,122 @@ void launch_score_keys(const float* score, const u32* counts, u32 m, u64* keys, 
   SW_LAUNCH_CHECK();
 }
 
+// sel[0 .. width) = the rows with the smallest score keys (their upper halves),
+// ascending; equal scores by layer key, then position.  One CTA: a radix select
+// over four bytes of the score, then the rows at the threshold ranked among
+// themselves (few: equal scores of different sets are rare).  Only the set of kept
+// rows matters to a beam, so nothing is sorted.  Bound by its ~20 barriers and
+// the histograms; with the unsorted duplicate removal before it a level of 8192
+// children takes 90 us, where sorting the children and then the scores took 210
+// (beam of 4096, n=256: 7 -> 3 ms).
+constexpr u32 kSelectThreads = 1024;
+template <int W>
+__global__ void __launch_bounds__(kSelectThreads) k_select(const u64* __restrict__ keys, u32 m, u32 width,
+                                                           const u64* __restrict__ rows, u32* __restrict__ sel) {
+  extern __shared__ __align__(16) u32 s_score[];
+  u32* const s_drop = s_score + m;  // bitmap: rows at the threshold that stay out
+  uint16_t* const s_ties = reinterpret_cast<uint16_t*>(s_drop + (m + 31) / 32);
+  __shared__ u32 s_hist[256], s_bin, s_before, s_count, s_sum[32];
+  const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rounds = (m + kSelectThreads - 1) / kSelectThreads;
+  for (u32 i = tid; i < m; i += kSelectThreads) s_score[i] = (u32)(keys[i] >> 32);
+  for (u32 i = tid; i < (m + 31) / 32; i += kSelectThreads) s_drop[i] = 0;
+  u32 prefix = 0, mask = 0, need = width, equal = 0;
+  for (int shift = 24; shift >= 0; shift -= 8) {
+    if (tid < 256) s_hist[tid] = 0;
+    __syncthreads();
+    for (u32 r = 0; r < rounds; ++r) {
+      const u32 i = r * kSelectThreads + tid;
+      const u32 v = i < m ? s_score[i] : 0u;
+      const bool in = i < m && (v & mask) == prefix;
+      const u32 who = __ballot_sync(kFull, in);
+      if (in) {
+        const u32 bin = (v >> shift) & 255u, peers = __match_any_sync(who, bin);
+        if ((int)lane == __ffs(peers) - 1) atomicAdd(&s_hist[bin], (u32)__popc(peers));
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      u32 c[8], sum = 0;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) sum += c[b] = s_hist[8 * lane + b];
+      u32 incl = sum;
+#pragma unroll
+      for (u32 d = 1; d < 32; d *= 2) {
+        const u32 o = __shfl_up_sync(kFull, incl, d);
+        if (lane >= d) incl += o;
+      }
+      u32 at = incl - sum;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        if (at < need && need <= at + c[b]) {
+          s_bin = 8 * lane + b;
+          s_before = at;
+          s_count = c[b];
+        }
+        at += c[b];
+      }
+    }
+    __syncthreads();
+    prefix |= s_bin << shift;
+    mask |= 255u << shift;
+    need -= s_before;
+    equal = s_count;
+  }
+  if (need < equal) {  // the same for every thread
+    __syncthreads();
+    if (tid == 0) s_count = 0;
+    __syncthreads();
+    for (u32 i = tid; i < m; i += kSelectThreads)
+      if (s_score[i] == prefix) s_ties[atomicAdd(&s_count, 1u)] = (uint16_t)i;
+    __syncthreads();
+    for (u32 t = tid; t < equal; t += kSelectThreads) {
+      const u32 i = s_ties[t];
+      u64 a0, a1;
+      layer_key<W>(rows + (size_t)i * W, KeyMap{}, a0, a1);
+      u32 rank = 0;
+      for (u32 j = 0; j < equal && rank < need; ++j) {
+        const u32 o = s_ties[j];
+        u64 b0, b1;
+        layer_key<W>(rows + (size_t)o * W, KeyMap{}, b0, b1);
+        rank += b0 < a0 || (b0 == a0 && (b1 < a1 || (b1 == a1 && o < i)));
+      }
+      if (rank >= need) atomicOr(&s_drop[i >> 5], 1u << (i & 31));
+    }
+  }
+  __syncthreads();
+  // each thread a run of rows
+  const u32 i0 = min(tid * rounds, m), i1 = min(i0 + rounds, m);
+  u32 mine = 0;
+  for (u32 i = i0; i < i1; ++i) {
+    const u32 v = s_score[i];
+    mine += v < prefix || (v == prefix && !((s_drop[i >> 5] >> (i & 31)) & 1u));
+  }
+  u32 incl = mine;
+#pragma unroll
+  for (u32 d = 1; d < 32; d *= 2) {
+    const u32 o = __shfl_up_sync(kFull, incl, d);
+    if (lane >= d) incl += o;
+  }
+  if (lane == 31) s_sum[warp] = incl;
+  __syncthreads();
+  const u32 other = s_sum[lane];
+  u32 at = __reduce_add_sync(kFull, lane < warp ? other : 0u) + incl - mine;
+  for (u32 i = i0; i < i1; ++i) {
+    const u32 v = s_score[i];
+    if (v < prefix || (v == prefix && !((s_drop[i >> 5] >> (i & 31)) & 1u))) sel[at++] = i;
+  }
+}
+
+void launch_select(int W, const u64* keys, u32 m, u32 width, const u64* rows, u32* sel, cudaStream_t s) {
+  if (m > kSelectMax || width == 0 || width > m) throw std::invalid_argument("select: size");
+  const size_t smem = sizeof(u32) * (m + (m + 31) / 32) + sizeof(uint16_t) * m;
+  SW_DISPATCH_W(W, {
+    ensure_smem_limit((const void*)k_select<WW>, (int)(sizeof(u32) * (kSelectMax + kSelectMax / 32) + sizeof(uint16_t) * kSelectMax));
+    k_select<WW><<<1, kSelectThreads, smem, s>>>(keys, m, width, rows, sel);
+  });
+  SW_LAUNCH_CHECK();
+}
+
 // One thread follows the chain of origins: a dependent load and a division per
 // layer (under 1 us), where a read-back per layer cost a copy and a stream
 // synchronisation each (about 10 us; 0.36 ms of an n = 200 solve of 37 layers).

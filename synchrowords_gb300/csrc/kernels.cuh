@@ -243,6 +243,10 @@ void launch_gather_u32(const u32* src, const u32* idx, u32 m, u32* dst, cudaStre
 // primary = the order-preserving bits of score[i] (counts null), counts[i]
 // (score null), or counts[i] << 16 | leading 16 bits of score[i] (both).
 void launch_score_keys(const float* score, const u32* counts, u32 m, u64* keys, cudaStream_t s);
+// sel[0 .. width) = positions, ascending, of the `width` rows with the smallest
+// score keys (upper halves; ties by layer key); 0 < width <= m <= kSelectMax.
+constexpr u32 kSelectMax = 1u << 14;
+void launch_select(int W, const u64* keys, u32 m, u32 width, const u64* rows, u32* sel, cudaStream_t s);
 
 // Walks a word back: step i reads o = steps[i].origin[idx], emits the letter
 // out[i] = o / parents and goes on at idx = o % parents; out[count] = the last idx.
