@@ -60,7 +60,7 @@ struct Side {
   // The last hashed step, and where its layer's count is while only the device
   // knows it (count is then an upper bound).
   struct Step {
-    u32 parents = 0, children = 0, base = 0, visited = 0;
+    u32 parents = 0, children = 0, base = 0, visited = 0, distinct = 0, kept = 0;
     bool forward = false, reduce = false, self = false, compacted = false, deferred = false;
     double t0 = 0;
   } step;
@@ -135,8 +135,9 @@ class Engine {
   }
   ~Engine() {
     for (auto e : ev_pool) cudaEventDestroy(e);
-    for (auto e : meet_ev)
-      if (e) cudaEventDestroy(e);
+    for (auto* p : {&reduce_span, &meet_span})
+      for (auto e : p->ev)
+        if (e) cudaEventDestroy(e);
     if (d_query_bytes) cudaFree(d_query_bytes);
     if (d_misc) cudaFree(d_misc);
     if (stream) cudaStreamDestroy(stream);
@@ -418,19 +419,19 @@ class Engine {
     if (!m_live && !q_live) count_query(m, q);
   }
 
-  // Device time of the last meet check.
-  cudaEvent_t meet_ev[2] = {nullptr, nullptr};
-  void meet_begin() {
-    for (cudaEvent_t& e : meet_ev)
-      if (!e) SW_CUDA(cudaEventCreate(&e));
-    SW_CUDA(cudaEventRecord(meet_ev[0], stream));
-  }
-  void meet_end() { SW_CUDA(cudaEventRecord(meet_ev[1], stream)); }
-  double meet_seconds() {
-    float ms = 0;
-    SW_CUDA(cudaEventElapsedTime(&ms, meet_ev[0], meet_ev[1]));
-    return 1e-3 * ms;
-  }
+  // Device time of a level's dominance checks and of its meet check.
+  struct Span {
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    void mark(int i, cudaStream_t s) {
+      if (!ev[i]) SW_CUDA(cudaEventCreate(&ev[i]));
+      SW_CUDA(cudaEventRecord(ev[i], s));
+    }
+    double seconds() const {
+      float ms = 0;
+      SW_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
+      return 1e-3 * ms;
+    }
+  } reduce_span, meet_span;
 
   // Step log on stderr when SYNCHRO_VERBOSE is set (synchronises per phase).
   const bool verbose = std::getenv("SYNCHRO_VERBOSE") != nullptr;
@@ -557,10 +558,12 @@ class Engine {
       if (reduce && u) {
         flags_a.reserve(sizeof(u32) * (size_t)u);
         SW_CUDA(cudaMemsetAsync(flags_a.p, 0, sizeof(u32) * (size_t)u, stream));
+        reduce_span.mark(0, stream);
         if (X.vis_count && visited_subsets)
           dominated(forward, W, X.vis.as<u64>(), X.vis_count, fresh, u, n, false, flags_a.as<u32>(), nullptr, fresh_live);
         if (self_check)
           dominated(forward, W, fresh, u, fresh, u, n, true, flags_a.as<u32>(), fresh_live, fresh_live);
+        reduce_span.mark(1, stream);
         const u32 epoch = next_dc_epoch(u);
         timed(3, (double)u * (4 + 2 * (8.0 * W + 4)), [&] {
           launch_keep_compact(W, fresh, fresh_origin, flags_a.as<u32>(), u, out, L->origin.as<u32>(), d_misc + 9,
@@ -605,6 +608,8 @@ class Engine {
       if (P.self) count_query(u, u);
     }
     if (X.split) X.met_count = P.base + u;
+    P.distinct = u;
+    P.kept = f;
     X.layers.back()->count = f;
     X.count = f;
     X.vis_count += f;
@@ -1319,6 +1324,18 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
   // levels before the bound, took 190 ms where 35 was enough).
   constexpr double kStepLaunch = 8e-5, kMeetLaunch = 1.5e-5;
   constexpr u32 kSwitchRows = 4096;
+  struct Reduction {
+    double seconds = 0, dropped = 0;  // of the last reduced level: time of the checks, share dropped
+    u32 parents = 0;
+  } reductions[2];
+  double rest = 0;  // projected seconds to the end of the search (0: not known)
+  // The checks must save kReduceGain times less than they cost to be left out, and
+  // a search that leaves them out switches at kSwitchUnreduced of the projection,
+  // since each further level then enlarges what the bounded phase starts from.
+  // Sum over 18 LearnedBeam + Exact n=256 / 12 Beam + Exact n=300 searches, ms: no
+  // rule 469 / 533; gain 0.6 333 / 640, 1 349 / 605, 1.4 with the earlier switch
+  // 365 / 519, 2 365 / 547 (512 with it), 4 388 / 544.
+  constexpr double kReduceGain = 1.4, kSwitchUnreduced = 0.5;
   double t_iter_last = 0, t_meet_per_query = 0, b_growth = k * 0.95;
   while (rt < max_rt) {  // meet_in_the_middle.cpp:73
     const auto t_iter0 = std::chrono::steady_clock::now();
@@ -1346,8 +1363,15 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
     // phase expands B from its size at the switch) or lists past a quarter
     // of the memory budget
     const bool pressure = 4 * (live + next) > budget;
-    E.self_check = E.visited_subsets = cfg.reductions == SW_REDUCE_ALWAYS ||
-                                       (cfg.reductions == SW_REDUCE_AUTO && b.has_word) || pressure;
+    bool reduce = cfg.reductions == SW_REDUCE_ALWAYS || (cfg.reductions == SW_REDUCE_AUTO && b.has_word);
+    // ... and, left to this rule, only while what they drop saves more of the
+    // projected rest of the search than they cost (their time grows with the square)
+    Reduction& red_last = reductions[fwd];
+    if (cfg.reductions == SW_REDUCE_AUTO && red_last.parents && rest > 0) {
+      const double g = (double)X.count / red_last.parents;
+      if (red_last.seconds * g * g > kReduceGain * red_last.dropped * rest) reduce = false;
+    }
+    E.self_check = E.visited_subsets = reduce || pressure;
     E.step(X, fwd, W, n, k, /*dominance=*/!bounded, false, /*defer=*/true);
     if (fwd) {
       st.bfs_steps++;
@@ -1359,11 +1383,11 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
     // the switch to the bounded phase prices the meet check per query: it is timed
     // while that switch is possible
     const bool time_meet = !bounded && b.has_word;
-    if (time_meet) E.meet_begin();
+    if (time_meet) E.meet_span.mark(0, E.stream);
     SW_CUDA(cudaMemsetAsync(E.d_misc, 0, 4 * sizeof(u32), E.stream));
     E.query(W, kQueryDisjoint, E.F.cur_rows(W), E.F.count, E.B.cur_rows(W), E.B.count, n, nullptr, true, E.F.live,
             E.B.live);
-    if (time_meet) E.meet_end();
+    if (time_meet) E.meet_span.mark(1, E.stream);
     // the one read-back of a level: witness, error, the step's counts (a reduced
     // level read back four times: n=100 plans of ~19 levels 2.7 -> 2.4 ms, plain
     // n=200 levels twice: 3.1 -> 2.9 ms)
@@ -1378,11 +1402,13 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
       E.count_query(E.F.count, E.B.count);
     }
     st.meet_pairs += (u64)E.F.count * E.B.count;
+    if (X.hashed && X.step.compacted && X.step.distinct && time_meet)
+      red_last = Reduction{E.reduce_span.seconds(), 1.0 - (double)X.step.kept / X.step.distinct, X.step.parents};
     // projected branching of the bounded levels: distinct children per parent
     // before pruning, never below 1.2
     if (!fwd && parents_before) b_growth = std::max(1.2, E.B.unique_growth);
     t_iter_last = std::chrono::duration<double>(t_end - t_iter0).count();
-    if (E.B.count && time_meet) t_meet_per_query = E.meet_seconds() / (double)E.B.count;
+    if (E.B.count && time_meet) t_meet_per_query = E.meet_span.seconds() / (double)E.B.count;
     if (!bounded && b.has_word && !w[0] && rt < max_rt && rt >= 4 && E.B.count >= kSwitchRows) {
       const u64 R = max_rt - rt;  // levels still to exclude
       // per child: expansion and hash table (0.12-0.25 ns measured at 10^7
@@ -1406,9 +1432,13 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
           fits = false;
         lvl *= b_growth;
       }
+      // without the checks' own time, which is what the rest is held against
+      const double checks = X.hashed && X.step.compacted ? std::min(red_last.seconds, t_iter_last) : 0.0;
+      const double plain = mitm * (1.0 - checks / std::max(t_iter_last, 1e-9));
+      rest = fits ? std::min(total, plain) : plain;
       // voluntary switch only when every projected level fits; chunking is the
       // safety net for an exhausted budget, not a plan
-      if (fits && total < mitm) {
+      if (fits && total * (reduce ? 1.0 : kSwitchUnreduced) < mitm) {
         bounded = true;
         if (E.verbose)
           std::fprintf(stderr, "[sw] bounded phase from length %llu: %llu levels left, |F|=%u |B|=%u, "
