@@ -244,7 +244,7 @@ typedef struct {
 /* What the last sw_solve_batch on this context did on the device (no
  * counterpart in the reference, which solves one automaton at a time). */
 typedef struct {
-  uint32_t small_solved;    /* automata finished by the shared-memory batched launch */
+  uint32_t small_solved;    /* automata finished by the batched launch (small clusters) */
   uint32_t cluster_solved;  /* automata finished by the cluster launch */
   uint32_t streamed;        /* automata solved on the worker streams */
   uint32_t launches;        /* batched kernel launches */

@@ -396,7 +396,7 @@ void start_round(sw_context* ctx, DeviceRound& D, const std::vector<uint32_t> sm
 }
 
 // Waits for a round, verifies and stores what it solved; returns the
-// instances it did not finish (those of the shared-memory launch go to
+// instances it did not finish (those of the small clusters' launch go to
 // *unfinished_small when given).
 std::vector<uint32_t> finish_round(sw_context* ctx, DeviceRound& D, const uint32_t* deltas,
                                    const std::vector<size_t>& off, const uint32_t* ns, const uint32_t* ks,

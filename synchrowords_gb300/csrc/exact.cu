@@ -29,6 +29,7 @@
 #include "exact.hpp"
 #include "kernels.cuh"
 #include "learn.hpp"
+#include "train.hpp"
 
 namespace sw {
 
@@ -146,6 +147,7 @@ class Engine {
   cudaStream_t stream = nullptr;
   HostPinned pinned;
   std::unique_ptr<MlpRunner> mlp;
+  std::unique_ptr<Trainer> trainer;  // of the first training call; its buffers are kept
 
   // ---- optional per-kernel-class timing (CUDA events on `stream`) ----
   // class 0: subset-query tree walks, 1: layer expansion, 2: radix sorts,
@@ -2202,25 +2204,38 @@ void Solver::mlp_forward(const Automaton& A, const uint64_t* sets, uint64_t coun
   SW_CUDA(cudaStreamSynchronize(E.stream));
 }
 
+// The trainer, with the loaded parameters and no moments.
+static Trainer& training(Engine& E) {
+  if (!E.mlp->has_params()) throw std::runtime_error("no distance model loaded");
+  if (!E.trainer) E.trainer = std::make_unique<Trainer>(E.stream);
+  std::vector<float> p(mlp::kParams);
+  E.mlp->get_params(p.data());
+  E.trainer->set_params(p.data());  // waits for the stream
+  return *E.trainer;
+}
+
 float Solver::mlp_gradient(const Automaton& A, const uint64_t* sets, const float* labels, uint64_t count,
                            float* grad) {
   SW_CUDA(cudaSetDevice(device_));
   Engine& E = *eng_;
   if (!count) throw std::invalid_argument("empty batch");
-  DevBuf d_rows, d_t;
+  DevBuf d_rows, d_y, d_t;
   d_rows.reserve(sizeof(u64) * 8 * count);
+  d_y.reserve(sizeof(float) * count);
   d_t.reserve(sizeof(float) * count);
   SW_CUDA(cudaMemcpyAsync(d_rows.p, sets, sizeof(u64) * 8 * count, cudaMemcpyHostToDevice, E.stream));
   launch_convert_rows(8, d_rows.as<u64>(), count, (int)A.n, true, E.stream);
   SW_CUDA(cudaMemcpyAsync(d_t.p, labels, sizeof(float) * count, cudaMemcpyHostToDevice, E.stream));
-  E.mlp->prepare(A);
-  E.mlp->zero_grad();
-  E.mlp->gradient(d_rows.as<u64>(), 8, (u32)count, d_t.as<float>(), nullptr, 0.0f, E.mlp->loss());
+  Trainer& T = training(E);
+  T.prepare(A);
+  T.zero_grad();
+  T.forward(d_rows.as<u64>(), 8, (u32)count, d_y.as<float>());
+  T.backward(d_t.as<float>(), (u32)count);
   float loss = 0;
-  SW_CUDA(cudaMemcpyAsync(grad, E.mlp->grad(), sizeof(float) * mlp::kParams, cudaMemcpyDeviceToHost, E.stream));
-  SW_CUDA(cudaMemcpyAsync(&loss, E.mlp->loss(), sizeof(float), cudaMemcpyDeviceToHost, E.stream));
+  SW_CUDA(cudaMemcpyAsync(grad, T.grad(), sizeof(float) * mlp::kParams, cudaMemcpyDeviceToHost, E.stream));
+  SW_CUDA(cudaMemcpyAsync(&loss, T.loss(), sizeof(float), cudaMemcpyDeviceToHost, E.stream));
   SW_CUDA(cudaStreamSynchronize(E.stream));
-  if (mlp::tc_error()) throw CudaError("distance model: a tensor-core wait ran out");
+  if (train::tc_error()) throw CudaError("distance model: a tensor-core wait ran out");
   return loss;
 }
 
@@ -2233,7 +2248,9 @@ float Solver::mlp_train(const std::vector<Automaton>& autos, const uint64_t* off
   const uint64_t total = offsets[A_n];
   if (!total || !batch) throw std::invalid_argument("no training pairs");
   // all pairs resident on the device as 8-word rows
-  DevBuf d_rows, d_lab, d_grp, d_loss;
+  Trainer& T = training(E);
+  DevBuf d_rows, d_lab, d_grp, d_y;
+  d_y.reserve(sizeof(float) * batch);
   d_rows.reserve(sizeof(u64) * 8 * total);
   d_lab.reserve(sizeof(float) * total);
   SW_CUDA(cudaMemcpyAsync(d_rows.p, sets, sizeof(u64) * 8 * total, cudaMemcpyHostToDevice, E.stream));
@@ -2245,11 +2262,6 @@ float Solver::mlp_train(const std::vector<Automaton>& autos, const uint64_t* off
     d_grp.reserve(sizeof(uint32_t) * total);
     SW_CUDA(cudaMemcpyAsync(d_grp.p, groups, sizeof(uint32_t) * total, cudaMemcpyHostToDevice, E.stream));
   }
-  // one loss per step, read once an epoch: the steps queue without waiting for each other
-  uint64_t steps = 0;
-  for (size_t a = 0; a < A_n; ++a) steps += (offsets[a + 1] - offsets[a] + batch - 1) / batch;
-  d_loss.reserve(sizeof(float) * steps);
-  std::vector<float> step_loss(steps);
   std::vector<size_t> order(A_n);
   for (size_t a = 0; a < A_n; ++a) order[a] = a;
   uint64_t state = seed;
@@ -2262,26 +2274,30 @@ float Solver::mlp_train(const std::vector<Automaton>& autos, const uint64_t* off
   double last = 0;
   for (uint32_t ep = 0; ep < epochs; ++ep) {
     for (size_t a = A_n; a > 1; --a) std::swap(order[a - 1], order[next() % a]);
-    SW_CUDA(cudaMemsetAsync(d_loss.p, 0, sizeof(float) * steps, E.stream));
-    E.mlp->zero_grad();
-    uint64_t step = 0;
+    double sum = 0;
+    uint64_t steps = 0;
     for (size_t oi = 0; oi < A_n; ++oi) {
       const size_t a = order[oi];
-      for (uint64_t o = offsets[a]; o < offsets[a + 1]; o += batch, ++step) {
+      for (uint64_t o = offsets[a]; o < offsets[a + 1]; o += batch) {
         const u32 c = (u32)std::min<uint64_t>(batch, offsets[a + 1] - o);
-        E.mlp->prepare(autos[a]);
-        E.mlp->gradient(d_rows.as<u64>() + o * 8, 8, c, d_lab.as<float>() + o,
-                        d_grp.p ? d_grp.as<uint32_t>() + o : nullptr, rank_w, d_loss.as<float>() + step);
-        E.mlp->adam_step(lr);
+        T.prepare(autos[a]);
+        T.zero_grad();
+        T.forward(d_rows.as<u64>() + o * 8, 8, c, d_y.as<float>());
+        T.backward(d_lab.as<float>() + o, c, d_grp.p ? d_grp.as<uint32_t>() + o : nullptr, rank_w);
+        T.adam_step(lr);
+        float l = 0;
+        SW_CUDA(cudaMemcpyAsync(&l, T.loss(), sizeof(float), cudaMemcpyDeviceToHost, E.stream));
+        SW_CUDA(cudaStreamSynchronize(E.stream));
+        sum += l;
+        ++steps;
       }
     }
-    SW_CUDA(cudaMemcpyAsync(step_loss.data(), d_loss.p, sizeof(float) * steps, cudaMemcpyDeviceToHost, E.stream));
-    SW_CUDA(cudaStreamSynchronize(E.stream));
-    double sum = 0;
-    for (float l : step_loss) sum += l;
     last = steps ? sum / steps : 0.0;
   }
-  if (mlp::tc_error()) throw CudaError("distance model: a tensor-core wait ran out");
+  if (train::tc_error()) throw CudaError("distance model: a tensor-core wait ran out");
+  std::vector<float> trained(mlp::kParams);
+  T.get_params(trained.data());
+  E.mlp->set_params(trained.data());
   return (float)last;
 }
 

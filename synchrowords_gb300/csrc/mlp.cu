@@ -1,12 +1,10 @@
-// Kernels of the learned distance model (mlp.cuh).
+// Scoring kernels of the learned distance model (mlp.cuh).
 //
-// A training step on a batch of a few hundred sets is 1.5 GFLOP: what it costs is
-// launches and the round trips between them.  So the whole forward pass of a
-// block of 128 sets is one block of one launch, and the whole backward pass
-// another: the activations of a block go from TMEM through registers into the
-// next product's shared-memory operand, and only what the other pass needs is
-// written out.  (One launch per product, bias and conversion took 45 launches and
-// 540 us a step at batch 512.)
+// Scoring some thousand sets is about 0.1 GFLOP: what it costs is launches and the
+// round trips between them.  So the whole forward pass of 128 sets is one block of
+// one launch: activations go from TMEM through registers into the next product's
+// shared-memory operand (18 us for 8192 sets at n = 256, where one launch per
+// product, bias and conversion took eleven).
 //
 // Every product runs on the fifth-generation tensor cores: tcgen05.mma
 // kind::f16 (bf16 x bf16 -> fp32), M = 128, N = 64 or 128, K = 16 per
@@ -38,10 +36,6 @@ constexpr u32 kSlice = kRows * 64 * 2;  // bytes of a 128-row operand slice; 64-
 constexpr u32 kFwdB = 2 * kSlice, kFwdBar = 4 * kSlice;
 constexpr u32 kFwdSmem = 100 * 1024;
 static_assert(kFwdBar + 32 <= kFwdSmem, "forward block's shared memory");
-// Backward block: four operands of two slices, the sets' rows, mbarrier; one block an SM (512 TMEM columns).
-constexpr u32 kBwdB = 2 * kSlice, kBwdC = 4 * kSlice, kBwdT = 6 * kSlice, kBwdRows = 8 * kSlice,
-              kBwdBar = kBwdRows + kRows * 8 * 8;
-constexpr u32 kBwdSmem = kBwdBar + 32;
 
 __device__ u32 g_tc_error = 0;
 
@@ -348,250 +342,8 @@ void forward(const u64* rows, int W, int n, u32 count, const bf16* staged_e, con
              float* y, const Activations& act, cudaStream_t s) {
   if (!count) return;
   const u32 blocks = (count + kRows - 1) / kRows;
-  if (act.h2) {
-    ensure_smem_limit((const void*)k_forward<true>, kFwdSmem);
-    k_forward<true><<<blocks, kThreads, kFwdSmem, s>>>(rows, W, n, count, staged_e, weights, params, y, act);
-  } else {
-    ensure_smem_limit((const void*)k_forward<false>, kFwdSmem);
-    k_forward<false><<<blocks, kThreads, kFwdSmem, s>>>(rows, W, n, count, staged_e, weights, params, y, act);
-  }
-  SW_LAUNCH_CHECK();
-}
-
-// ---- loss ----
-// Warp per row.  The ranking term pairs the rows of one group (one BFS layer):
-// for t_a < t_b, w / rows * softplus(y_a - y_b), so that a set nearer to a
-// singleton scores lower than its sibling.  (One thread per row walked the batch
-// with dependent loads: 75 us at 512 rows.)
-__global__ void __launch_bounds__(256) k_loss(const float* __restrict__ y, const float* __restrict__ tgt,
-                                              const uint32_t* __restrict__ grp, int rows, float w,
-                                              float* __restrict__ dy, float* loss) {
-  __shared__ float s_sum[8];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * 8 + warp;
-  float l = 0.0f;
-  if (i < rows) {
-    const float yi = y[i], ti = tgt[i];
-    float g = 0.0f;
-    if (grp) {
-      const uint32_t gi = grp[i];
-      for (int j0 = 0; j0 < rows; j0 += 32) {
-        const int j = j0 + lane;
-        float term = 0.0f;
-        if (j < rows && grp[j] == gi) {
-          const float tj = tgt[j];
-          if (ti < tj) {  // i should score below j
-            const float z = yi - y[j];
-            term = 1.0f / (1.0f + __expf(-z));
-            l += z > 20.0f ? z : log1pf(__expf(z));
-          } else if (tj < ti) {  // j should score below i
-            term = -(1.0f / (1.0f + __expf(-(y[j] - yi))));
-          }
-        }
-#pragma unroll
-        for (int x = 0; x < 32; ++x) g += __shfl_sync(0xffffffffu, term, x);  // in the order of j
-      }
-#pragma unroll
-      for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-      l *= w / (float)rows;
-    }
-    if (lane == 0) {
-      const float d = yi - ti;
-      l += d * d / (float)rows;
-      dy[i] = 2.0f * d / (float)rows + (grp ? w * g / (float)rows : 0.0f);
-    }
-  }
-  if (lane == 0) s_sum[warp] = i < rows ? l : 0.0f;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float b = 0.0f;
-    for (int x = 0; x < 8; ++x) b += s_sum[x];
-    atomicAdd(loss, b);
-  }
-}
-
-void loss(const float* y, const float* t, const uint32_t* grp, int rows, float w, float* dy, float* loss,
-          cudaStream_t s) {
-  if (!rows) return;
-  k_loss<<<(rows + 7) / 8, 256, 0, s>>>(y, t, w > 0.0f ? grp : nullptr, rows, w, dy, loss);
-  SW_LAUNCH_CHECK();
-}
-
-// ---- backward ----
-// TMEM columns: dH1 and then the dE tiles 0 .. 127, dW2 128 .. 255, dX 256 .. 319,
-// dW1 384 .. 511.
-__global__ void __launch_bounds__(kThreads, 1) k_backward(const u64* __restrict__ rows, int W, int n, u32 count,
-                                                          const float* __restrict__ dy,
-                                                          const bf16* __restrict__ weights,
-                                                          const float* __restrict__ params, Activations act,
-                                                          float* grad, float* de) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t *const sA = smem, *const sB = smem + kBwdB, *const sC = smem + kBwdC, *const sT = smem + kBwdT;
-  u64* const s_rows = reinterpret_cast<u64*>(smem + kBwdRows);  // [128][8]
-  u32* const slot = reinterpret_cast<u32*>(smem + kBwdBar + 16);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = warp & 3, half = warp >> 2;
-  const u32 i0 = blockIdx.x * kRows;
-  const int r = q * 32 + lane;
-  const u32 row = i0 + r;
-  const bool in = row < count;
-  const int words = (n + 63) / 64;
-  Tc tc;
-  tc.open(sm_addr(smem + kBwdBar), sm_addr(slot), slot, 512);
-  for (int e = tid; e < kRows * words; e += kThreads) {
-    const int rr = e / words, w = e - rr * words;
-    s_rows[rr * 8 + w] = i0 + rr < count ? rows[(size_t)(i0 + rr) * W + w] : 0ULL;
-  }
-  const float d = in ? dy[row] : 0.0f;
-  if (half == 0) {
-    float b = d;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
-    if (lane == 0) atomicAdd(grad + kOffB3, b);
-  }
-  // head: dw3, db2, dH2 = dy w3^T * [h2 open] (rows and columns); h1 by columns
-#pragma unroll
-  for (int cb = 0; cb < 2; ++cb) {
-    const int c = half * 64 + cb * 32;
-    const u32 open = in ? act.open2[(size_t)row * 4 + (c >> 5)] : 0u;
-    float v[32];
-    u32 p[16];
-    const uint4* h = reinterpret_cast<const uint4*>(act.h2 + (size_t)row * kHidden + c);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint4 x = in ? h[i] : make_uint4(0, 0, 0, 0);
-      p[4 * i] = x.x;
-      p[4 * i + 1] = x.y;
-      p[4 * i + 2] = x.z;
-      p[4 * i + 3] = x.w;
-    }
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = d * unpack(p[i / 2], i & 1);
-    atomicAdd(grad + kOffW3 + c + lane, column_sums(v));
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = (open >> i) & 1u ? d * __ldg(params + kOffW3 + c + i) : 0.0f;
-    put_rows(v, r, c, sA, nullptr);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) p[i] = pack2(v[2 * i], v[2 * i + 1]);
-    put_columns(p, r, c, sT, kSlice);
-    atomicAdd(grad + kOffB2 + c + lane, column_sums(v));
-    h = reinterpret_cast<const uint4*>(act.h1 + (size_t)row * kHidden + c);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint4 x = in ? h[i] : make_uint4(0, 0, 0, 0);
-      p[4 * i] = x.x;
-      p[4 * i + 1] = x.y;
-      p[4 * i + 2] = x.z;
-      p[4 * i + 3] = x.w;
-    }
-    put_columns(p, r, c, sC, kSlice);
-  }
-  copy_in(sB, weights + kOffW2B, kStagedW2 * 2);
-  tc.publish();
-  if (tid == 0) {
-    issue_mma(tc.tmem, sm_addr(sA), sm_addr(sB), kSlice, 2, kHidden, false);        // dH1 = dH2 · W2^T
-    issue_mma(tc.tmem + 128, sm_addr(sC), sm_addr(sT), kSlice, 2, kHidden, false);  // dW2 = h1^T · dH2
-    tc.commit();
-  }
-  bool ok = tc.wait();
-  if (ok) {
-#pragma unroll
-    for (int cb = 0; cb < 2; ++cb) {
-      const int c = half * 64 + cb * 32;
-      const u32 open = in ? act.open1[(size_t)row * 4 + (c >> 5)] : 0u;
-      float v[32];
-      ld32(tc.tmem, q * 32, c, v);
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = (open >> i) & 1u ? v[i] : 0.0f;
-      put_rows(v, r, c, sA, nullptr);
-      u32 p[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) p[i] = pack2(v[2 * i], v[2 * i + 1]);
-      put_columns(p, r, c, sT, kSlice);
-      atomicAdd(grad + kOffB1 + c + lane, column_sums(v));
-      ld32(tc.tmem + 128, q * 32, c, v);
-      float4* const g = reinterpret_cast<float4*>(grad + kOffW2 + (size_t)r * kHidden + c);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) atomicAdd(g + i, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
-    }
-    {  // x by columns: rows 0 .. 63 of the operand, the others zero
-      u32 p[16];
-      const uint4* const h = reinterpret_cast<const uint4*>(act.x + (size_t)row * kEmb + half * 32);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint4 x = in ? h[i] : make_uint4(0, 0, 0, 0);
-        p[4 * i] = x.x;
-        p[4 * i + 1] = x.y;
-        p[4 * i + 2] = x.z;
-        p[4 * i + 3] = x.w;
-      }
-      put_columns(p, r, half * 32, sC, kSlice);
-      for (int e = tid; e < 1024; e += kThreads)
-        *reinterpret_cast<uint4*>(sC + (e >> 9) * kSlice + kSlice / 2 + (e & 511) * 16) = make_uint4(0, 0, 0, 0);
-    }
-    copy_in(sB, weights + kOffW1B, kStagedW1 * 2);
-    tc.publish();
-    if (tid == 0) {
-      issue_mma(tc.tmem + 256, sm_addr(sA), sm_addr(sB), kSlice / 2, 2, kEmb, false);  // dX = dH1 · W1^T
-      issue_mma(tc.tmem + 384, sm_addr(sC), sm_addr(sT), kSlice, 2, kHidden, false);   // dW1 = x^T · dH1
-      tc.commit();
-    }
-    ok = tc.wait();
-  }
-  if (ok) {
-    float v[32];
-    if (q < 2) {
-#pragma unroll
-      for (int cb = 0; cb < 2; ++cb) {
-        const int c = half * 64 + cb * 32;
-        ld32(tc.tmem + 384, q * 32, c, v);
-        float4* const g = reinterpret_cast<float4*>(grad + kOffW1 + (size_t)r * kHidden + c);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) atomicAdd(g + i, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
-      }
-    }
-    ld32(tc.tmem + 256, q * 32, half * 32, v);
-    u32 p[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) p[i] = pack2(v[2 * i], v[2 * i + 1]);
-    put_columns(p, r, half * 32, sB, kSlice / 2);
-  }
-  // dE += bits^T · dX, 128 states at a time
-  for (int t0 = 0; t0 < n && ok; t0 += kRows) {
-    for (int e = tid; e < kRows * 16; e += kThreads) {
-      const int m = e & 127, kg = e >> 7, s = t0 + m;  // state s, rows 8 kg .. 8 kg + 7
-      u32 b[4] = {0, 0, 0, 0};
-      if (s < n) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if ((s_rows[(8 * kg + j) * 8 + (s >> 6)] >> (63 - (s & 63))) & 1ULL) b[j >> 1] |= j & 1 ? 0x3F800000u : 0x3F80u;
-      }
-      *reinterpret_cast<uint4*>(sA + (kg >> 3) * kSlice + core_offset(m, (kg & 7) * 8)) =
-          make_uint4(b[0], b[1], b[2], b[3]);
-    }
-    tc.publish();
-    if (tid == 0) {
-      issue_mma(tc.tmem, sm_addr(sA), sm_addr(sB), kSlice / 2, 2, kEmb, false);
-      tc.commit();
-    }
-    ok = tc.wait();
-    if (ok) {
-      float v[32];
-      ld32(tc.tmem, q * 32, half * 32, v);
-      if (t0 + r < n) {
-        float4* const g = reinterpret_cast<float4*>(de + (size_t)(t0 + r) * kEmb + half * 32);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) atomicAdd(g + i, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
-      }
-    }
-  }
-  tc.close(512);
-}
-
-void backward(const u64* rows, int W, int n, u32 count, const float* dy, const bf16* weights, const float* params,
-              const Activations& act, float* grad, float* de, cudaStream_t s) {
-  if (!count) return;
-  ensure_smem_limit((const void*)k_backward, kBwdSmem);
-  k_backward<<<(count + kRows - 1) / kRows, kThreads, kBwdSmem, s>>>(rows, W, n, count, dy, weights, params, act, grad,
-                                                                    de);
+  ensure_smem_limit((const void*)k_forward<false>, kFwdSmem);
+  k_forward<false><<<blocks, kThreads, kFwdSmem, s>>>(rows, W, n, count, staged_e, weights, params, y, act);
   SW_LAUNCH_CHECK();
 }
 
@@ -657,47 +409,6 @@ void embed(const float* feat, const float* params, int n, float* epre, bf16* sta
   SW_LAUNCH_CHECK();
 }
 
-// Block of 32 states, thread (feature f, columns): dPhi += feat^T · bf16(de open),
-// dc += column sums; de cleared.
-constexpr int kEbStates = 32;
-__global__ void __launch_bounds__(256) k_embed_back(const float* __restrict__ feat, const float* __restrict__ epre, int n,
-                                                    float* __restrict__ de, float* grad) {
-  __shared__ float s_d[kEbStates][kEmb];   // masked, fp32
-  __shared__ float s_f[kEbStates][kFeat];  // rounded to bf16
-  const int s0 = blockIdx.x * kEbStates, tid = threadIdx.x;
-  for (int e = tid; e < kEbStates * kEmb; e += 256) {
-    const int s = s0 + e / kEmb;
-    float v = 0.0f;
-    if (s < n) {
-      const size_t at = (size_t)s * kEmb + e % kEmb;
-      v = epre[at] > 0.0f ? de[at] : 0.0f;
-      de[at] = 0.0f;
-    }
-    s_d[e / kEmb][e % kEmb] = v;
-  }
-  for (int e = tid; e < kEbStates * kFeat; e += 256) {
-    const int s = s0 + e / kFeat;
-    s_f[e / kFeat][e % kFeat] = s < n ? __bfloat162float(__float2bfloat16(feat[(size_t)s * kFeat + e % kFeat])) : 0.0f;
-  }
-  __syncthreads();
-  const int j = tid & 63, fq = tid >> 6;  // features 4 fq .. 4 fq + 3
-  float a[4] = {0, 0, 0, 0}, c = 0.0f;
-  for (int s = 0; s < kEbStates; ++s) {
-    const float v = s_d[s][j], b = __bfloat162float(__float2bfloat16(v));
-    c += v;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] += s_f[s][4 * fq + i] * b;
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) atomicAdd(grad + kOffPhi + (4 * fq + i) * kEmb + j, a[i]);
-  if (fq == 0) atomicAdd(grad + kOffC + j, c);
-}
-
-void embed_back(const float* feat, const float* epre, int n, float* de, float* grad, cudaStream_t s) {
-  k_embed_back<<<(n + kEbStates - 1) / kEbStates, 256, 0, s>>>(feat, epre, n, de, grad);
-  SW_LAUNCH_CHECK();
-}
-
 // ---- weights ----
 // bf16 copies of W1[i][j] and W2[i][j] where the products read them: forward as
 // B(N = j, K = i), backward as B(N = i, K = j).
@@ -721,27 +432,6 @@ __global__ void k_stage_weights(const float* __restrict__ p, bf16* __restrict__ 
 
 void stage_weights(const float* p, bf16* weights, cudaStream_t s) {
   k_stage_weights<<<(kParams + 255) / 256, 256, 0, s>>>(p, weights);
-  SW_LAUNCH_CHECK();
-}
-
-// Adam (Kingma & Ba 2015) with beta1 = 0.9, beta2 = 0.999, eps = 1e-8.
-__global__ void k_adam(float* p, float* g, float* m, float* v, bf16* w, float lr, float c1, float c2) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= kParams) return;
-  const float gr = g[e];
-  g[e] = 0.0f;
-  const float mm = 0.9f * m[e] + 0.1f * gr;
-  const float vv = 0.999f * v[e] + 0.001f * gr * gr;
-  m[e] = mm;
-  v[e] = vv;
-  const float np = p[e] - lr * (mm / c1) / (sqrtf(vv / c2) + 1e-8f);
-  p[e] = np;
-  stage_weight(w, e, np);
-}
-
-void adam(float* p, float* g, float* m, float* v, bf16* weights, float lr, int t, cudaStream_t s) {
-  const float c1 = 1.0f - std::pow(0.9f, (float)t), c2 = 1.0f - std::pow(0.999f, (float)t);
-  k_adam<<<(kParams + 255) / 256, 256, 0, s>>>(p, g, m, v, weights, lr, c1, c2);
   SW_LAUNCH_CHECK();
 }
 

@@ -55,18 +55,6 @@ void embed(const float* feat, const float* params, int n, float* epre, bf16* sta
 // y of `count` sets (device rows of W words).
 void forward(const u64* rows, int W, int n, u32 count, const bf16* staged_e, const bf16* weights, const float* params,
              float* y, const Activations& act, cudaStream_t s);
-// loss[0] += mean (y - t)^2 plus, with grp and w > 0, w / rows sum over pairs of one
-// group with t_a < t_b of softplus(y_a - y_b); dy = its gradient in y.
-void loss(const float* y, const float* t, const uint32_t* grp, int rows, float w, float* dy, float* loss,
-          cudaStream_t s);
-// grad += the gradients of W1, b1, W2, b2, w3, b3; de (n x 64, zero before) += the embeddings'.
-void backward(const u64* rows, int W, int n, u32 count, const float* dy, const bf16* weights, const float* params,
-              const Activations& act, float* grad, float* de, cudaStream_t s);
-// grad += the gradients of Phi and c; de is cleared.
-void embed_back(const float* feat, const float* epre, int n, float* de, float* grad, cudaStream_t s);
-// Adam step t (1-based) on the parameters, which also refreshes the staged
-// weights and clears the gradient.
-void adam(float* p, float* g, float* m, float* v, bf16* weights, float lr, int t, cudaStream_t s);
 void stage_weights(const float* p, bf16* weights, cudaStream_t s);
 
 // True once a product's bounded wait for its tensor-core work ran out (its

@@ -13,7 +13,7 @@ enough that an ncu capture of a few launches ends in seconds:
   n320     one Beam(dynamic)+Exact solve (the reference's configs/exact.json
            Beam and Exact entries), n = 320: large subset checks of the
            bounded inverse phase
-  gemm     one LearnedBeam(4096) run, n = 200 (the model's k_gemm products)
+  gemm     one LearnedBeam(4096) run, n = 200 (the model's k_forward)
 
 Usage: python -m synchrowords_gb300.profile_cases <case>
 """
