@@ -27,7 +27,8 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "-Xc
 
 LIB_SOURCES = ["kernels.cu", "subset_check.cu", "dominance.cu", "noalloc.cu", "pairs.cu", "brute.cu", "beam.cu",
                "batch_cluster.cu", "mlp.cu",
-               "learn.cu", "train_steps.cu", "train.cu", "exact.cu", "plan.cpp", "automaton.cpp", "abi.cpp"]
+               "learn.cu", "train_steps.cu", "train.cu", "exact.cu", "plan.cpp", "automaton.cpp", "abi.cpp",
+               "testing.cpp"]
 CLI_SOURCES = ["cli.cpp"]
 
 

@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cstdio>
 #include <stdexcept>
 #include <string>
@@ -26,12 +27,17 @@ struct CudaError : std::runtime_error {
   explicit CudaError(const std::string& s) : std::runtime_error(s) {}
 };
 
+// A failed call also leaves its error on the thread, where the next launch check
+// would find it; reported here, it is taken off (an error that ended the context
+// comes back with every later call all the same).
 #define SW_CUDA(call)                                                                      \
   do {                                                                                     \
     cudaError_t _e = (call);                                                               \
-    if (_e != cudaSuccess)                                                                 \
+    if (_e != cudaSuccess) {                                                               \
+      (void)cudaGetLastError();                                                            \
       throw ::sw::CudaError(std::string(#call) + " failed: " + cudaGetErrorString(_e) +  \
                             " at " + __FILE__ + ":" + std::to_string(__LINE__));           \
+    }                                                                                      \
   } while (0)
 
 #define SW_LAUNCH_CHECK() SW_CUDA(cudaGetLastError())
@@ -79,6 +85,14 @@ struct AllocScope {
   AllocScope& operator=(const AllocScope&) = delete;
 };
 
+// How many buffer growths from now on succeed before one fails as it does when
+// the device is full (negative: none fails).  Only tests set it (testing.cpp).
+inline std::atomic<int> g_growths_until_failure{-1};
+inline size_t growth_bytes(size_t want) {
+  if (g_growths_until_failure.load(std::memory_order_relaxed) < 0) return want;
+  return g_growths_until_failure.fetch_sub(1) == 0 ? (size_t)1 << 60 : want;
+}
+
 // Grow-only device buffer (the context keeps them across steps and solves,
 // so a solve performs no per-step cudaMalloc).
 struct DevBuf {
@@ -92,7 +106,7 @@ struct DevBuf {
   }
   void reserve(size_t bytes) {
     if (bytes <= cap) return;
-    const size_t want = bytes + bytes / 4 + 256;
+    const size_t want = growth_bytes(bytes + bytes / 4 + 256);
     if (cudaStream_t s = alloc_stream()) {
       if (p) SW_CUDA(cudaFreeAsync(p, s));
       p = nullptr;
