@@ -412,6 +412,7 @@ class Engine {
       else  // complements: the set of c lies in the set of s
         launch_dominance(W, true, false, S, m, Q, q, n, proper, flags, sc, stream, m_live, q_live);
     });
+    if (tm > kDomOrderRows) scanned();
     if (prof_on) {
       cudaEvent_t e1 = next_event();
       SW_CUDA(cudaEventRecord(e1, stream));
@@ -462,17 +463,27 @@ class Engine {
 
   // ---- duplicate removal by hash table ----
   DevBuf bk_counts, bk_first, bk_place, level_table;
+  // Bucket counts are zero between steps: the scan that reads them clears them.
+  // A step that ends before that scan (its buffers did not fit) leaves counts
+  // behind, and the next step would move its rows past their list; so every use
+  // starts with buckets(), which zeroes what such a step left, and ends with
+  // scanned() once the scan is launched.
+  bool bk_open = true;
   BucketScratch buckets(u64 children) {
     const size_t bytes = sizeof(u32) << kBucketBitsLarge;
-    if (bk_counts.cap < bytes) {
-      bk_counts.reserve(bytes);
-      SW_CUDA(cudaMemsetAsync(bk_counts.p, 0, bk_counts.cap, stream));
-    }
+    bk_counts.reserve(bytes);
     bk_first.reserve(bytes);
     bk_place.reserve(sizeof(uint2) * children);
+    if (bk_open) {
+      SW_CUDA(cudaMemsetAsync(bk_counts.p, 0, bk_counts.cap, stream));
+      SW_CUDA(cudaMemsetAsync(d_misc + 6, 0, 2 * sizeof(u32), stream));
+      SW_CUDA(cudaMemsetAsync(d_misc + 14, 0, 2 * sizeof(u32), stream));
+    }
+    bk_open = true;
     return BucketScratch{bucket_bits(children), bk_counts.as<u32>(), bk_first.as<u32>(), bk_place.as<uint2>(),
                          d_misc + 6};
   }
+  void scanned() { bk_open = false; }
   // Power-of-two slots, two to four per row.
   static u64 slots_for(u64 rows) {
     u64 s = 1024;
@@ -547,6 +558,7 @@ class Engine {
       launch_bucket_scatter(W, ch_rows.as<u64>(), Nc, bk, base, fresh, fresh_origin, X.table.as<u64>(), d_misc + 8,
                             stream);
     });
+    scanned();
     count_launch(3);
     defer = defer && Nc && (reduce || !X.split);
     u32 u = Nc;
@@ -641,6 +653,7 @@ class Engine {
       launch_bucket_scatter(W, ch_rows.as<u64>(), Nc, bk, 0, X.rows_alt.as<u64>(), L->origin.as<u32>(), nullptr,
                             d_misc + 8, stream);
     });
+    scanned();
     count_launch(3);
     if (st) st->subsets_expanded += Nc;
     std::swap(X.rows.p, X.rows_alt.p);
@@ -888,6 +901,7 @@ class Engine {
       launch_bucket_scatter(W, ch_rows.as<u64>(), Nc, bk, 0, out_rows.as<u64>(), out_origin.as<u32>(), nullptr,
                             d_misc + 8, stream);
     });
+    scanned();
     count_launch(3);
     if (st) st->subsets_expanded += N;
     out_count = read_total_checked();
@@ -1026,6 +1040,7 @@ class Engine {
       launch_bucket_rank(W, cur, cnt, bk, stream);
       launch_bucket_scatter(W, cur, cnt, bk, base, X.vis.as<u64>() + (size_t)base * W, ch_vals.as<u32>(), nullptr,
                             d_misc + 8, stream);
+      scanned();
       count_launch(4);
       X.hashed = X.in_vis = true;
       X.cur_off = base;

@@ -1,9 +1,12 @@
 """Calls that end for want of device memory leave their context usable: the
 next calls on it give what a fresh context gives."""
+import json
+
 import numpy as np
 import pytest
 
 import synchrowords_gb300 as sw
+from synchrowords_gb300.generate import random_dfa
 
 pytestmark = pytest.mark.gpu
 
@@ -22,3 +25,66 @@ def test_error_stays_with_its_call(fail_growth):
         with pytest.raises(sw.SynchroError):
             c.sort_unique(40, sets)
         assert len(c.sort_unique(40, sets)) == 3
+
+
+def plan(*algorithms, **top):
+    return json.dumps({**top, "algorithms": [{"name": name, "config": config} for name, config in algorithms]})
+
+
+PLANS = {
+    "plain": plan(("Exact", {})),
+    "always": plan(("Exact", {"reductions": "always"})),
+    "reduce": plan(("Eppstein", {}), ("Beam", {"presort": "indeg", "beam_size": "10"}),
+                   ("Reduce", {"min_n": "40", "list_size_threshold": "AUT_N * 16"}), ("Exact", {})),
+    # the bounded phase, in chunks
+    "bounded": plan(("Beam", {"presort": "indeg", "beam_size": "AUT_N * 4"}),
+                    ("Exact", {"max_memory_mb": "4", "dfs_min_list_size": "512"})),
+}
+
+
+def answers(results):
+    return [(r.non_synchro, r.lower, r.upper, r.word is not None) for r in results]
+
+
+# at n = 200 the lists pass 2^16 children and the size where the dominance checks order them
+@pytest.mark.parametrize("name,n,k,seed", [("plain", 200, 2, 12), ("always", 65, 3, 1), ("always", 200, 2, 12),
+                                           ("reduce", 100, 3, 4), ("bounded", 120, 2, 7700)])
+def test_solves_after_a_failed_growth(fail_growth, name, n, k, seed):
+    big, small = random_dfa(n, k, seed), random_dfa(70, 2, 5)
+    with sw.Context(0) as c:
+        want = answers([c.solve(big, n, k, PLANS[name]), c.solve(small, 70, 2, PLANS["always"])])
+    failed = 0
+    for successes in range(500):
+        with sw.Context(0) as c:
+            fail_growth(successes)
+            try:
+                c.solve(big, n, k, PLANS[name])
+            except sw.SynchroError:
+                failed += 1
+            else:
+                break
+            finally:
+                fail_growth(-1)
+            assert answers([c.solve(small, 70, 2, PLANS["always"])]) == want[1:]
+            assert answers([c.solve(big, n, k, PLANS[name]), c.solve(small, 70, 2, PLANS["always"])]) == want
+    assert 10 < failed < 500
+
+
+def test_batches_after_a_failed_growth(fail_growth):
+    automata = [(n, 2, random_dfa(n, 2, 300 + n)) for n in (40, 70, 101, 130, 170, 190, 200)]
+    with sw.Context(0) as c:
+        want = answers(c.solve_batch(automata, PLANS["plain"]))
+    failed = 0
+    for successes in range(0, 400, 3):
+        with sw.Context(0) as c:
+            fail_growth(successes)
+            try:
+                c.solve_batch(automata, PLANS["plain"])
+            except sw.SynchroError:
+                failed += 1
+            else:
+                break
+            finally:
+                fail_growth(-1)
+            assert answers(c.solve_batch(automata, PLANS["plain"])) == want
+    assert 3 < failed < 130
