@@ -280,7 +280,13 @@ class Engine {
   }
   Side F, B;
   Side R;  // the list of the last Reduce, from which a search of the reduced automaton starts
+  // Where the running call counts; the caller's record, so only for that long.
   sw_stats* st = nullptr;
+  struct Counting {
+    Engine& E;
+    Counting(Engine& e, sw_stats& st) : E(e) { E.st = &st; }
+    ~Counting() { E.st = nullptr; }
+  };
   std::vector<std::unique_ptr<DLevel>> dlevel_pool;  // the bounded phase's per-depth levels
   // scratch of the beams and of Reduce, kept across calls
   DevBuf lb_counts, lb_scores, lb_keys, lb_vals, lb_alt_k, lb_alt_v, lb_sel_rows, lb_sel_origin, red_states;
@@ -1221,7 +1227,7 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
   SW_CUDA(cudaSetDevice(device_));
   Engine& E = *eng_;
   AllocScope alloc_scope(E.stream);  // buffer growth ordered on this solve's stream only
-  E.st = &st;
+  const Engine::Counting counting(E, st);
   auto t0 = std::chrono::steady_clock::now();
   const int n = (int)A.n, k = (int)A.k, W = words_for(n);
   const size_t budget = (size_t)cfg.max_memory_mb * 1024 * 1024;
@@ -1236,7 +1242,6 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
   E.B.reset();
   auto finish = [&] {
     st.device_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-    E.st = nullptr;
   };
   // A search with duplicate removal only starts on one thread-block cluster
   // (the other reductions and reduced forward seeds are the streamed path's).
@@ -1688,7 +1693,7 @@ void Solver::beam(const Automaton& A0, const sw_beam_config& cfg, Bounds& b, sw_
   SW_CUDA(cudaSetDevice(device_));
   Engine& E = *eng_;
   AllocScope alloc_scope(E.stream);  // buffer growth ordered on this solve's stream only
-  E.st = &st;
+  const Engine::Counting counting(E, st);
   auto t0 = std::chrono::steady_clock::now();
   // presort (beam.hpp:54-63, 351-369): states ordered by in-degree ascending
   std::vector<uint32_t> perm(A0.n);
@@ -1730,7 +1735,6 @@ void Solver::beam(const Automaton& A0, const sw_beam_config& cfg, Bounds& b, sw_
     b.has_word = false;
   }
   st.device_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-  E.st = nullptr;
 }
 
 // ---------------------------------------------------------------------------
@@ -1970,7 +1974,7 @@ void Solver::reduce(const Automaton& A, const sw_reduce_config& cfg, Bounds& b, 
   if (A.n < cfg.min_n) return;                      // reduce.hpp:48-50
   SW_CUDA(cudaSetDevice(device_));
   Engine& E = *eng_;
-  E.st = &st;
+  const Engine::Counting counting(E, st);
   auto t0 = std::chrono::steady_clock::now();
   const int n = (int)A.n, k = (int)A.k, W = words_for(n);
   E.upload_tables(A);
@@ -1988,7 +1992,6 @@ void Solver::reduce(const Automaton& A, const sw_reduce_config& cfg, Bounds& b, 
   std::vector<uint32_t> word;
   auto done = [&] {
     st.device_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-    E.st = nullptr;
   };
   u64* const sum = reinterpret_cast<u64*>(E.d_misc + 32);  // the list's union, then ~(its first single-state set)
   const size_t sum_bytes = 8 * sizeof(u64) + sizeof(u32);
@@ -2328,7 +2331,7 @@ void Solver::learned_beam(const Automaton& A, const sw_learned_beam_config& cfg,
   }
   SW_CUDA(cudaSetDevice(device_));
   Engine& E = *eng_;
-  E.st = &st;
+  const Engine::Counting counting(E, st);
   auto t0 = std::chrono::steady_clock::now();
   const int n = (int)A.n, k = (int)A.k, W = words_for(n);
   E.upload_tables(A);
@@ -2420,7 +2423,6 @@ void Solver::learned_beam(const Automaton& A, const sw_learned_beam_config& cfg,
     b.word = word;
   }
   st.device_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-  E.st = nullptr;
 }
 
 }  // namespace sw

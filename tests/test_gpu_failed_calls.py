@@ -1,5 +1,6 @@
 """Calls that end for want of device memory leave their context usable: the
 next calls on it give what a fresh context gives."""
+import ctypes
 import json
 
 import numpy as np
@@ -88,3 +89,19 @@ def test_batches_after_a_failed_growth(fail_growth):
                 fail_growth(-1)
             assert answers(c.solve_batch(automata, PLANS["plain"])) == want
     assert 3 < failed < 130
+
+
+@pytest.mark.parametrize("name", ["plain", "reduce"])
+def test_later_calls_leave_the_record_of_a_failed_one(native_lib, fail_growth, name):
+    n, k = 100, 3
+    d = np.array(random_dfa(n, k, 4), dtype=np.uint32)
+    sets = np.arange(1, 200, dtype=np.uint64).reshape(-1, 1)
+    with sw.Context(0) as c:
+        record = sw._Result()
+        fail_growth(5)
+        assert native_lib.sw_solve_json(c._h, d.ctypes.data_as(sw._U32P), n, k, PLANS[name].encode(),
+                                        ctypes.byref(record)) != 0
+        fail_growth(-1)
+        before = bytes(record)
+        c.subsets_check(60, sets, sets)
+        assert bytes(record) == before
