@@ -49,6 +49,7 @@ void Trainer::prepare(const Automaton& A) {
   std::vector<uint32_t> key{A.n, A.k};
   key.insert(key.end(), A.t.begin(), A.t.end());
   if (key != feat_key_) {  // features depend on the automaton only: computed once per automaton
+    feat_key_.clear();  // until they are there: growing the buffer gives up the ones it holds
     const std::vector<float> f = state_features(A);
     feat_.reserve(sizeof(float) * f.size());
     feat_b_.reserve(sizeof(bf16) * f.size());

@@ -105,3 +105,58 @@ def test_later_calls_leave_the_record_of_a_failed_one(native_lib, fail_growth, n
         before = bytes(record)
         c.subsets_check(60, sets, sets)
         assert bytes(record) == before
+
+
+@pytest.mark.parametrize("what", ["forward", "gradient"])
+def test_scores_after_a_failed_growth(fail_growth, what):
+    rng = np.random.default_rng(2)
+    small, big = (40, 2, random_dfa(40, 2, 1)), (300, 2, random_dfa(300, 2, 2))
+    params = rng.normal(0, 0.1, sw.MLP_PARAMS).astype(np.float32)
+    labels = rng.normal(10, 3, 300).astype(np.float32)
+
+    def call(c, automaton):
+        n, k, d = automaton
+        sets = np.packbits(np.random.default_rng(n).random((300, 512)) < 0.2, axis=1, bitorder="little").view(np.uint64)
+        if what == "forward":
+            return c.mlp_forward(params, d, n, k, sets)
+        return c.mlp_gradient(params, d, n, k, sets, labels)[0]
+
+    with sw.Context(0) as c:
+        want = [call(c, small), call(c, big)]
+    failed = 0
+    for successes in range(200):
+        with sw.Context(0) as c:
+            call(c, small)
+            fail_growth(successes)
+            try:
+                call(c, big)
+            except sw.SynchroError:
+                failed += 1
+            else:
+                break
+            finally:
+                fail_growth(-1)
+            for automaton, w in zip((small, big), want):
+                np.testing.assert_allclose(call(c, automaton), w, rtol=1e-4, atol=1e-4 * np.abs(w).max())
+    assert 3 < failed < 200
+
+
+def test_learned_plans_after_a_failed_growth(fail_growth):
+    learned = plan(("LearnedBeam", {"beam_size": "1024", "order": "model"}), ("Exact", {}), upper_bound="4 * AUT_N")
+    n, d = 130, random_dfa(130, 2, 6)
+    with sw.Context(0) as c:
+        want = answers([c.solve(d, n, 2, learned)])
+    failed = 0
+    for successes in range(300):
+        with sw.Context(0) as c:
+            fail_growth(successes)
+            try:
+                c.solve(d, n, 2, learned)
+            except sw.SynchroError:
+                failed += 1
+            else:
+                break
+            finally:
+                fail_growth(-1)
+            assert answers([c.solve(d, n, 2, learned)]) == want
+    assert 10 < failed < 300
