@@ -1152,4 +1152,12 @@ int sw_mlp_train_ranked(sw_context* ctx, float* params, uint32_t automata, const
   });
 }
 
+// For tests, outside the public header (as testing.cpp).
+int sw_testing_plant_error(sw_context* ctx, uint32_t code) {
+  return guarded([&] {
+    ctx->solver->plant_error(code);
+    return SW_OK;
+  });
+}
+
 }  // extern "C"

@@ -132,7 +132,7 @@ class Engine {
     pinned.reserve(4096);
     SW_CUDA(cudaMalloc(&d_misc, 64 * sizeof(u32)));
     SW_CUDA(cudaMemset(d_misc, 0, 64 * sizeof(u32)));
-    mlp = std::make_unique<MlpRunner>(stream);
+    mlp = std::make_unique<MlpRunner>(stream, d_misc + kScanErrWord);
   }
   ~Engine() {
     for (auto e : ev_pool) cudaEventDestroy(e);
@@ -222,13 +222,17 @@ class Engine {
   }
   u32* d_misc = nullptr;  // [0..2] witness, [3] the subset check's size floor, [6, 7] children met before, [8] scan total, [9] rows kept by the reductions, [kScanErrWord] bounded-wait timeouts
   static constexpr int kScanErrWord = 4;  // read back with the witness, never cleared by it
-  // Throws if a launch reported a bounded wait that ran out: 2 = a compaction
-  // tile's look-back never saw its predecessor, 3 = a hash table's probe found
-  // no slot; `w` is the pinned copy of d_misc[kScanErrWord].
-  static void check_scan_error(u32 w) {
+  // Throws, and clears the word, if a launch reported a bounded wait that ran out:
+  // 2 = a compaction tile's look-back never saw its predecessor, 3 = a hash
+  // table's probe found no slot, mlp::kErrorWait; `w` is the pinned copy of
+  // d_misc[kScanErrWord].
+  void check_scan_error(u32 w) {
+    if (!w) return;
+    SW_CUDA(cudaMemsetAsync(d_misc + kScanErrWord, 0, sizeof(u32), stream));
+    if (w == mlp::kErrorWait) throw CudaError("distance model: a tensor-core wait ran out");
     if (w == 2) throw CudaError("layer compaction: a look-back wait ran out");
     if (w == 3) throw CudaError("duplicate removal: a hash table ran out of slots");
-    if (w) throw CudaError("a launch reported error " + std::to_string(w));
+    throw CudaError("a launch reported error " + std::to_string(w));
   }
   // Single-pass duplicate removal (launch_dedup_compact): its tile status
   // words (zero-filled when allocated), tile counter and launch epoch.
@@ -1418,7 +1422,7 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
     const auto t_end = std::chrono::steady_clock::now();
     u32 w[Engine::kStepWords];
     std::copy(E.pinned.as<u32>(), E.pinned.as<u32>() + Engine::kStepWords, w);
-    Engine::check_scan_error(w[Engine::kScanErrWord]);
+    E.check_scan_error(w[Engine::kScanErrWord]);
     if (X.live) {
       E.finish_step(X, w);
       E.count_query(E.F.count, E.B.count);
@@ -2219,6 +2223,13 @@ void Solver::mlp_forward(const Automaton& A, const uint64_t* sets, uint64_t coun
   E.mlp->prepare(A);
   E.mlp->forward(d_rows.as<u64>(), 8, (u32)count, d_y.as<float>());
   SW_CUDA(cudaMemcpyAsync(out, d_y.p, sizeof(float) * count, cudaMemcpyDeviceToHost, E.stream));
+  E.check_scan_error(E.read_u32(E.d_misc + Engine::kScanErrWord));
+}
+
+void Solver::plant_error(uint32_t code) {
+  SW_CUDA(cudaSetDevice(device_));
+  Engine& E = *eng_;
+  launch_fill_u32(E.d_misc + Engine::kScanErrWord, code, 1, E.stream);
   SW_CUDA(cudaStreamSynchronize(E.stream));
 }
 
@@ -2367,7 +2378,7 @@ void Solver::learned_beam(const Automaton& A, const sw_learned_beam_config& cfg,
                         select ? E.d_misc + 8 : nullptr);
     SW_CUDA(cudaMemcpyAsync(E.pinned.p, E.d_misc, 32 * sizeof(u32) + sum_bytes, cudaMemcpyDeviceToHost, E.stream));
     SW_CUDA(cudaStreamSynchronize(E.stream));
-    Engine::check_scan_error(E.pinned.as<u32>()[Engine::kScanErrWord]);
+    E.check_scan_error(E.pinned.as<u32>()[Engine::kScanErrWord]);
     const u32 single = E.pinned.as<u32>()[48];
     if (select) {
       E.F.count = E.F.layers.back()->count = E.pinned.as<u32>()[8];

@@ -79,6 +79,8 @@ class Solver {
   void subsets_check(uint32_t n, const uint64_t* sets, uint64_t set_count, const uint64_t* checks,
                      uint64_t check_count, bool proper, uint8_t* results);
   uint64_t sort_unique(uint32_t n, uint64_t* sets, uint64_t count);
+  // For tests: as if a launch had reported `code`.
+  void plant_error(uint32_t code);
 
   int device() const { return device_; }
   void* stream() const;  // the cudaStream_t every kernel of this solver runs on

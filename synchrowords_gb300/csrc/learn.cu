@@ -35,12 +35,12 @@ void MlpRunner::prepare(const Automaton& A) {
   }
   epre_.reserve(sizeof(float) * n_ * mlp::kEmb);
   e_.reserve(sizeof(bf16) * mlp::staged_embeddings(n_));
-  mlp::embed(feat_.as<float>(), params_.as<float>(), n_, epre_.as<float>(), e_.as<bf16>(), stream_);
+  mlp::embed(feat_.as<float>(), params_.as<float>(), n_, epre_.as<float>(), e_.as<bf16>(), error_, stream_);
 }
 
 void MlpRunner::forward(const u64* rows, int W, u32 count, float* y) {
   mlp::forward(rows, W, n_, count, e_.as<bf16>(), weights_.as<bf16>(), params_.as<float>(), y, mlp::Activations{},
-               stream_);
+               error_, stream_);
 }
 
 }  // namespace sw

@@ -13,7 +13,9 @@ namespace sw {
 
 class MlpRunner {
  public:
-  explicit MlpRunner(cudaStream_t s) : stream_(s) {}
+  // error: device word that a launch whose tensor-core wait ran out sets
+  // (mlp::kErrorWait); whoever reads a launch's results back reads it with them.
+  MlpRunner(cudaStream_t s, u32* error) : stream_(s), error_(error) {}
 
   // Parameters: host vector of mlp::kParams floats (layout in mlp.cuh).
   void set_params(const float* host);
@@ -29,6 +31,7 @@ class MlpRunner {
 
  private:
   cudaStream_t stream_;
+  u32* error_;
   bool loaded_ = false;
   int n_ = 0;
   std::vector<uint32_t> feat_key_;  // automaton whose features are in feat_ (n, k, table)

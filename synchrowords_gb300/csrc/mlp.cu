@@ -14,8 +14,8 @@
 // matrices" of 128 contiguous bytes, K-adjacent cores 128 bytes apart, 8-row
 // groups 1024 bytes apart); the weights and embeddings are kept in that layout in
 // global memory, so they are copied as they are.  Every wait is bounded: a wait
-// that runs out sets an error word (tc_error()) and the block frees its TMEM and
-// stops.
+// that runs out sets the caller's error word to kErrorWait and the block frees its
+// TMEM and stops.
 #include "mlp.cuh"
 
 #include <algorithm>
@@ -36,8 +36,6 @@ constexpr u32 kSlice = kRows * 64 * 2;  // bytes of a 128-row operand slice; 64-
 constexpr u32 kFwdB = 2 * kSlice, kFwdBar = 4 * kSlice;
 constexpr u32 kFwdSmem = 100 * 1024;
 static_assert(kFwdBar + 32 <= kFwdSmem, "forward block's shared memory");
-
-__device__ u32 g_tc_error = 0;
 
 __device__ __forceinline__ u32 sm_addr(const void* p) { return (u32)__cvta_generic_to_shared(p); }
 
@@ -94,8 +92,10 @@ __device__ __forceinline__ bool bar_wait(u32 bar, u32 parity) {
 // A block's tensor-core state.
 struct Tc {
   u32 tmem, bar, parity;
-  __device__ void open(u32 bar_addr, u32 slot_addr, const u32* slot, u32 columns) {
+  u32* err;
+  __device__ void open(u32 bar_addr, u32 slot_addr, const u32* slot, u32 columns, u32* error) {
     bar = bar_addr;
+    err = error;
     parity = 0;
     if (threadIdx.x == 0) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
@@ -126,7 +126,7 @@ struct Tc {
     const bool ok = __syncthreads_and(bar_wait(bar, parity));
     parity ^= 1u;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (!ok && threadIdx.x == 0) atomicExch(&g_tc_error, 1u);
+    if (!ok && threadIdx.x == 0) atomicExch(err, kErrorWait);
     return ok;
   }
   __device__ void close(u32 columns) {
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kThreads) k_forward(const u64* __restrict__ ro
                                                       const bf16* __restrict__ staged_e,
                                                       const bf16* __restrict__ weights,
                                                       const float* __restrict__ params, float* __restrict__ y,
-                                                      Activations act) {
+                                                      Activations act, u32* err) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t *const sA = smem, *const sB = smem + kFwdB;
   u32* const slot = reinterpret_cast<u32*>(smem + kFwdBar + 16);
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kThreads) k_forward(const u64* __restrict__ ro
   const u32 row = i0 + r;
   const bool in = row < count;
   Tc tc;
-  tc.open(sm_addr(smem + kFwdBar), sm_addr(slot), slot, 256);
+  tc.open(sm_addr(smem + kFwdBar), sm_addr(slot), slot, 256, err);
   bool ok = true;
   // x = bits · E: columns 0 .. 63, two 64-state slices at a time
   const int slices = (n + 63) / 64;
@@ -339,24 +339,19 @@ __global__ void __launch_bounds__(kThreads) k_forward(const u64* __restrict__ ro
 }
 
 void forward(const u64* rows, int W, int n, u32 count, const bf16* staged_e, const bf16* weights, const float* params,
-             float* y, const Activations& act, cudaStream_t s) {
+             float* y, const Activations& act, u32* err, cudaStream_t s) {
   if (!count) return;
   const u32 blocks = (count + kRows - 1) / kRows;
   ensure_smem_limit((const void*)k_forward<false>, kFwdSmem);
-  k_forward<false><<<blocks, kThreads, kFwdSmem, s>>>(rows, W, n, count, staged_e, weights, params, y, act);
+  k_forward<false><<<blocks, kThreads, kFwdSmem, s>>>(rows, W, n, count, staged_e, weights, params, y, act, err);
   SW_LAUNCH_CHECK();
-}
-
-bool tc_error() {
-  u32 v = 0;
-  SW_CUDA(cudaMemcpyFromSymbol(&v, g_tc_error, sizeof(u32)));
-  return v != 0;
 }
 
 // ---- embeddings ----
 // Block of 128 states: feat · Phi is one K = 16 product.
 __global__ void __launch_bounds__(kThreads) k_embed(const float* __restrict__ feat, const float* __restrict__ params,
-                                                    int n, float* __restrict__ epre, bf16* __restrict__ staged) {
+                                                    int n, float* __restrict__ epre, bf16* __restrict__ staged,
+                                                    u32* err) {
   __shared__ __align__(1024) uint8_t sA[kSlice];
   __shared__ __align__(1024) uint8_t sB[kSlice / 2];
   __shared__ __align__(16) uint64_t s_bar[2];
@@ -364,7 +359,7 @@ __global__ void __launch_bounds__(kThreads) k_embed(const float* __restrict__ fe
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = warp & 3, half = warp >> 2;
   const int s0 = blockIdx.x * kRows;
   Tc tc;
-  tc.open(sm_addr(s_bar), sm_addr(&slot), &slot, 64);
+  tc.open(sm_addr(s_bar), sm_addr(&slot), &slot, 64, err);
   for (int e = tid; e < kRows * kFeat; e += kThreads) {
     const int m = e / kFeat, f = e % kFeat;
     const float v = s0 + m < n ? feat[(size_t)(s0 + m) * kFeat + f] : 0.0f;
@@ -404,8 +399,8 @@ __global__ void __launch_bounds__(kThreads) k_embed(const float* __restrict__ fe
   tc.close(64);
 }
 
-void embed(const float* feat, const float* params, int n, float* epre, bf16* staged, cudaStream_t s) {
-  k_embed<<<(n + kRows - 1) / kRows, kThreads, 0, s>>>(feat, params, n, epre, staged);
+void embed(const float* feat, const float* params, int n, float* epre, bf16* staged, u32* err, cudaStream_t s) {
+  k_embed<<<(n + kRows - 1) / kRows, kThreads, 0, s>>>(feat, params, n, epre, staged, err);
   SW_LAUNCH_CHECK();
 }
 

@@ -50,16 +50,16 @@ struct Activations {
   u32 *open1 = nullptr, *open2 = nullptr;           // [rows][4]: bit c of word c / 32 = pre-activation above zero
 };
 
+// What a launch leaves in the error word it was given when a bounded wait for its
+// tensor-core work ran out (its results are then incomplete).
+constexpr u32 kErrorWait = 4;
+
 // epre = feat · Phi + c (fp32, n x 64), staged = bf16(relu(epre)).
-void embed(const float* feat, const float* params, int n, float* epre, bf16* staged, cudaStream_t s);
+void embed(const float* feat, const float* params, int n, float* epre, bf16* staged, u32* err, cudaStream_t s);
 // y of `count` sets (device rows of W words).
 void forward(const u64* rows, int W, int n, u32 count, const bf16* staged_e, const bf16* weights, const float* params,
-             float* y, const Activations& act, cudaStream_t s);
+             float* y, const Activations& act, u32* err, cudaStream_t s);
 void stage_weights(const float* p, bf16* weights, cudaStream_t s);
-
-// True once a product's bounded wait for its tensor-core work ran out (its
-// results are then incomplete); synchronises with the device.
-bool tc_error();
 
 }  // namespace mlp
 }  // namespace sw

@@ -160,3 +160,20 @@ def test_learned_plans_after_a_failed_growth(fail_growth):
                 fail_growth(-1)
             assert answers([c.solve(d, n, 2, learned)]) == want
     assert 10 < failed < 300
+
+
+@pytest.mark.parametrize("what", ["forward", "beam"])
+def test_a_scoring_wait_that_ran_out_is_reported(native_lib, what):
+    n, d = 130, random_dfa(130, 2, 6)
+    rows = np.packbits(np.random.default_rng(1).random((100, 512)) < 0.1, axis=1, bitorder="little").view(np.uint64)
+    learned = plan(("LearnedBeam", {"beam_size": "256", "order": "model"}), upper_bound="4 * AUT_N")
+
+    def call(c):
+        return c.mlp_forward(c.get_model(), d, n, 2, rows).tolist() if what == "forward" else c.solve(d, n, 2, learned).upper
+
+    with sw.Context(0) as c:
+        want = call(c)
+        assert native_lib.sw_testing_plant_error(c._h, 4) == 0  # what the kernel stores (mlp::kErrorWait)
+        with pytest.raises(sw.SynchroError, match="tensor-core wait"):
+            call(c)
+        assert call(c) == want
