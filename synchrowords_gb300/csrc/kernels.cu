@@ -1606,20 +1606,50 @@ void launch_score_keys(const float* score, const u32* counts, u32 m, u64* keys, 
 
 // sel[0 .. width) = the rows with the smallest score keys (their upper halves),
 // ascending; equal scores by layer key, then position.  One CTA: a radix select
-// over four bytes of the score, then the rows at the threshold ranked among
-// themselves (few: equal scores of different sets are rare).  Only the set of kept
-// rows matters to a beam, so nothing is sorted.  Bound by its ~20 barriers and
-// the histograms; with the unsorted duplicate removal before it a level of 8192
-// children takes 90 us, where sorting the children and then the scores took 210
-// (beam of 4096, n=256: 7 -> 3 ms).
-constexpr u32 kSelectThreads = 1024;
+// over four bytes of the score, then, over the rows at the threshold, over the
+// bytes of their layer keys until kFewTies are left, which are ranked among
+// themselves.  Only the set of kept rows matters to a beam, so nothing is
+// sorted.  Bound by its ~20 barriers and the histograms; with the unsorted
+// duplicate removal before it a level of 8192 children takes 90 us, where
+// sorting the children and then the scores took 210 (beam of 4096, n=256: 7 ->
+// 3 ms).  Ranking every row at the threshold against every other took 40 ms a
+// level of 16 384 equal scores (a model whose units are all off: beam of 4096,
+// n=150, k=4, 28 levels 1180 -> 3.5 ms).
+constexpr u32 kSelectThreads = 1024, kFewTies = 128;
+
+// The bin that holds the need-th element of the counts: its number, the elements
+// before it and in it.  Warp 0; the caller synchronises.
+__device__ __forceinline__ void select_bin(const u32* s_hist, u32 need, u32* s_bin, u32* s_before, u32* s_count) {
+  const u32 lane = threadIdx.x & 31;
+  u32 c[8], sum = 0;
+#pragma unroll
+  for (int b = 0; b < 8; ++b) sum += c[b] = s_hist[8 * lane + b];
+  u32 incl = sum;
+#pragma unroll
+  for (u32 d = 1; d < 32; d *= 2) {
+    const u32 o = __shfl_up_sync(kFull, incl, d);
+    if (lane >= d) incl += o;
+  }
+  u32 at = incl - sum;
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    if (at < need && need <= at + c[b]) {
+      *s_bin = 8 * lane + b;
+      *s_before = at;
+      *s_count = c[b];
+    }
+    at += c[b];
+  }
+}
+
 template <int W>
 __global__ void __launch_bounds__(kSelectThreads) k_select(const u64* __restrict__ keys, u32 m, u32 width,
                                                            const u64* __restrict__ rows, u32* __restrict__ sel) {
   extern __shared__ __align__(16) u32 s_score[];
   u32* const s_drop = s_score + m;  // bitmap: rows at the threshold that stay out
-  uint16_t* const s_ties = reinterpret_cast<uint16_t*>(s_drop + (m + 31) / 32);
-  __shared__ u32 s_hist[256], s_bin, s_before, s_count, s_sum[32];
+  uint16_t* s_ties = reinterpret_cast<uint16_t*>(s_drop + (m + 31) / 32);
+  uint16_t* s_next = s_ties + m;
+  __shared__ u32 s_hist[256], s_bin, s_before, s_count, s_kept, s_sum[32];
   const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rounds = (m + kSelectThreads - 1) / kSelectThreads;
   for (u32 i = tid; i < m; i += kSelectThreads) s_score[i] = (u32)(keys[i] >> 32);
   for (u32 i = tid; i < (m + 31) / 32; i += kSelectThreads) s_drop[i] = 0;
@@ -1638,27 +1668,7 @@ __global__ void __launch_bounds__(kSelectThreads) k_select(const u64* __restrict
       }
     }
     __syncthreads();
-    if (warp == 0) {
-      u32 c[8], sum = 0;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) sum += c[b] = s_hist[8 * lane + b];
-      u32 incl = sum;
-#pragma unroll
-      for (u32 d = 1; d < 32; d *= 2) {
-        const u32 o = __shfl_up_sync(kFull, incl, d);
-        if (lane >= d) incl += o;
-      }
-      u32 at = incl - sum;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        if (at < need && need <= at + c[b]) {
-          s_bin = 8 * lane + b;
-          s_before = at;
-          s_count = c[b];
-        }
-        at += c[b];
-      }
-    }
+    if (warp == 0) select_bin(s_hist, need, &s_bin, &s_before, &s_count);
     __syncthreads();
     prefix |= s_bin << shift;
     mask |= 255u << shift;
@@ -1666,13 +1676,38 @@ __global__ void __launch_bounds__(kSelectThreads) k_select(const u64* __restrict
     equal = s_count;
   }
   if (need < equal) {  // the same for every thread
-    __syncthreads();
-    if (tid == 0) s_count = 0;
+    if (tid == 0) s_kept = 0;
     __syncthreads();
     for (u32 i = tid; i < m; i += kSelectThreads)
-      if (s_score[i] == prefix) s_ties[atomicAdd(&s_count, 1u)] = (uint16_t)i;
+      if (s_score[i] == prefix) s_ties[atomicAdd(&s_kept, 1u)] = (uint16_t)i;
+    // the rows in s_ties are undecided, and `need` of them are kept
+    for (int byte = 0; byte < 16 && equal > kFewTies && need < equal; ++byte) {
+      const auto digit = [&](u32 i) {  // of the layer key, most significant byte first
+        u64 a0, a1;
+        layer_key<W>(rows + (size_t)i * W, KeyMap{}, a0, a1);
+        return (u32)((byte < 8 ? a0 : a1) >> (56 - 8 * (byte & 7))) & 255u;
+      };
+      if (tid < 256) s_hist[tid] = 0;
+      __syncthreads();
+      if (tid == 0) s_kept = 0;
+      for (u32 t = tid; t < equal; t += kSelectThreads) atomicAdd(&s_hist[digit(s_ties[t])], 1u);
+      __syncthreads();
+      if (warp == 0) select_bin(s_hist, need, &s_bin, &s_before, &s_count);
+      __syncthreads();
+      const u32 bin = s_bin;
+      for (u32 t = tid; t < equal; t += kSelectThreads) {
+        const u32 i = s_ties[t], d = digit(i);
+        if (d > bin) atomicOr(&s_drop[i >> 5], 1u << (i & 31));
+        if (d == bin) s_next[atomicAdd(&s_kept, 1u)] = (uint16_t)i;
+      }
+      need -= s_before;
+      equal = s_count;
+      uint16_t* const o = s_ties;
+      s_ties = s_next;
+      s_next = o;
+    }
     __syncthreads();
-    for (u32 t = tid; t < equal; t += kSelectThreads) {
+    for (u32 t = tid; t < equal && need < equal; t += kSelectThreads) {
       const u32 i = s_ties[t];
       u64 a0, a1;
       layer_key<W>(rows + (size_t)i * W, KeyMap{}, a0, a1);
@@ -1712,10 +1747,10 @@ __global__ void __launch_bounds__(kSelectThreads) k_select(const u64* __restrict
 
 void launch_select(int W, const u64* keys, u32 m, u32 width, const u64* rows, u32* sel, cudaStream_t s) {
   if (m > kSelectMax || width == 0 || width > m) throw std::invalid_argument("select: size");
-  const size_t smem = sizeof(u32) * (m + (m + 31) / 32) + sizeof(uint16_t) * m;
+  const auto bytes = [](u32 r) { return sizeof(u32) * (r + (r + 31) / 32) + 2 * sizeof(uint16_t) * r; };
   SW_DISPATCH_W(W, {
-    ensure_smem_limit((const void*)k_select<WW>, (int)(sizeof(u32) * (kSelectMax + kSelectMax / 32) + sizeof(uint16_t) * kSelectMax));
-    k_select<WW><<<1, kSelectThreads, smem, s>>>(keys, m, width, rows, sel);
+    ensure_smem_limit((const void*)k_select<WW>, (int)bytes(kSelectMax));
+    k_select<WW><<<1, kSelectThreads, bytes(m), s>>>(keys, m, width, rows, sel);
   });
   SW_LAUNCH_CHECK();
 }
