@@ -1,0 +1,19 @@
+"""What the rule that leaves reductions out of a search may not change."""
+import json
+
+import pytest
+
+from synchrowords_gb300.generate import random_dfa
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,seed,mb", [(300, 5, 300), (300, 6, 100), (320, 7, 100), (320, 7, 180)])
+def test_bounds_where_memory_ends_the_search(ctx, n, seed, mb):
+    bounds = []
+    for reductions in ("always", "auto"):
+        r = ctx.solve(random_dfa(n, 2, seed), n, 2, json.dumps({"algorithms": [
+            {"name": "Beam", "config": {"presort": "indeg", "beam_size": "AUT_N * 4"}},
+            {"name": "Exact", "config": {"max_memory_mb": mb, "dfs": False, "reductions": reductions}}]}))
+        bounds.append((r.lower, r.upper))
+    assert bounds[0] == bounds[1]  # a bound with a word behind it is always searched reduced
