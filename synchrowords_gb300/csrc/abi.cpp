@@ -1153,6 +1153,13 @@ int sw_mlp_train_ranked(sw_context* ctx, float* params, uint32_t automata, const
 }
 
 // For tests, outside the public header (as testing.cpp).
+int sw_testing_dominated(sw_context* ctx, uint32_t n, int forward, int proper, const uint64_t* S, uint32_t m,
+                         const uint64_t* Q, uint32_t q, int live, int masked, uint32_t* flags, float* ms) {
+  return guarded([&] {
+    *ms = ctx->solver->check_dominated(n, forward != 0, proper != 0, S, m, Q, q, live != 0, masked != 0, flags);
+    return SW_OK;
+  });
+}
 int sw_testing_plant_error(sw_context* ctx, uint32_t code) {
   return guarded([&] {
     ctx->solver->plant_error(code);

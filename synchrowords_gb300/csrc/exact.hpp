@@ -79,6 +79,12 @@ class Solver {
   void subsets_check(uint32_t n, const uint64_t* sets, uint64_t set_count, const uint64_t* checks,
                      uint64_t check_count, bool proper, uint8_t* results);
   uint64_t sort_unique(uint32_t n, uint64_t* sets, uint64_t count);
+  // For tests: what the dominance checks of a level flag of Q's rows (words_for(n)
+  // words each, as on the device) for the rows S, with each list's count on the
+  // device when `live`; masked: by the tiled check, whatever the rule says.
+  // Returns the device's milliseconds.
+  float check_dominated(uint32_t n, bool forward, bool proper, const uint64_t* S, uint32_t m, const uint64_t* Q,
+                        uint32_t q, bool live, bool masked, uint32_t* flags);
   // For tests: as if a launch had reported `code`.
   void plant_error(uint32_t code);
 
