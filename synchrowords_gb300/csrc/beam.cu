@@ -15,6 +15,13 @@ namespace {
 constexpr u32 kBeamThreads = 1024;
 constexpr u32 kBeamBins = 2 * kBeamThreads;
 constexpr u32 kDuplicate = 0x8000u;  // in a child's key: an earlier child is the same set
+// Pairs a child, within the bins, above which a level's children are sorted instead:
+// us a level by 16 / 64 / 128 / 256 / never, random automata n=256 beam 2048 62 / 53 /
+// 54 / 66 / 67, n=60 k=16 beam 500 107 / 69 / 64 / 64 / 82; letters that permute all
+// states but one, whose sets differ in few states, n=128 beam 3000 101 / 100 / 100 /
+// 101 / 1730, n=60 k=16 beam 500 118 / 101 / 97 / 101 / 520 (launches over the whole GPU
+// 113 and 116).
+constexpr u32 kBeamPairs = 128;
 
 struct BeamLayout {
   size_t child, col, delta, bins, key, list, kept, bytes;
@@ -53,6 +60,60 @@ __device__ __forceinline__ void scan_bins(u32* count, u32* out, u32* s_sum) {
   out[2 * tid + 1] = count[2 * tid + 1] = at + c0;
   if (tid == kBeamThreads - 1) out[kBeamBins] = count[kBeamBins] = at + c0 + c1;
 }
+
+template <int W>
+__device__ __forceinline__ bool same_child(const u64* child, size_t cap, u32 i, u32 j) {
+  if (child[i] != child[j]) return false;
+  bool same = true;
+#pragma unroll
+  for (int w = 1; w < W; ++w) same = same && child[w * cap + i] == child[w * cap + j];
+  return same;
+}
+
+// list[0 .. N) = the children by (key, set in the beam's order, number): a bitonic
+// network whose exchanges all ascend, so that places past N (larger than any
+// child) need no storage.  The whole block.
+template <int W>
+__device__ __forceinline__ void sort_children(uint16_t* list, const uint16_t* key, const u64* child, size_t cap,
+                                              u32 N) {
+  const auto less = [&](u32 i, u32 j) {
+    if (key[i] != key[j]) return key[i] < key[j];
+    u64 d = child[i] ^ child[j], y = child[j];
+#pragma unroll
+    for (int w = 1; w < W; ++w)
+      if (!d) {
+        y = child[w * cap + j];
+        d = child[w * cap + i] ^ y;
+      }
+    return d ? (y & (d & (~d + 1))) != 0 : i < j;  // the lowest differing bit decides
+  };
+  const auto exchange = [&](u32 a, u32 b) {
+    if (b >= N) return;
+    const uint16_t i = list[a], j = list[b];
+    if (less(j, i)) {
+      list[a] = j;
+      list[b] = i;
+    }
+  };
+  u32 half = 1;  // exchanges of a stage
+  while (2 * half < N) half *= 2;
+  for (u32 p = threadIdx.x; p < N; p += kBeamThreads) list[p] = (uint16_t)p;
+  for (u32 size = 1; size <= half; size *= 2) {  // merges runs of `size`
+    __syncthreads();
+    for (u32 t = threadIdx.x; t < half; t += kBeamThreads) {
+      const u32 at = 2 * (t & ~(size - 1)), o = t & (size - 1);
+      exchange(at + o, at + 2 * size - 1 - o);
+    }
+    for (u32 step = size / 2; step; step /= 2) {
+      __syncthreads();
+      for (u32 t = threadIdx.x; t < half; t += kBeamThreads) {
+        const u32 a = 2 * (t & ~(step - 1)) + (t & (step - 1));
+        exchange(a, a + step);
+      }
+    }
+  }
+  __syncthreads();
+}
 }  // namespace
 
 // Every level of the beam in one CTA: over the whole GPU a level of a few
@@ -62,8 +123,9 @@ __device__ __forceinline__ void scan_bins(u32* count, u32* out, u32* s_sum) {
 // columns of 32 (one letter's preimages of 32 sets are then 2 W table reads and
 // transposes per lane).  Ordering: a counting sort by cardinality and the next
 // bits of the order, then each child counts the smaller ones in its bin; bins by
-// cardinality alone were 2-3x slower from 1500 children.  What bounds a level is
-// that count (shared memory) and ~14 barriers.  Per level, launches over the
+// cardinality alone were 2-3x slower from 1500 children, and where bins hold too
+// many (kBeamPairs) the level is sorted by a bitonic network.  What bounds a level
+// is that count (shared memory) and ~14 barriers, or the network's stages.  Per level, launches over the
 // whole GPU -> here: n=100 k=3 beam 10 73 -> 6.2 us, n=64 beam 4000 105 -> 31,
 // n=128 beam 896 114 -> 17, n=200 beam 1528 121 -> 43.
 template <int W>
@@ -80,7 +142,7 @@ __global__ void __launch_bounds__(kBeamThreads, 1) k_beam(const uint16_t* __rest
   uint16_t* const key = (uint16_t*)(s_raw + L.key);
   uint16_t* const list = (uint16_t*)(s_raw + L.list);
   uint16_t* const kept = (uint16_t*)(s_raw + L.kept);
-  __shared__ u32 s_full, s_least, s_most, s_sum[32];
+  __shared__ u32 s_full, s_least, s_most, s_pairs, s_sum[32];
   const u32 tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, warps = kBeamThreads / 32;
   const u32 cap = parents * k;
   const u32 low = W == 1 ? 64 - n : 0;  // the first word's last state, whose bit leads the order
@@ -97,7 +159,7 @@ __global__ void __launch_bounds__(kBeamThreads, 1) k_beam(const uint16_t* __rest
     for (u32 b = tid; b <= kBeamBins; b += kBeamThreads) count[b] = 0;
     if (tid == 0) {
       s_full = s_least = ~0u;
-      s_most = 0;
+      s_most = s_pairs = 0;
     }
     __syncthreads();
     for (u32 t = warp; t < k * groups; t += warps) {
@@ -141,57 +203,80 @@ __global__ void __launch_bounds__(kBeamThreads, 1) k_beam(const uint16_t* __rest
       atomicAdd(&count[b], 1u);
     }
     __syncthreads();
+    // pairs that ranking within the bins would compare
+    const u32 c0 = count[2 * tid], c1 = count[2 * tid + 1];
+    const u32 pairs = __reduce_add_sync(0xffffffffu, c0 * c0 + c1 * c1);
+    if (lane == 0) atomicAdd(&s_pairs, pairs);
     scan_bins(count, first, s_sum);
     __syncthreads();
-    for (u32 i = tid; i < N; i += kBeamThreads) list[atomicAdd(&count[key[i]], 1u)] = (uint16_t)i;
-    __syncthreads();
-    for (u32 b = tid; b <= kBeamBins; b += kBeamThreads) count[b] = 0;
-    __syncthreads();
-    for (u32 p = tid; p < N; p += kBeamThreads) {
-      const u32 i = list[p], b = key[i], end = first[b + 1];
-      u64 x[W];
+    u32 unique;
+    if (s_pairs > kBeamPairs * N) {
+      sort_children<W>(list, key, child, cap, N);
+      // runs of `run` places: the first of equal sets is kept, in order
+      const u32 run = (N + kBeamThreads - 1) / kBeamThreads, p0 = min(tid * run, N), p1 = min(p0 + run, N);
+      const auto fresh = [&](u32 p) { return p == 0 || !same_child<W>(child, cap, list[p], list[p - 1]); };
+      u32 mine = 0;
+      for (u32 p = p0; p < p1; ++p) mine += fresh(p);
+      count[2 * tid] = mine;
+      count[2 * tid + 1] = 0;
+      __syncthreads();
+      scan_bins(count, count, s_sum);
+      __syncthreads();
+      u32 r = count[2 * tid];
+      for (u32 p = p0; p < p1 && r < beam; ++p)
+        if (fresh(p)) kept[r++] = list[p];
+      unique = count[kBeamBins];
+    } else {
+      for (u32 i = tid; i < N; i += kBeamThreads) list[atomicAdd(&count[key[i]], 1u)] = (uint16_t)i;
+      __syncthreads();
+      for (u32 b = tid; b <= kBeamBins; b += kBeamThreads) count[b] = 0;
+      __syncthreads();
+      for (u32 p = tid; p < N; p += kBeamThreads) {
+        const u32 i = list[p], b = key[i], end = first[b + 1];
+        u64 x[W];
 #pragma unroll
-      for (int w = 0; w < W; ++w) x[w] = child[(size_t)w * cap + i];
-      bool dup = false;
-      for (u32 j = first[b]; j < end && !dup; ++j) {
-        const u32 o = list[j];
-        if (child[o] != x[0] || o >= i) continue;
-        bool same = true;
+        for (int w = 0; w < W; ++w) x[w] = child[(size_t)w * cap + i];
+        bool dup = false;
+        for (u32 j = first[b]; j < end && !dup; ++j) {
+          const u32 o = list[j];
+          if (child[o] != x[0] || o >= i) continue;
+          bool same = true;
 #pragma unroll
-        for (int w = 1; w < W; ++w) same = same && child[(size_t)w * cap + o] == x[w];
-        dup = same;
+          for (int w = 1; w < W; ++w) same = same && child[(size_t)w * cap + o] == x[w];
+          dup = same;
+        }
+        if (dup)
+          key[i] = (uint16_t)(b | kDuplicate);
+        else
+          atomicAdd(&count[b], 1u);
       }
-      if (dup)
-        key[i] = (uint16_t)(b | kDuplicate);
-      else
-        atomicAdd(&count[b], 1u);
-    }
-    __syncthreads();
-    scan_bins(count, count, s_sum);  // distinct sets before each bin; first keeps the bins' places
-    __syncthreads();
-    const u32 unique = count[kBeamBins];
-    for (u32 p = tid; p < N; p += kBeamThreads) {
-      const u32 i = list[p], b = key[i];
-      if (b & kDuplicate) continue;
-      u32 r = count[b];
-      if (r >= beam) continue;
-      u64 x[W];
+      __syncthreads();
+      scan_bins(count, count, s_sum);  // distinct sets before each bin; first keeps the bins' places
+      __syncthreads();
+      unique = count[kBeamBins];
+      for (u32 p = tid; p < N; p += kBeamThreads) {
+        const u32 i = list[p], b = key[i];
+        if (b & kDuplicate) continue;
+        u32 r = count[b];
+        if (r >= beam) continue;
+        u64 x[W];
 #pragma unroll
-      for (int w = 0; w < W; ++w) x[w] = child[(size_t)w * cap + i];
-      const u32 end = first[b + 1];
-      for (u32 j = first[b]; j < end; ++j) {
-        const u32 o = list[j];
-        // order of the bit-reversed words: the lowest differing bit decides
-        u64 d = child[o] ^ x[0], y = x[0];
+        for (int w = 0; w < W; ++w) x[w] = child[(size_t)w * cap + i];
+        const u32 end = first[b + 1];
+        for (u32 j = first[b]; j < end; ++j) {
+          const u32 o = list[j];
+          // order of the bit-reversed words: the lowest differing bit decides
+          u64 d = child[o] ^ x[0], y = x[0];
 #pragma unroll
-        for (int w = 1; w < W; ++w)
-          if (!d) {
-            y = x[w];
-            d = child[(size_t)w * cap + o] ^ y;
-          }
-        r += (y & (d & (~d + 1))) != 0 && !(key[o] & kDuplicate);
+          for (int w = 1; w < W; ++w)
+            if (!d) {
+              y = x[w];
+              d = child[(size_t)w * cap + o] ^ y;
+            }
+          r += (y & (d & (~d + 1))) != 0 && !(key[o] & kDuplicate);
+        }
+        if (r < beam) kept[r] = (uint16_t)i;
       }
-      if (r < beam) kept[r] = (uint16_t)i;
     }
     __syncthreads();
     m = min(unique, beam);
