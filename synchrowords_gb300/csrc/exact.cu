@@ -29,6 +29,7 @@
 #include "exact.hpp"
 #include "kernels.cuh"
 #include "learn.hpp"
+#include "search_rules.hpp"
 #include "train.hpp"
 
 namespace sw {
@@ -1365,18 +1366,8 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
   // levels before the bound, took 190 ms where 35 was enough).
   constexpr double kStepLaunch = 8e-5, kMeetLaunch = 1.5e-5;
   constexpr u32 kSwitchRows = 4096;
-  struct Reduction {
-    double seconds = 0, dropped = 0;  // of the last reduced level: time of the checks, share dropped
-    u32 parents = 0;
-  } reductions[2];
+  Reduction reductions[2];
   double rest = 0;  // projected seconds to the end of the search (0: not known)
-  // The checks must save kReduceGain times less than they cost to be left out, and
-  // a search that leaves them out switches at kSwitchUnreduced of the projection,
-  // since each further level then enlarges what the bounded phase starts from.
-  // Sum over 18 LearnedBeam + Exact n=256 / 12 Beam + Exact n=300 searches, ms: no
-  // rule 469 / 533; gain 0.6 333 / 640, 1 349 / 605, 1.4 with the earlier switch
-  // 365 / 519, 2 365 / 547 (512 with it), 4 388 / 544.
-  constexpr double kReduceGain = 1.4, kSwitchUnreduced = 0.5;
   double t_iter_last = 0, t_meet_per_query = 0, b_growth = k * 0.95;
   while (rt < max_rt) {  // meet_in_the_middle.cpp:73
     const auto t_iter0 = std::chrono::steady_clock::now();
@@ -1400,22 +1391,11 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
     }
     rt++;
     const u32 parents_before = X.count;
-    // self reduction only where it pays: a word-backed bound (the bounded
-    // phase expands B from its size at the switch) or lists past a quarter
-    // of the memory budget
     const bool pressure = 4 * (live + next) > budget;
-    bool reduce = cfg.reductions == SW_REDUCE_ALWAYS || (cfg.reductions == SW_REDUCE_AUTO && b.has_word);
-    // ... and, left to this rule, only while what they drop saves more of the
-    // projected rest of the search than they cost (their time grows with the
-    // square).  Where running out of memory would end the search (no bounded
-    // phase to go on in) they stay: the larger lists ran out up to two lengths
-    // earlier (n = 320, 100 MB)
     Reduction& red_last = reductions[fwd];
-    if (cfg.reductions == SW_REDUCE_AUTO && cfg.dfs && red_last.parents && rest > 0) {
-      const double g = (double)X.count / red_last.parents;
-      if (red_last.seconds * g * g > kReduceGain * red_last.dropped * rest) reduce = false;
-    }
-    E.self_check = E.visited_subsets = reduce || pressure;
+    const LevelRule level =
+        reductions_of_level((int)cfg.reductions, b.has_word, cfg.dfs != 0, pressure, red_last, X.count, rest);
+    E.self_check = E.visited_subsets = level.reduce;
     E.step(X, fwd, W, n, k, /*dominance=*/!bounded, false, /*defer=*/true);
     if (fwd) {
       st.bfs_steps++;
@@ -1482,7 +1462,7 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
       rest = fits ? std::min(total, plain) : plain;
       // voluntary switch only when every projected level fits; chunking is the
       // safety net for an exhausted budget, not a plan
-      if (fits && total * (reduce ? 1.0 : kSwitchUnreduced) < mitm) {
+      if (fits && total * (level.left_out ? kSwitchUnreduced : 1.0) < mitm) {
         bounded = true;
         if (E.verbose)
           std::fprintf(stderr, "[sw] bounded phase from length %llu: %llu levels left, |F|=%u |B|=%u, "
