@@ -77,7 +77,7 @@ struct SmallResult {
 
 // Device-resident search on thread-block clusters (batch_cluster.cu): one
 // cluster of `cs` CTAs per automaton (n <= 256, n * k <= 4096), lists in a
-// per-cluster global region.  Status 1 may also report why 6 (a hash-table probe ran out), status 2 why 8
+// per-cluster global region.  Status 1 may also report why 6 (a hash-table probe ran out) or 7 (given up), status 2 why 8
 // (a side died out) or 9 (max_len reached), and status 3 says that the search
 // stopped at a work limit; where no word was found, `length` counts the
 // lengths excluded so far.
@@ -90,12 +90,16 @@ struct ClusterCaps {
 // max_children children, after a level of more than max_pairs meet pairs, and
 // once its lists and the next level pass a quarter of `budget` bytes by the
 // streamed search's count (which then changes its reductions).
+constexpr u32 kClusterPoll = 4;
 struct ClusterLimits {
   u64 max_pairs = ~0ull;
   u64 budget = ~0ull;
   u32 max_children = ~0u;
   u32 counter_ready = 0;    // the caller zeroed the counter on the launch's stream
   size_t header_bytes = 0;  // bytes before the first region; 0: room for every cluster index
+  // Word in pinned host memory (may be null) that the host sets to have the search
+  // given up at one of its next kClusterPoll levels (status 1, why 7).
+  const u32* cancel = nullptr;
 };
 // How a single search ended (written at kClusterExitOffset of its scratch):
 // meet pairs, children and meet queries (backward rows, summed over levels),

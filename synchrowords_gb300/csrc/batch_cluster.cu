@@ -110,7 +110,7 @@ __device__ __forceinline__ bool table_insert(u64* vt, u32 vmask, u64 tag, const 
     }
     slot = (slot + 1) & vmask;
   }
-  atomicExch(overflow, 1u);
+  atomicOr(overflow, 1u);
   return false;
 }
 
@@ -127,7 +127,7 @@ __device__ __forceinline__ uint4 ld_volatile128(const void* p) {
 // four are read together).
 struct ClusterCtl {
   u32 fcount[2];  // kept children of the step (by step parity)
-  u32 overflow;   // a table probe ran out (never expected: tables hold more slots than rows)
+  u32 overflow;   // bit 0: a table probe ran out (never expected: tables hold more slots than rows); bit 1: given up
   u32 found;      // meet flag
   u32 inst;       // automaton being solved
   u32 vtag;       // tag of this search's table slots
@@ -335,6 +335,9 @@ __global__ void __launch_bounds__(kCtThreads, 1)
         status = 3;  // a level of this size belongs to the whole GPU
         break;
       }
+      // read now, used at the level's end: the word lies in host memory, a microsecond away
+      u32 given_up = 0;
+      if (lim.cancel && rank == 0 && tid == 0 && rt % kClusterPoll == kClusterPoll - 1) given_up = ld_volatile(lim.cancel);
       // ---- expansion and duplicate removal ----
       const u32* const P = LX + curX;  // the parents' row slots
       const u32 par = rt & 1u;
@@ -411,6 +414,7 @@ __global__ void __launch_bounds__(kCtThreads, 1)
         }
       }
       my_children += c;
+      if (given_up) atomicOr(&ctl->overflow, 2u);
       cluster_barrier();
       lap(0);
       const uint4 now = ld_volatile128(ctl);  // both counts, overflow, meet flag
@@ -437,7 +441,7 @@ __global__ void __launch_bounds__(kCtThreads, 1)
       ++steps;
       if (now.z) {
         status = 1;
-        why = 6;
+        why = now.z & 1u ? 6 : 7;
         break;
       }
       if (f == 0) {  // a side died out: no reset word within reach
