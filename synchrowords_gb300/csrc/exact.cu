@@ -1385,8 +1385,13 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
       // meet_in_the_middle.cpp:98-101 + exact.cpp:139-145: out of memory, the
       // search continues in the memory-bounded inverse phase when DFS is
       // enabled and the remaining depth is bounded (word-backed bound or at
-      // most 64 levels); otherwise only a lower bound results
-      if (cfg.dfs && !bounded && E.B.count && (b.has_word || max_rt - rt <= 64)) {
+      // most 64 levels); otherwise only a lower bound results.  Plans that reduce
+      // for memory only and have a word behind the bound switch there by cost at
+      // any level, DFS or not, and so go on at the budget too: while the switch
+      // still came within the first levels of such plans (below kSwitchRows) they
+      // never met the budget
+      const bool goes_on = cfg.dfs || (b.has_word && cfg.reductions == SW_REDUCE_MEMORY);
+      if (goes_on && !bounded && E.B.count && (b.has_word || max_rt - rt <= 64)) {
         bounded = true;
         if (E.verbose)
           std::fprintf(stderr, "[sw] memory budget reached at length %llu: bounded phase\n", (unsigned long long)rt);

@@ -17,3 +17,14 @@ def test_bounds_where_memory_ends_the_search(ctx, n, seed, mb):
             {"name": "Exact", "config": {"max_memory_mb": mb, "dfs": False, "reductions": reductions}}]}))
         bounds.append((r.lower, r.upper))
     assert bounds[0] == bounds[1]  # a bound with a word behind it is always searched reduced
+
+
+@pytest.mark.parametrize("n,k,seed,mb", [(106, 3, 902, 1), (106, 3, 903, 3), (130, 2, 901, 1), (160, 2, 900, 3),
+                                         (200, 2, 901, 5)])
+def test_searches_reduced_for_memory_only_end(ctx, n, k, seed, mb):
+    bounds = []
+    for config in ({"max_memory_mb": mb, "dfs": False, "reductions": "memory"}, {}):
+        r = ctx.solve(random_dfa(n, k, seed), n, k, json.dumps({"upper_bound": "AUT_N", "algorithms": [
+            {"name": "Beam", "config": {"presort": "indeg", "beam_size": "500"}}, {"name": "Exact", "config": config}]}))
+        bounds.append((r.lower, r.upper))
+    assert bounds[0] == bounds[1] and bounds[0][0] == bounds[0][1]
