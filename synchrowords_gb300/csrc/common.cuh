@@ -121,7 +121,11 @@ struct DevBuf {
     cap = want;
   }
   void release() {
-    if (p) cudaFree(p);
+    if (cudaStream_t s = alloc_stream()) {
+      if (p) cudaFreeAsync(p, s);
+    } else if (p) {
+      cudaFree(p);
+    }
     p = nullptr;
     cap = 0;
   }

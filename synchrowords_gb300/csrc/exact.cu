@@ -67,6 +67,7 @@ struct Side {
     double t0 = 0;
   } step;
   const u32* live = nullptr;
+  size_t list_bytes() const { return vis.cap + vis_alt.cap + met.cap + table.cap; }
   const u64* cur_rows(int W) const { return in_vis ? vis.as<u64>() + (size_t)cur_off * W : rows.as<u64>(); }
   std::vector<std::unique_ptr<Layer>> layers;
   std::vector<u64> seed_states;  // backward side: the state of each seed row
@@ -290,7 +291,10 @@ class Engine {
   struct Counting {
     Engine& E;
     Counting(Engine& e, sw_stats& st) : E(e) { E.st = &st; }
-    ~Counting() { E.st = nullptr; }
+    ~Counting() {
+      E.st = nullptr;
+      E.list_budget = ~(size_t)0;
+    }
   };
   std::vector<std::unique_ptr<DLevel>> dlevel_pool;  // the bounded phase's per-depth levels
   // scratch of the beams and of Reduce, kept across calls
@@ -365,7 +369,8 @@ class Engine {
     if (!m || !q) return;
     const ScanShape& sh = scan_shapes.pick(W, m);
     tile_and.reserve(subset_check_temp_bytes(W, m, sh));
-    scan_items.reserve(sizeof(uint2) * kSubsetItems + sizeof(u32) * kSubsetCounterWords);
+    static_assert(kSubsetCounterWords % 2 == 0, "the list lies behind the counters");
+    scan_items.reserve(sizeof(u32) * kSubsetCounterWords + sizeof(uint2) * subset_check_items(m, q, sh));
     cudaEvent_t e0 = nullptr;
     if (prof_on) {
       e0 = next_event();
@@ -377,8 +382,9 @@ class Engine {
     // algorithmic bytes: the query rows plus every row of S a query is tested against
     timed(0, (double)q * 8.0 * W, [&] {
       launch_subset_check(W, mode, S, m, tile_and.as<u64>(), size_floor, Q, q, n, flags, d_misc, stop, sh, stream,
-                          prof_on ? d_query_bytes : nullptr, scan_items.as<uint2>(),
-                          reinterpret_cast<u32*>(scan_items.as<uint2>() + kSubsetItems), m_live, q_live);
+                          prof_on ? d_query_bytes : nullptr,
+                          reinterpret_cast<uint2*>(scan_items.as<u32>() + kSubsetCounterWords), scan_items.as<u32>(),
+                          m_live, q_live);
     });
     if (prof_on) {
       cudaEvent_t e1 = next_event();
@@ -404,9 +410,10 @@ class Engine {
   // 300 50K x 50K 0.28 / 0.28, 1.1M x 1.1M 22 / 34.  Backward the bitmaps are
   // faster throughout (n = 42 283K 2.7 / 1.4, n = 300 280K 27 / 2.5).
   static constexpr u32 kMaskedChildren = 1u << 16, kMaskedChildrenOneWord = 1u << 15;
+  // `order`: scratch for the rows in the order the check takes them.
   DevBuf dom_rows, dom_index;
   void dominated(bool forward, int W, const u64* S, u32 m, const u64* Q, u32 q, int n, bool proper, u32* flags,
-                 const u32* m_live = nullptr, const u32* q_live = nullptr) {
+                 DevBuf& order, const u32* m_live = nullptr, const u32* q_live = nullptr) {
     if (!m || !q) return;
     if (forward && q > (W == 1 ? kMaskedChildrenOneWord : kMaskedChildren))
       return query(W, proper ? kQueryProperSubset : kQuerySubset, S, m, Q, q, n, flags, false, m_live, q_live);
@@ -420,9 +427,9 @@ class Engine {
     if (tm > kDomOrderRows) {
       sc.bucket = buckets(tm);
       sc.bucket.met = d_misc + 14;  // not the step's
-      dom_rows.reserve(sizeof(u64) * W * (size_t)tm);
+      order.reserve(sizeof(u64) * W * (size_t)tm);
       dom_index.reserve(sizeof(u32) * (size_t)tm);
-      sc.rows = dom_rows.as<u64>();
+      sc.rows = order.as<u64>();
       sc.index = dom_index.as<u32>();
       sc.total = d_misc + 10;
       count_launch(3);
@@ -512,20 +519,46 @@ class Engine {
     return s;
   }
   // Room for `rows` more rows behind the first `count` of `buf`, which are kept.
-  void grow_rows(DevBuf& buf, DevBuf& spare, int W, u64 count, u64 rows) {
+  void grow_rows(DevBuf& buf, int W, u64 count, u64 rows) {
     const size_t need = sizeof(u64) * W * (count + rows);
     if (buf.cap >= need) return;
-    spare.reserve(std::max(need, 2 * buf.cap));
-    SW_CUDA(cudaMemcpyAsync(spare.p, buf.p, sizeof(u64) * W * (size_t)count, cudaMemcpyDeviceToDevice, stream));
-    std::swap(buf.p, spare.p);
-    std::swap(buf.cap, spare.cap);
+    DevBuf larger;
+    larger.reserve(need);
+    SW_CUDA(cudaMemcpyAsync(larger.p, buf.p, sizeof(u64) * W * (size_t)count, cudaMemcpyDeviceToDevice, stream));
+    std::swap(buf.p, larger.p);
+    std::swap(buf.cap, larger.cap);
+    larger.release();
   }
-  // Lists up to this size are hashed; larger ones, whose table and spare copies
-  // would take several times as much again, are kept sorted.
+  // Lists up to this size are hashed; larger ones, whose table and second list
+  // would take several times as much again, are kept sorted.  So are lists that,
+  // with table and second list, would pass the search's memory budget, which
+  // counts rows only.
   static constexpr u64 kHashBytes = 16ull << 30;
-  static bool hashable(const Side& X, int W, u64 children) {
+  size_t list_budget = ~(size_t)0;
+  bool hashable(const Side& X, int W, u64 children) const {
     const u64 rows = (X.split ? X.met_count : X.vis_count) + children + 1;
-    return !X.sorted_only && 2 * rows <= 1ull << 32 && rows * 8 * W <= kHashBytes;
+    if (X.sorted_only || 2 * rows > 1ull << 32 || rows * 8 * W > kHashBytes) return false;
+    if (list_budget == ~(size_t)0) return true;
+    // what the step's buffers come to, and the list that is copied while it grows
+    size_t copied = 0;
+    const auto list = [&](const DevBuf& b, u64 count) {
+      const size_t need = sizeof(u64) * W * (count + children);
+      if (b.cap >= need) return b.cap;
+      copied = std::max(copied, b.cap);
+      return need + need / 4;
+    };
+    size_t bytes = list(X.vis, X.vis_count);
+    if (X.split || self_check || visited_subsets) bytes += list(X.met, X.split ? X.met_count : X.vis_count);
+    bytes += 2 * X.table_slots < 3 * rows ? sizeof(u64) * slots_for(rows) / 4 * 5 : X.table.cap;
+    return bytes + copied + X.vis_alt.cap + (&X == &F ? B : F).list_bytes() <= list_budget;
+  }
+  // Gives back what the bounded phase, whose levels are counted row by row, has no use for.
+  void release_tables() {
+    for (Side* X : {&F, &B}) {
+      X->table.release();
+      X->met.release();
+      X->table_slots = 0;
+    }
   }
   // One layer on a hashed side: children equal to a row met before or to a sibling
   // are dropped by the table, then, with the reductions on, those that a visited
@@ -552,7 +585,7 @@ class Engine {
     }
     DevBuf& list = X.split ? X.met : X.vis;
     const u32 base = X.split ? X.met_count : X.vis_count;
-    grow_rows(list, X.vis_alt, W, base, Nc);
+    grow_rows(list, W, base, Nc);
     if (2 * X.table_slots < 3 * ((u64)base + Nc)) {  // fewer than 1.5 slots a row: rebuild
       X.table_slots = slots_for((u64)base + Nc);
       X.table.reserve(sizeof(u64) * X.table_slots);
@@ -593,16 +626,17 @@ class Engine {
     if (X.split) {
       P.visited = visited_subsets ? X.vis_count : 0;
       P.self = self_check;
-      grow_rows(X.vis, X.vis_alt, W, X.vis_count, u);
+      grow_rows(X.vis, W, X.vis_count, u);
       u64* const out = X.vis.as<u64>() + (size_t)X.vis_count * W;
       if (reduce && u) {
         flags_a.reserve(sizeof(u32) * (size_t)u);
         SW_CUDA(cudaMemsetAsync(flags_a.p, 0, sizeof(u32) * (size_t)u, stream));
         reduce_span.mark(0, stream);
         if (X.vis_count && visited_subsets)
-          dominated(forward, W, X.vis.as<u64>(), X.vis_count, fresh, u, n, false, flags_a.as<u32>(), nullptr, fresh_live);
+          dominated(forward, W, X.vis.as<u64>(), X.vis_count, fresh, u, n, false, flags_a.as<u32>(), dom_rows,
+                    nullptr, fresh_live);
         if (self_check)
-          dominated(forward, W, fresh, u, fresh, u, n, true, flags_a.as<u32>(), fresh_live, fresh_live);
+          dominated(forward, W, fresh, u, fresh, u, n, true, flags_a.as<u32>(), dom_rows, fresh_live, fresh_live);
         reduce_span.mark(1, stream);
         const u32 epoch = next_dc_epoch(u);
         timed(3, (double)u * (4 + 2 * (8.0 * W + 4)), [&] {
@@ -698,6 +732,9 @@ class Engine {
     }
     X.hashed = X.in_vis = X.split = false;
     X.table_slots = 0;
+    X.table.release();
+    X.met.release();
+    dom_rows.release();
     sort_by_layer_key(W, X.vis.as<u64>(), X.vis_count, X.keymap);
   }
 
@@ -794,7 +831,9 @@ class Engine {
     const double t_sort = vclock();
     if (X.vis_count) {
       if (visited_subsets) {
-        dominated(forward, W, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, n, false, flags_a.as<u32>());
+        // the list the layer is merged into afterwards is free until then
+        dominated(forward, W, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, n, false, flags_a.as<u32>(),
+                  X.vis_alt);
       } else {
         timed(3, (double)u * 8.0 * W, [&] {
           launch_member_key(W, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, flags_a.as<u32>(), stream,
@@ -805,7 +844,7 @@ class Engine {
     }
     const double t_vis = vclock();
     if (self_check)
-      dominated(forward, W, uq_rows.as<u64>(), u, uq_rows.as<u64>(), u, n, true, flags_b.as<u32>());
+      dominated(forward, W, uq_rows.as<u64>(), u, uq_rows.as<u64>(), u, n, true, flags_b.as<u32>(), X.vis_alt);
     const double t_self = vclock();
     if (verbose) {
       std::vector<u32> fa(u), fb(u);
@@ -1265,6 +1304,10 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
   const std::vector<uint32_t> seeds = backward_seeds(A);
   E.F.reset();
   E.B.reset();
+  E.list_budget = budget;
+  if (E.F.list_bytes() + E.B.list_bytes() > budget)  // left by a search of a larger budget
+    for (DevBuf* b : {&E.F.vis, &E.F.vis_alt, &E.F.met, &E.F.table, &E.B.vis, &E.B.vis_alt, &E.B.met, &E.B.table})
+      b->release();
   auto finish = [&] {
     st.device_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   };
@@ -1497,6 +1540,7 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
   if (bounded && !found) {
     BoundedSearch S{E, A, W, n, k, budget, row_bytes, std::max<u64>(cfg.dfs_min_list_size, 1), max_rt, 0, {}, 0,
                     {}, {}, st};
+    E.release_tables();
     S.pool.swap(E.dlevel_pool);  // levels (and their device buffers) kept across solves
     S.levels.push_back(nullptr);
     S.explore(0, 0, E.B.count, rt);
@@ -2262,7 +2306,7 @@ float Solver::check_dominated(uint32_t n, bool forward, bool proper, const uint6
               d_flags.as<u32>(), false, live ? counts : nullptr, live ? counts + 1 : nullptr);
     else
       E.dominated(forward, W, s_rows.as<u64>(), mm, q_rows.as<u64>(), qq, (int)n, proper, d_flags.as<u32>(),
-                  live ? counts : nullptr, live ? counts + 1 : nullptr);
+                  E.dom_rows, live ? counts : nullptr, live ? counts + 1 : nullptr);
     E.reduce_span.mark(1, E.stream);
     SW_CUDA(cudaStreamSynchronize(E.stream));
     ms = (float)(1e3 * E.reduce_span.seconds());

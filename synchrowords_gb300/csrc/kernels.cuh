@@ -111,7 +111,7 @@ enum QueryMode : int {
 // index).  S is cut into tiles of sh.tile_rows rows and super-tiles of
 // sh.tiles_per_super tiles; `masks` (subset_check_temp_bytes) and *size_floor
 // (zero beforehand) come from launch_tile_and with the same shape.  `flags`
-// must start zeroed (non-stop mode).  `items` (kSubsetItems entries) and
+// must start zeroed (non-stop mode).  `items` (subset_check_items entries) and
 // item_counts (kSubsetCounterWords words) list the parts of S that a large check's queries need; without them
 // (nullptr) it goes over all of S.  `bytes_ctr` (optional) accumulates the
 // bytes of S rows tested.
@@ -139,6 +139,8 @@ struct ScanShapes {
 bool scan_shape_valid(int W, const ScanShape& sh);
 size_t scan_smem_bytes(int W, const ScanShape& sh);
 size_t subset_check_temp_bytes(int W, u32 m, const ScanShape& sh);
+// Entries of `items` that a check of q queries against m rows can use.
+u64 subset_check_items(u32 m, u32 q, const ScanShape& sh);
 void launch_tile_and(int W, const u64* S, u32 m, u64* masks, u32* size_floor, const ScanShape& sh, cudaStream_t s,
                      const u32* m_live = nullptr);
 void launch_subset_check(int W, int mode, const u64* S, u32 m, const u64* masks, const u32* size_floor, const u64* Q,

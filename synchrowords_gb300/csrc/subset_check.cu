@@ -459,6 +459,11 @@ size_t subset_check_temp_bytes(int W, u32 m, const ScanShape& sh) {
   return sizeof(u64) * mask_layout(W, mm, n_tiles(mm, sh), n_supers(mm, sh)).words;
 }
 
+u64 subset_check_items(u32 m, u32 q, const ScanShape& sh) {
+  const u64 pairs = (u64)((q + 31) / 32) * n_supers(m, sh);
+  return pairs > kDirectUnits ? std::min(pairs, kSubsetItems) : 0;
+}
+
 void launch_tile_and(int W, const u64* S, u32 m, u64* masks, u32* size_floor, const ScanShape& sh, cudaStream_t s,
                      const u32* m_live) {
   if (!m) return;
