@@ -294,6 +294,7 @@ class Engine {
     ~Counting() {
       E.st = nullptr;
       E.list_budget = ~(size_t)0;
+      E.states_ordered = false;
     }
   };
   std::vector<std::unique_ptr<DLevel>> dlevel_pool;  // the bounded phase's per-depth levels
@@ -409,13 +410,26 @@ class Engine {
   // permutations 0.39 / 0.63; n = 128 50K x 50K 0.21 / 0.21, 170K x 170K 0.66 / 1.1; n =
   // 300 50K x 50K 0.28 / 0.28, 1.1M x 1.1M 22 / 34.  Backward the bitmaps are
   // faster throughout (n = 42 283K 2.7 / 1.4, n = 300 280K 27 / 2.5).
-  static constexpr u32 kMaskedChildren = 1u << 16, kMaskedChildrenOneWord = 1u << 15;
-  // `order`: scratch for the rows in the order the check takes them.
+  // That is with states ordered by how often images hold them, as in the exact
+  // search.  In the caller's order (distance_pairs) the masks say less: from 2^18
+  // children, and not among siblings once the layers shrink against the visited
+  // list: n = 130 839K x 1228K 8.4 / 34, siblings 10 / 24, at the end 822K x 5851K 52 /
+  // 109, siblings 26 / 18; n = 160 129K 0.5 / 0.9; n = 200 168K x 414K 3.5 / 1.9,
+  // siblings 3.8 / 0.9.
+  static constexpr u32 kMaskedChildren = 1u << 16, kMaskedChildrenOneWord = 1u << 15, kMaskedUnordered = 1u << 18;
+  bool states_ordered = false;
+  bool masked_check(bool forward, int W, u32 q, bool siblings, u32 visited) const {
+    if (!forward) return false;
+    if (states_ordered) return q > (W == 1 ? kMaskedChildrenOneWord : kMaskedChildren);
+    return q > kMaskedUnordered && (!siblings || 2 * (u64)q > visited);
+  }
+  // Siblings (proper) are checked beside `visited` visited rows.  `order`: scratch
+  // for the rows in the order the check takes them.
   DevBuf dom_rows, dom_index;
-  void dominated(bool forward, int W, const u64* S, u32 m, const u64* Q, u32 q, int n, bool proper, u32* flags,
+  void dominated(bool forward, int W, const u64* S, u32 m, const u64* Q, u32 q, int n, bool proper, u32 visited, u32* flags,
                  DevBuf& order, const u32* m_live = nullptr, const u32* q_live = nullptr) {
     if (!m || !q) return;
-    if (forward && q > (W == 1 ? kMaskedChildrenOneWord : kMaskedChildren))
+    if (masked_check(forward, W, q, proper, visited))
       return query(W, proper ? kQueryProperSubset : kQuerySubset, S, m, Q, q, n, flags, false, m_live, q_live);
     cudaEvent_t e0 = nullptr;
     if (prof_on) {
@@ -633,10 +647,10 @@ class Engine {
         SW_CUDA(cudaMemsetAsync(flags_a.p, 0, sizeof(u32) * (size_t)u, stream));
         reduce_span.mark(0, stream);
         if (X.vis_count && visited_subsets)
-          dominated(forward, W, X.vis.as<u64>(), X.vis_count, fresh, u, n, false, flags_a.as<u32>(), dom_rows,
+          dominated(forward, W, X.vis.as<u64>(), X.vis_count, fresh, u, n, false, X.vis_count, flags_a.as<u32>(), dom_rows,
                     nullptr, fresh_live);
         if (self_check)
-          dominated(forward, W, fresh, u, fresh, u, n, true, flags_a.as<u32>(), dom_rows, fresh_live, fresh_live);
+          dominated(forward, W, fresh, u, fresh, u, n, true, X.vis_count, flags_a.as<u32>(), dom_rows, fresh_live, fresh_live);
         reduce_span.mark(1, stream);
         const u32 epoch = next_dc_epoch(u);
         timed(3, (double)u * (4 + 2 * (8.0 * W + 4)), [&] {
@@ -832,8 +846,8 @@ class Engine {
     if (X.vis_count) {
       if (visited_subsets) {
         // the list the layer is merged into afterwards is free until then
-        dominated(forward, W, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, n, false, flags_a.as<u32>(),
-                  X.vis_alt);
+        dominated(forward, W, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, n, false, X.vis_count,
+                  flags_a.as<u32>(), X.vis_alt);
       } else {
         timed(3, (double)u * 8.0 * W, [&] {
           launch_member_key(W, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, flags_a.as<u32>(), stream,
@@ -844,7 +858,8 @@ class Engine {
     }
     const double t_vis = vclock();
     if (self_check)
-      dominated(forward, W, uq_rows.as<u64>(), u, uq_rows.as<u64>(), u, n, true, flags_b.as<u32>(), X.vis_alt);
+      dominated(forward, W, uq_rows.as<u64>(), u, uq_rows.as<u64>(), u, n, true, X.vis_count, flags_b.as<u32>(),
+                X.vis_alt);
     const double t_self = vclock();
     if (verbose) {
       std::vector<u32> fa(u), fb(u);
@@ -1305,6 +1320,7 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
   E.F.reset();
   E.B.reset();
   E.list_budget = budget;
+  E.states_ordered = true;
   if (E.F.list_bytes() + E.B.list_bytes() > budget)  // left by a search of a larger budget
     for (DevBuf* b : {&E.F.vis, &E.F.vis_alt, &E.F.met, &E.F.table, &E.B.vis, &E.B.vis_alt, &E.B.met, &E.B.table})
       b->release();
@@ -2298,6 +2314,7 @@ float Solver::check_dominated(uint32_t n, bool forward, bool proper, const uint6
   launch_fill_u32(counts, m, 1, E.stream);
   launch_fill_u32(counts + 1, q, 1, E.stream);
   float ms = 0;
+  E.states_ordered = true;
   for (int run = 0; run < 2; ++run) {  // the first grows the buffers
     SW_CUDA(cudaMemcpyAsync(d_flags.p, flags, sizeof(u32) * (size_t)q, cudaMemcpyHostToDevice, E.stream));
     E.reduce_span.mark(0, E.stream);
@@ -2305,12 +2322,13 @@ float Solver::check_dominated(uint32_t n, bool forward, bool proper, const uint6
       E.query(W, proper ? kQueryProperSubset : kQuerySubset, s_rows.as<u64>(), mm, q_rows.as<u64>(), qq, (int)n,
               d_flags.as<u32>(), false, live ? counts : nullptr, live ? counts + 1 : nullptr);
     else
-      E.dominated(forward, W, s_rows.as<u64>(), mm, q_rows.as<u64>(), qq, (int)n, proper, d_flags.as<u32>(),
+      E.dominated(forward, W, s_rows.as<u64>(), mm, q_rows.as<u64>(), qq, (int)n, proper, mm, d_flags.as<u32>(),
                   E.dom_rows, live ? counts : nullptr, live ? counts + 1 : nullptr);
     E.reduce_span.mark(1, E.stream);
     SW_CUDA(cudaStreamSynchronize(E.stream));
     ms = (float)(1e3 * E.reduce_span.seconds());
   }
+  E.states_ordered = false;
   SW_CUDA(cudaMemcpy(flags, d_flags.p, sizeof(u32) * (size_t)q, cudaMemcpyDeviceToHost));
   return ms;
 }
