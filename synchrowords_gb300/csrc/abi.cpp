@@ -49,7 +49,7 @@ struct ClusterScratch {
 struct SmallBatchState {
   cudaStream_t stream = nullptr;
   sw::DevBuf inst, delta, seeds, results, words, counter, c_stats;
-  ClusterScratch scratch[2];  // the batched launch's small regions, the cluster launch's large ones
+  ClusterScratch scratch[3];  // the batched launch's small regions, the cluster launch's large ones, the batched launch's tiny ones
   sw_batch_profile last{};
   // CUDA graphs of recent device rounds, keyed by everything their launches
   // bake in (buffers, per-width counts, cluster geometry): a batch of a shape
@@ -69,6 +69,11 @@ constexpr uint64_t kClusterMaxPairs = 1ull << 28;
 // batches: 1.8 / 4.9 / 1.03 ms with 4, 2.0 / 12.8 / 1.08 with 1, 1.9 / 3.8 /
 // 1.29 with 8; 1024 of them 17.4, 21.6, 20.9).
 constexpr int kSmallClusterCtas = 4;
+// Below this n * log2(k) an automaton's levels are too small to split: one CTA each,
+// in smaller regions.  ms with 1 / 2 / 4 CTAs: 2000 of n = 10 10.8 / 11.5 / 12.8, 1000
+// of n = 12, k = 4 5.5 / 5.8 / 6.3, 1000 of n = 24 8.1 / 8.5 / 9.7, 64 of n = 24 0.88 / 0.89 /
+// 0.90; 1000 of n = 32 14.4 / 11.9 / 10.8 (a few hard ones end the launch).
+constexpr double kTinySize = 32.0;
 
 struct sw_context {
   std::unique_ptr<sw::Solver> solver;
@@ -309,19 +314,28 @@ void start_round(sw_context* ctx, DeviceRound& D, const std::vector<uint32_t> sm
   S.words.reserve((size_t)D.word_stride * inst.size());
   S.counter.reserve(sizeof(uint32_t) * 2);
   // geometry and scratch of the two launches (class c: c / 4 = launch)
-  const int cs[2] = {kSmallClusterCtas,
-                     ctx->tuning.cluster_size > 0 ? std::min<int>(ctx->tuning.cluster_size, 16) : 8};
-  const sw::ClusterCaps caps[2] = {sw::cluster_single_caps(), sw::cluster_default_caps()};
+  const int cs[3] = {kSmallClusterCtas,
+                     ctx->tuning.cluster_size > 0 ? std::min<int>(ctx->tuning.cluster_size, 16) : 8, 1};
+  const sw::ClusterCaps caps[3] = {sw::cluster_single_caps(), sw::cluster_default_caps(), sw::cluster_tiny_caps()};
+  int launch_of[8];  // index of the class's launch in cs, caps and S.scratch
+  for (int c = 0; c < 8; ++c) {
+    launch_of[c] = c / 4;
+    if (c >= 4) continue;
+    bool tiny = true;
+    for (uint32_t i : small[c]) tiny = tiny && (double)ns[i] * std::log2((double)ks[i]) < kTinySize;
+    if (tiny) launch_of[c] = 2;
+  }
   // A cluster gives an automaton back (to the worker streams, which search it
   // with the whole GPU) after a level of more than kClusterMaxPairs meet pairs,
   // unless the caller raised cluster_limit to have larger automata searched here.
   sw::ClusterLimits limits;
   if (ctx->tuning.cluster_limit <= kDefaultClusterLimit) limits.max_pairs = kClusterMaxPairs;
   uint32_t clusters[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int l = 0; l < 2; ++l) {
+  for (int l = 0; l < 3; ++l) {
     uint32_t most = 0;
     uint64_t tags = 0;
-    for (int c = 4 * l; c < 4 * l + 4; ++c) {
+    for (int c = 0; c < 8; ++c) {
+      if (launch_of[c] != l) continue;
       const uint32_t cnt = (uint32_t)(class_start[c + 1] - class_start[c]);
       if (!cnt) continue;
       clusters[c] = std::min<uint32_t>({cnt, sw::cluster_batch_max_clusters(c % 4 + 1, cs[l]),
@@ -347,11 +361,11 @@ void start_round(sw_context* ctx, DeviceRound& D, const std::vector<uint32_t> sm
     for (int c = 0; c < 8; ++c) {
       const size_t a = class_start[c], b = class_start[c + 1];
       if (a == b) continue;
-      const int l = c / 4;
+      const int l = launch_of[c];
       sw::launch_cluster_batch(c % 4 + 1, cs[l], clusters[c], S.inst.as<sw::SmallInstance>() + a, (uint32_t)(b - a),
                                S.delta.as<uint8_t>(), S.seeds.as<uint8_t>(), S.results.as<sw::SmallResult>() + a,
                                S.words.as<uint8_t>() + a * D.word_stride, D.word_stride, S.scratch[l].buf.p, caps[l],
-                               limits, S.counter.as<uint32_t>(), l ? S.c_stats.as<sw::u64>() : nullptr, S.stream);
+                               limits, S.counter.as<uint32_t>(), c < 4 ? nullptr : S.c_stats.as<sw::u64>(), S.stream);
     }
   };
   for (int c = 0; c < 8; ++c) D.launches += class_start[c] != class_start[c + 1];
@@ -359,10 +373,10 @@ void start_round(sw_context* ctx, DeviceRound& D, const std::vector<uint32_t> sm
                             (uint64_t)(uintptr_t)S.delta.p, (uint64_t)(uintptr_t)S.seeds.p,
                             (uint64_t)(uintptr_t)S.results.p, (uint64_t)(uintptr_t)S.words.p,
                             (uint64_t)(uintptr_t)S.counter.p, (uint64_t)(uintptr_t)S.scratch[0].buf.p,
-                            (uint64_t)(uintptr_t)S.scratch[1].buf.p, (uint64_t)(uintptr_t)S.c_stats.p,
-                            limits.max_pairs};
+                            (uint64_t)(uintptr_t)S.scratch[1].buf.p, (uint64_t)(uintptr_t)S.scratch[2].buf.p,
+                            (uint64_t)(uintptr_t)S.c_stats.p, limits.max_pairs};
   for (int c = 0; c < 9; ++c) key.push_back(class_start[c]);
-  for (int c = 0; c < 8; ++c) key.push_back(clusters[c]);
+  for (int c = 0; c < 8; ++c) key.push_back(clusters[c]), key.push_back(launch_of[c]);
   cudaGraphExec_t exec = nullptr;
   for (auto& g : S.graphs)
     if (g.first == key) exec = g.second;

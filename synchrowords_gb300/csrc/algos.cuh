@@ -115,6 +115,7 @@ constexpr size_t kClusterSingleResult = 512, kClusterSingleWords = 576, kCluster
 constexpr u32 kClusterSingleWord = 1024;
 ClusterCaps cluster_default_caps();
 ClusterCaps cluster_single_caps();
+ClusterCaps cluster_tiny_caps();
 // Bytes of scratch for `clusters` clusters.  It must be zero-filled before its
 // first launch, and again before the tags the launches take from its counter
 // (cluster_tags_per_launch) could pass kClusterTagLimit.

@@ -703,6 +703,14 @@ ClusterCaps cluster_single_caps() {
   return c;
 }
 
+ClusterCaps cluster_tiny_caps() {
+  ClusterCaps c;
+  c.vis = 1u << 16;
+  c.ch = 1u << 15;
+  c.vtab_bits = 17;
+  return c;
+}
+
 size_t cluster_scratch_bytes(u32 clusters, const ClusterCaps& c) {
   return kCtHeaderBytes + (size_t)clusters * cluster_region<4>(c).bytes;
 }
