@@ -2344,9 +2344,7 @@ void Solver::plant_error(uint32_t code) {
 static Trainer& training(Engine& E) {
   if (!E.mlp->has_params()) throw std::runtime_error("no distance model loaded");
   if (!E.trainer) E.trainer = std::make_unique<Trainer>(E.stream);
-  std::vector<float> p(mlp::kParams);
-  E.mlp->get_params(p.data());
-  E.trainer->set_params(p.data());  // waits for the stream
+  E.trainer->set_params(E.mlp->params());
   return *E.trainer;
 }
 

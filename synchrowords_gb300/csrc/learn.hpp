@@ -21,6 +21,7 @@ class MlpRunner {
   void set_params(const float* host);
   void get_params(float* host);
   bool has_params() const { return loaded_; }
+  const float* params() const { return params_.as<float>(); }  // on the device
 
   // Embedding table of automaton A (its state features through Phi, c, relu).
   void prepare(const Automaton& A);

@@ -13,18 +13,17 @@ View view(const bf16* p, long long si, long long sk) { return View{p, si, sk}; }
 int splits_for(u32 k_rows) { return (int)std::max<u32>(1, std::min<u32>(64, k_rows / 512)); }
 }  // namespace
 
-void Trainer::set_params(const float* host) {
+void Trainer::set_params(const float* device) {
   params_.reserve(sizeof(float) * mlp::kParams);
   grad_.reserve(sizeof(float) * mlp::kParams);
   m_.reserve(sizeof(float) * mlp::kParams);
   v_.reserve(sizeof(float) * mlp::kParams);
   loss_.reserve(sizeof(float) * 4);
-  SW_CUDA(cudaMemcpyAsync(params_.p, host, sizeof(float) * mlp::kParams, cudaMemcpyHostToDevice, stream_));
+  SW_CUDA(cudaMemcpyAsync(params_.p, device, sizeof(float) * mlp::kParams, cudaMemcpyDeviceToDevice, stream_));
   SW_CUDA(cudaMemsetAsync(m_.p, 0, sizeof(float) * mlp::kParams, stream_));
   SW_CUDA(cudaMemsetAsync(v_.p, 0, sizeof(float) * mlp::kParams, stream_));
   step_ = 0;
   refresh_bf16();
-  SW_CUDA(cudaStreamSynchronize(stream_));
   loaded_ = true;
 }
 

@@ -72,8 +72,8 @@ class Trainer {
  public:
   explicit Trainer(cudaStream_t s) : stream_(s) {}
 
-  // Parameters: host vector of mlp::kParams floats (layout in mlp.cuh).
-  void set_params(const float* host);
+  // Parameters: mlp::kParams floats on the device (layout in mlp.cuh); no moments.
+  void set_params(const float* device);
   void get_params(float* host);
   bool has_params() const { return loaded_; }
 
