@@ -63,7 +63,7 @@ struct Side {
   // knows it (count is then an upper bound).
   struct Step {
     u32 parents = 0, children = 0, base = 0, visited = 0, distinct = 0, kept = 0;
-    bool forward = false, reduce = false, self = false, compacted = false, deferred = false;
+    bool forward = false, reduce = false, self = false, compacted = false, deferred = false, counted = false;
     double t0 = 0;
   } step;
   const u32* live = nullptr;
@@ -630,13 +630,16 @@ class Engine {
     count_launch(3);
     // The checks of a reduced level are cut for the rows they are told of, and
     // where most children are duplicates few of those rows are there: from
-    // kDomSmallRows children on the count is read back first (searches whose
+    // kDomOrderRows children on the count is read back first (searches whose
     // letters permute all states but one: n = 60, k = 16 55 -> 26 ms, n = 40, k = 8
-    // 35 -> 20; n = 200, k = 2 6.9 -> 7.1)
-    defer = defer && Nc && (reduce ? Nc <= kDomSmallRows : !X.split);
+    // 35 -> 20; below, a read-back costs more than it saves: n = 100, k = 3 plans
+    // of ten levels of 10 000 to 30 000 children 2.4 -> 2.6 ms)
+    defer = defer && Nc && (reduce || !X.split);
+    P.counted = reduce && Nc > kDomOrderRows;
     u32 u = Nc;
-    const u32* const fresh_live = defer ? d_misc + 8 : nullptr;
-    if (!defer) u = read_total_checked();
+    if (!defer || P.counted) u = read_total_checked();
+    defer = defer && u;
+    const u32* const fresh_live = defer && !P.counted ? d_misc + 8 : nullptr;
     if (X.split) {
       P.visited = visited_subsets ? X.vis_count : 0;
       P.self = self_check;
@@ -691,7 +694,7 @@ class Engine {
       st->subsets_expanded += P.children;
       st->subsets_kept += f;
     }
-    if (P.deferred && P.compacted) {
+    if (P.deferred && P.compacted && !P.counted) {
       if (P.visited) count_query(P.visited, u);
       if (P.self) count_query(u, u);
     }
@@ -1556,7 +1559,7 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
   if (bounded && !found) {
     BoundedSearch S{E, A, W, n, k, budget, row_bytes, std::max<u64>(cfg.dfs_min_list_size, 1), max_rt, 0, {}, 0,
                     {}, {}, st};
-    E.release_tables();
+    if (4 * (E.F.list_bytes() + E.B.list_bytes()) > budget) E.release_tables();
     S.pool.swap(E.dlevel_pool);  // levels (and their device buffers) kept across solves
     S.levels.push_back(nullptr);
     S.explore(0, 0, E.B.count, rt);
