@@ -8,9 +8,9 @@
 // B is stored as complements: the preimage of a complement is the complement
 // of the preimage, so the same expansion, dedup and dominance code serves both
 // sides.  One step expands the smaller side (meet_in_the_middle.cpp:355-358),
-// sorts and deduplicates the children, drops every child that has a visited
-// set inside it or a proper subset in its own layer
-// (meet_in_the_middle.cpp:179-344 on complements for B), and then asks
+// drops duplicates by hash table (or by sorting, past its limits), drops where it
+// pays every child that has a visited set inside it or a proper subset in its own
+// layer (meet_in_the_middle.cpp:179-344 on complements for B), and then asks
 // whether some F is disjoint from some B-complement (F ⊆ B,
 // meet_in_the_middle.cpp:90).  Each kept child records (letter, parent) so the
 // meeting pair yields a word, which is verified on the host before it is
@@ -63,14 +63,13 @@ struct Side {
   // knows it (count is then an upper bound).
   struct Step {
     u32 parents = 0, children = 0, base = 0, visited = 0, distinct = 0, kept = 0;
-    bool forward = false, reduce = false, self = false, compacted = false, deferred = false, counted = false;
+    bool forward = false, reduce = false, compacted = false, deferred = false, counted = false;
     double t0 = 0;
   } step;
   const u32* live = nullptr;
   size_t list_bytes() const { return vis.cap + vis_alt.cap + met.cap + table.cap; }
   const u64* cur_rows(int W) const { return in_vis ? vis.as<u64>() + (size_t)cur_off * W : rows.as<u64>(); }
   std::vector<std::unique_ptr<Layer>> layers;
-  std::vector<u64> seed_states;  // backward side: the state of each seed row
   double unique_growth = 0;      // distinct children per parent at the last step
   KeyMap keymap;                 // sort key of this side's layers and visited list
   bool keymap_chosen = false;
@@ -104,7 +103,6 @@ struct Side {
     keymap_chosen = false;
     for (auto& L : layers) spare.push_back(std::move(L));
     layers.clear();
-    seed_states.clear();
   }
 };
 
@@ -489,19 +487,13 @@ class Engine {
   // One BFS layer on side X (forward = image, backward = preimage of complements).
   // With `dominance` false only duplicates are removed and the visited list is
   // left alone (the bounded inverse phase, see Solver::exact).
-  // Dominance reductions (the reference's self and visited reductions).
-  // self_check: drop children with a proper subset in their own layer;
-  // visited_subsets: drop children containing a visited set (false: only
-  // children equal to a visited set, by a sorted-membership search).
-  // Solver::exact runs the full reductions only where they pay: each removes
-  // ~15% of a layer for a layer-by-layer subset query, which repays itself
-  // when the lists are large or feed the bounded phase.  Measured (ms per
-  // DFA): n = 200 plain Exact 4.8 with duplicates only, 7.3 with the visited
-  // subset check, 10.3 with both reductions; n = 320 Beam+Exact 949 without
-  // the self reduction, 863 with both.  Lengths are the same either way:
-  // every kept set is still a set of its layer and the meet check is exact.
-  bool self_check = true;
-  bool visited_subsets = true;
+  // Dominance reductions (the reference's self and visited reductions): drop
+  // children that hold a visited set or a proper subset in their own layer.
+  // Solver::exact runs them only where they pay: each removes ~15% of a layer for a
+  // check of the layer, which repays itself when the lists are large or feed the
+  // bounded phase.  Lengths are the same either way: every kept set is still a set
+  // of its layer and the meet check is exact.
+  bool reductions = true;
 
   // ---- duplicate removal by hash table ----
   DevBuf bk_counts, bk_first, bk_place, level_table;
@@ -562,7 +554,7 @@ class Engine {
       return need + need / 4;
     };
     size_t bytes = list(X.vis, X.vis_count);
-    if (X.split || self_check || visited_subsets) bytes += list(X.met, X.split ? X.met_count : X.vis_count);
+    if (X.split || reductions) bytes += list(X.met, X.split ? X.met_count : X.vis_count);
     bytes += 2 * X.table_slots < 3 * rows ? sizeof(u64) * slots_for(rows) / 4 * 5 : X.table.cap;
     return bytes + copied + X.vis_alt.cap + (&X == &F ? B : F).list_bytes() <= list_budget;
   }
@@ -581,7 +573,7 @@ class Engine {
   // the launches that follow are sized for every child.
   void step_hashed(Side& X, bool forward, int W, int n, int k, bool defer) {
     const u32 m = X.count, Nc = m * (u32)k;
-    const bool reduce = self_check || visited_subsets;
+    const bool reduce = reductions;
     Side::Step& P = X.step;
     P = Side::Step{};
     P.t0 = vclock();
@@ -641,19 +633,18 @@ class Engine {
     defer = defer && u;
     const u32* const fresh_live = defer && !P.counted ? d_misc + 8 : nullptr;
     if (X.split) {
-      P.visited = visited_subsets ? X.vis_count : 0;
-      P.self = self_check;
+      P.visited = X.vis_count;
       grow_rows(X.vis, W, X.vis_count, u);
       u64* const out = X.vis.as<u64>() + (size_t)X.vis_count * W;
       if (reduce && u) {
         flags_a.reserve(sizeof(u32) * (size_t)u);
         SW_CUDA(cudaMemsetAsync(flags_a.p, 0, sizeof(u32) * (size_t)u, stream));
         reduce_span.mark(0, stream);
-        if (X.vis_count && visited_subsets)
-          dominated(forward, W, X.vis.as<u64>(), X.vis_count, fresh, u, n, false, X.vis_count, flags_a.as<u32>(), dom_rows,
-                    nullptr, fresh_live);
-        if (self_check)
-          dominated(forward, W, fresh, u, fresh, u, n, true, X.vis_count, flags_a.as<u32>(), dom_rows, fresh_live, fresh_live);
+        if (X.vis_count)
+          dominated(forward, W, X.vis.as<u64>(), X.vis_count, fresh, u, n, false, X.vis_count, flags_a.as<u32>(),
+                    dom_rows, nullptr, fresh_live);
+        dominated(forward, W, fresh, u, fresh, u, n, true, X.vis_count, flags_a.as<u32>(), dom_rows, fresh_live,
+                  fresh_live);
         reduce_span.mark(1, stream);
         const u32 epoch = next_dc_epoch(u);
         timed(3, (double)u * (4 + 2 * (8.0 * W + 4)), [&] {
@@ -696,7 +687,7 @@ class Engine {
     }
     if (P.deferred && P.compacted && !P.counted) {
       if (P.visited) count_query(P.visited, u);
-      if (P.self) count_query(u, u);
+      count_query(u, u);
     }
     if (X.split) X.met_count = P.base + u;
     P.distinct = u;
@@ -789,7 +780,7 @@ class Engine {
     if (st) st->subsets_expanded += N;
     // sort the children by layer key
     sort_rows(2, keys.as<u64>(), ch_vals.as<u32>(), Nc);
-    if (dominance && !self_check && !visited_subsets) {
+    if (dominance && !reductions) {
       // duplicates only: a child is dropped when it equals its predecessor in
       // the sorted layer or a visited set.  One launch flags the children in
       // sort order (rows read through the sort's permutation), counts the
@@ -846,22 +837,11 @@ class Engine {
     launch_fill_u32(flags_b.as<u32>(), 0, u, stream);
     count_launch(2);
     const double t_sort = vclock();
-    if (X.vis_count) {
-      if (visited_subsets) {
-        // the list the layer is merged into afterwards is free until then
-        dominated(forward, W, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, n, false, X.vis_count,
-                  flags_a.as<u32>(), X.vis_alt);
-      } else {
-        timed(3, (double)u * 8.0 * W, [&] {
-          launch_member_key(W, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, flags_a.as<u32>(), stream,
-                            X.keymap);
-        });
-        count_launch();
-      }
-    }
+    if (X.vis_count)  // the list the layer is merged into afterwards is free until then
+      dominated(forward, W, X.vis.as<u64>(), X.vis_count, uq_rows.as<u64>(), u, n, false, X.vis_count,
+                flags_a.as<u32>(), X.vis_alt);
     const double t_vis = vclock();
-    if (self_check)
-      dominated(forward, W, uq_rows.as<u64>(), u, uq_rows.as<u64>(), u, n, true, X.vis_count, flags_b.as<u32>(),
+    dominated(forward, W, uq_rows.as<u64>(), u, uq_rows.as<u64>(), u, n, true, X.vis_count, flags_b.as<u32>(),
                 X.vis_alt);
     const double t_self = vclock();
     if (verbose) {
@@ -1395,7 +1375,6 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
     for (size_t i = 0; i < seeds.size(); ++i) {
       for (int q = 0; q < n; ++q)
         if ((uint32_t)q != seeds[i]) rows[i * W + (q >> 6)] |= state_bit(q);  // complement of {seed}
-      E.B.seed_states.push_back(seeds[i]);
     }
     E.B.rows.reserve(sizeof(u64) * rows.size());
     SW_CUDA(cudaMemcpyAsync(E.B.rows.p, rows.data(), sizeof(u64) * W * seeds.size(), cudaMemcpyHostToDevice,
@@ -1468,7 +1447,7 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
     Reduction& red_last = reductions[fwd];
     const LevelRule level =
         reductions_of_level((int)cfg.reductions, b.has_word, cfg.dfs != 0, pressure, red_last, X.count, rest);
-    E.self_check = E.visited_subsets = level.reduce;
+    E.reductions = level.reduce;
     E.step(X, fwd, W, n, k, /*dominance=*/!bounded, false, /*defer=*/true);
     if (fwd) {
       st.bfs_steps++;
@@ -2054,7 +2033,7 @@ void Solver::reduce(const Automaton& A, const sw_reduce_config& cfg, Bounds& b, 
   auto t0 = std::chrono::steady_clock::now();
   const int n = (int)A.n, k = (int)A.k, W = words_for(n);
   E.upload_tables(A);
-  E.self_check = E.visited_subsets = true;  // the reference's step (reduce.hpp:186-187): its list sizes decide the reduction
+  E.reductions = true;  // the reference's step (reduce.hpp:186-187): its list sizes decide the reduction
   E.R.reset();
   std::vector<u64> full(W, 0);
   for (int q = 0; q < n; ++q) full[q >> 6] |= state_bit(q);
@@ -2198,7 +2177,7 @@ uint32_t Solver::distance_pairs(const Automaton& A, uint32_t per_layer, uint64_t
   Engine& E = *eng_;
   const int n = (int)A.n, k = (int)A.k, W = words_for(n);
   E.upload_tables(A);
-  E.self_check = E.visited_subsets = true;  // labelled layers are the fully reduced ones
+  E.reductions = true;  // labelled layers are the fully reduced ones
   // inverse layers (complements of the maximal preimage sets), depth 0..D
   E.B.reset();
   std::vector<uint32_t> seeds = backward_seeds(A);

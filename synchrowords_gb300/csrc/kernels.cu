@@ -1,8 +1,8 @@
-// Device kernels of the exact search: warp-per-subset layer expansion, radix
-// sort / unique, stream compaction, the binary radix tree over a sorted layer
-// and the tree-walking subset queries.  All integer bitset work; see
-// common.cuh for the row layout and kernels.cuh for the reference functions
-// each kernel replaces.
+// Device kernels of the searches: layer expansion 32 parents a warp, duplicate
+// removal by hash table and bucket order, sorts of rows by layer key with unique
+// and compaction, merges, and the learned beam's selection.  All integer bitset
+// work; see common.cuh for the row layout and kernels.cuh for the reference
+// functions each kernel replaces.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -971,14 +971,6 @@ __global__ void k_compact(const u64* __restrict__ rows, const u32* __restrict__ 
   if (out_vals) out_vals[d] = vals[i];
 }
 
-template <int W>
-__global__ void k_complement(u64* rows, u32 m, int n) {
-  u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-#pragma unroll
-  for (int w = 0; w < W; ++w) rows[(size_t)i * W + w] = ~rows[(size_t)i * W + w] & valid_mask(n, w);
-}
-
 // Reference layout <-> device layout, one word per thread: both put state q in
 // word q / 64, so a row converts by reversing the bits of its words.  Bound by
 // the words' way through memory; a few microseconds beside the copies of the
@@ -1051,12 +1043,6 @@ void launch_compact(int W, const u64* rows, const u32* vals, const u32* flags, c
                     u32* out_vals, cudaStream_t s) {
   if (!m) return;
   SW_DISPATCH_R(W, (k_compact<RR><<<(m + 255) / 256, 256, 0, s>>>(rows, vals, flags, pos, m, out_rows, out_vals)));
-  SW_LAUNCH_CHECK();
-}
-
-void launch_complement(int W, u64* rows, u32 m, int n, cudaStream_t s) {
-  if (!m) return;
-  SW_DISPATCH_W(W, (k_complement<WW><<<(m + 255) / 256, 256, 0, s>>>(rows, m, n)));
   SW_LAUNCH_CHECK();
 }
 
@@ -1147,34 +1133,6 @@ void launch_fill_u32(u32* p, u32 value, u32 m, cudaStream_t s) {
 }
 
 // ===========================================================================
-// Merge of two sorted disjoint row arrays: each element finds its output
-// position by a binary search in the other array (merge path per element).
-// ===========================================================================
-template <int W>
-__global__ void k_merge(const u64* __restrict__ A, u32 na, const u64* __restrict__ B, u32 nb, u64* __restrict__ out) {
-  const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= na + nb) return;
-  const bool fromA = i < na;
-  const u64* x = fromA ? A + (size_t)i * W : B + (size_t)(i - na) * W;
-  const u64* other = fromA ? B : A;
-  u32 lo = 0, hi = fromA ? nb : na;
-  while (lo < hi) {
-    u32 mid = (lo + hi) >> 1;
-    if (row_less<W>(other + (size_t)mid * W, x)) lo = mid + 1;
-    else hi = mid;
-  }
-  const size_t pos = (size_t)(fromA ? i : i - na) + lo;
-#pragma unroll
-  for (int w = 0; w < W; ++w) out[pos * W + w] = x[w];
-}
-
-void launch_merge(int W, const u64* A, u32 na, const u64* B, u32 nb, u64* out, cudaStream_t s) {
-  if (na + nb == 0) return;
-  SW_DISPATCH_W(W, (k_merge<WW><<<(na + nb + 255) / 256, 256, 0, s>>>(A, na, B, nb, out)));
-  SW_LAUNCH_CHECK();
-}
-
-// ===========================================================================
 // Layer keys: (64 chosen states packed into one word, 32-bit mix of the row).
 // Sorting by this key groups sets by the pattern of their side's most
 // frequent states and makes equal sets adjacent; distinct sets with equal
@@ -1228,73 +1186,6 @@ void launch_merge_key(int W, const u64* A, u32 na, const u64* B, u32 nb, u64* ou
                       const KeyMap& map) {
   if (na + nb == 0) return;
   SW_DISPATCH_W(W, (k_merge_key<WW><<<(na + nb + 255) / 256, 256, 0, s>>>(A, na, B, nb, map, out)));
-  SW_LAUNCH_CHECK();
-}
-
-// flags[i] = 1 when row i of C equals some row of V (both sorted by the same
-// layer key): a binary search for C's key in V, then a scan of V's rows with
-// that key.
-template <int W>
-__global__ void k_member_key(const u64* __restrict__ V, u32 nv, const u64* __restrict__ C, u32 nc, KeyMap map,
-                             u32* __restrict__ flags) {
-  const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nc) return;
-  const u64* x = C + (size_t)i * W;
-  u64 x0, x1;
-  layer_key<W>(x, map, x0, x1);
-  u32 lo = 0, hi = nv;
-  while (lo < hi) {
-    const u32 mid = (lo + hi) >> 1;
-    u64 y0, y1;
-    layer_key<W>(V + (size_t)mid * W, map, y0, y1);
-    if (y0 < x0 || (y0 == x0 && y1 < x1)) lo = mid + 1;
-    else hi = mid;
-  }
-  for (u32 j = lo; j < nv; ++j) {
-    const u64* y = V + (size_t)j * W;
-    u64 y0, y1;
-    layer_key<W>(y, map, y0, y1);
-    if (y0 != x0 || y1 != x1) break;
-    if (row_eq<W>(x, y)) {
-      flags[i] = 1u;
-      return;
-    }
-  }
-}
-
-// flags[i] = 0 for rows of C (with flags[i] = 1) equal to some row of V.
-template <int W>
-__global__ void k_clear_members(const u64* __restrict__ V, u32 nv, const u64* __restrict__ C, u32 nc, KeyMap map,
-                                u32* __restrict__ flags) {
-  const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nc || !flags[i]) return;
-  const u64* x = C + (size_t)i * W;
-  u64 x0, x1;
-  layer_key<W>(x, map, x0, x1);
-  u32 lo = 0, hi = nv;
-  while (lo < hi) {
-    const u32 mid = (lo + hi) >> 1;
-    u64 y0, y1;
-    layer_key<W>(V + (size_t)mid * W, map, y0, y1);
-    if (y0 < x0 || (y0 == x0 && y1 < x1)) lo = mid + 1;
-    else hi = mid;
-  }
-  for (u32 j = lo; j < nv; ++j) {
-    const u64* y = V + (size_t)j * W;
-    u64 y0, y1;
-    layer_key<W>(y, map, y0, y1);
-    if (y0 != x0 || y1 != x1) break;
-    if (row_eq<W>(x, y)) {
-      flags[i] = 0u;
-      return;
-    }
-  }
-}
-
-void launch_clear_members(int W, const u64* V, u32 nv, const u64* C, u32 nc, u32* flags, cudaStream_t s,
-                          const KeyMap& map) {
-  if (!nc || !nv) return;
-  SW_DISPATCH_W(W, (k_clear_members<WW><<<(nc + 255) / 256, 256, 0, s>>>(V, nv, C, nc, map, flags)));
   SW_LAUNCH_CHECK();
 }
 
@@ -1475,13 +1366,6 @@ void launch_dedup_compact(int W, const u64* C, const u32* vals, const u64* keys,
   const u32 blocks = (m + kDcTile - 1) / kDcTile;
   SW_DISPATCH_W(W, (k_dedup_compact<WW><<<blocks, kDcTile, 0, s>>>(C, vals, keys, m, V, nv, map, out_rows, out_vals,
                                                                   total, status, ctr, epoch, err)));
-  SW_LAUNCH_CHECK();
-}
-
-void launch_member_key(int W, const u64* V, u32 nv, const u64* C, u32 nc, u32* flags, cudaStream_t s,
-                       const KeyMap& map) {
-  if (!nc || !nv) return;
-  SW_DISPATCH_W(W, (k_member_key<WW><<<(nc + 255) / 256, 256, 0, s>>>(V, nv, C, nc, map, flags)));
   SW_LAUNCH_CHECK();
 }
 

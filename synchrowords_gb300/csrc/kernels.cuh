@@ -169,12 +169,6 @@ void launch_dominance(int W, bool comp, bool hit_t, const u64* T, u32 tm, const 
                       u32* flags, const DominanceScratch& sc, cudaStream_t s, const u32* t_live = nullptr,
                       const u32* x_live = nullptr);
 
-// out = sorted merge of two sorted, mutually disjoint row arrays.
-void launch_merge(int W, const u64* A, u32 na, const u64* B, u32 nb, u64* out, cudaStream_t s);
-
-// rows[i] = complement of rows[i] within n states.
-void launch_complement(int W, u64* rows, u32 m, int n, cudaStream_t s);
-
 // In-place conversion of `count` rows between the reference bit layout (state
 // q = bit q % 64 of word q / 64) and the device layout (bit 63 - q % 64); bits
 // of states >= n come out zero.
@@ -220,12 +214,6 @@ void launch_dedup_compact(int W, const u64* C, const u32* vals, const u64* keys,
 // by launch_dedup_compact (same status, ctr and epoch).
 void launch_keep_compact(int W, const u64* rows, const u32* vals, const u32* flags, u32 m, u64* out_rows, u32* out_vals,
                          u32* total, u64* status, u32* ctr, u32 epoch, u32* err, cudaStream_t s, const u32* live = nullptr);
-void launch_member_key(int W, const u64* V, u32 nv, const u64* C, u32 nc, u32* flags, cudaStream_t s,
-                       const KeyMap& map = KeyMap{});
-// flags[i] = 0 where flags[i] = 1 and row i of C equals a row of V (same
-// layer-key order as launch_member_key).
-void launch_clear_members(int W, const u64* V, u32 nv, const u64* C, u32 nc, u32* flags, cudaStream_t s,
-                          const KeyMap& map = KeyMap{});
 // counts[q] += rows containing state q (counts: 64*W entries, caller-zeroed).
 void launch_state_counts(int W, const u64* rows, u32 m, u32* counts, cudaStream_t s);
 

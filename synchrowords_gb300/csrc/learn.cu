@@ -1,5 +1,4 @@
-// MlpRunner (learn.hpp): the forward and backward passes of the learned
-// distance model as sequences of the launches of mlp.cu.
+// MlpRunner (learn.hpp): scoring with the learned distance model (mlp.cu).
 #include "learn.hpp"
 
 namespace sw {
@@ -33,14 +32,13 @@ void MlpRunner::prepare(const Automaton& A) {
     SW_CUDA(cudaStreamSynchronize(stream_));  // f is released at the end of this block
     feat_key_ = std::move(key);
   }
-  epre_.reserve(sizeof(float) * n_ * mlp::kEmb);
   e_.reserve(sizeof(bf16) * mlp::staged_embeddings(n_));
-  mlp::embed(feat_.as<float>(), params_.as<float>(), n_, epre_.as<float>(), e_.as<bf16>(), error_, stream_);
+  mlp::embed(feat_.as<float>(), params_.as<float>(), n_, e_.as<bf16>(), error_, stream_);
 }
 
 void MlpRunner::forward(const u64* rows, int W, u32 count, float* y) {
-  mlp::forward(rows, W, n_, count, e_.as<bf16>(), weights_.as<bf16>(), params_.as<float>(), y, mlp::Activations{},
-               error_, stream_);
+  mlp::forward(rows, W, n_, count, e_.as<bf16>(), weights_.as<bf16>(), params_.as<float>(), y, error_,
+               stream_);
 }
 
 }  // namespace sw

@@ -37,7 +37,7 @@ class MlpRunner {
   int n_ = 0;
   std::vector<uint32_t> feat_key_;  // automaton whose features are in feat_ (n, k, table)
   DevBuf params_, weights_;
-  DevBuf feat_, epre_, e_;               // features, embeddings before and after the relu (staged bf16)
+  DevBuf feat_, e_;                 // features, embeddings (staged bf16)
 };
 
 }  // namespace sw

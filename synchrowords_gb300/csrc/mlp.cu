@@ -165,8 +165,8 @@ __device__ __forceinline__ float unpack(u32 pair, int i) {
 }
 
 // 32 values of row r, columns c .. c + 31 (c % 32 == 0): bf16 into a K-major
-// operand (K = columns) and, if given, into a global row.
-__device__ __forceinline__ void put_rows(const float* v, int r, int c, uint8_t* op, bf16* global) {
+// operand (K = columns).
+__device__ __forceinline__ void put_rows(const float* v, int r, int c, uint8_t* op) {
   u32 p[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) p[i] = pack2(v[2 * i], v[2 * i + 1]);
@@ -174,32 +174,8 @@ __device__ __forceinline__ void put_rows(const float* v, int r, int c, uint8_t* 
   for (int i = 0; i < 4; ++i) {
     const uint4 q = make_uint4(p[4 * i], p[4 * i + 1], p[4 * i + 2], p[4 * i + 3]);
     *reinterpret_cast<uint4*>(op + (c >> 6) * kSlice + core_offset(r, (c & 63) + 8 * i)) = q;
-    if (global) reinterpret_cast<uint4*>(global)[i] = q;
   }
 }
-// ... transposed: bf16 pairs p (columns c ..) into an operand whose K is the row.
-__device__ __forceinline__ void put_columns(const u32* p, int r, int c, uint8_t* op, u32 slice) {
-  uint8_t* const o = op + (r >> 6) * slice;
-#pragma unroll
-  for (int i = 0; i < 32; ++i)
-    *reinterpret_cast<uint16_t*>(o + core_offset(c + i, r & 63)) = (uint16_t)(i & 1 ? p[i / 2] >> 16 : p[i / 2]);
-}
-
-// Sums of 32 columns over the warp's rows: lane l gets column l's (31 exchanges).
-__device__ __forceinline__ float column_sums(float* v) {
-  const u32 lane = threadIdx.x & 31;
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int i = 0; i < o; ++i) {
-      const float send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  return v[0];
-}
-
 __device__ __forceinline__ void copy_in(uint8_t* dst, const bf16* src, int bytes) {
   for (int i = threadIdx.x; i < bytes / 16; i += kThreads)
     reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
@@ -207,12 +183,11 @@ __device__ __forceinline__ void copy_in(uint8_t* dst, const bf16* src, int bytes
 }  // namespace
 
 // ---- forward ----
-template <bool kTrain>
 __global__ void __launch_bounds__(kThreads) k_forward(const u64* __restrict__ rows, int W, int n, u32 count,
                                                       const bf16* __restrict__ staged_e,
                                                       const bf16* __restrict__ weights,
                                                       const float* __restrict__ params, float* __restrict__ y,
-                                                      Activations act, u32* err) {
+                                                      u32* err) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t *const sA = smem, *const sB = smem + kFwdB;
   u32* const slot = reinterpret_cast<u32*>(smem + kFwdBar + 16);
@@ -250,7 +225,7 @@ __global__ void __launch_bounds__(kThreads) k_forward(const u64* __restrict__ ro
   if (ok) {
     float v[32];
     ld32(tc.tmem, q * 32, half * 32, v);
-    put_rows(v, r, half * 32, sA, kTrain && in ? act.x + (size_t)row * kEmb + half * 32 : nullptr);
+    put_rows(v, r, half * 32, sA);
     // h1 = relu(x · W1 + b1): columns 128 .. 255
     copy_in(sB, weights + kOffW1F, kStagedW1 * 2);
     tc.publish();
@@ -266,15 +241,9 @@ __global__ void __launch_bounds__(kThreads) k_forward(const u64* __restrict__ ro
       const int c = half * 64 + cb * 32;
       float v[32];
       ld32(tc.tmem + 128, q * 32, c, v);
-      u32 open = 0;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        v[i] += __ldg(params + kOffB1 + c + i);
-        open |= v[i] > 0.0f ? 1u << i : 0u;
-        v[i] = fmaxf(v[i], 0.0f);
-      }
-      put_rows(v, r, c, sA, kTrain && in ? act.h1 + (size_t)row * kHidden + c : nullptr);
-      if (kTrain && in) act.open1[(size_t)row * 4 + (c >> 5)] = open;
+      for (int i = 0; i < 32; ++i) v[i] = fmaxf(v[i] + __ldg(params + kOffB1 + c + i), 0.0f);
+      put_rows(v, r, c, sA);
     }
     // h2 = relu(h1 · W2 + b2): columns 0 .. 127
     copy_in(sB, weights + kOffW2F, kStagedW2 * 2);
@@ -295,24 +264,13 @@ __global__ void __launch_bounds__(kThreads) k_forward(const u64* __restrict__ ro
       const int c = half * 64 + cb * 32;
       float v[32];
       ld32(tc.tmem, q * 32, c, v);
-      u32 open = 0;
       u32 p[16];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        v[i] += __ldg(params + kOffB2 + c + i);
-        open |= v[i] > 0.0f ? 1u << i : 0u;
-        v[i] = fmaxf(v[i], 0.0f);
-      }
+      for (int i = 0; i < 32; ++i) v[i] = fmaxf(v[i] + __ldg(params + kOffB2 + c + i), 0.0f);
 #pragma unroll
       for (int i = 0; i < 16; ++i) p[i] = pack2(v[2 * i], v[2 * i + 1]);
 #pragma unroll
       for (int i = 0; i < 32; ++i) part[i] += unpack(p[i / 2], i & 1) * __ldg(params + kOffW3 + c + i);
-      if (kTrain && in) {
-        uint4* const o = reinterpret_cast<uint4*>(act.h2 + (size_t)row * kHidden + c);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) o[i] = make_uint4(p[4 * i], p[4 * i + 1], p[4 * i + 2], p[4 * i + 3]);
-        act.open2[(size_t)row * 4 + (c >> 5)] = open;
-      }
     };
     if (half == 0) {
 #pragma unroll
@@ -339,19 +297,18 @@ __global__ void __launch_bounds__(kThreads) k_forward(const u64* __restrict__ ro
 }
 
 void forward(const u64* rows, int W, int n, u32 count, const bf16* staged_e, const bf16* weights, const float* params,
-             float* y, const Activations& act, u32* err, cudaStream_t s) {
+             float* y, u32* err, cudaStream_t s) {
   if (!count) return;
   const u32 blocks = (count + kRows - 1) / kRows;
-  ensure_smem_limit((const void*)k_forward<false>, kFwdSmem);
-  k_forward<false><<<blocks, kThreads, kFwdSmem, s>>>(rows, W, n, count, staged_e, weights, params, y, act, err);
+  ensure_smem_limit((const void*)k_forward, kFwdSmem);
+  k_forward<<<blocks, kThreads, kFwdSmem, s>>>(rows, W, n, count, staged_e, weights, params, y, err);
   SW_LAUNCH_CHECK();
 }
 
 // ---- embeddings ----
 // Block of 128 states: feat · Phi is one K = 16 product.
 __global__ void __launch_bounds__(kThreads) k_embed(const float* __restrict__ feat, const float* __restrict__ params,
-                                                    int n, float* __restrict__ epre, bf16* __restrict__ staged,
-                                                    u32* err) {
+                                                    int n, bf16* __restrict__ staged, u32* err) {
   __shared__ __align__(1024) uint8_t sA[kSlice];
   __shared__ __align__(1024) uint8_t sB[kSlice / 2];
   __shared__ __align__(16) uint64_t s_bar[2];
@@ -387,11 +344,7 @@ __global__ void __launch_bounds__(kThreads) k_embed(const float* __restrict__ fe
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
         const int j = half * 32 + i;
-        float a = 0.0f;
-        if (st < n) {
-          a = v[i] + params[kOffC + j];
-          epre[(size_t)st * kEmb + j] = a;
-        }
+        const float a = st < n ? v[i] + params[kOffC + j] : 0.0f;
         staged[(size_t)(st >> 6) * 64 * kEmb + core_offset(j, st & 63) / 2] = __float2bfloat16(fmaxf(a, 0.0f));
       }
     }
@@ -399,24 +352,22 @@ __global__ void __launch_bounds__(kThreads) k_embed(const float* __restrict__ fe
   tc.close(64);
 }
 
-void embed(const float* feat, const float* params, int n, float* epre, bf16* staged, u32* err, cudaStream_t s) {
-  k_embed<<<(n + kRows - 1) / kRows, kThreads, 0, s>>>(feat, params, n, epre, staged, err);
+void embed(const float* feat, const float* params, int n, bf16* staged, u32* err, cudaStream_t s) {
+  k_embed<<<(n + kRows - 1) / kRows, kThreads, 0, s>>>(feat, params, n, staged, err);
   SW_LAUNCH_CHECK();
 }
 
 // ---- weights ----
-// bf16 copies of W1[i][j] and W2[i][j] where the products read them: forward as
-// B(N = j, K = i), backward as B(N = i, K = j).
+// bf16 copies of W1[i][j] and W2[i][j] where the products read them, as B(N = j,
+// K = i).
 __device__ __forceinline__ void stage_weight(bf16* w, int e, float value) {
   const bf16 b = __float2bfloat16(value);
   if (e >= kOffW1 && e < kOffB1) {
     const int i = (e - kOffW1) / kHidden, j = (e - kOffW1) % kHidden;
     w[kOffW1F + core_offset(j, i) / 2] = b;
-    w[kOffW1B + (j >> 6) * (64 * 64) + core_offset(i, j & 63) / 2] = b;
   } else if (e >= kOffW2 && e < kOffB2) {
     const int i = (e - kOffW2) / kHidden, j = (e - kOffW2) % kHidden;
     w[kOffW2F + (i >> 6) * (128 * 64) + core_offset(j, i & 63) / 2] = b;
-    w[kOffW2B + (j >> 6) * (128 * 64) + core_offset(i, j & 63) / 2] = b;
   }
 }
 
