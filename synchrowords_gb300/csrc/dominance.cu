@@ -261,7 +261,8 @@ void launch_dom_w(bool comp, bool hit_t, const u64* T, u32 tm, const u64* X, u32
     k_size_rank<W, true><<<blocks, 256, 0, s>>>(T, tm, n, sc.bucket.counts, sc.bucket.place, t_live);
   else
     k_size_rank<W, false><<<blocks, 256, 0, s>>>(T, tm, n, sc.bucket.counts, sc.bucket.place, t_live);
-  launch_bucket_scan(BucketScratch{kBucketBitsSmall, sc.bucket.counts, sc.bucket.first, sc.bucket.place, sc.bucket.met},
+  launch_bucket_scan(BucketScratch{kBucketBitsSmall, sc.bucket.counts, sc.bucket.first, sc.bucket.place, nullptr,
+                                   sc.bucket.met},
                      sc.total, s);
   k_size_scatter<W><<<blocks, 256, 0, s>>>(T, tm, sc.bucket.place, sc.bucket.first, sc.rows, sc.index, t_live);
   SW_LAUNCH_CHECK();

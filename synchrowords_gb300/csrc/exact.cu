@@ -496,7 +496,7 @@ class Engine {
   bool reductions = true;
 
   // ---- duplicate removal by hash table ----
-  DevBuf bk_counts, bk_first, bk_place, level_table;
+  DevBuf bk_counts, bk_first, bk_place, bk_scan, level_table;
   // Bucket counts are zero between steps: the scan that reads them clears them.
   // A step that ends before that scan (its buffers did not fit) leaves counts
   // behind, and the next step would move its rows past their list; so every use
@@ -504,18 +504,20 @@ class Engine {
   // scanned() once the scan is launched.
   bool bk_open = true;
   BucketScratch buckets(u64 children) {
-    const size_t bytes = sizeof(u32) << kBucketBitsLarge;
+    const int bits = bucket_bits(children);
+    const size_t bytes = sizeof(u32) << std::max(bits, kBucketBitsLarge);
+    if (bk_counts.cap < bytes) bk_open = true;
     bk_counts.reserve(bytes);
     bk_first.reserve(bytes);
     bk_place.reserve(sizeof(uint2) * children);
+    bk_scan.reserve(scan_temp_bytes(1u << bits));
     if (bk_open) {
       SW_CUDA(cudaMemsetAsync(bk_counts.p, 0, bk_counts.cap, stream));
       SW_CUDA(cudaMemsetAsync(d_misc + 6, 0, 2 * sizeof(u32), stream));
       SW_CUDA(cudaMemsetAsync(d_misc + 14, 0, 2 * sizeof(u32), stream));
     }
     bk_open = true;
-    return BucketScratch{bucket_bits(children), bk_counts.as<u32>(), bk_first.as<u32>(), bk_place.as<uint2>(),
-                         d_misc + 6};
+    return BucketScratch{bits, bk_counts.as<u32>(), bk_first.as<u32>(), bk_place.as<uint2>(), bk_scan.p, d_misc + 6};
   }
   void scanned() { bk_open = false; }
   // Power-of-two slots, two to four per row.

@@ -569,7 +569,19 @@ void launch_bucket_rank(int W, const u64* C, u32 m, const BucketScratch& b, cuda
   SW_LAUNCH_CHECK();
 }
 
+__global__ void k_bucket_close(u32* met) {
+  met[1] = met[0];
+  met[0] = 0;
+}
+
 void launch_bucket_scan(const BucketScratch& b, u32* total, cudaStream_t s) {
+  if (b.bits > kBucketBitsLarge) {
+    launch_scan(b.counts, b.first, 1u << b.bits, total, b.scan, s);
+    SW_CUDA(cudaMemsetAsync(b.counts, 0, sizeof(u32) << b.bits, s));
+    k_bucket_close<<<1, 1, 0, s>>>(b.met);
+    SW_LAUNCH_CHECK();
+    return;
+  }
   k_bucket_scan<<<1, kScanThreads, 0, s>>>(b.counts, b.first, 1u << b.bits, total, b.met);
   SW_LAUNCH_CHECK();
 }

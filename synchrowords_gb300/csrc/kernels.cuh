@@ -62,11 +62,23 @@ struct BucketScratch {
   u32* counts = nullptr;
   u32* first = nullptr;
   uint2* place = nullptr;
+  void* scan = nullptr;  // launch_scan's scratch, above kBucketBitsLarge
   u32* met = nullptr;  // two words, the first zero before the first launch; the second gets the children found in V
 };
-// 12 leading bits below 2^16 children (one round of the bucket scan), 16 above.
-constexpr int kBucketBitsSmall = 12, kBucketBitsLarge = 16;
-inline int bucket_bits(u64 children) { return children < (1u << 16) ? kBucketBitsSmall : kBucketBitsLarge; }
+// Leading bits by the layer's children: up to 4096 buckets take one round of the
+// bucket scan; above 2^20 children 16 bits leave tiles of the subset check and the
+// dominance checks with few shared states, and the checks, which grow with the
+// square, cost more than any scan (launch_scan's three launches).  Sums of searches
+// in ms by bits above 2^20 children, 16 / 20 / 22 / 24 (sorted lists): plain Exact n = 200
+// 31 / 31 / 31 / 31 (84), n = 280 1572 / 909 / 735 / 629 (760), n = 320 381 / 256 / 227 / 211
+// (505); Beam + Exact n = 340 7125 / 4268 / 3882 / 3646 (7821), n = 384 14040 / 8715 /
+// 7476 / 6740 (10882).  22 below 2^22 children keeps the counts small against the rows.
+constexpr int kBucketBitsSmall = 12, kBucketBitsLarge = 16, kBucketBitsHuge = 22, kBucketBitsMost = 24;
+inline int bucket_bits(u64 children) {
+  if (children < (1u << 16)) return kBucketBitsSmall;
+  if (children < (1u << 20)) return kBucketBitsLarge;
+  return children < (1u << 22) ? kBucketBitsHuge : kBucketBitsMost;
+}
 void launch_expand_hash(int W, bool image, const u64* in, u32 m, const TransTables& t, u64* C, const u64* V, u32 base,
                         u64* tab, u32 tmask, const BucketScratch& b, u32* err, cudaStream_t s);
 // Ranks m rows that are all kept.
