@@ -1513,7 +1513,9 @@ void Solver::exact(const Automaton& A0, const sw_exact_config& cfg, Bounds& b, s
       // without the checks' own time, which is what the rest is held against
       const double checks = X.hashed && X.step.compacted ? std::min(red_last.seconds, t_iter_last) : 0.0;
       const double plain = mitm * (1.0 - checks / std::max(t_iter_last, 1e-9));
-      rest = fits ? std::min(total, plain) : plain;
+      const double lists =
+          (double)(E.F.count + E.F.vis_count + E.B.count + E.B.vis_count) * (double)row_bytes;
+      rest = fits ? std::min(total, plain) : lists_stay_small(lists, R, (double)budget) ? plain : 0.0;
       // voluntary switch only when every projected level fits; chunking is the
       // safety net for an exhausted budget, not a plan
       if (fits && total * (level.left_out ? kSwitchUnreduced : 1.0) < mitm) {

@@ -1,5 +1,6 @@
 // Which levels of an exact search run the dominance reductions (exact.cu).
 #pragma once
+#include <cmath>
 #include <cstdint>
 
 #include "synchrowords.h"
@@ -25,6 +26,16 @@ struct LevelRule {
 // searches, ms: no rule 469 / 533; gain 0.6 333 / 640, 1 349 / 605, 1.4 with the
 // earlier switch 365 / 519, 2 365 / 547 (512 with it), 4 388 / 544.
 constexpr double kReduceGain = 1.4, kSwitchUnreduced = 0.5;
+
+// Whether lists of `bytes` now stay below a quarter of the budget, where the checks
+// come on again, for `levels` more lengths (each side grows ~1.7x when its turn
+// comes, 1.3x a length).  A search that will get there gains nothing by larger
+// lists: Beam + Exact n = 384, 12 GB, 10.6 s with its checks left out until then, 5.6 with
+// them; the others of n = 320 to 384 whose bounded phase does not fit take 4.3 s
+// without, 4.9 with this limit, 6.3 with their checks throughout.
+inline bool lists_stay_small(double bytes, uint64_t levels, double budget) {
+  return 4.0 * bytes * std::pow(1.3, (double)levels) <= budget;
+}
 
 // A level expanded from `rows` rows, `rest` seconds (0: not known) before the
 // projected end of the search.  The checks pay with a word behind the bound (the

@@ -42,3 +42,17 @@ def test_rule(tmp_path):
         assert got == f"{int(bool(pressure) or wanted and not left_out)}{int(left_out)}"
         seen.add((got, mode, pressure))
     assert ("00", memory, 0) in seen and ("10", auto, 1) in seen and ("01", auto, 0) in seen
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="g++ not available")
+def test_lists_stay_small(tmp_path):
+    (tmp_path / "small.cpp").write_text("#include <cstdio>\n#include \"search_rules.hpp\"\nint main() {\n"
+                                        "  double b, m; unsigned long long l;\n"
+                                        "  while (std::scanf(\"%lf %llu %lf\", &b, &l, &m) == 3)\n"
+                                        "    std::printf(\"%d\", (int)sw::lists_stay_small(b, l, m));\n}\n")
+    subprocess.run(["g++", "-std=c++17", "-O1", f"-I{ROOT / 'include'}", f"-I{ROOT / 'synchrowords_gb300' / 'csrc'}",
+                    str(tmp_path / "small.cpp"), "-o", str(tmp_path / "small")], check=True)
+    cases = [(b, l, m) for b in (1e6, 1e8, 1e9) for l in (0, 1, 5, 20) for m in (4e6, 1e9, 12e9)]
+    out = subprocess.run([str(tmp_path / "small")], input="".join(f"{b} {l} {m}\n" for b, l, m in cases),
+                         capture_output=True, text=True, check=True).stdout
+    assert out == "".join(str(int(4 * b * 1.3 ** l <= m)) for b, l, m in cases)
