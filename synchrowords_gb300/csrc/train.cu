@@ -24,6 +24,7 @@ void Trainer::set_params(const float* device) {
   SW_CUDA(cudaMemsetAsync(v_.p, 0, sizeof(float) * mlp::kParams, stream_));
   step_ = 0;
   refresh_bf16();
+  SW_CUDA(cudaStreamSynchronize(stream_));  // the first step's atomics arrive as on an idle device, call after call
   loaded_ = true;
 }
 
