@@ -35,7 +35,10 @@ import subprocess
 import sys
 from pathlib import Path
 
-REF_ROOT = Path(os.environ.get("SYNCHRO_REF_ROOT", "/root/reference"))
+_CHECKOUT = Path(os.environ.get("SYNCHRO_REF_ROOT", "/root/reference"))
+# REF_ROOT.is_dir() says whether there is a checkout: an empty folder (a mount point
+# with nothing in it) holds none, so the path then names what is missing in it.
+REF_ROOT = _CHECKOUT if (_CHECKOUT / "synchrolib").is_dir() else _CHECKOUT / "synchrolib"
 HERE = Path(__file__).resolve().parent
 OUT_ROOT = HERE / "_ref"
 
