@@ -221,8 +221,8 @@ int sw_solve_json(sw_context* ctx, const uint32_t* delta, uint32_t n, uint32_t k
  * Exact run are solved on the device without host round trips:
  *   - those with n * log2(k) at most the context's batched_limit (default
  *     104: binary automata up to 104 states, ternary up to 65; k <= 4) by one
- *     persistent launch per set width, one GPU block per automaton at a time,
- *     lists in shared memory;
+ *     persistent launch per set width, a cluster of four CTAs with small
+ *     regions per automaton (one CTA where every n * log2(k) is below 32);
  *   - the others, and those the first launch cannot finish within its
  *     capacities, by one persistent launch per set width on thread-block
  *     clusters (cluster_size CTAs per automaton, lists in the cluster's

@@ -444,8 +444,8 @@ class Context:
     def solve_batch(self, automata: Sequence[Tuple[int, int, Sequence[int]]], plan_json: str,
                     workers: int = 0) -> List[Result]:
         """Solve many automata: plain-Exact automata of up to 256 states are
-        searched on the device (a shared-memory persistent launch for the
-        smallest, a thread-block-cluster launch for the rest), everything else
+        searched on the device (persistent launches of a thread-block cluster an
+        automaton, smaller clusters for the smallest), everything else
         and what those launches cannot finish on concurrent worker streams
         (workers = 0: the autotuned count, else min(count, 16))."""
         if len(automata) == 0:
